@@ -595,6 +595,33 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
   }
 }
 
+// The current device (which the entry points make the stream's device) and what belongs to it: the status
+// word's address and the number of SMs, looked up once per device and remembered (`remember`: so may be the
+// shared-memory attribute of a (function, device) pair; nothing learnt from a pretended device is kept).
+cudaError_t fwd_device_facts(int* dev, unsigned int** status, int* sms, bool* remember) {
+  static std::atomic<unsigned int*> status_of[64];
+  static std::atomic<int> sms_of[64];
+  cudaError_t e = host().get_device(dev);
+  if (e != cudaSuccess) return e;
+  *remember = *dev >= 0 && *dev < 64 && !host_pretends();
+  *status = *remember ? status_of[*dev].load(std::memory_order_acquire) : nullptr;
+  if (*status == nullptr) {
+    e = host().symbol_address(reinterpret_cast<void**>(status), reinterpret_cast<const void*>(&g_sm100_fwd_status));
+    if (e != cudaSuccess) return e;
+    if (*remember) status_of[*dev].store(*status, std::memory_order_release);
+  }
+  if (sms != nullptr) {
+    *sms = *remember ? sms_of[*dev].load(std::memory_order_acquire) : 0;
+    if (*sms == 0) {
+      if ((e = host().device_attr(sms, cudaDevAttrMultiProcessorCount, *dev)) != cudaSuccess) return e;
+      if (*remember) sms_of[*dev].store(*sms, std::memory_order_release);
+    }
+  }
+  return cudaSuccess;
+}
+
+#include "sm100_fwd_decode.cuh"
+
 inline bool exact_tiles(const Params& p, int hd) {
   return p.varlen_mode == 0 && p.max_sq % 128 == 0 && p.max_sk % 128 == 0 && p.dqk == hd && p.dvo == hd;
 }
@@ -606,25 +633,16 @@ cudaError_t launch_fwd_TE(const Params& p, cudaStream_t st) {
   if (!make_tile_map_16bit(&tq, p.q, p.dqk, p.q.n[2], kBM) || !make_tile_map_16bit(&tk, p.k, p.dqk, p.k.n[2], kBN) ||
       !make_tile_map_16bit(&tv, p.v, p.dvo, p.v.n[2], kBN))
     return cudaErrorInvalidValue;
-  // The shared-memory attribute belongs to the (function, device) pair and the status word's
-  // address to the device: both are looked up once per device (the current one, which the entry
-  // points make the stream's device) and remembered.
-  static std::atomic<unsigned int*> status_of[64];
   static std::atomic<bool> attr_set[64];
   int dev = 0;
-  cudaError_t e = host().get_device(&dev);
+  unsigned int* status = nullptr;
+  bool remember = false;
+  cudaError_t e = fwd_device_facts(&dev, &status, nullptr, &remember);
   if (e != cudaSuccess) return e;
-  const bool cached = dev >= 0 && dev < 64 && !host_pretends();
-  if (!cached || !attr_set[dev].load(std::memory_order_acquire)) {
+  if (!remember || !attr_set[dev].load(std::memory_order_acquire)) {
     e = host().func_set_smem(reinterpret_cast<const void*>(sm100_fwd_kernel<T, HD, EXACT>), L::kDynamic);
     if (e != cudaSuccess) return e;
-    if (cached) attr_set[dev].store(true, std::memory_order_release);
-  }
-  unsigned int* status = cached ? status_of[dev].load(std::memory_order_acquire) : nullptr;
-  if (status == nullptr) {
-    e = host().symbol_address(reinterpret_cast<void**>(&status), reinterpret_cast<const void*>(&g_sm100_fwd_status));
-    if (e != cudaSuccess) return e;
-    if (cached) status_of[dev].store(status, std::memory_order_release);
+    if (remember) attr_set[dev].store(true, std::memory_order_release);
   }
   dim3 grid((p.max_sq + L::kCtaRows - 1) / L::kCtaRows, p.hq, p.batch);
   e = launch_kernel(sm100_fwd_kernel<T, HD, EXACT>, grid, dim3(kFwdThreads), L::kDynamic, st, p, tq, tk, tv, status);
@@ -651,6 +669,7 @@ bool sm100_fwd_supported(int dtype, const Params& p) {
 }
 
 cudaError_t launch_sm100_fwd(int dtype, const Params& p, cudaStream_t st) {
+  if (decode_shape(p)) return dtype == 2 ? launch_decode_T<__half>(p, st) : launch_decode_T<__nv_bfloat16>(p, st);
   const int dmax = p.dqk > p.dvo ? p.dqk : p.dvo;
   if (dtype == 2)
     return dmax <= 64 ? launch_fwd_T<__half, 64>(p, st)
