@@ -3,7 +3,8 @@
 // three flavours, bias/dBias, dropout, Dqk != Dvo -- with plain CUDA cores and fp32
 // math, and back the shapes the tcgen05 kernels do not take.
 //
-// All three matmul-bearing kernels share one scheme.  A CTA of 256 threads owns a
+// Head dims up to 128 run the register-tiled kernels of general_tiled.cuh.  Above that, all three
+// matmul-bearing kernels share one scheme.  A CTA of 256 threads owns a
 // 16x16 tile of (query, key) pairs:
 //   pair phase        thread (r, c) computes the dot products of query r with key c
 //                     from fp32 tiles staged in shared memory, applies scale, bias,
@@ -370,6 +371,8 @@ __global__ void __launch_bounds__(kThreads) general_bwd_dq_kernel(const __grid_c
   }
 }
 
+#include "general_tiled.cuh"
+
 // ---------------------------------------------------------------------------
 // delta[m] = sum_d O[m,d] * dO[m,d] in fp32, written with the LSE layout.  HBM-bound.
 // grid = (cdiv(max_sq, 128), Hq, batch); a CTA of 8 warps owns 128 rows of one (sequence, head).
@@ -525,11 +528,27 @@ cudaError_t launch_general_T(int which, const Params& p, cudaStream_t st) {
   return e;
 }
 
+template <typename T, int DP>
+cudaError_t launch_tiled_T(int which, const Params& p, cudaStream_t st) {
+  using C = Tiled<DP>;
+  const size_t rows = which == 0 ? C::kBM + 2 * C::kBN : 2 * C::kBM + 2 * C::kBN;      // staged rows of DP + 4 floats
+  const size_t tiles = which == 1 ? 2 : 1;                                             // P and dS, or one of them
+  const size_t sm = (rows * C::kLd + tiles * C::kBM * C::kLdP + (which == 1 ? 2 * C::kBN : 0)) * sizeof(float);
+  auto kern = which == 0 ? tiled_fwd_kernel<T, DP> : (which == 1 ? tiled_bwd_dkdv_kernel<T, DP> : tiled_bwd_dq_kernel<T, DP>);
+  cudaError_t e = set_smem(kern, sm);
+  if (e != cudaSuccess) return e;
+  const int rows_total = which == 1 ? p.max_sk : p.max_sq;
+  dim3 grid((rows_total + C::kBM - 1) / C::kBM, which == 1 ? p.hk : p.hq, p.batch);
+  e = launch_kernel(kern, grid, dim3(C::kThreads), sm, st, p);
+  if (e == cudaSuccess) count_launch();
+  return e;
+}
+
 template <typename T>
 cudaError_t launch_general_D(int which, const Params& p, cudaStream_t st) {
   int d = p.dqk > p.dvo ? p.dqk : p.dvo;
-  if (d <= 64) return launch_general_T<T, 2>(which, p, st);
-  if (d <= 128) return launch_general_T<T, 4>(which, p, st);
+  if (d <= 64) return launch_tiled_T<T, 64>(which, p, st);
+  if (d <= 128) return launch_tiled_T<T, 128>(which, p, st);
   if (d <= 256) return launch_general_T<T, 8>(which, p, st);
   return launch_general_T<T, 16>(which, p, st);
 }

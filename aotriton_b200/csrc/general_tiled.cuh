@@ -1,0 +1,402 @@
+// General attention kernels for head dims up to 128: register tiles on the fp32 arithmetic units.
+// Included by general_kernels.cu inside its namespaces.
+//
+// What bounds them: 16-byte shared-memory reads (an 8-read step feeds 64 multiply-adds per thread) where the
+// grid fills the chip, the latency of a block's chain -- stage, scores, softmax, accumulate -- where it does
+// not.  The 16x16-tile kernels (kept for head dims above 128) compute one dot product per thread, two
+// reads for every four multiply-adds.  Here a CTA of 128 threads owns 32 rows (queries; keys for
+// dK / dV) and walks the other sequence dimension in blocks of BN columns; a thread holds a 4 x BN/16
+// tile of scores (rows ty*4.., columns tx + 16 j) and a 4 x DP/16 tile of each accumulator (columns tx*4.. + 64 j),
+// so that a 16-byte read feeds 8 or more multiply-adds.  32 rows and not 64: at the sizes single precision is
+// used at, the number of CTAs is what is short.  Measured, fp32: 2 x 8 heads x 500 tokens, head dim 64, causal:
+// forward 114 -> 68 us, dK/dV 176 -> 101, dQ 141 -> 86; 4 x 8 x 1024, head dim 128: 1471 -> 719, 2684 -> 1820,
+// 2038 -> 1244.
+//
+// All tiles are row-major fp32 with four floats of padding: (DP + 4) / 4 is odd, so the 16 lanes that
+// read 16 different rows at one column hit different banks.  The P / dS rows that a warp writes are read
+// back by that warp only.
+template <int DP> struct Tiled {
+  static constexpr int kThreads = 128, kBM = 32;
+  static constexpr int kBN = DP > 64 ? 32 : 64;
+  static constexpr int kNC = kBN / 16;        // score columns per thread
+  static constexpr int kND = DP / 64;         // float4 accumulator columns per thread
+  static constexpr int kLd = DP + 4, kLdP = kBN + 4;
+};
+
+// 16-byte (fp32) or 8-byte (16-bit types) loads of four elements are possible on every row of the view.
+template <typename T>
+__device__ __forceinline__ bool rows_vec4(const View4& v, int d) {
+  return ((reinterpret_cast<uintptr_t>(v.ptr) & (4 * sizeof(T) - 1)) == 0) && ((v.s[0] | v.s[1] | v.s[2]) & 3) == 0 && (d & 3) == 0;
+}
+
+// Rows row0.. of one head into dst[ROWS][DP + 4]; rows at or beyond nrows and columns at or beyond d
+// are zero (columns up to the next multiple of four: the contractions stop there, the accumulators' ones
+// are never stored).
+template <typename T, int DP, int ROWS>
+__device__ __forceinline__ void stage_tile(float* dst, const View4& v, int b, int h, int64_t tok0, int row0, int nrows, int d, bool vec) {
+  constexpr int kThreadsT = Tiled<DP>::kThreads, kLd = Tiled<DP>::kLd, kC4 = DP / 4;
+  const T* base = row_ptr<T>(v, b, h, tok0 + row0);
+#pragma unroll 4
+  for (int idx = threadIdx.x; idx < ROWS * kC4; idx += kThreadsT) {
+    const int r = idx / kC4, c = (idx - r * kC4) * 4;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (row0 + r < nrows && c < d) {
+      const T* src = base + (int64_t)r * v.s[2] + c;
+      if (vec) {
+        if constexpr (sizeof(T) == 4) {
+          x = __ldg(reinterpret_cast<const float4*>(src));
+        } else {
+          const uint2 w = __ldg(reinterpret_cast<const uint2*>(src));
+          const T* e = reinterpret_cast<const T*>(&w);
+          x = make_float4(to_f32<T>(e[0]), to_f32<T>(e[1]), to_f32<T>(e[2]), to_f32<T>(e[3]));
+        }
+      } else {
+        x.x = to_f32<T>(src[0]);
+        if (c + 1 < d) x.y = to_f32<T>(src[1]);
+        if (c + 2 < d) x.z = to_f32<T>(src[2]);
+        if (c + 3 < d) x.w = to_f32<T>(src[3]);
+      }
+    }
+    *reinterpret_cast<float4*>(dst + r * kLd + c) = x;
+  }
+}
+
+// s[i][j] = A[ty*4 + i] . B[tx + 16 j] over d4 groups of four columns
+template <int DP>
+__device__ __forceinline__ void tile_dots(float (&s)[4][Tiled<DP>::kNC], const float* A, const float* B, int d4, int ty, int tx) {
+  using C = Tiled<DP>;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < C::kNC; ++j) s[i][j] = 0.f;
+  const float* a0 = A + ty * 4 * C::kLd;
+  const float* b0 = B + tx * C::kLd;
+#pragma unroll 2
+  for (int c = 0; c < d4; ++c) {
+    float4 a[4], b[C::kNC];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(a0 + i * C::kLd + c * 4);
+#pragma unroll
+    for (int j = 0; j < C::kNC; ++j) b[j] = *reinterpret_cast<const float4*>(b0 + j * 16 * C::kLd + c * 4);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < C::kNC; ++j) {
+        s[i][j] = fmaf(a[i].x, b[j].x, s[i][j]);
+        s[i][j] = fmaf(a[i].y, b[j].y, s[i][j]);
+        s[i][j] = fmaf(a[i].z, b[j].z, s[i][j]);
+        s[i][j] = fmaf(a[i].w, b[j].w, s[i][j]);
+      }
+  }
+}
+
+// acc[i][j] += P[ty*4 + i][0..BN) x X[0..BN)[tx*4 + 64 j ..]
+template <int DP>
+__device__ __forceinline__ void tile_accumulate(float4 (&acc)[4][Tiled<DP>::kND], const float* P, const float* X, int ty, int tx) {
+  using C = Tiled<DP>;
+  const float* p0 = P + ty * 4 * C::kLdP;
+  const float* x0 = X + tx * 4;
+#pragma unroll 2
+  for (int k = 0; k < C::kBN; k += 4) {
+    float4 a[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(p0 + i * C::kLdP + k);
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+      for (int j = 0; j < C::kND; ++j) {
+        const float4 x = *reinterpret_cast<const float4*>(x0 + (k + kk) * C::kLd + 64 * j);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float w = kk == 0 ? a[i].x : (kk == 1 ? a[i].y : (kk == 2 ? a[i].z : a[i].w));
+          acc[i][j].x = fmaf(w, x.x, acc[i][j].x);
+          acc[i][j].y = fmaf(w, x.y, acc[i][j].y);
+          acc[i][j].z = fmaf(w, x.z, acc[i][j].z);
+          acc[i][j].w = fmaf(w, x.w, acc[i][j].w);
+        }
+      }
+  }
+}
+
+template <typename T, int DP>
+__device__ __forceinline__ void store_acc_row(T* dst, const float4 (&acc)[Tiled<DP>::kND], float scale, int d, int tx) {
+#pragma unroll
+  for (int j = 0; j < Tiled<DP>::kND; ++j) {
+    const int c = tx * 4 + 64 * j;
+    if (c + 0 < d) dst[c + 0] = from_f32<T>(acc[j].x * scale);
+    if (c + 1 < d) dst[c + 1] = from_f32<T>(acc[j].y * scale);
+    if (c + 2 < d) dst[c + 2] = from_f32<T>(acc[j].z * scale);
+    if (c + 3 < d) dst[c + 3] = from_f32<T>(acc[j].w * scale);
+  }
+}
+
+// Keep bits of a thread's scores when rows are queries: the four lanes of a quad own the four keys of
+// a Philox counter for each (row, j); each lane draws one of the quad's four rows and they exchange.
+// Bit 4*j + i of the result: row ty*4 + i, column tx + 16 j.
+template <int NC>
+__device__ __forceinline__ uint32_t tile_keep_bits(const DropoutCtx& d, int m_first, int n_first, int tx) {
+  const int lane = threadIdx.x & 31, q = lane & 3;
+  uint32_t mine = 0u, keep = 0u;
+#pragma unroll
+  for (int j = 0; j < NC; ++j) mine |= dropout_keep4(d, m_first + q, (n_first + (tx & ~3) + 16 * j) >> 2) << (4 * j);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t w = __shfl_sync(0xffffffffu, mine, (lane & ~3) | i);
+#pragma unroll
+    for (int j = 0; j < NC; ++j) keep |= ((w >> (4 * j + q)) & 1u) << (4 * j + i);
+  }
+  return keep;
+}
+
+template <typename T>
+__device__ __forceinline__ const T* bias_at(const Params& p, const Seq& sq, int h, int m, int n) {
+  return reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] + (int64_t)h * p.bias.s[1] +
+         (int64_t)m * p.bias.s[2] + (int64_t)n * p.bias.s[3];
+}
+
+// Forward.  grid = (cdiv(max_sq, 32), Hq, batch); the last rows of a causal problem see the most keys and start first.
+template <typename T, int DP>
+__global__ void __launch_bounds__(128) tiled_fwd_kernel(const __grid_constant__ Params p) {
+  using C = Tiled<DP>;
+  extern __shared__ float smem[];
+  float* Qs = smem;                       // [32][LD]
+  float* Ks = Qs + C::kBM * C::kLd;       // [BN][LD]
+  float* Vs = Ks + C::kBN * C::kLd;       // [BN][LD]
+  float* Ps = Vs + C::kBN * C::kLd;       // [32][BN + 4]
+  const int z = blockIdx.z, h = blockIdx.y, m0 = (int)(gridDim.x - 1 - blockIdx.x) * C::kBM;
+  // One thread of the grid reports the seed and offset actually used, before any early exit
+  // (the first sequence of a varlen batch may be empty).
+  if (p.dropout_on && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) {
+    if (p.seed_out) *p.seed_out = p.seed_ptr ? *p.seed_ptr : 0ull;
+    if (p.off_out) *p.off_out = p.off2 + (p.off1_ptr ? *p.off1_ptr : 0ull);
+  }
+  const Seq sq = resolve_seq(p, z);
+  if (m0 >= sq.sq) return;
+  const int hk = h / p.group, ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const bool kvec = rows_vec4<T>(p.k, p.dqk), vvec = rows_vec4<T>(p.v, p.dvo);
+  DropoutCtx dctx;
+  if (p.dropout_on) dctx = dropout_ctx(p, z, h);
+  stage_tile<T, DP, C::kBM>(Qs, p.q, sq.bidx, h, sq.q0, m0, sq.sq, p.dqk, rows_vec4<T>(p.q, p.dqk));
+  float m_i[4], l_i[4];
+  float4 acc[4][C::kND];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m_i[i] = -INFINITY;
+    l_i[i] = 0.f;
+#pragma unroll
+    for (int j = 0; j < C::kND; ++j) acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  int n_lo, n_hi;
+  key_range(p, sq, m0, min(m0 + C::kBM, sq.sq) - 1, n_lo, n_hi);
+  const int d4 = (p.dqk + 3) >> 2;
+  for (int n0 = n_lo / C::kBN * C::kBN; n0 <= n_hi; n0 += C::kBN) {
+    __syncthreads();   // the previous block's tiles have been read
+    stage_tile<T, DP, C::kBN>(Ks, p.k, sq.bidx, hk, sq.k0, n0, sq.sk, p.dqk, kvec);
+    stage_tile<T, DP, C::kBN>(Vs, p.v, sq.bidx, hk, sq.k0, n0, sq.sk, p.dvo, vvec);
+    __syncthreads();
+    float s[4][C::kNC];
+    tile_dots<DP>(s, Qs, Ks, d4, ty, tx);
+    const uint32_t keep = p.dropout_on ? tile_keep_bits<C::kNC>(dctx, m0 + ty * 4, n0, tx) : 0xffffffffu;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int m = m0 + ty * 4 + i;
+      float mx = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < C::kNC; ++j) {
+        const int n = n0 + tx + 16 * j;
+        const bool ok = score_valid(p, sq, m, n);
+        s[i][j] *= p.qk_scale;
+        if (ok && p.has_bias) s[i][j] += to_f32<T>(*bias_at<T>(p, sq, h, m, n)) * kLog2e;
+        if (!ok) s[i][j] = -INFINITY;
+        mx = fmaxf(mx, s[i][j]);
+      }
+      const float m_new = fmaxf(m_i[i], half_warp_max(mx));
+      const float ms = m_new == -INFINITY ? 0.f : m_new, alpha = exp2f(m_i[i] - ms);   // m_i == -inf -> 0
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < C::kNC; ++j) {
+        float pv = exp2f(s[i][j] - ms);
+        sum += pv;
+        if (!((keep >> (4 * j + i)) & 1u)) pv = 0.f;
+        Ps[(ty * 4 + i) * C::kLdP + tx + 16 * j] = round_to<T>(pv);
+      }
+      l_i[i] = l_i[i] * alpha + sum;      // this lane's columns: the row's sums meet after the loop
+      m_i[i] = m_new;
+#pragma unroll
+      for (int j = 0; j < C::kND; ++j) {
+        acc[i][j].x *= alpha; acc[i][j].y *= alpha; acc[i][j].z *= alpha; acc[i][j].w *= alpha;
+      }
+    }
+    __syncwarp();
+    tile_accumulate<DP>(acc, Ps, Vs, ty, tx);
+    __syncwarp();
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = m0 + ty * 4 + i;
+    const float l = half_warp_sum(l_i[i]);
+    if (m >= sq.sq) continue;
+    // natural-log LSE of the scaled, biased logits; rows without any valid key get O = 0, LSE = +inf
+    if (tx == 0 && p.lse != nullptr) p.lse[lse_offset(p, sq, h) + m] = l > 0.f ? (m_i[i] + log2f(l)) * kLn2 : INFINITY;
+    store_acc_row<T, DP>(row_ptr_mut<T>(p.out, sq.bidx, h, sq.q0 + m), acc[i], l > 0.f ? (1.f / l) * p.dropout_scale : 0.f, p.dvo, tx);
+  }
+}
+
+// dK / dV.  grid = (cdiv(max_sk, 32), Hk, batch)
+template <typename T, int DP>
+__global__ void __launch_bounds__(128) tiled_bwd_dkdv_kernel(const __grid_constant__ Params p) {
+  using C = Tiled<DP>;
+  extern __shared__ float smem[];
+  float* Ks = smem;                       // [32][LD]
+  float* Vs = Ks + C::kBM * C::kLd;
+  float* Qs = Vs + C::kBM * C::kLd;       // [BN][LD]
+  float* dOs = Qs + C::kBN * C::kLd;
+  float* Ps = dOs + C::kBN * C::kLd;      // [32][BN + 4]
+  float* dSs = Ps + C::kBM * C::kLdP;
+  float* lse_s = dSs + C::kBM * C::kLdP;  // [BN]
+  float* dl_s = lse_s + C::kBN;
+  const int z = blockIdx.z, hk = blockIdx.y, n0 = blockIdx.x * C::kBM;
+  const Seq sq = resolve_seq(p, z);
+  if (n0 >= sq.sk) return;
+  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const bool qvec = rows_vec4<T>(p.q, p.dqk), dovec = rows_vec4<T>(p.dout, p.dvo);
+  stage_tile<T, DP, C::kBM>(Ks, p.k, sq.bidx, hk, sq.k0, n0, sq.sk, p.dqk, rows_vec4<T>(p.k, p.dqk));
+  stage_tile<T, DP, C::kBM>(Vs, p.v, sq.bidx, hk, sq.k0, n0, sq.sk, p.dvo, rows_vec4<T>(p.v, p.dvo));
+  float4 adv[4][C::kND], adk[4][C::kND];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < C::kND; ++j) adv[i][j] = adk[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+  int m_lo, m_hi;
+  query_range(p, sq, n0, min(n0 + C::kBM, sq.sk) - 1, m_lo, m_hi);
+  const int dq4 = (p.dqk + 3) >> 2, dv4 = (p.dvo + 3) >> 2;
+  for (int g = 0; g < p.group; ++g) {
+    const int h = hk * p.group + g;
+    DropoutCtx dctx;
+    if (p.dropout_on) dctx = dropout_ctx(p, z, h);
+    const int64_t lrow = lse_offset(p, sq, h);
+    for (int m0 = m_lo / C::kBN * C::kBN; m0 <= m_hi; m0 += C::kBN) {
+      __syncthreads();
+      stage_tile<T, DP, C::kBN>(Qs, p.q, sq.bidx, h, sq.q0, m0, sq.sq, p.dqk, qvec);
+      stage_tile<T, DP, C::kBN>(dOs, p.dout, sq.bidx, h, sq.q0, m0, sq.sq, p.dvo, dovec);
+      if (threadIdx.x < C::kBN) {
+        const int m = m0 + threadIdx.x;
+        lse_s[threadIdx.x] = m < sq.sq ? p.lse[lrow + m] * kLog2e : INFINITY;
+        dl_s[threadIdx.x] = m < sq.sq ? p.delta[lrow + m] : 0.f;
+      }
+      __syncthreads();
+      float s[4][C::kNC], dp[4][C::kNC];
+      tile_dots<DP>(s, Ks, Qs, dq4, ty, tx);
+      tile_dots<DP>(dp, Vs, dOs, dv4, ty, tx);
+#pragma unroll
+      for (int j = 0; j < C::kNC; ++j) {
+        const int c = tx + 16 * j, m = m0 + c;
+        // (a thread's four keys are the four columns of one Philox counter)
+        const uint32_t keep = p.dropout_on ? dropout_keep4(dctx, m, (n0 + ty * 4) >> 2) : 15u;
+        const float lse = lse_s[c], dl = dl_s[c];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int n = n0 + ty * 4 + i;
+          float pd = 0.f, ds = 0.f;
+          if (score_valid(p, sq, m, n)) {
+            float x = s[i][j] * p.qk_scale;
+            if (p.has_bias) x += to_f32<T>(*bias_at<T>(p, sq, h, m, n)) * kLog2e;
+            const float pr = exp2f(x - lse);      // lse = +inf on dead rows -> 0
+            const bool kept = (keep >> i) & 1u;
+            pd = kept ? pr * p.dropout_scale : 0.f;
+            ds = pr * ((kept ? dp[i][j] * p.dropout_scale : 0.f) - dl);
+          }
+          Ps[(ty * 4 + i) * C::kLdP + c] = round_to<T>(pd);
+          dSs[(ty * 4 + i) * C::kLdP + c] = round_to<T>(ds);
+        }
+      }
+      __syncwarp();
+      tile_accumulate<DP>(adv, Ps, dOs, ty, tx);
+      tile_accumulate<DP>(adk, dSs, Qs, ty, tx);
+      __syncwarp();
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int n = n0 + ty * 4 + i;
+    if (n >= sq.sk) continue;
+    store_acc_row<T, DP>(row_ptr_mut<T>(p.dk, sq.bidx, hk, sq.k0 + n), adk[i], p.sm_scale, p.dqk, tx);
+    store_acc_row<T, DP>(row_ptr_mut<T>(p.dv, sq.bidx, hk, sq.k0 + n), adv[i], 1.f, p.dvo, tx);
+  }
+}
+
+// dQ (+ dBias).  grid = (cdiv(max_sq, 32), Hq, batch), last rows first
+template <typename T, int DP>
+__global__ void __launch_bounds__(128) tiled_bwd_dq_kernel(const __grid_constant__ Params p) {
+  using C = Tiled<DP>;
+  extern __shared__ float smem[];
+  float* Qs = smem;                       // [32][LD]
+  float* dOs = Qs + C::kBM * C::kLd;
+  float* Ks = dOs + C::kBM * C::kLd;      // [BN][LD]
+  float* Vs = Ks + C::kBN * C::kLd;
+  float* dSs = Vs + C::kBN * C::kLd;      // [32][BN + 4]
+  const int z = blockIdx.z, h = blockIdx.y, m0 = (int)(gridDim.x - 1 - blockIdx.x) * C::kBM;
+  const Seq sq = resolve_seq(p, z);
+  if (m0 >= sq.sq) return;
+  const int hk = h / p.group, ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const bool kvec = rows_vec4<T>(p.k, p.dqk), vvec = rows_vec4<T>(p.v, p.dvo);
+  DropoutCtx dctx;
+  if (p.dropout_on) dctx = dropout_ctx(p, z, h);
+  stage_tile<T, DP, C::kBM>(Qs, p.q, sq.bidx, h, sq.q0, m0, sq.sq, p.dqk, rows_vec4<T>(p.q, p.dqk));
+  stage_tile<T, DP, C::kBM>(dOs, p.dout, sq.bidx, h, sq.q0, m0, sq.sq, p.dvo, rows_vec4<T>(p.dout, p.dvo));
+  const int64_t lrow = lse_offset(p, sq, h);
+  float lse[4], dl[4];
+  float4 adq[4][C::kND];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = m0 + ty * 4 + i;
+    lse[i] = m < sq.sq ? p.lse[lrow + m] * kLog2e : INFINITY;
+    dl[i] = m < sq.sq ? p.delta[lrow + m] : 0.f;
+#pragma unroll
+    for (int j = 0; j < C::kND; ++j) adq[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  int n_lo, n_hi;
+  key_range(p, sq, m0, min(m0 + C::kBM, sq.sq) - 1, n_lo, n_hi);
+  if (n_hi >= n_lo) zero_dbias_outside<T>(p, sq, h, m0, C::kBM, n_lo / C::kBN * C::kBN, (n_hi / C::kBN + 1) * C::kBN);
+  else zero_dbias_outside<T>(p, sq, h, m0, C::kBM, 0, 0);
+  const int dq4 = (p.dqk + 3) >> 2, dv4 = (p.dvo + 3) >> 2;
+  for (int n0 = n_lo / C::kBN * C::kBN; n0 <= n_hi; n0 += C::kBN) {
+    __syncthreads();
+    stage_tile<T, DP, C::kBN>(Ks, p.k, sq.bidx, hk, sq.k0, n0, sq.sk, p.dqk, kvec);
+    stage_tile<T, DP, C::kBN>(Vs, p.v, sq.bidx, hk, sq.k0, n0, sq.sk, p.dvo, vvec);
+    __syncthreads();
+    float s[4][C::kNC], dp[4][C::kNC];
+    tile_dots<DP>(s, Qs, Ks, dq4, ty, tx);
+    tile_dots<DP>(dp, dOs, Vs, dv4, ty, tx);
+    const uint32_t keep = p.dropout_on ? tile_keep_bits<C::kNC>(dctx, m0 + ty * 4, n0, tx) : 0xffffffffu;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int m = m0 + ty * 4 + i;
+#pragma unroll
+      for (int j = 0; j < C::kNC; ++j) {
+        const int n = n0 + tx + 16 * j;
+        float ds = 0.f;
+        if (score_valid(p, sq, m, n)) {
+          float x = s[i][j] * p.qk_scale;
+          if (p.has_bias) x += to_f32<T>(*bias_at<T>(p, sq, h, m, n)) * kLog2e;
+          const float pr = exp2f(x - lse[i]);
+          ds = pr * (((keep >> (4 * j + i)) & 1u ? dp[i][j] * p.dropout_scale : 0.f) - dl[i]);
+        }
+        if (p.has_dbias && m < sq.sq && n < sq.sk) {
+          T* dbp = reinterpret_cast<T*>(p.dbias.ptr) + (int64_t)sq.bidx * p.dbias.s[0] + (int64_t)h * p.dbias.s[1] +
+                   (int64_t)m * p.dbias.s[2] + (int64_t)n * p.dbias.s[3];
+          *dbp = from_f32<T>(ds);
+        }
+        dSs[(ty * 4 + i) * C::kLdP + tx + 16 * j] = round_to<T>(ds);
+      }
+    }
+    __syncwarp();
+    tile_accumulate<DP>(adq, dSs, Ks, ty, tx);
+    __syncwarp();
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = m0 + ty * 4 + i;
+    if (m < sq.sq) store_acc_row<T, DP>(row_ptr_mut<T>(p.dq, sq.bidx, h, sq.q0 + m), adq[i], p.sm_scale, p.dqk, tx);
+  }
+}
