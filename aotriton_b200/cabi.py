@@ -24,8 +24,8 @@ SYMBOLS = [
     "ab200_bwd_fused", "ab200_bwd_postprocess", "ab200_bwd_preprocess", "ab200_bwd_dkdv", "ab200_bwd_dq",
     "ab200_debug_simulate_encoded_softmax", "ab200_check_gpu", "ab200_multiprocessor_count",
     "ab200_set_kernel_family", "ab200_select_variant", "ab200_last_fwd_family", "ab200_last_bwd_family",
-    "ab200_kernel_status", "ab200_stream_check", "ab200_debug_bounded_wait_test", "ab200_debug_host_calls",
-    "ab200_debug_host_call_count", "ab200_launch_count", "ab200_version",
+    "ab200_kernel_status", "ab200_stream_check", "ab200_debug_bounded_wait_test", "ab200_debug_keep_tiles",
+    "ab200_debug_host_calls", "ab200_debug_host_call_count", "ab200_launch_count", "ab200_version",
 ]
 
 
@@ -90,6 +90,7 @@ def lib() -> C.CDLL:
         L.ab200_stream_check.argtypes = [C.c_void_p]
         L.ab200_debug_bounded_wait_test.argtypes = [C.c_int, C.c_uint]
         L.ab200_debug_bounded_wait_test.restype = None
+        L.ab200_debug_keep_tiles.argtypes = [C.POINTER(BwdArgs)]
         L.ab200_debug_host_calls.argtypes = [C.c_int] * 4
         L.ab200_debug_host_calls.restype = None
         L.ab200_debug_host_call_count.argtypes = [C.c_int]

@@ -270,6 +270,70 @@ constexpr SelectionRow kSelection[] = {
     {kOpBwd, kHalfTypes, 256, 256, kVarTcgen05}, {kOpBwd, kAllTypes, 512, 0, kVarGeneral},
 };
 
+// ---- keep bits shared between the kernels of one backward (KeepShare in common.cuh) ---------
+// Bytes [lo, hi) a view of 16-bit elements reaches.  False: extents or strides that say nothing.
+bool view_range(const View4& v, uintptr_t* lo, uintptr_t* hi) {
+  int64_t last = 0;
+  for (int i = 0; i < 4; ++i) {
+    if (v.n[i] <= 0 || (v.n[i] > 1 && v.s[i] < 0)) return false;
+    last += (v.n[i] - 1) * (v.n[i] > 1 ? v.s[i] : 0);
+  }
+  *lo = reinterpret_cast<uintptr_t>(v.ptr);
+  *hi = *lo + 2 * (uintptr_t)(last + 1);
+  return true;
+}
+
+// Decides whether (and for how many 32-key tiles) dQ's rows carry keep bits from the dK/dV kernel to the dQ
+// kernel.  dQ must be a tensor in which no two rows share memory, shaped like q, and apart from everything
+// the kernels still read when the bits are written: a caller may hand in the same memory for dQ and an
+// input, which works as long as dQ is only written by the kernel that no longer needs that input.  Head
+// dims below 64 have no room for a tile (128 bytes) in a row.
+void keep_share_setup(Params& p) {
+  p.keep_tiles = 0;
+  p.keep_shift = 0;
+  if (!p.dropout_on || p.dqk < 64 || p.dq.s[3] != 1 || (reinterpret_cast<uintptr_t>(p.dq.ptr) & 15u) != 0) return;
+  for (int i = 0; i < 3; ++i)
+    if (p.dq.n[i] != p.q.n[i] || p.dq.s[i] % 8 != 0) return;
+  if (p.dq.n[3] != p.dqk) return;
+  uintptr_t lo, hi;
+  if (!view_range(p.dq, &lo, &hi)) return;
+  // no two elements at one address: sorted by stride, each dimension steps over the whole of the ones below
+  int order[3] = {0, 1, 2};
+  for (int i = 0; i < 2; ++i)
+    for (int j = 0; j < 2 - i; ++j)
+      if (p.dq.s[order[j]] > p.dq.s[order[j + 1]]) { const int t = order[j]; order[j] = order[j + 1]; order[j + 1] = t; }
+  int64_t extent = p.dqk;
+  for (int i = 0; i < 3; ++i) {
+    const int d = order[i];
+    if (p.dq.n[d] == 1) continue;
+    if (p.dq.s[d] < extent) return;
+    extent += (p.dq.n[d] - 1) * p.dq.s[d];
+  }
+  auto apart = [&](uintptr_t b, uintptr_t e) { return e <= lo || b >= hi; };
+  for (const View4* v : {&p.q, &p.k, &p.v, &p.dout, &p.bias, &p.dk, &p.dv}) {
+    if (v->ptr == nullptr) continue;
+    uintptr_t b, e;
+    if (!view_range(*v, &b, &e) || !apart(b, e)) return;
+  }
+  // logsumexp and delta: dense fp32, one per (batch, q head, query row); token-packed: per (q head, token)
+  const uintptr_t rows = (uintptr_t)p.hq * (p.varlen_mode == 1 ? (uintptr_t)p.q.n[2] : (uintptr_t)p.batch * (uintptr_t)p.max_sq);
+  for (const float* f : {static_cast<const float*>(p.lse), static_cast<const float*>(p.delta)}) {
+    const uintptr_t b = reinterpret_cast<uintptr_t>(f);
+    if (!apart(b, b + 4 * rows)) return;
+  }
+  const uintptr_t cu_bytes = 4 * ((uintptr_t)p.batch + 1);
+  for (const int32_t* c : {p.cu_q, p.cu_k, p.ss_q, p.ss_k}) {
+    const uintptr_t b = reinterpret_cast<uintptr_t>(c);
+    if (c != nullptr && !apart(b, b + cu_bytes)) return;
+  }
+  for (const uint64_t* c : {p.seed_ptr, p.off1_ptr}) {
+    const uintptr_t b = reinterpret_cast<uintptr_t>(c);
+    if (c != nullptr && !apart(b, b + 8)) return;
+  }
+  p.keep_shift = p.dqk >= 256 ? 2 : (p.dqk >= 128 ? 1 : 0);
+  p.keep_tiles = std::min(32 << p.keep_shift, (p.max_sk + 31) / 32);
+}
+
 bool want_sm100(int family) { return family != 1; }
 int family_flags(int family) {
   return family == 1 ? AB200_SELECT_FORCE_GENERAL : (family == 2 ? AB200_SELECT_FORCE_TCGEN05 : 0);
@@ -439,7 +503,8 @@ int ab200_bwd_preprocess(const ab200_attn_bwd_args* a, void* stream) {
   return (int)launch_preprocess(a->prob.dtype, p, st);
 }
 
-int ab200_bwd_dkdv(const ab200_attn_bwd_args* a, void* stream) {
+// `share`: dK/dV and dQ run in one call, so that keep bits may pass from one to the other.
+static int run_dkdv(const ab200_attn_bwd_args* a, void* stream, bool share) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   Params p{};
   if (int e = fill_bwd(a, p, true)) return e;
@@ -451,13 +516,14 @@ int ab200_bwd_dkdv(const ab200_attn_bwd_args* a, void* stream) {
   if (sel < 0) return -sel;
   if ((sel & 0xff) >= kVarTcgen05) {
     t_last_bwd = 2;
+    if (share) keep_share_setup(p);
     return (int)launch_sm100_bwd_dkdv(a->prob.dtype, p, st);
   }
   t_last_bwd = 1;
   return (int)launch_general(1, a->prob.dtype, p, st);
 }
 
-int ab200_bwd_dq(const ab200_attn_bwd_args* a, void* stream) {
+static int run_dq(const ab200_attn_bwd_args* a, void* stream, bool share) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   Params p{};
   if (int e = fill_bwd(a, p, true)) return e;
@@ -469,11 +535,15 @@ int ab200_bwd_dq(const ab200_attn_bwd_args* a, void* stream) {
   if (sel < 0) return -sel;
   if ((sel & 0xff) >= kVarTcgen05) {
     t_last_bwd = 2;
+    if (share) keep_share_setup(p);
     return (int)launch_sm100_bwd_dq(a->prob.dtype, p, st);
   }
   t_last_bwd = 1;
   return (int)launch_general(2, a->prob.dtype, p, st);
 }
+
+int ab200_bwd_dkdv(const ab200_attn_bwd_args* a, void* stream) { return run_dkdv(a, stream, false); }
+int ab200_bwd_dq(const ab200_attn_bwd_args* a, void* stream) { return run_dq(a, stream, false); }
 
 int ab200_bwd_uses_dq_acc(const ab200_attn_bwd_args* a, void* stream) {
   if (a == nullptr || a->deterministic || !want_fused(g_family)) return 0;
@@ -519,8 +589,15 @@ int ab200_attn_bwd(const ab200_attn_bwd_args* a, void* stream) {
     if (int e = ab200_bwd_fused(a, stream)) return e;
     return ab200_bwd_postprocess(a, stream);
   }
-  if (int e = ab200_bwd_dkdv(a, stream)) return e;
-  return ab200_bwd_dq(a, stream);
+  if (int e = run_dkdv(a, stream, true)) return e;
+  return run_dq(a, stream, true);
+}
+
+int ab200_debug_keep_tiles(const ab200_attn_bwd_args* a) {
+  Params p{};
+  if (int e = fill_bwd(a, p, true)) return -e;
+  keep_share_setup(p);
+  return p.keep_tiles;
 }
 
 // --- backward with the delta scratch inside the library image -----------------------------

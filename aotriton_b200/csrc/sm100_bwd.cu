@@ -781,6 +781,8 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
 #pragma unroll
           for (int k = 0; k < 8; ++k)
             mine |= dropout_keep4_keys(dctx, pkeys, min(mbase + q4 + 4 * k, p.max_sq - 1), n >> 2) << (4 * k);
+          if (keep_shared(p, sq, mbase, it.n0 + quarter * 32))
+            *keep_share_word(p, sq, h, mbase, it.n0 + quarter * 32, lane) = keep_rows_from_quads(mine, lane);
           keep = 0u;
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -1212,6 +1214,10 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
       const uint32_t par = (uint32_t)i & 1u;
       const int nbase = (jb_lo + i) * kBlk + cbase;     // first key of this thread's columns
       if (threadIdx.x == AB200_TRACE_TID) AB200_STAMPQ(i, 4);
+      // keep bits the dK/dV kernel left behind: on their way while the tensor pipe computes S
+      const bool shared = keep_shared(p, sq, m0 + quarter * 32, nbase);
+      uint32_t shared_bits = 0u;
+      if (shared) shared_bits = *keep_share_word(p, sq, h, m0 + quarter * 32, nbase, lane);
       // (the thread's 64 bytes of bias for this block: on their way to L2 while the tensor pipe computes S)
       if (p.has_bias && p.bias_vec) asm volatile("prefetch.global.L2 [%0];" ::"l"(bias_row + nbase));
       if (!mbar_wait(&bars[L::bSFull], par, abort_flag, status, 0x2600 + i)) { ok = false; break; }
@@ -1269,7 +1275,9 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
         }
       }
       uint32_t keep = 0xffffffffu;
-      if (p.dropout_on) {
+      if (shared) {
+        keep = shared_bits;
+      } else if (p.dropout_on) {
         keep = 0u;
         const int md = min(m, p.max_sq - 1);
 #pragma unroll

@@ -370,6 +370,10 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         if (++cb == ncb) { cb = 0; ++hg; }
         const uint32_t lse2 = aux_s + (uint32_t)(s * 2 * kNB + cbase) * 4u;      // shared-space addresses
         const uint32_t dlt = lse2 + (uint32_t)kNB * 4u;
+        // dK: keep bits the dV launch left behind, on their way while the tensor pipe computes S'
+        const bool shared = MODE == kWideDK && keep_shared(p, sq, mbase, r0 + quarter * 32);
+        uint32_t shared_bits = 0u;
+        if (shared) shared_bits = *keep_share_word(p, sq, h, mbase, r0 + quarter * 32, lane);
         if (p.has_bias && p.bias_vec)      // the warp's 32 x 32 bias tile, one 64-byte row per lane, towards L2
           asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
                                                        (int64_t)h * p.bias.s[1] + (int64_t)min(mbase + lane, sq.sq - 1) * p.bias.s[2] +
@@ -431,7 +435,9 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           }
         }
         uint32_t keep = 0xffffffffu;
-        if (p.dropout_on) {
+        if (shared) {
+          keep = transpose_bits32(shared_bits, lane);      // (this lane's key, query rows in the bits)
+        } else if (p.dropout_on) {
           // One Philox counter serves four consecutive keys of one query row, and the four lanes of
           // a quad own exactly such keys: lane q4 of the quad draws the counters of query rows
           // mbase + q4 + 4k (k = 0..7) for all four keys, then the quad exchanges them.
@@ -441,6 +447,10 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
 #pragma unroll
           for (int k = 0; k < 8; ++k)
             mine |= dropout_keep4_keys(dctx, pkeys, min(mbase + q4 + 4 * k, p.max_sq - 1), n >> 2) << (4 * k);
+          if constexpr (MODE == kWideDV) {
+            if (keep_shared(p, sq, mbase, r0 + quarter * 32))
+              *keep_share_word(p, sq, h, mbase, r0 + quarter * 32, lane) = keep_rows_from_quads(mine, lane);
+          }
           keep = 0u;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -511,6 +521,9 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         const int s = i & 1;
         const uint32_t par2 = (uint32_t)(i >> 1) & 1u;
         const int nbase = (cb_lo + i) * kNB + cbase;     // first key of this thread's columns
+        const bool shared = keep_shared(p, sq, r0 + quarter * 32, nbase);
+        uint32_t shared_bits = 0u;
+        if (shared) shared_bits = *keep_share_word(p, sq, hrow, r0 + quarter * 32, nbase, lane);
         if (p.has_bias && p.bias_vec) asm volatile("prefetch.global.L2 [%0];" ::"l"(bias_row + nbase));
         if (!mbar_wait(&bars[L::bSFull], (uint32_t)i & 1u, abort_flag, status, 0x3C00)) { ok = false; break; }
         tc_fence_after();
@@ -564,7 +577,9 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           }
         }
         uint32_t keep = 0xffffffffu;
-        if (p.dropout_on) {
+        if (shared) {
+          keep = shared_bits;
+        } else if (p.dropout_on) {
           keep = 0u;
           const int md = min(m, p.max_sq - 1);
 #pragma unroll

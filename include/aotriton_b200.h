@@ -253,6 +253,10 @@ AB200_API int ab200_stream_check(void* stream);
  * the kernel takes a few limits to drain.  Call with (0, 0) to restore normal operation. */
 AB200_API void ab200_debug_bounded_wait_test(int drop_copy, unsigned int wait_limit_kcycles);
 
+/* Number of 32-key tiles whose dropout keep bits ab200_attn_bwd hands from the dK/dV kernel to the dQ kernel
+ * through rows of dQ (0: each draws its own); negative: error.  Launches nothing. */
+AB200_API int ab200_debug_keep_tiles(const ab200_attn_bwd_args* args);
+
 /* Test hooks for the host side of the launch path; no counterpart in the reference.  Every CUDA
  * call the library makes on that path goes through one table.  fake_device != 0 makes the table
  * pretend an sm_100 device (148 SMs): device queries answer, symbol look-ups, attribute settings
