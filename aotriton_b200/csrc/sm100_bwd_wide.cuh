@@ -62,7 +62,7 @@ static __device__ __noinline__ void zero_tail_rows_streamed(uint8_t* tile, int v
 }
 
 // grid = (cdiv(rows, 128), heads, batch): rows/heads are keys/kv heads (dV, dK) or queries/q heads (dQ)
-template <typename T, int MODE>
+template <typename T, int MODE, bool PLAIN>
 __global__ void __launch_bounds__(kWideThreads, 1)
 sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm_r1,
                       const __grid_constant__ CUtensorMap tm_r2, const __grid_constant__ CUtensorMap tm_late,
@@ -84,6 +84,8 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
   volatile uint32_t* aux_flag = reinterpret_cast<volatile uint32_t*>(smem + L::kAuxFlag);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (constants where PLAIN: nothing of dropout, bias or its gradient is compiled in)
+  const bool drop_on = !PLAIN && p.dropout_on != 0, bias_on = !PLAIN && p.has_bias != 0, dbias_on = !PLAIN && p.has_dbias != 0;
   if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile unsigned int*>(status) != 0u)) return;
   if ((int)(smem - smem_raw) + L::kUsed > L::kDynamic) {      // the alignment padding did not fit
     if (threadIdx.x == 0) atomicCAS(status, 0u, 0x3F00u);
@@ -104,12 +106,12 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
   const int64_t row_tok0 = kKeys ? sq.k0 : sq.q0, col_tok0 = kKeys ? sq.q0 : sq.k0;
   if (c_hi < c_lo) {      // rows nothing attends to / that attend to nothing: the gradient is zero
     zero_rows<T>(outv, sq.bidx, hrow, row_tok0, r0, rows_total, d_out);
-    if constexpr (MODE == kWideDQ) zero_dbias_outside<T>(p, sq, hrow, r0, kBlk, 0, 0);
+    if constexpr (MODE == kWideDQ) { if (dbias_on) zero_dbias_outside<T>(p, sq, hrow, r0, kBlk, 0, 0); }
     return;
   }
   const int cb_lo = c_lo / kNB;
   const int ncb = c_hi / kNB - cb_lo + 1;
-  if constexpr (MODE == kWideDQ) zero_dbias_outside<T>(p, sq, hrow, r0, kBlk, cb_lo * kNB, (cb_lo + ncb) * kNB);
+  if constexpr (MODE == kWideDQ) { if (dbias_on) zero_dbias_outside<T>(p, sq, hrow, r0, kBlk, cb_lo * kNB, (cb_lo + ncb) * kNB); }
   const int niter = kKeys ? ncb * p.group : ncb;      // dV / dK walk the q heads of the kv head's group
   const int hk = kKeys ? hrow : hrow / p.group;
 
@@ -356,10 +358,10 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
     const int warp_lo = __reduce_max_sync(0xffffffffu, v_lo), warp_hi = __reduce_min_sync(0xffffffffu, v_hi);
     bool ok = true;
     // Philox seed and offset are read once; the round keys depend on the seed only
-    const uint64_t ph_seed = (p.dropout_on && p.seed_ptr) ? *p.seed_ptr : 0ull;
-    const uint64_t ph_off = p.off2 + ((p.dropout_on && p.off1_ptr) ? *p.off1_ptr : 0ull);
+    const uint64_t ph_seed = (drop_on && p.seed_ptr) ? *p.seed_ptr : 0ull;
+    const uint64_t ph_off = p.off2 + ((drop_on && p.off1_ptr) ? *p.off1_ptr : 0ull);
     PhiloxKeys pkeys;
-    if (p.dropout_on) pkeys = philox_keys(ph_seed);
+    if (drop_on) pkeys = philox_keys(ph_seed);
     if constexpr (kKeys) {
       const int n = row;
       for (int i = 0, hg = 0, cb = 0; i < niter; ++i) {
@@ -371,10 +373,10 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         const uint32_t lse2 = aux_s + (uint32_t)(s * 2 * kNB + cbase) * 4u;      // shared-space addresses
         const uint32_t dlt = lse2 + (uint32_t)kNB * 4u;
         // dK: keep bits the dV launch left behind, on their way while the tensor pipe computes S'
-        const bool shared = MODE == kWideDK && keep_shared(p, sq, mbase, r0 + quarter * 32);
+        const bool shared = MODE == kWideDK && drop_on && keep_shared(p, sq, mbase, r0 + quarter * 32);
         uint32_t shared_bits = 0u;
         if (shared) shared_bits = *keep_share_word(p, sq, h, mbase, r0 + quarter * 32, lane);
-        if (p.has_bias && p.bias_vec)      // the warp's 32 x 32 bias tile, one 64-byte row per lane, towards L2
+        if (bias_on && p.bias_vec)      // the warp's 32 x 32 bias tile, one 64-byte row per lane, towards L2
           asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
                                                        (int64_t)h * p.bias.s[1] + (int64_t)min(mbase + lane, sq.sq - 1) * p.bias.s[2] +
                                                        (r0 + quarter * 32)));
@@ -388,7 +390,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars[L::bSRead]);
         const bool any_mask = !(mbase >= warp_lo && mbase + kWgCols - 1 <= warp_hi);
-        if (!p.has_bias && aux_flag[s] == 0) {
+        if (!bias_on && aux_flag[s] == 0) {
           const float2 sc2 = make_float2(p.qk_scale, p.qk_scale);
 #pragma unroll
           for (int c4 = 0; c4 < 8; ++c4) {
@@ -403,12 +405,12 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         } else {
 #pragma unroll
           for (int c = 0; c < 32; ++c) pr[c] *= p.qk_scale;
-          if (p.has_bias && p.bias_vec && mbase + 32 <= sq.sq && r0 + quarter * 32 + 32 <= sq.sk) {
+          if (bias_on && p.bias_vec && mbase + 32 <= sq.sq && r0 + quarter * 32 + 32 <= sq.sk) {
             // the warp's whole 32 x 32 bias tile is inside the sequence: vector loads and a transpose
             add_bias_column32<T>(pr, reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
                                          (int64_t)h * p.bias.s[1] + (int64_t)mbase * p.bias.s[2] + (r0 + quarter * 32),
                                  p.bias.s[2], lane);
-          } else if (p.has_bias && n < sq.sk) {
+          } else if (bias_on && n < sq.sk) {
             const T* bcol = reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
                             (int64_t)h * p.bias.s[1] + (int64_t)n * p.bias.s[3];
 #pragma unroll
@@ -437,7 +439,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         uint32_t keep = 0xffffffffu;
         if (shared) {
           keep = transpose_bits32(shared_bits, lane);      // (this lane's key, query rows in the bits)
-        } else if (p.dropout_on) {
+        } else if (drop_on) {
           // One Philox counter serves four consecutive keys of one query row, and the four lanes of
           // a quad own exactly such keys: lane q4 of the quad draws the counters of query rows
           // mbase + q4 + 4k (k = 0..7) for all four keys, then the quad exchanges them.
@@ -448,7 +450,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           for (int k = 0; k < 8; ++k)
             mine |= dropout_keep4_keys(dctx, pkeys, min(mbase + q4 + 4 * k, p.max_sq - 1), n >> 2) << (4 * k);
           if constexpr (MODE == kWideDV) {
-            if (keep_shared(p, sq, mbase, r0 + quarter * 32))
+            if (drop_on && keep_shared(p, sq, mbase, r0 + quarter * 32))
               *keep_share_word(p, sq, h, mbase, r0 + quarter * 32, lane) = keep_rows_from_quads(mine, lane);
           }
           keep = 0u;
@@ -468,7 +470,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
 #pragma unroll
           for (int c = 0; c < 16; ++c) {
             float a = pr[2 * c], b = pr[2 * c + 1];
-            if (p.dropout_on) {
+            if (drop_on) {
               a = ((keep >> (2 * c)) & 1u) ? a * p.dropout_scale : 0.f;
               b = ((keep >> (2 * c + 1)) & 1u) ? b * p.dropout_scale : 0.f;
             }
@@ -478,7 +480,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           float dp[32];
           tmem_ld32f(a_col, dp);
           tmem_wait_ld();
-          if (p.dropout_on) {
+          if (drop_on) {
 #pragma unroll
             for (int c = 0; c < 32; ++c) dp[c] = ((keep >> c) & 1u) ? dp[c] * p.dropout_scale : 0.f;
           }
@@ -507,24 +509,24 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
       const int64_t lrow = lse_offset(p, sq, hrow);
       const float lse2 = (m < sq.sq) ? p.lse[lrow + m] * kLog2e : INFINITY;
       const float dlt = (m < sq.sq) ? p.delta[lrow + m] : 0.f;
-      const bool simple = !p.has_bias && !__any_sync(0xffffffffu, fabsf(lse2) > 1.0e6f && lse2 != INFINITY);
+      const bool simple = !bias_on && !__any_sync(0xffffffffu, fabsf(lse2) > 1.0e6f && lse2 != INFINITY);
       DropoutCtx dctx;
-      if (p.dropout_on) dctx = dropout_ctx_from(p, ph_seed, ph_off, z, hrow);
+      if (drop_on) dctx = dropout_ctx_from(p, ph_seed, ph_off, z, hrow);
       const int mm = min(m, sq.sq - 1);
-      const T* bias_row = p.has_bias ? reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
+      const T* bias_row = bias_on ? reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
                                            (int64_t)hrow * p.bias.s[1] + (int64_t)mm * p.bias.s[2]
                                      : nullptr;
-      T* db_row = p.has_dbias ? reinterpret_cast<T*>(p.dbias.ptr) + (int64_t)sq.bidx * p.dbias.s[0] +
+      T* db_row = dbias_on ? reinterpret_cast<T*>(p.dbias.ptr) + (int64_t)sq.bidx * p.dbias.s[0] +
                                     (int64_t)hrow * p.dbias.s[1] + (int64_t)mm * p.dbias.s[2]
                               : nullptr;
       for (int i = 0; i < niter; ++i) {
         const int s = i & 1;
         const uint32_t par2 = (uint32_t)(i >> 1) & 1u;
         const int nbase = (cb_lo + i) * kNB + cbase;     // first key of this thread's columns
-        const bool shared = keep_shared(p, sq, r0 + quarter * 32, nbase);
+        const bool shared = drop_on && keep_shared(p, sq, r0 + quarter * 32, nbase);
         uint32_t shared_bits = 0u;
         if (shared) shared_bits = *keep_share_word(p, sq, hrow, r0 + quarter * 32, nbase, lane);
-        if (p.has_bias && p.bias_vec) asm volatile("prefetch.global.L2 [%0];" ::"l"(bias_row + nbase));
+        if (bias_on && p.bias_vec) asm volatile("prefetch.global.L2 [%0];" ::"l"(bias_row + nbase));
         if (!mbar_wait(&bars[L::bSFull], (uint32_t)i & 1u, abort_flag, status, 0x3C00)) { ok = false; break; }
         tc_fence_after();
         float pr[32];
@@ -545,7 +547,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         } else {
 #pragma unroll
           for (int c = 0; c < 32; ++c) pr[c] *= p.qk_scale;
-          if (p.has_bias) {
+          if (bias_on) {
             if (p.bias_vec && nbase + kWgCols <= sq.sk) {
               // the thread's 32 bias values are 64 contiguous bytes: four 16-byte loads
               const uint4* bp = reinterpret_cast<const uint4*>(bias_row + nbase);
@@ -579,7 +581,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         uint32_t keep = 0xffffffffu;
         if (shared) {
           keep = shared_bits;
-        } else if (p.dropout_on) {
+        } else if (drop_on) {
           keep = 0u;
           const int md = min(m, p.max_sq - 1);
 #pragma unroll
@@ -592,7 +594,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           float dp[32];
           tmem_ld32f(a_col, dp);
           tmem_wait_ld();
-          if (p.dropout_on) {
+          if (drop_on) {
 #pragma unroll
             for (int c = 0; c < 32; ++c) dp[c] = ((keep >> c) & 1u) ? dp[c] * p.dropout_scale : 0.f;
           }
@@ -604,7 +606,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
             pk[c] = pack2<T>(a.x, a.y);
           }
           tmem_st16(a_col, pk);
-          if (p.has_dbias && m < sq.sq) {
+          if (dbias_on && m < sq.sq) {
             // dB = cast(dS): the packed pairs are exactly the values to store
             if (p.dbias.s[3] == 1 && nbase + 32 <= sq.sk && (reinterpret_cast<uintptr_t>(db_row + nbase) & 15u) == 0) {
 #pragma unroll
@@ -676,7 +678,8 @@ cudaError_t launch_bwd_wide_T(int which, const Params& p, cudaStream_t st) {
       return cudaErrorInvalidValue;
   }
   static std::atomic<unsigned int*> status_of[64];
-  static std::atomic<bool> attr_set[64][3];
+  static std::atomic<bool> attr_set[64][6];
+  const bool plain = !p.dropout_on && !p.has_bias && !p.has_dbias;
   int dev = 0;
   cudaError_t e = host().get_device(&dev);
   if (e != cudaSuccess) return e;
@@ -694,18 +697,18 @@ cudaError_t launch_bwd_wide_T(int which, const Params& p, cudaStream_t st) {
     return r;
   };
   if (which == 1) {
-    auto kern_dv = sm100_bwd_wide_kernel<T, kWideDV>;
-    auto kern_dk = sm100_bwd_wide_kernel<T, kWideDK>;
-    if ((e = set_smem(0, reinterpret_cast<const void*>(kern_dv))) != cudaSuccess) return e;
-    if ((e = set_smem(1, reinterpret_cast<const void*>(kern_dk))) != cudaSuccess) return e;
+    auto kern_dv = plain ? sm100_bwd_wide_kernel<T, kWideDV, true> : sm100_bwd_wide_kernel<T, kWideDV, false>;
+    auto kern_dk = plain ? sm100_bwd_wide_kernel<T, kWideDK, true> : sm100_bwd_wide_kernel<T, kWideDK, false>;
+    if ((e = set_smem(0 + (plain ? 3 : 0), reinterpret_cast<const void*>(kern_dv))) != cudaSuccess) return e;
+    if ((e = set_smem(1 + (plain ? 3 : 0), reinterpret_cast<const void*>(kern_dk))) != cudaSuccess) return e;
     dim3 grid((p.max_sk + kBlk - 1) / kBlk, p.hk, p.batch);
     e = launch_kernel(kern_dv, grid, dim3(kWideThreads), L::kDynamic, st, p, k128, k128, do64, q64, status);
     if (e != cudaSuccess) return e;
     count_launch();
     e = launch_kernel(kern_dk, grid, dim3(kWideThreads), L::kDynamic, st, p, k128, v128, q64, do64, status);
   } else {
-    auto kern_dq = sm100_bwd_wide_kernel<T, kWideDQ>;
-    if ((e = set_smem(2, reinterpret_cast<const void*>(kern_dq))) != cudaSuccess) return e;
+    auto kern_dq = plain ? sm100_bwd_wide_kernel<T, kWideDQ, true> : sm100_bwd_wide_kernel<T, kWideDQ, false>;
+    if ((e = set_smem(2 + (plain ? 3 : 0), reinterpret_cast<const void*>(kern_dq))) != cudaSuccess) return e;
     dim3 grid((p.max_sq + kBlk - 1) / kBlk, p.hq, p.batch);
     e = launch_kernel(kern_dq, grid, dim3(kWideThreads), L::kDynamic, st, p, q128, do128, k64, v64, status);
   }
