@@ -388,12 +388,15 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
   const int row0 = blockIdx.x * 128;
   if (row0 >= sq.sq) return;
   const int64_t lrow = lse_offset(p, sq, h);
-  const bool vec_ok = (sizeof(T) == 2) && (d == 64 || d == 128 || d == 256) &&
+  // 16-byte loads wherever rows allow them: a row goes to the smallest power of two of lanes that
+  // covers its d / 8 loads.
+  const bool vec_ok = (sizeof(T) == 2) && d % 8 == 0 && d <= 256 &&
                       ((reinterpret_cast<uintptr_t>(p.out.ptr) | reinterpret_cast<uintptr_t>(p.dout.ptr)) % 16 == 0) &&
                       (p.out.s[0] % 8 == 0) && (p.out.s[1] % 8 == 0) && (p.out.s[2] % 8 == 0) &&
                       (p.dout.s[0] % 8 == 0) && (p.dout.s[1] % 8 == 0) && (p.dout.s[2] % 8 == 0);
   if (vec_ok) {
-    const int lpr = d >> 3;                 // lanes per row: 8, 16 or 32
+    const int loads = d >> 3;
+    const int lpr = loads <= 4 ? 4 : (loads <= 8 ? 8 : (loads <= 16 ? 16 : 32));      // lanes per row
     const int rpw = 32 / lpr;               // rows per warp pass
     const int sub = lane / lpr, col = (lane % lpr) * 8;
     // warp w covers rows row0 + 16w .. +15 in passes of rpw rows, four passes in flight
@@ -404,7 +407,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         rows[u] = wrow0 + (pass + u) * rpw + sub;
-        const bool in = (pass + u) * rpw < 16 && rows[u] < sq.sq;
+        const bool in = (pass + u) * rpw < 16 && rows[u] < sq.sq && col < d;
         if (in) {
           a[u] = *reinterpret_cast<const uint4*>(row_ptr<T>(p.out, sq.bidx, h, sq.q0 + rows[u]) + col);
           b[u] = *reinterpret_cast<const uint4*>(row_ptr<T>(p.dout, sq.bidx, h, sq.q0 + rows[u]) + col);
