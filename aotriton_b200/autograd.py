@@ -22,12 +22,28 @@ def _check(err, what):
         raise RuntimeError(f"{what} failed: {err}")
 
 
+# A null device scalar: no elements, so no address on any device.
+_NULL_SCALAR = torch.empty([0], dtype=torch.uint64)
+# The counter of a persistent kernel: the kernels bring their own.
+_NULL_COUNTER = torch.empty([0], dtype=torch.int32)
+
+
+def _device_u64(device, value):
+    """One uint64 on the device.  Filled by a kernel on the current stream: torch.tensor(..., device=...) copies
+    from pageable host memory and waits for the stream."""
+    if type(value) is int and 0 <= value < 1 << 64:
+        return torch.full([1], value - (value >> 63 << 64), device=device, dtype=torch.int64).view(torch.uint64)
+    return torch.tensor([value], device=device, dtype=torch.uint64)
+
+
 def _philox_tensors(device, dropout_p, seed, offset1):
-    null = torch.empty([0], device=device, dtype=torch.uint64)
+    """(philox seed, philox offset) of a call as device scalars.  The offset is the whole of it (offset1 +
+    offset2), so the backward takes both as they are with a second offset of 0."""
     if dropout_p <= 0.0:
-        return null, null, 0, null, null
-    mk = lambda v: torch.tensor([v], device=device, dtype=torch.uint64)
-    return mk(seed), mk(offset1), DEFAULT_PHILOX_OFFSET_2, mk(0), mk(0)
+        return _NULL_SCALAR, _NULL_SCALAR
+    if type(offset1) is not int or not 0 <= offset1 < 1 << 64:
+        offset1 = int(torch.tensor([offset1], dtype=torch.uint64).item())
+    return _device_u64(device, seed), _device_u64(device, (offset1 + DEFAULT_PHILOX_OFFSET_2) % (1 << 64))
 
 
 # Kernel family of the most recent backward (the library keeps it per thread, and autograd runs
@@ -47,14 +63,12 @@ class _Attention(torch.autograd.Function):
                 philox_seed=DEFAULT_PHILOX_SEED, philox_offset1=DEFAULT_PHILOX_OFFSET_1):
         o = torch.empty((q.shape[0], q.shape[1], q.shape[2], v.shape[3]), device=q.device, dtype=q.dtype)
         M = torch.empty((q.shape[0] * q.shape[1], q.shape[2]), device=q.device, dtype=torch.float32)
-        seed, off1, off2, seed_out, off_out = _philox_tensors(q.device, dropout_p, philox_seed, philox_offset1)
-        atomic = torch.zeros([1], device=q.device, dtype=torch.int32) if causal else \
-            torch.empty([0], device=q.device, dtype=torch.int32)
-        _check(flash.attn_fwd(q, k, v, b, sm_scale, M, o, dropout_p, seed, off1, off2, seed_out, off_out,
-                              None, causal, atomic), "attn_fwd")
+        seed, offset = _philox_tensors(q.device, dropout_p, philox_seed, philox_offset1)
+        _check(flash.attn_fwd(q, k, v, b, sm_scale, M, o, dropout_p, seed, offset, 0, _NULL_SCALAR, _NULL_SCALAR,
+                              None, causal, _NULL_COUNTER), "attn_fwd")
         ctx.save_for_backward(q, k, v, b, o, M)
         ctx.sm_scale, ctx.causal, ctx.dropout_p = sm_scale, causal, dropout_p
-        ctx.philox_seed, ctx.philox_offset = seed_out, off_out
+        ctx.philox_seed, ctx.philox_offset = seed, offset
         return (o, M) if return_lse else o
 
     @staticmethod
@@ -86,15 +100,14 @@ class _VarlenAttention(torch.autograd.Function):
         # q, k, v: (1, H, total_tokens, D) views of THD storage
         o = torch.empty((1, q.shape[2], q.shape[1], v.shape[3]), device=q.device, dtype=q.dtype).transpose(1, 2)
         M = torch.empty((q.shape[1], q.shape[2]), device=q.device, dtype=torch.float32)
-        seed, off1, off2, seed_out, off_out = _philox_tensors(q.device, dropout_p, philox_seed, philox_offset1)
-        atomic = torch.empty([0], device=q.device, dtype=torch.int32)
+        seed, offset = _philox_tensors(q.device, dropout_p, philox_seed, philox_offset1)
         _check(flash.attn_fwd_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, None, None,
-                                     None, sm_scale, M, o, dropout_p, seed, off1, off2, seed_out, off_out, None,
-                                     causal, atomic, "compact"), "attn_fwd (varlen)")
+                                     None, sm_scale, M, o, dropout_p, seed, offset, 0, _NULL_SCALAR, _NULL_SCALAR, None,
+                                     causal, _NULL_COUNTER, "compact"), "attn_fwd (varlen)")
         ctx.save_for_backward(q, k, v, o, M, cu_seqlens_q, cu_seqlens_k)
         ctx.max_seqlens = (max_seqlen_q, max_seqlen_k)
         ctx.sm_scale, ctx.causal, ctx.dropout_p = sm_scale, causal, dropout_p
-        ctx.philox_seed, ctx.philox_offset = seed_out, off_out
+        ctx.philox_seed, ctx.philox_offset = seed, offset
         return (o, M) if return_lse else o
 
     @staticmethod
@@ -135,15 +148,14 @@ def op_attn_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, bias: torch.T
     """Returns (out, logsumexp, philox seed used, philox offset used)."""
     o = torch.empty((q.shape[0], q.shape[1], q.shape[2], v.shape[3]), device=q.device, dtype=q.dtype)
     M = torch.empty(_lse_rows(q), device=q.device, dtype=torch.float32)
-    seed, off1, off2, seed_out, off_out = _philox_tensors(q.device, dropout_p, philox_seed, philox_offset1)
+    seed, offset = _philox_tensors(q.device, dropout_p, philox_seed, philox_offset1)
     causal = (window_left, window_right) if causal_type == flash.CausalType.WINDOWED else False
-    atomic = torch.zeros([1], device=q.device, dtype=torch.int32)
-    _check(flash.attn_fwd(q, k, v, bias, sm_scale, M, o, dropout_p, seed, off1, off2, seed_out, off_out, None,
-                          causal, atomic), "attn_fwd")
+    _check(flash.attn_fwd(q, k, v, bias, sm_scale, M, o, dropout_p, seed, offset, 0, _NULL_SCALAR, _NULL_SCALAR, None,
+                          causal, _NULL_COUNTER), "attn_fwd")
     if dropout_p <= 0.0:
-        seed_out = torch.zeros([1], device=q.device, dtype=torch.uint64)
-        off_out = torch.zeros([1], device=q.device, dtype=torch.uint64)
-    return o, M, seed_out, off_out
+        seed = torch.zeros([1], device=q.device, dtype=torch.uint64)
+        offset = torch.zeros([1], device=q.device, dtype=torch.uint64)
+    return o, M, seed, offset
 
 
 @op_attn_fwd.register_fake
@@ -164,12 +176,11 @@ def op_attn_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, bias: torch.T
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
     db = torch.empty_like(bias) if bias is not None else None
     causal = (window_left, window_right) if causal_type == flash.CausalType.WINDOWED else False
-    null = torch.empty([0], device=q.device, dtype=torch.uint64)
     opts = flash.attn_options()
     opts.deterministic = bool(deterministic)
     _check(flash.attn_bwd(q, k, v, bias, sm_scale, out, dout, dq, dk, dv, db, flash.lazy_dq_acc(dq), lse,
-                          flash.lazy_delta(lse), dropout_p, philox_seed if dropout_p > 0 else null,
-                          philox_offset if dropout_p > 0 else null, 0, causal, opts), "attn_bwd")
+                          flash.lazy_delta(lse), dropout_p, philox_seed if dropout_p > 0 else _NULL_SCALAR,
+                          philox_offset if dropout_p > 0 else _NULL_SCALAR, 0, causal, opts), "attn_bwd")
     _note_bwd_family()
     return dq, dk, dv, db if db is not None else q.new_empty([0])
 

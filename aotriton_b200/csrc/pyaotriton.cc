@@ -327,6 +327,115 @@ void def_v3(py::module_& root) {
         py::arg("stream") = aotriton::Stream(), py::arg("options") = nullptr);
 }
 
+// ---- torch tensors straight into a parameter struct ----------------------------------------------
+// Building every TensorView as a Python object (tuples to std::array and back) and assigning it costs 5 to 6
+// us a tensor: 66 us of host time for a forward call and 91 us for a backward, several times what the kernels
+// of a small call take.  These fill the structs from the tensors' data_ptr() / shape / stride() in one call (6 and
+// 8 us).  They take the ordinary forms only and return false for everything else (the caller then goes the long
+// way, which also words the errors).
+struct TorchNames {
+  PyObject *data_ptr = PyUnicode_InternFromString("data_ptr"), *shape = PyUnicode_InternFromString("shape"),
+           *stride = PyUnicode_InternFromString("stride"), *dtype = PyUnicode_InternFromString("dtype");
+};
+const TorchNames& torch_names() {
+  static const TorchNames* n = new TorchNames;
+  return *n;
+}
+
+// `dtypes`: dict torch.dtype -> DType value as int.
+class ViewReader {
+ public:
+  explicit ViewReader(py::dict dtypes) : dtypes_(std::move(dtypes)) {}
+
+  template <int Rank>
+  bool read(py::handle t, aotriton::TensorView<Rank>* out) const {
+    const TorchNames& n = torch_names();
+    aotriton::DType dt;
+    if (t.is_none() || !dtype(t, &dt)) return false;
+    const py::object shape = py::reinterpret_steal<py::object>(PyObject_GetAttr(t.ptr(), n.shape));
+    if (!shape) throw py::error_already_set();
+    if (!PyTuple_Check(shape.ptr()) || PyTuple_GET_SIZE(shape.ptr()) != Rank) return false;
+    const py::object stride = py::reinterpret_steal<py::object>(PyObject_CallMethodNoArgs(t.ptr(), n.stride));
+    if (!stride) throw py::error_already_set();
+    if (!PyTuple_Check(stride.ptr()) || PyTuple_GET_SIZE(stride.ptr()) != Rank) return false;
+    std::array<uint64_t, Rank> sizes, strides;
+    for (int i = 0; i < Rank; ++i) {
+      sizes[i] = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(shape.ptr(), i));
+      strides[i] = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(stride.ptr(), i));
+      if (PyErr_Occurred()) { PyErr_Clear(); return false; }
+    }
+    if (strides[Rank - 1] != 1) return false;
+    intptr_t ptr;
+    if (!pointer(t, &ptr)) return false;
+    *out = aotriton::TensorView<Rank>(ptr, sizes, strides, dt);
+    return true;
+  }
+
+  // None: a null view of the other tensor's type
+  template <int Rank>
+  bool read_or_null(py::handle t, aotriton::DType like, aotriton::TensorView<Rank>* out) const {
+    if (!t.is_none()) return read(t, out);
+    *out = aotriton::TensorView<Rank>(0, {}, {}, like);
+    return true;
+  }
+
+  // a device scalar: a rank-1 tensor of one element, or of none (null)
+  bool read_scalar(py::handle t, aotriton::TensorView<0>* out) const {
+    aotriton::DType dt;
+    if (t.is_none() || !dtype(t, &dt)) return false;
+    const py::object shape = py::reinterpret_steal<py::object>(PyObject_GetAttr(t.ptr(), torch_names().shape));
+    if (!shape) throw py::error_already_set();
+    if (!PyTuple_Check(shape.ptr()) || PyTuple_GET_SIZE(shape.ptr()) != 1) return false;
+    const long long count = PyLong_AsLongLong(PyTuple_GET_ITEM(shape.ptr(), 0));
+    if (PyErr_Occurred()) { PyErr_Clear(); return false; }
+    intptr_t ptr;
+    if ((count != 0 && count != 1) || !pointer(t, &ptr)) return false;
+    *out = aotriton::TensorView<0>(ptr, dt);
+    return true;
+  }
+
+ private:
+  bool dtype(py::handle t, aotriton::DType* out) const {
+    const py::object d = py::reinterpret_steal<py::object>(PyObject_GetAttr(t.ptr(), torch_names().dtype));
+    if (!d) throw py::error_already_set();
+    PyObject* v = PyDict_GetItemWithError(dtypes_.ptr(), d.ptr());      // (borrowed)
+    if (v == nullptr) { if (PyErr_Occurred()) throw py::error_already_set(); return false; }
+    *out = static_cast<aotriton::DType>(PyLong_AsLong(v));
+    return true;
+  }
+  static bool pointer(py::handle t, intptr_t* out) {
+    const py::object p = py::reinterpret_steal<py::object>(PyObject_CallMethodNoArgs(t.ptr(), torch_names().data_ptr));
+    if (!p) throw py::error_already_set();
+    *out = (intptr_t)PyLong_AsUnsignedLongLong(p.ptr());
+    if (PyErr_Occurred()) { PyErr_Clear(); return false; }
+    return true;
+  }
+  py::dict dtypes_;
+};
+
+bool set_fwd_views(aotriton::v3::flash::attn_fwd_params& p, py::dict dtypes, py::handle q, py::handle k, py::handle v,
+                   py::handle b, py::handle lse, py::handle out, py::handle seed, py::handle off1, py::handle seed_out,
+                   py::handle off_out, py::handle enc, py::handle atomic) {
+  const ViewReader r(std::move(dtypes));
+  if (!r.read(q, &p.Q)) return false;
+  return r.read(k, &p.K) && r.read(v, &p.V) && r.read_or_null(b, p.Q.dtype(), &p.B) &&
+         r.read_or_null(lse, aotriton::kFloat32, &p.L) && r.read(out, &p.Out) && r.read_scalar(seed, &p.philox_seed_ptr) &&
+         r.read_scalar(off1, &p.philox_offset1) && r.read_scalar(seed_out, &p.philox_seed_output) &&
+         r.read_scalar(off_out, &p.philox_offset_output) && r.read_or_null(enc, p.Q.dtype(), &p.encoded_softmax) &&
+         r.read_scalar(atomic, &p.persistent_atomic_counter);
+}
+
+bool set_bwd_views(aotriton::v3::flash::attn_bwd_params& p, py::dict dtypes, py::handle q, py::handle k, py::handle v,
+                   py::handle b, py::handle out, py::handle dout, py::handle dk, py::handle dv, py::handle dq, py::handle db,
+                   py::handle lse, py::handle seed, py::handle off1) {
+  const ViewReader r(std::move(dtypes));
+  if (!r.read(q, &p.Q)) return false;
+  return r.read(k, &p.K) && r.read(v, &p.V) && r.read_or_null(b, p.Q.dtype(), &p.B) && r.read(out, &p.Out) &&
+         r.read(dout, &p.DO) && r.read(dk, &p.DK) && r.read(dv, &p.DV) && r.read(dq, &p.DQ) &&
+         r.read_or_null(db, p.Q.dtype(), &p.DB) && r.read(lse, &p.L) && r.read_scalar(seed, &p.philox_seed_ptr) &&
+         r.read_scalar(off1, &p.philox_offset1);
+}
+
 void def_lazy(py::module_& root) {
   py::module_ m = root.def_submodule("lazy_tensor", "lazy_tensor API namespace");
   py::class_<aotriton::LazyTensor<4>>(m, "LT4");
@@ -336,6 +445,22 @@ void def_lazy(py::module_& root) {
   m.def("dq_acc_from", &PyLazy<4>::make, py::arg("like"), py::arg("factory"));
   m.def("delta_from", &PyLazy<2>::make, py::arg("like"), py::arg("factory"));
   m.def("eager_delta", &LazyHelper<2, false>::make_eager);
+  // (the same straight from a tensor; None: not an ordinary one)
+  m.def("dq_acc_of", [](py::dict dtypes, py::handle t, py::object factory) -> py::object {
+    aotriton::TensorView<4> like;
+    if (!ViewReader(std::move(dtypes)).read(t, &like)) return py::none();
+    return py::cast(PyLazy<4>::make(like, std::move(factory)));
+  });
+  m.def("delta_of", [](py::dict dtypes, py::handle t, py::object factory) -> py::object {
+    aotriton::TensorView<2> like;
+    if (!ViewReader(std::move(dtypes)).read(t, &like)) return py::none();
+    return py::cast(PyLazy<2>::make(like, std::move(factory)));
+  });
+  m.def("eager_delta_of", [](py::dict dtypes, py::handle t) -> py::object {
+    aotriton::TensorView<2> view;
+    if (!ViewReader(std::move(dtypes)).read(t, &view)) return py::none();
+    return py::cast(LazyHelper<2, false>::make_eager(view));
+  });
   m.def("eager_null_dq_acc", &LazyHelper<4, false>::make_eager);
 }
 
@@ -385,6 +510,8 @@ PYBIND11_MODULE(pyaotriton, m) {
 #define AB200_STR2(x) #x
 #define AB200_STR(x) AB200_STR2(x)
   m.def("get_name_suffix", []() -> std::string { return AB200_STR(AOTRITON_NAME_SUFFIX); });
+  m.def("set_fwd_views", &set_fwd_views);
+  m.def("set_bwd_views", &set_bwd_views);
   m.def("launch_count", []() { return ab200_launch_count(); });
   m.def("set_kernel_family", [](int f) { return ab200_set_kernel_family(f); });
   m.def("last_fwd_family", []() { return ab200_last_fwd_family(); });

@@ -52,13 +52,24 @@ def translate_causal(causal):
     return CausalType.NONE, 0, 0
 
 
-def cast_dtype(dtype):
+def _dtype_by_name(dtype):
     bits = dtype.itemsize * 8
     if dtype.is_floating_point:
         main = "BFloat" if dtype == torch.bfloat16 else "Float"
     else:
         main = "UInt" if "uint" in str(dtype) else "Int"
     return getattr(DType, f"k{main}{bits}")
+
+
+_DTYPE_VALUES = {t: _dtype_by_name(t) for t in (torch.float32, torch.float16, torch.bfloat16, torch.int8, torch.int16,
+                                                torch.int32, torch.int64, torch.uint8, torch.uint16, torch.uint32,
+                                                torch.uint64)}
+_DTYPES = {t: int(v) for t, v in _DTYPE_VALUES.items()}      # as the native readers of tensors take them
+
+
+def cast_dtype(dtype):
+    found = _DTYPE_VALUES.get(dtype)
+    return found if found is not None else _dtype_by_name(dtype)
 
 
 def mk_aotensor(t, if_empty_then_like=None):
@@ -82,19 +93,21 @@ def _stream():
 
 def _fill_fwd(params, q, k, v, b, sm_scale, M, o, dropout_p, philox_seed, philox_offset1, philox_offset2,
               philox_seed_output, philox_offset_output, encoded_softmax, causal, atomic):
-    params.Q, params.K, params.V = mk_aotensor(q), mk_aotensor(k), mk_aotensor(v)
-    params.B = mk_aotensor(b, if_empty_then_like=q)
+    if not _p.set_fwd_views(params, _DTYPES, q, k, v, b, M, o, philox_seed, philox_offset1, philox_seed_output,
+                            philox_offset_output, encoded_softmax, atomic):
+        params.Q, params.K, params.V = mk_aotensor(q), mk_aotensor(k), mk_aotensor(v)
+        params.B = mk_aotensor(b, if_empty_then_like=q)
+        params.L = mk_aotensor(M, if_empty_then_like=torch.empty(0, 0, dtype=torch.float32))
+        params.Out = mk_aotensor(o)
+        params.philox_seed_ptr = mk_aotensor(philox_seed)
+        params.philox_offset1 = mk_aotensor(philox_offset1)
+        params.philox_seed_output = mk_aotensor(philox_seed_output)
+        params.philox_offset_output = mk_aotensor(philox_offset_output)
+        params.encoded_softmax = mk_aotensor(encoded_softmax, if_empty_then_like=q)
+        params.persistent_atomic_counter = mk_aotensor(atomic)
     params.Sm_scale = float(sm_scale)
-    params.L = mk_aotensor(M, if_empty_then_like=torch.empty(0, 0, dtype=torch.float32))
-    params.Out = mk_aotensor(o)
     params.dropout_p = float(dropout_p)
-    params.philox_seed_ptr = mk_aotensor(philox_seed)
-    params.philox_offset1 = mk_aotensor(philox_offset1)
     params.philox_offset2 = philox_offset2
-    params.philox_seed_output = mk_aotensor(philox_seed_output)
-    params.philox_offset_output = mk_aotensor(philox_offset_output)
-    params.encoded_softmax = mk_aotensor(encoded_softmax, if_empty_then_like=q)
-    params.persistent_atomic_counter = mk_aotensor(atomic)
     params.causal_type, params.window_left, params.window_right = translate_causal(causal)
 
 
@@ -124,19 +137,20 @@ def attn_fwd_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqle
 
 def _fill_bwd(params, q, k, v, b, sm_scale, o, dout, dq, dk, dv, db, dq_acc, L, delta, dropout_p, philox_seed,
               philox_offset1, philox_offset2, causal):
-    params.Q, params.K, params.V = mk_aotensor(q), mk_aotensor(k), mk_aotensor(v)
-    params.B = mk_aotensor(b, if_empty_then_like=q)
+    if not _p.set_bwd_views(params, _DTYPES, q, k, v, b, o, dout, dk, dv, dq, db, L, philox_seed, philox_offset1):
+        params.Q, params.K, params.V = mk_aotensor(q), mk_aotensor(k), mk_aotensor(v)
+        params.B = mk_aotensor(b, if_empty_then_like=q)
+        params.Out, params.DO = mk_aotensor(o), mk_aotensor(dout)
+        params.DK, params.DV, params.DQ = mk_aotensor(dk), mk_aotensor(dv), mk_aotensor(dq)
+        params.DB = mk_aotensor(db, if_empty_then_like=q)
+        params.L = mk_aotensor(L)
+        params.philox_seed_ptr = mk_aotensor(philox_seed)
+        params.philox_offset1 = mk_aotensor(philox_offset1)
     params.Sm_scale = float(sm_scale)
-    params.Out, params.DO = mk_aotensor(o), mk_aotensor(dout)
-    params.DK, params.DV, params.DQ = mk_aotensor(dk), mk_aotensor(dv), mk_aotensor(dq)
-    params.DB = mk_aotensor(db, if_empty_then_like=q)
-    params.L = mk_aotensor(L)
     params.D = delta
     if dq_acc is not None:
         params.DQ_ACC = dq_acc
     params.dropout_p = float(dropout_p)
-    params.philox_seed_ptr = mk_aotensor(philox_seed)
-    params.philox_offset1 = mk_aotensor(philox_offset1)
     params.philox_offset2 = philox_offset2
     params.causal_type, params.window_left, params.window_right = translate_causal(causal)
 
@@ -172,15 +186,19 @@ def debug_simulate_encoded_softmax(R, dropout_p, philox_seed, philox_offset1, ph
 def lazy_dq_acc(dq: torch.Tensor):
     """fp32 zero-initialised dQ accumulator shaped like dq, allocated by torch only if the backward
     asks for it (reference: bindings/lazy_tensor/lazy_tensor_template.h:19-58, at::zeros)."""
-    like = T4(dq.data_ptr(), tuple(dq.size()), tuple(dq.stride()), cast_dtype(dq.dtype))
-    return _p.lazy_tensor.dq_acc_from(like, lambda: torch.zeros(dq.shape, dtype=torch.float32, device=dq.device))
+    make = lambda: torch.zeros(dq.shape, dtype=torch.float32, device=dq.device)
+    lazy = _p.lazy_tensor.dq_acc_of(_DTYPES, dq, make)
+    return lazy if lazy is not None else _p.lazy_tensor.dq_acc_from(
+        T4(dq.data_ptr(), tuple(dq.size()), tuple(dq.stride()), cast_dtype(dq.dtype)), make)
 
 
 def lazy_delta(L: torch.Tensor):
     """fp32 delta scratch shaped like the logsumexp tensor, allocated by torch when the backward
     acquires it (reference: lazy_tensor_template.h:60-97, at::empty)."""
-    like = T2(L.data_ptr(), tuple(L.size()), tuple(L.stride()), cast_dtype(L.dtype))
-    return _p.lazy_tensor.delta_from(like, lambda: torch.empty(L.shape, dtype=torch.float32, device=L.device))
+    make = lambda: torch.empty(L.shape, dtype=torch.float32, device=L.device)
+    lazy = _p.lazy_tensor.delta_of(_DTYPES, L, make)
+    return lazy if lazy is not None else _p.lazy_tensor.delta_from(
+        T2(L.data_ptr(), tuple(L.size()), tuple(L.stride()), cast_dtype(L.dtype)), make)
 
 
 def pooled_lazy_delta(L: torch.Tensor):
@@ -209,5 +227,6 @@ def reset_kernel_status():
 
 def eager_delta(delta: torch.Tensor):
     """Wrap a caller-owned fp32 tensor shaped like L as the backward's delta scratch."""
-    return _p.lazy_tensor.eager_delta(
+    lazy = _p.lazy_tensor.eager_delta_of(_DTYPES, delta)
+    return lazy if lazy is not None else _p.lazy_tensor.eager_delta(
         T2(delta.data_ptr(), tuple(delta.size()), tuple(delta.stride()), cast_dtype(delta.dtype)))
