@@ -270,24 +270,71 @@ constexpr SelectionRow kSelection[] = {
     {kOpBwd, kHalfTypes, 256, 256, kVarTcgen05}, {kOpBwd, kAllTypes, 512, 0, kVarGeneral},
 };
 
-// ---- keep bits shared between the kernels of one backward (KeepShare in common.cuh) ---------
-// Bytes [lo, hi) a view of 16-bit elements reaches.  False: extents or strides that say nothing.
-bool view_range(const View4& v, uintptr_t* lo, uintptr_t* hi) {
+// ---- outputs that share no memory with what is still read ------------------------------------------
+// Bytes [lo, hi) a view of `elt`-byte elements reaches.  False: extents or strides that say nothing.
+bool view_range(const View4& v, int elt, uintptr_t* lo, uintptr_t* hi) {
   int64_t last = 0;
   for (int i = 0; i < 4; ++i) {
     if (v.n[i] <= 0 || (v.n[i] > 1 && v.s[i] < 0)) return false;
     last += (v.n[i] - 1) * (v.n[i] > 1 ? v.s[i] : 0);
   }
   *lo = reinterpret_cast<uintptr_t>(v.ptr);
-  *hi = *lo + 2 * (uintptr_t)(last + 1);
+  *hi = *lo + (uintptr_t)elt * (uintptr_t)(last + 1);
   return true;
 }
 
+// True when the backward's output `o` (dQ or dBias) shares no memory with an input of the backward or with dK, dV
+// and the other of the two.  A caller may hand in the same memory for dQ and, say, dO: that works as long as the
+// kernel that writes dQ runs last and a CTA reads only its own rows of dO, and must go on working.
+bool apart_from_inputs(const View4& o, const Params& p, int elt) {
+  uintptr_t lo, hi;
+  if (!view_range(o, elt, &lo, &hi)) return false;
+  auto apart = [&](uintptr_t b, uintptr_t e) { return e <= lo || b >= hi; };
+  for (const View4* v : {&p.q, &p.k, &p.v, &p.dout, &p.bias, &p.dq, &p.dk, &p.dv, &p.dbias}) {
+    if (v->ptr == nullptr || v == &o || (v == &p.dbias && !p.has_dbias)) continue;
+    uintptr_t b, e;
+    if (!view_range(*v, elt, &b, &e) || !apart(b, e)) return false;
+  }
+  // logsumexp and delta: dense fp32, one per (batch, q head, query row); token-packed: per (q head, token)
+  const uintptr_t rows = (uintptr_t)p.hq * (p.varlen_mode == 1 ? (uintptr_t)p.q.n[2] : (uintptr_t)p.batch * (uintptr_t)p.max_sq);
+  for (const float* f : {static_cast<const float*>(p.lse), static_cast<const float*>(p.delta)}) {
+    const uintptr_t b = reinterpret_cast<uintptr_t>(f);
+    if (!apart(b, b + 4 * rows)) return false;
+  }
+  const uintptr_t cu_bytes = 4 * ((uintptr_t)p.batch + 1);
+  for (const int32_t* c : {p.cu_q, p.cu_k, p.ss_q, p.ss_k}) {
+    const uintptr_t b = reinterpret_cast<uintptr_t>(c);
+    if (c != nullptr && !apart(b, b + cu_bytes)) return false;
+  }
+  for (const uint64_t* c : {p.seed_ptr, p.off1_ptr}) {
+    const uintptr_t b = reinterpret_cast<uintptr_t>(c);
+    if (c != nullptr && !apart(b, b + 8)) return false;
+  }
+  return true;
+}
+
+// No two elements at one address, rows of `inner` elements: sorted by stride, each dimension steps over the whole
+// of the ones below.
+bool rows_disjoint(const View4& v, int64_t inner) {
+  int order[3] = {0, 1, 2};
+  for (int i = 0; i < 2; ++i)
+    for (int j = 0; j < 2 - i; ++j)
+      if (v.s[order[j]] > v.s[order[j + 1]]) std::swap(order[j], order[j + 1]);
+  int64_t extent = inner;
+  for (int i = 0; i < 3; ++i) {
+    const int d = order[i];
+    if (v.n[d] == 1) continue;
+    if (v.s[d] < extent) return false;
+    extent += (v.n[d] - 1) * v.s[d];
+  }
+  return true;
+}
+
+// ---- keep bits shared between the kernels of one backward (KeepShare in common.cuh) ---------
 // Decides whether (and for how many 32-key tiles) dQ's rows carry keep bits from the dK/dV kernel to the dQ
 // kernel.  dQ must be a tensor in which no two rows share memory, shaped like q, and apart from everything
-// the kernels still read when the bits are written: a caller may hand in the same memory for dQ and an
-// input, which works as long as dQ is only written by the kernel that no longer needs that input.  Head
-// dims below 64 have no room for a tile (128 bytes) in a row.
+// the kernels still read when the bits are written.  Head dims below 64 have no room for a tile (128 bytes)
+// in a row.
 void keep_share_setup(Params& p) {
   p.keep_tiles = 0;
   p.keep_shift = 0;
@@ -295,41 +342,7 @@ void keep_share_setup(Params& p) {
   for (int i = 0; i < 3; ++i)
     if (p.dq.n[i] != p.q.n[i] || p.dq.s[i] % 8 != 0) return;
   if (p.dq.n[3] != p.dqk) return;
-  uintptr_t lo, hi;
-  if (!view_range(p.dq, &lo, &hi)) return;
-  // no two elements at one address: sorted by stride, each dimension steps over the whole of the ones below
-  int order[3] = {0, 1, 2};
-  for (int i = 0; i < 2; ++i)
-    for (int j = 0; j < 2 - i; ++j)
-      if (p.dq.s[order[j]] > p.dq.s[order[j + 1]]) { const int t = order[j]; order[j] = order[j + 1]; order[j + 1] = t; }
-  int64_t extent = p.dqk;
-  for (int i = 0; i < 3; ++i) {
-    const int d = order[i];
-    if (p.dq.n[d] == 1) continue;
-    if (p.dq.s[d] < extent) return;
-    extent += (p.dq.n[d] - 1) * p.dq.s[d];
-  }
-  auto apart = [&](uintptr_t b, uintptr_t e) { return e <= lo || b >= hi; };
-  for (const View4* v : {&p.q, &p.k, &p.v, &p.dout, &p.bias, &p.dk, &p.dv}) {
-    if (v->ptr == nullptr) continue;
-    uintptr_t b, e;
-    if (!view_range(*v, &b, &e) || !apart(b, e)) return;
-  }
-  // logsumexp and delta: dense fp32, one per (batch, q head, query row); token-packed: per (q head, token)
-  const uintptr_t rows = (uintptr_t)p.hq * (p.varlen_mode == 1 ? (uintptr_t)p.q.n[2] : (uintptr_t)p.batch * (uintptr_t)p.max_sq);
-  for (const float* f : {static_cast<const float*>(p.lse), static_cast<const float*>(p.delta)}) {
-    const uintptr_t b = reinterpret_cast<uintptr_t>(f);
-    if (!apart(b, b + 4 * rows)) return;
-  }
-  const uintptr_t cu_bytes = 4 * ((uintptr_t)p.batch + 1);
-  for (const int32_t* c : {p.cu_q, p.cu_k, p.ss_q, p.ss_k}) {
-    const uintptr_t b = reinterpret_cast<uintptr_t>(c);
-    if (c != nullptr && !apart(b, b + cu_bytes)) return;
-  }
-  for (const uint64_t* c : {p.seed_ptr, p.off1_ptr}) {
-    const uintptr_t b = reinterpret_cast<uintptr_t>(c);
-    if (c != nullptr && !apart(b, b + 8)) return;
-  }
+  if (!rows_disjoint(p.dq, p.dqk) || !apart_from_inputs(p.dq, p, 2)) return;
   p.keep_shift = p.dqk >= 256 ? 2 : (p.dqk >= 128 ? 1 : 0);
   p.keep_tiles = std::min(32 << p.keep_shift, (p.max_sk + 31) / 32);
 }
@@ -542,6 +555,24 @@ static int run_dq(const ab200_attn_bwd_args* a, void* stream, bool share) {
   return (int)launch_general(2, a->prob.dtype, p, st);
 }
 
+// dK/dV and dQ of the general kernels in one launch.  -1: done; 0: not a case for it; else an error.
+static int run_general_bwd(const ab200_attn_bwd_args* a, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  Params p{};
+  if (int e = fill_bwd(a, p, true)) return e;
+  if (int e = check_device(st)) return e;
+  DeviceGuard guard(st);
+  const int sel = ab200_select_variant(kOpBwd, a->prob.dtype, p.dqk, p.dvo,
+                                       family_flags(g_family) | (sm100_bwd_supported(a->prob.dtype, p) ? AB200_SELECT_ALIGNED : 0));
+  if (sel < 0) return -sel;
+  const int elt = a->prob.dtype == AB200_DTYPE_FP32 ? 4 : 2;
+  if ((sel & 0xff) != kVarGeneral || !apart_from_inputs(p.dq, p, elt) || (p.has_dbias && !apart_from_inputs(p.dbias, p, elt)))
+    return 0;
+  t_last_bwd = 1;
+  const int e = (int)launch_general(3, a->prob.dtype, p, st);
+  return e ? e : -1;
+}
+
 int ab200_bwd_dkdv(const ab200_attn_bwd_args* a, void* stream) { return run_dkdv(a, stream, false); }
 int ab200_bwd_dq(const ab200_attn_bwd_args* a, void* stream) { return run_dq(a, stream, false); }
 
@@ -589,6 +620,7 @@ int ab200_attn_bwd(const ab200_attn_bwd_args* a, void* stream) {
     if (int e = ab200_bwd_fused(a, stream)) return e;
     return ab200_bwd_postprocess(a, stream);
   }
+  if (int e = run_general_bwd(a, stream)) return e > 0 ? e : 0;
   if (int e = run_dkdv(a, stream, true)) return e;
   return run_dq(a, stream, true);
 }

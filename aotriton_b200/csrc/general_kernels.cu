@@ -535,13 +535,17 @@ template <typename T, int DP>
 cudaError_t launch_tiled_T(int which, const Params& p, cudaStream_t st) {
   using C = Tiled<DP>;
   const size_t rows = which == 0 ? C::kBM + 2 * C::kBN : 2 * C::kBM + 2 * C::kBN;      // staged rows of DP + 4 floats
-  const size_t tiles = which == 1 ? 2 : 1;                                             // P and dS, or one of them
-  const size_t sm = (rows * C::kLd + tiles * C::kBM * C::kLdP + (which == 1 ? 2 * C::kBN : 0)) * sizeof(float);
-  auto kern = which == 0 ? tiled_fwd_kernel<T, DP> : (which == 1 ? tiled_bwd_dkdv_kernel<T, DP> : tiled_bwd_dq_kernel<T, DP>);
+  const size_t tiles = which & 1 ? 2 : 1;                                              // P and dS, or one of them
+  const size_t sm = (rows * C::kLd + tiles * C::kBM * C::kLdP + (which & 1 ? 2 * C::kBN : 0)) * sizeof(float);
+  auto kern = which == 0   ? tiled_fwd_kernel<T, DP>
+              : which == 1 ? tiled_bwd_kernel<T, DP, 1>
+              : which == 2 ? tiled_bwd_kernel<T, DP, 2>
+                           : tiled_bwd_kernel<T, DP, 3>;
   cudaError_t e = set_smem(kern, sm);
   if (e != cudaSuccess) return e;
-  const int rows_total = which == 1 ? p.max_sk : p.max_sq;
-  dim3 grid((rows_total + C::kBM - 1) / C::kBM, which == 1 ? p.hk : p.hq, p.batch);
+  const int rows_total = which == 1 ? p.max_sk : (which == 3 && p.max_sk > p.max_sq ? p.max_sk : p.max_sq);
+  const int blocks = (rows_total + C::kBM - 1) / C::kBM;
+  dim3 grid(which == 3 ? 2 * blocks : blocks, which == 1 ? p.hk : p.hq, p.batch);
   e = launch_kernel(kern, grid, dim3(C::kThreads), sm, st, p);
   if (e == cudaSuccess) count_launch();
   return e;
@@ -552,6 +556,10 @@ cudaError_t launch_general_D(int which, const Params& p, cudaStream_t st) {
   int d = p.dqk > p.dvo ? p.dqk : p.dvo;
   if (d <= 64) return launch_tiled_T<T, 64>(which, p, st);
   if (d <= 128) return launch_tiled_T<T, 128>(which, p, st);
+  if (which == 3) {
+    const cudaError_t e = launch_general_D<T>(1, p, st);
+    return e != cudaSuccess ? e : launch_general_D<T>(2, p, st);
+  }
   if (d <= 256) return launch_general_T<T, 8>(which, p, st);
   return launch_general_T<T, 16>(which, p, st);
 }

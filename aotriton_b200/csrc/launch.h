@@ -66,7 +66,8 @@ cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
   return host().launch(reinterpret_cast<const void*>(kernel), grid, block, ptrs, smem, st);
 }
 
-// which: 0 forward, 1 dK/dV, 2 dQ(+dBias).  dtype: ab200_dtype value.
+// which: 0 forward, 1 dK/dV, 2 dQ(+dBias), 3 both (dQ and dBias share no memory with an input).  dtype:
+// ab200_dtype value.
 cudaError_t launch_general(int which, int dtype, const Params& p, cudaStream_t st);
 cudaError_t launch_preprocess(int dtype, const Params& p, cudaStream_t st);
 cudaError_t launch_dropout_sign(int dtype, const View4& r, int batch, int heads, int rows, int cols, float dropout_p,
