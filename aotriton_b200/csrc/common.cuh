@@ -51,6 +51,7 @@ struct Params {
   uint32_t wait_limit_kcycles;    // bound of every in-kernel wait, in units of 1024 SM cycles (0 = about a second)
   int32_t drop_copy;              // test hook of the bounded waits: the producer leaves out one tile copy
                                   // (1 = first V block of the forward, 2 = first Q/dO block of dK/dV, 3 = first V block of dQ)
+  int32_t packed_tiles;           // token-packed: the grid counts row tiles of all sequences instead of max_sq's per sequence
   int32_t keep_tiles, keep_shift; // keep bits of the first keep_tiles 32-key tiles pass through dQ's rows (0: none); see KeepShare
 };
 
@@ -88,6 +89,45 @@ __device__ __forceinline__ Seq resolve_seq(const Params& p, int z) {
   else if (p.causal_type == 2 || p.window_right == kBottomRight) s.wr = s.sk - s.sq;
   else s.wr = p.window_right;
   return s;
+}
+
+// Row tile `tile` of a token-packed batch, when the tiles of all sequences are counted through (within a
+// sequence the last rows, which a causal mask lets see the most keys, come first).  A grid of max_sq's tiles
+// for every sequence starts a CTA for each tile a shorter sequence does not have: at one CTA per SM each of
+// them takes its turn.  Sequences are looked at 32 at a time by the whole warp.  False: beyond the last tile.
+// Measured: 24 packed prompts of 32 to 2048 tokens, 32:8 heads of 128, 399 -> 372 us.
+template <int ROWS>
+__device__ __forceinline__ bool packed_tile(const Params& p, int tile, int lane, int& z, int& m0) {
+  const int cap = (p.max_sq + ROWS - 1) / ROWS;      // a sequence longer than max_sq has no more tiles than that
+  int before = 0;
+  for (int b0 = 0; b0 < p.batch; b0 += 32) {
+    int n = 0;
+    if (b0 + lane < p.batch) n = max(0, min(cap, (p.cu_q[b0 + lane + 1] - p.cu_q[b0 + lane] + ROWS - 1) / ROWS));
+    int upto = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const uint32_t past = __ballot_sync(0xffffffffu, before + upto > tile);
+    if (past != 0u) {
+      const int src = __ffs(past) - 1;
+      z = b0 + src;
+      m0 = (before + __shfl_sync(0xffffffffu, upto, src) - 1 - tile) * ROWS;
+      return true;
+    }
+    before += __shfl_sync(0xffffffffu, upto, 31);
+  }
+  return false;
+}
+// Upper bound of the number of tiles packed_tile() counts, from what the host knows: the packed token count.
+// 0: not a batch for it (only consecutive sequences are bounded by that count; and past a few rounds of 32
+// sequences the search costs a CTA more than the empty CTAs did).
+inline int packed_tiles_bound(const Params& p, int rows) {
+  if (p.varlen_mode != 1 || p.ss_q != nullptr || p.batch > 128) return 0;
+  const int64_t per_seq = (int64_t)p.batch * ((p.max_sq + rows - 1) / rows);
+  const int64_t by_tokens = p.q.n[2] / rows + p.batch;
+  return by_tokens < per_seq ? (int)by_tokens : 0;
 }
 
 __device__ __forceinline__ int64_t lse_offset(const Params& p, const Seq& s, int h) {

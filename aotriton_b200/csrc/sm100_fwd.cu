@@ -155,6 +155,11 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
     if (p.seed_out) *p.seed_out = seed;
     if (p.off_out) *p.off_out = base;
   }
+  if (!EXACT && p.packed_tiles > 0) {      // one-dimensional grid: the heads of a tile next to each other
+    const int tile = (int)blockIdx.x / p.hq;
+    h = (int)blockIdx.x - tile * p.hq;
+    if (!packed_tile<kCtaRows>(p, tile, lane, z, m0)) return;
+  }
   const Seq sq = resolve_seq(p, z);
   if (m0 >= sq.sq) return;
   const int hk = h / p.group;
@@ -650,7 +655,10 @@ cudaError_t launch_fwd_TE(const Params& p, cudaStream_t st) {
     if (remember) attr_set[dev].store(true, std::memory_order_release);
   }
   dim3 grid((p.max_sq + L::kCtaRows - 1) / L::kCtaRows, p.hq, p.batch);
-  e = launch_kernel(sm100_fwd_kernel<T, HD, EXACT, PLAIN>, grid, dim3(kFwdThreads), L::kDynamic, st, p, tq, tk, tv, status);
+  Params pp = p;
+  pp.packed_tiles = packed_tiles_bound(p, L::kCtaRows);
+  if (pp.packed_tiles > 0) grid = dim3(pp.packed_tiles * p.hq);
+  e = launch_kernel(sm100_fwd_kernel<T, HD, EXACT, PLAIN>, grid, dim3(kFwdThreads), L::kDynamic, st, pp, tq, tk, tv, status);
   if (e == cudaSuccess) count_launch();
   return e;
 }
