@@ -206,9 +206,9 @@ struct DeviceGuard {
   ~DeviceGuard() { if (switched_) { (void)host().set_device(old_); } }
 };
 
-bool rows_16byte(const ab200_view4& v) {
-  return v.ptr != nullptr && (reinterpret_cast<uintptr_t>(v.ptr) & 15u) == 0 && v.stride[3] == 1 &&
-         v.stride[0] % 8 == 0 && v.stride[1] % 8 == 0 && v.stride[2] % 8 == 0;
+bool rows_16byte(const void* ptr, const int64_t* stride) {
+  return ptr != nullptr && (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0 && stride[3] == 1 && stride[0] % 8 == 0 &&
+         stride[1] % 8 == 0 && stride[2] % 8 == 0;
 }
 
 View4 to_view(const ab200_view4& v) {
@@ -347,6 +347,16 @@ void keep_share_setup(Params& p) {
   p.keep_tiles = std::min(32 << p.keep_shift, (p.max_sk + 31) / 32);
 }
 
+// dK from dBias (wide heads; dense, the only layout with a bias gradient whose rows a tile map can describe).  dBias
+// must keep every value the dQ kernel wrote (a broadcast one does not), and dQ, written before dK is formed, must
+// leave Q alone.
+bool dk_from_db_possible(const Params& p) {
+  if (!p.has_dbias || p.varlen_mode != 0 || (p.dqk <= 128 && p.dvo <= 128)) return false;
+  const View4& d = p.dbias;
+  if (d.n[0] != p.batch || d.n[1] != p.hq || d.n[2] != p.max_sq || d.n[3] != p.max_sk) return false;
+  return rows_16byte(d.ptr, d.s) && rows_disjoint(d, p.max_sk) && apart_from_inputs(d, p, 2) && apart_from_inputs(p.dq, p, 2);
+}
+
 bool want_sm100(int family) { return family != 1; }
 int family_flags(int family) {
   return family == 1 ? AB200_SELECT_FORCE_GENERAL : (family == 2 ? AB200_SELECT_FORCE_TCGEN05 : 0);
@@ -457,7 +467,7 @@ int ab200_attn_fwd(const ab200_attn_fwd_args* a, void* stream) {
   if (int e = check_device(st)) return e;
   DeviceGuard guard(st);
   p.q = to_view(a->q); p.k = to_view(a->k); p.v = to_view(a->v); p.out = to_view(a->out);
-  p.bias = to_view(a->bias); p.has_bias = a->bias.ptr != nullptr; p.bias_vec = rows_16byte(a->bias);
+  p.bias = to_view(a->bias); p.has_bias = a->bias.ptr != nullptr; p.bias_vec = rows_16byte(a->bias.ptr, a->bias.stride);
   p.lse = a->lse;
   p.seed_out = a->philox_seed_output; p.off_out = a->philox_offset_output;
 
@@ -498,7 +508,7 @@ static int fill_bwd(const ab200_attn_bwd_args* a, Params& p, bool need_outputs) 
       return kErrInvalidValue;
   }
   p.q = to_view(a->q); p.k = to_view(a->k); p.v = to_view(a->v);
-  p.bias = to_view(a->bias); p.has_bias = a->bias.ptr != nullptr; p.bias_vec = rows_16byte(a->bias);
+  p.bias = to_view(a->bias); p.has_bias = a->bias.ptr != nullptr; p.bias_vec = rows_16byte(a->bias.ptr, a->bias.stride);
   p.dq = to_view(a->dq); p.dk = to_view(a->dk); p.dv = to_view(a->dv); p.dbias = to_view(a->dbias);
   // dBias is skipped when absent or when all its strides are zero
   // (modules/flash/kernel/bwd_kernel_dq.py:265-266).
@@ -516,7 +526,7 @@ int ab200_bwd_preprocess(const ab200_attn_bwd_args* a, void* stream) {
   return (int)launch_preprocess(a->prob.dtype, p, st);
 }
 
-// `share`: dK/dV and dQ run in one call, so that keep bits may pass from one to the other.
+// `share`: dK/dV and dQ run in one call, so that keep bits may pass from one to the other, and dK come out of the second.
 static int run_dkdv(const ab200_attn_bwd_args* a, void* stream, bool share) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   Params p{};
@@ -529,7 +539,7 @@ static int run_dkdv(const ab200_attn_bwd_args* a, void* stream, bool share) {
   if (sel < 0) return -sel;
   if ((sel & 0xff) >= kVarTcgen05) {
     t_last_bwd = 2;
-    if (share) keep_share_setup(p);
+    if (share) { keep_share_setup(p); p.dk_from_db = dk_from_db_possible(p); }
     return (int)launch_sm100_bwd_dkdv(a->prob.dtype, p, st);
   }
   t_last_bwd = 1;
@@ -548,7 +558,7 @@ static int run_dq(const ab200_attn_bwd_args* a, void* stream, bool share) {
   if (sel < 0) return -sel;
   if ((sel & 0xff) >= kVarTcgen05) {
     t_last_bwd = 2;
-    if (share) keep_share_setup(p);
+    if (share) { keep_share_setup(p); p.dk_from_db = dk_from_db_possible(p); }
     return (int)launch_sm100_bwd_dq(a->prob.dtype, p, st);
   }
   t_last_bwd = 1;
