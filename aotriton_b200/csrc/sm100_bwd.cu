@@ -623,11 +623,9 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
     const int cbase = kWgCols * wg;
     uint32_t G = 0, live = 0, drawn = 0;
     bool ok = true;
-    // Philox seed and offset are read once; the round keys depend on the seed only
+    // Philox seed and offset are read once
     const uint64_t ph_seed = (drop_on && p.seed_ptr) ? *p.seed_ptr : 0ull;
     const uint64_t ph_off = p.off2 + ((drop_on && p.off1_ptr) ? *p.off1_ptr : 0ull);
-    PhiloxKeys pkeys;
-    if (drop_on) pkeys = philox_keys(ph_seed);
     for (int w = blockIdx.x; ok && w < nitems; w = next_item(drawn++, true)) {
       const DkdvItem it = dkdv_item(p, w);
       if (!it.valid) continue;
@@ -799,8 +797,10 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           const int q4 = lane & 3;
           uint32_t mine = 0u;            // nibble k: keep bits of keys 4a..4a+3 for query row mbase + q4 + 4k
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            mine |= dropout_keep4_keys(dctx, pkeys, min(mbase + q4 + 4 * k, p.max_sq - 1), n >> 2) << (4 * k);
+          for (int k = 0; k < 8; k += 4)
+            mine |= dropout_keep_nibbles<4>(dctx.seed, dctx.threshold, [&](int u) {
+                      return dctx.base + (uint64_t)min(mbase + q4 + 4 * (k + u), p.max_sq - 1) * dctx.stride + (uint64_t)(n >> 2);
+                    }) << (4 * k);
           if (drop_on && keep_shared(p, sq, mbase, it.n0 + quarter * 32))
             *keep_share_word(p, sq, h, mbase, it.n0 + quarter * 32, lane) = keep_rows_from_quads(mine, lane);
           keep = 0u;
@@ -1232,8 +1232,6 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
     const bool simple = !bias_on && !__any_sync(0xffffffffu, fabsf(lse2) > 1.0e6f && lse2 != INFINITY);
     DropoutCtx dctx;
     if (drop_on) dctx = dropout_ctx(p, z, h);
-    PhiloxKeys pkeys;      // Philox round keys: they depend on the seed only
-    if (drop_on) pkeys = philox_keys(dctx.seed);
     const int mm = min(m, sq.sq - 1);
     const T* bias_row = bias_on ? reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
                                          (int64_t)h * p.bias.s[1] + (int64_t)mm * p.bias.s[2]
@@ -1313,7 +1311,10 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
         keep = 0u;
         const int md = min(m, p.max_sq - 1);
 #pragma unroll
-        for (int c4 = 0; c4 < 8; ++c4) keep |= dropout_keep4_keys(dctx, pkeys, md, (nbase >> 2) + c4) << (4 * c4);
+        for (int c4 = 0; c4 < 8; c4 += 4)
+          keep |= dropout_keep_nibbles<4>(dctx.seed, dctx.threshold, [&](int u) {
+                    return dctx.base + (uint64_t)md * dctx.stride + (uint64_t)((nbase >> 2) + c4 + u);
+                  }) << (4 * c4);
       }
       const uint32_t dp_col = tmem_base + lane_addr + kColDP + (uint32_t)(i & 1) * 128u + cbase;
       if (threadIdx.x == AB200_TRACE_TID) AB200_STAMPQ(i, 7);

@@ -357,11 +357,9 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
     // the tightest bounds over the warp's rows: a block needs masking iff it is not inside them
     const int warp_lo = __reduce_max_sync(0xffffffffu, v_lo), warp_hi = __reduce_min_sync(0xffffffffu, v_hi);
     bool ok = true;
-    // Philox seed and offset are read once; the round keys depend on the seed only
+    // Philox seed and offset are read once
     const uint64_t ph_seed = (drop_on && p.seed_ptr) ? *p.seed_ptr : 0ull;
     const uint64_t ph_off = p.off2 + ((drop_on && p.off1_ptr) ? *p.off1_ptr : 0ull);
-    PhiloxKeys pkeys;
-    if (drop_on) pkeys = philox_keys(ph_seed);
     if constexpr (kKeys) {
       const int n = row;
       for (int i = 0, hg = 0, cb = 0; i < niter; ++i) {
@@ -447,8 +445,10 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           const int q4 = lane & 3;
           uint32_t mine = 0u;
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            mine |= dropout_keep4_keys(dctx, pkeys, min(mbase + q4 + 4 * k, p.max_sq - 1), n >> 2) << (4 * k);
+          for (int k = 0; k < 8; k += 4)
+            mine |= dropout_keep_nibbles<4>(dctx.seed, dctx.threshold, [&](int u) {
+                      return dctx.base + (uint64_t)min(mbase + q4 + 4 * (k + u), p.max_sq - 1) * dctx.stride + (uint64_t)(n >> 2);
+                    }) << (4 * k);
           if constexpr (MODE == kWideDV) {
             if (drop_on && keep_shared(p, sq, mbase, r0 + quarter * 32))
               *keep_share_word(p, sq, h, mbase, r0 + quarter * 32, lane) = keep_rows_from_quads(mine, lane);
@@ -585,7 +585,10 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           keep = 0u;
           const int md = min(m, p.max_sq - 1);
 #pragma unroll
-          for (int c4 = 0; c4 < 8; ++c4) keep |= dropout_keep4_keys(dctx, pkeys, md, (nbase >> 2) + c4) << (4 * c4);
+          for (int c4 = 0; c4 < 8; c4 += 4)
+          keep |= dropout_keep_nibbles<4>(dctx.seed, dctx.threshold, [&](int u) {
+                    return dctx.base + (uint64_t)md * dctx.stride + (uint64_t)((nbase >> 2) + c4 + u);
+                  }) << (4 * c4);
         }
         const uint32_t a_col = tmem_base + lane_addr + kWColDP + (uint32_t)s * 64u + cbase;
         if (!mbar_wait(&bars[L::bDpFull + s], par2, abort_flag, status, 0x3D00)) { ok = false; break; }

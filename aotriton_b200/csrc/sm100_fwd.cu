@@ -366,10 +366,6 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
     const int warp_lo = __reduce_max_sync(0xffffffffu, row_lo), warp_hi = __reduce_min_sync(0xffffffffu, row_hi);
     DropoutCtx dctx;
     if (drop_on) dctx = dropout_ctx(p, z, h);
-    // (the ten round keys of Philox depend on the seed only: kept in registers, they save every counter
-    // two additions per round, 13 to 18 % of a dropout forward)
-    PhiloxKeys pkeys;
-    if (drop_on) pkeys = philox_keys(dctx.seed);
     const T* bias_row = nullptr;
     if (bias_on)
       bias_row = reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] + (int64_t)h * p.bias.s[1] +
@@ -542,7 +538,25 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
         if (drop_on) {
           const int mm = min(m, p.max_sq - 1);
 #pragma unroll
-          for (int c4 = half * 16; c4 < half * 16 + 16; ++c4) dropout_zero4_keys(dctx, pkeys, mm, (n0 >> 2) + c4, &sc[c4 * 4]);
+          for (int c4 = half * 16; c4 < half * 16 + 16; c4 += 4) {
+            const uint64_t first = dctx.base + (uint64_t)mm * dctx.stride + (uint64_t)((n0 >> 2) + c4);
+            uint32_t w[4][4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              w[u][0] = (uint32_t)(first + (uint64_t)u);
+              w[u][1] = (uint32_t)((first + (uint64_t)u) >> 32);
+            }
+            philox4x32_10_lockstep<4>(dctx.seed, w);
+            // (the four words of a counter are its columns 0, 2, 1, 3)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              float* v = &sc[(c4 + u) * 4];
+              v[0] = ((int32_t)w[u][0] > dctx.threshold) ? v[0] : 0.f;
+              v[1] = ((int32_t)w[u][2] > dctx.threshold) ? v[1] : 0.f;
+              v[2] = ((int32_t)w[u][1] > dctx.threshold) ? v[2] : 0.f;
+              v[3] = ((int32_t)w[u][3] > dctx.threshold) ? v[3] : 0.f;
+            }
+          }
         }
         // P over the first 64 columns of this S buffer, two 16-bit values per column.
         {
