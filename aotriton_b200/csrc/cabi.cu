@@ -347,11 +347,11 @@ void keep_share_setup(Params& p) {
   p.keep_tiles = std::min(32 << p.keep_shift, (p.max_sk + 31) / 32);
 }
 
-// dK from dBias (dense, the only layout with a bias gradient whose rows a tile map can describe).  dBias
+// dK from dBias (wide heads; dense, the only layout with a bias gradient whose rows a tile map can describe).  dBias
 // must keep every value the dQ kernel wrote (a broadcast one does not), and dQ, written before dK is formed, must
 // leave Q alone.
 bool dk_from_db_possible(const Params& p) {
-  if (!p.has_dbias || p.varlen_mode != 0) return false;
+  if (!p.has_dbias || p.varlen_mode != 0 || (p.dqk <= 128 && p.dvo <= 128)) return false;
   const View4& d = p.dbias;
   if (d.n[0] != p.batch || d.n[1] != p.hq || d.n[2] != p.max_sq || d.n[3] != p.max_sk) return false;
   return rows_16byte(d.ptr, d.s) && rows_disjoint(d, p.max_sk) && apart_from_inputs(d, p, 2) && apart_from_inputs(p.dq, p, 2);

@@ -282,10 +282,7 @@ __device__ __forceinline__ DkdvItem dkdv_item(const Params& p, int w) {
 // what it keeps for these (Philox round keys, row pointers, strides) is most of it: with them 176 bytes stored in dK/dV
 // and 28 in dQ, without 52 and none.  Measured, forward + backward: dense causal 4 x 32 heads x 4096, head dim 128,
 // 2.85 -> 2.72 ms; 64:8 heads x 16384, window 4096, 8.90 -> 8.48.
-// DVONLY: dK comes out of the bias gradient afterwards (sm100_bwd_dk_db.cuh): no V, no dP, no dS, one accumulator.
-// Measured, training step with bias and dropout 0.2, 8 x 16 heads x 2048, head dim 72: 3.59 -> 3.51 ms (Philox in
-// lockstep included).
-template <typename T, int HD, bool FUSED, bool EXACT, bool PLAIN, bool DVONLY = false>
+template <typename T, int HD, bool FUSED, bool EXACT, bool PLAIN>
 __global__ void __launch_bounds__(FUSED ? kFusedThreads : kBwdThreads, 1)
 sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm_q,
                       const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -351,11 +348,10 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         // K and V of the previous item are free once its last S and dP GEMMs have run.
         if (!mbar_wait(&bars[L::bResEmpty], (live & 1u) ^ 1u, abort_flag, status, 0x1000)) break;
         const int krow = (int)(it.sq.k0 + it.n0);
-        mbar_expect_tx(&bars[L::bResFull], (DVONLY ? 1 : 2) * L::kTile);
+        mbar_expect_tx(&bars[L::bResFull], 2 * L::kTile);
         for (int hf = 0; hf < L::kHalves; ++hf) {
           tma_load_4d(smem + L::kResA + hf * 16384, &tm_k, &bars[L::bResFull], hf * 64, krow, it.hk, it.sq.bidx);
-          if constexpr (!DVONLY)
-            tma_load_4d(smem + L::kResB + hf * 16384, &tm_v, &bars[L::bResFull], hf * 64, krow, it.hk, it.sq.bidx);
+          tma_load_4d(smem + L::kResB + hf * 16384, &tm_v, &bars[L::bResFull], hf * 64, krow, it.hk, it.sq.bidx);
         }
         for (int i = 0, hg = 0, mb = 0; i < it.niter; ++i, ++G) {     // hg, mb: i / nmb, i % nmb
           const int s = (int)(G & 1u);
@@ -417,14 +413,13 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
       }
       __syncwarp();
     };
-    // dP^T = V dO_g^T; `release_kv`: these are the last readers of the item's K and V.  (DVONLY: nothing is computed; the
-    // commit says that dV has read the previous P^T, and releases K behind S^T)
+    // dP^T = V dO_g^T; `release_kv`: these are the last readers of the item's K and V
     auto issue_dp = [&](uint32_t g, bool release_kv) {
       const uint64_t da = do_km + (uint64_t)((g & 1u) * kStageStep);
       if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk)
-          if (!DVONLY && kk < ksteps_vo)
+          if (kk < ksteps_vo)
             mma_ss(tmem_base + kColDP, v_km + kmajor_step(kk), da + kmajor_step(kk), kIdescSS, kk > 0 ? 1u : 0u);
         mma_commit(&bars[L::bDpFull]);
         if (release_kv) mma_commit(&bars[L::bResEmpty]);
@@ -445,7 +440,7 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
       if constexpr (!EXACT) {
         if (it.sq.sk - it.n0 < kBlk) {
           zero_tail_rows(smem + L::kResA, it.sq.sk - it.n0, L::kHalves, lane);
-          if constexpr (!DVONLY) zero_tail_rows(smem + L::kResB, it.sq.sk - it.n0, L::kHalves, lane);
+          zero_tail_rows(smem + L::kResB, it.sq.sk - it.n0, L::kHalves, lane);
         }
       }
       if (G > 0 && !wait(L::bSRead, (G - 1) & 1u, 0x1201)) break;
@@ -518,15 +513,6 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
                    kk > 0 ? 1u : first);
         }
         __syncwarp();
-        if constexpr (DVONLY) {
-          if (elect_one()) {
-            mma_commit(&bars[L::bRingEmpty + s]);
-            if (i + 1 == it.niter) mma_commit(&bars[L::bAccDone]);
-          }
-          __syncwarp();
-          if (i + 1 < it.niter) issue_dp(G + 1, i + 2 == it.niter);
-          continue;
-        }
         if (!wait(L::bDsFull, par, 0x1500)) { ok = false; break; }
         if (lane == 0) AB200_STAMP(G, 5);
         tc_fence_after();
@@ -816,10 +802,8 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         tc_fence_after();
         {
           float dp[32];
-          if constexpr (!DVONLY) {
-            tmem_ld32f(tmem_base + lane_addr + kColDP + cbase, dp);
-            tmem_wait_ld();
-          }
+          tmem_ld32f(tmem_base + lane_addr + kColDP + cbase, dp);
+          tmem_wait_ld();
           if (threadIdx.x == AB200_TRACE_TID) AB200_STAMP(G, 10);
           // This thread has now read its 32 columns of dP: they can take P^T (packed, 16 columns)
           // followed by dS^T (packed, 16 columns).
@@ -838,10 +822,6 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars[L::bPFull]);
-          if constexpr (DVONLY) {
-            if (lane == 0) mbar_arrive(&bars[L::bAuxEmpty + s]);
-            continue;
-          }
           if (drop_on) {
 #pragma unroll
             for (int c = 0; c < 32; ++c) dp[c] = ((keep >> c) & 1u) ? dp[c] * p.dropout_scale : 0.f;
@@ -921,21 +901,17 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         warp_copy_out<T, 4>(stage, reinterpret_cast<T*>(p.dv.ptr) + (int64_t)sq.bidx * p.dv.s[0] + (int64_t)hk * p.dv.s[1] +
                                        (sq.k0 + it.n0) * p.dv.s[2],
                             p.dv.s[2], nrows, p.dvo, quarter * 32, wg * 4, lane, HD * 2);
-        if constexpr (!DVONLY) {
-          tmem_ld32f(tmem_base + lane_addr + kColAcc1 + d0, v);
-          tmem_wait_ld();
-        }
+        tmem_ld32f(tmem_base + lane_addr + kColAcc1 + d0, v);
+        tmem_wait_ld();
         // The accumulators are in registers now: the next item's first dV/dK GEMMs (which start from
         // zero) are only issued after this thread's next hand-off, i.e. after these loads.
         tc_fence_before();
         __syncwarp();
-        if constexpr (!DVONLY) {
-          stage_put32<T>(stage, r, d0, v, p.sm_scale, HD * 2);
-          __syncwarp();
-          warp_copy_out<T, 4>(stage, reinterpret_cast<T*>(p.dk.ptr) + (int64_t)sq.bidx * p.dk.s[0] + (int64_t)hk * p.dk.s[1] +
-                                         (sq.k0 + it.n0) * p.dk.s[2],
-                              p.dk.s[2], nrows, p.dqk, quarter * 32, wg * 4, lane, HD * 2);
-        }
+        stage_put32<T>(stage, r, d0, v, p.sm_scale, HD * 2);
+        __syncwarp();
+        warp_copy_out<T, 4>(stage, reinterpret_cast<T*>(p.dk.ptr) + (int64_t)sq.bidx * p.dk.s[0] + (int64_t)hk * p.dk.s[1] +
+                                       (sq.k0 + it.n0) * p.dk.s[2],
+                            p.dk.s[2], nrows, p.dqk, quarter * 32, wg * 4, lane, HD * 2);
         __syncwarp();
       }
       // The staging tile is the next item's dS^T tile: no compute warp may write dS^T there while
@@ -1390,10 +1366,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
   }
 }
 
-#include "sm100_bwd_dk_db.cuh"
-
-// which: 1 dK/dV, 2 dQ(+dBias), 3 dK/dV fused with dQ accumulation into `dq_acc` (HD == 128 only);
-// p.dk_from_db: 1 dV, 2 dQ and dBias, then dK from dBias
+// which: 1 dK/dV, 2 dQ(+dBias), 3 dK/dV fused with dQ accumulation into `dq_acc` (HD == 128 only)
 template <typename T, int HD>
 cudaError_t launch_bwd_T(int which, const Params& p, cudaStream_t st, float* dq_acc) {
   using L = BwdSmem<HD>;
@@ -1407,7 +1380,7 @@ cudaError_t launch_bwd_T(int which, const Params& p, cudaStream_t st, float* dq_
   // make the stream's device, and remembered.
   struct PerDevice { std::atomic<unsigned int*> status{nullptr}, tickets{nullptr}; std::atomic<int> sms{0}; };
   static PerDevice per_device[64];
-  static std::atomic<bool> attr_set[64][11];
+  static std::atomic<bool> attr_set[64][10];
   const bool exact = p.varlen_mode == 0 && p.max_sq % 128 == 0 && p.max_sk % 128 == 0 && p.dqk == HD && p.dvo == HD;
   const bool plain = !p.dropout_on && !p.has_bias && !p.has_dbias;
   int dev = 0;
@@ -1434,10 +1407,9 @@ cudaError_t launch_bwd_T(int which, const Params& p, cudaStream_t st, float* dq_
     if (fused && HD != 128) return cudaErrorInvalidValue;
     auto kern_split = plain ? (exact ? sm100_bwd_dkdv_kernel<T, HD, false, true, true> : sm100_bwd_dkdv_kernel<T, HD, false, false, true>)
                             : (exact ? sm100_bwd_dkdv_kernel<T, HD, false, true, false> : sm100_bwd_dkdv_kernel<T, HD, false, false, false>);
-    if (p.dk_from_db) kern_split = sm100_bwd_dkdv_kernel<T, HD, false, false, false, true>;
     auto kern_fused = sm100_bwd_dkdv_kernel<T, 128, true, false, false>;
     e = fused ? set_smem(2, reinterpret_cast<const void*>(kern_fused), BwdSmem<128>::kDynamic)
-              : set_smem(p.dk_from_db ? 10 : (exact ? 3 : 0) + (plain ? 5 : 0), reinterpret_cast<const void*>(kern_split), L::kDynamic);
+              : set_smem((exact ? 3 : 0) + (plain ? 5 : 0), reinterpret_cast<const void*>(kern_split), L::kDynamic);
     if (e != cudaSuccess) return e;
     const int nitems = ((p.max_sk + kBlk - 1) / kBlk) * ((p.hk * p.batch + 7) / 8) * 8;
     int sms = pd.sms.load(std::memory_order_acquire);
@@ -1468,10 +1440,6 @@ cudaError_t launch_bwd_T(int which, const Params& p, cudaStream_t st, float* dq_
     if (e != cudaSuccess) return e;
     dim3 grid((p.max_sq + kBlk - 1) / kBlk, p.hq, p.batch);
     e = launch_kernel(kern_dq, grid, dim3(kBwdThreads), DqSmem<HD>::kDynamic, st, p, tq, tk, tv, tdo, status);
-    if (e == cudaSuccess && p.dk_from_db) {
-      count_launch();
-      e = launch_dk_db<T>(p, st, status, dev);
-    }
   }
   if (e == cudaSuccess) count_launch();
   return e;

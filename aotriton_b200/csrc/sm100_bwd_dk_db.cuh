@@ -1,5 +1,5 @@
-// dK from a dBias that is already written: dK = sm_scale * dB^T Q.
-// Included by sm100_bwd.cu inside its namespaces.
+// dK of wide heads from a dBias that is already written: dK = sm_scale * dB^T Q.
+// Included by sm100_bwd_wide.cuh inside its namespaces.
 //
 // Bias enters the scores with factor one, so dB is dS: the 16-bit values the dK kernel would form again (scores,
 // exponentials, bias, keep bits, dP) to feed its accumulating GEMM.  When the caller wants dB, the dQ kernel runs
@@ -141,22 +141,4 @@ sm100_bwd_dk_db_kernel(const __grid_constant__ Params p, const __grid_constant__
     tc_fence_after();
     tmem_dealloc(tmem_base, kCols);
   }
-}
-
-template <typename T>
-cudaError_t launch_dk_db(const Params& p, cudaStream_t st, unsigned int* status, int dev) {
-  CUtensorMap db, q;
-  if (!make_tile_map_16bit(&q, p.q, p.dqk, p.q.n[2], DkDbSmem::kRows) ||
-      !make_tile_map_16bit(&db, p.dbias, p.max_sk, p.max_sq, DkDbSmem::kRows))
-    return cudaErrorInvalidValue;
-  static std::atomic<bool> attr_set[64];
-  auto kern = sm100_bwd_dk_db_kernel<T>;
-  const bool pretend = host_pretends();
-  if (pretend || !attr_set[dev].load(std::memory_order_acquire)) {
-    const cudaError_t e = host().func_set_smem(reinterpret_cast<const void*>(kern), DkDbSmem::kDynamic);
-    if (e != cudaSuccess) return e;
-    if (!pretend) attr_set[dev].store(true, std::memory_order_release);
-  }
-  dim3 grid((p.max_sk + kBlk - 1) / kBlk, p.hk, p.batch);
-  return launch_kernel(kern, grid, dim3(kDkDbThreads), DkDbSmem::kDynamic, st, p, db, q, status);
 }

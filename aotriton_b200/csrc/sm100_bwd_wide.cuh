@@ -665,11 +665,13 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
   }
 }
 
+#include "sm100_bwd_dk_db.cuh"
+
 // which: 1 dV and dK (two launches), 2 dQ(+dBias); p.dk_from_db: 1 dV, 2 dQ and dBias, then dK from dBias
 template <typename T>
 cudaError_t launch_bwd_wide_T(int which, const Params& p, cudaStream_t st) {
   using L = WideSmem;
-  CUtensorMap q128, k128, v128, do128, q64, k64, v64, do64;
+  CUtensorMap q128, k128, v128, do128, q64, k64, v64, do64, db64;
   if (which == 1) {
     if (!make_tile_map_16bit(&k128, p.k, p.dqk, p.k.n[2], kBlk) || !make_tile_map_16bit(&v128, p.v, p.dvo, p.v.n[2], kBlk) ||
         !make_tile_map_16bit(&q64, p.q, p.dqk, p.q.n[2], kNB) || !make_tile_map_16bit(&do64, p.dout, p.dvo, p.dout.n[2], kNB))
@@ -679,9 +681,12 @@ cudaError_t launch_bwd_wide_T(int which, const Params& p, cudaStream_t st) {
         !make_tile_map_16bit(&do128, p.dout, p.dvo, p.dout.n[2], kBlk) ||
         !make_tile_map_16bit(&k64, p.k, p.dqk, p.k.n[2], kNB) || !make_tile_map_16bit(&v64, p.v, p.dvo, p.v.n[2], kNB))
       return cudaErrorInvalidValue;
+    if (p.dk_from_db && (!make_tile_map_16bit(&q64, p.q, p.dqk, p.q.n[2], DkDbSmem::kRows) ||
+                         !make_tile_map_16bit(&db64, p.dbias, p.max_sk, p.max_sq, DkDbSmem::kRows)))
+      return cudaErrorInvalidValue;
   }
   static std::atomic<unsigned int*> status_of[64];
-  static std::atomic<bool> attr_set[64][6];
+  static std::atomic<bool> attr_set[64][7];
   const bool plain = !p.dropout_on && !p.has_bias && !p.has_dbias;
   int dev = 0;
   cudaError_t e = host().get_device(&dev);
@@ -693,9 +698,9 @@ cudaError_t launch_bwd_wide_T(int which, const Params& p, cudaStream_t st) {
     if ((e = host().symbol_address(reinterpret_cast<void**>(&status), reinterpret_cast<const void*>(&g_sm100_bwd_status))) != cudaSuccess) return e;
     if (!pretend) status_of[dev].store(status, std::memory_order_release);
   }
-  auto set_smem = [&](int slot, const void* fn) -> cudaError_t {
+  auto set_smem = [&](int slot, const void* fn, int bytes = L::kDynamic) -> cudaError_t {
     if (!pretend && attr_set[dev][slot].load(std::memory_order_acquire)) return cudaSuccess;
-    cudaError_t r = host().func_set_smem(fn, L::kDynamic);
+    cudaError_t r = host().func_set_smem(fn, bytes);
     if (r == cudaSuccess && !pretend) attr_set[dev][slot].store(true, std::memory_order_release);
     return r;
   };
@@ -718,7 +723,10 @@ cudaError_t launch_bwd_wide_T(int which, const Params& p, cudaStream_t st) {
     e = launch_kernel(kern_dq, grid, dim3(kWideThreads), L::kDynamic, st, p, q128, do128, k64, v64, status);
     if (e == cudaSuccess && p.dk_from_db) {
       count_launch();
-      e = launch_dk_db<T>(p, st, status, dev);
+      auto kern_db = sm100_bwd_dk_db_kernel<T>;
+      if ((e = set_smem(6, reinterpret_cast<const void*>(kern_db), DkDbSmem::kDynamic)) != cudaSuccess) return e;
+      dim3 grid_k((p.max_sk + kBlk - 1) / kBlk, p.hk, p.batch);
+      e = launch_kernel(kern_db, grid_k, dim3(kDkDbThreads), DkDbSmem::kDynamic, st, p, db64, q64, status);
     }
   }
   if (e == cudaSuccess) count_launch();

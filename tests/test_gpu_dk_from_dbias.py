@@ -24,12 +24,6 @@ TL, BR = -2147483647, -2147483646
     (1, 2, 2, 130, 136, 256, (0, 0, 0), "bshd"),
     (1, 2, 2, 130, 131, 256, (0, 0, 0), "odd"),          # rows of dBias off a 16-byte boundary
     (2, 2, 2, 130, 136, 256, (0, 0, 0), "in place"),     # dQ over Q
-    (1, 1, 1, 1, 8, 64, (0, 0, 0), ""),                  # head dims up to 128
-    (2, 4, 2, 300, 264, 72, (0, 0, 0), ""),
-    (1, 2, 2, 384, 640, 128, (3, BR, BR), "bshd"),
-    (1, 4, 1, 640, 384, 128, (3, 200, 10), ""),
-    (1, 2, 2, 200, 131, 64, (0, 0, 0), "odd"),
-    (2, 2, 2, 200, 136, 64, (0, 0, 0), "in place"),
 ])
 def test_equal_to_separate_stages(B, Hq, Hk, Sq, Sk, D, causal, how, p, dt):
     from aotriton_b200 import cabi
