@@ -228,20 +228,12 @@ __device__ __forceinline__ uint32_t dropout_keep4(const DropoutCtx& d, int m, in
   return k;
 }
 
-// Both halves of a 32 x 32-bit product, by two instructions.  Left to itself the compiler forms the 64-bit
-// product with one wide multiply, which has twice the latency (measured alone, per counter and warp, 8 warps per SM:
-// 158 scheduler cycles against 116 one counter at a time, 105 against 99 eight at a time; the high halves through
-// the fp64 unit 102 to 157).
-__device__ __forceinline__ void mul_hi_lo(uint32_t a, uint32_t b, uint32_t& hi, uint32_t& lo) {
-  hi = __umulhi(a, b);
-  lo = a * b;
-  asm("" : "+r"(lo));      // (keeps the two apart)
-}
-
 // N counters of one seed in lockstep: independent chains side by side, and the two key additions of a round
 // serve all of them.  (Ten round keys held in registers save the additions too, but twenty registers is what the
 // compute warps do not have: dK/dV spilled 228 bytes with them, 156 without.  Measured, training step of 16
-// packed sequences of 64 to 8192 tokens, 32:8 heads of 128, dropout 0.1: 22.96 -> 21.87 ms.)
+// packed sequences of 64 to 8192 tokens, 32:8 heads of 128, dropout 0.1: 22.73 -> 21.85 ms; bias, dropout 0.2,
+// 8 x 16 heads x 2048: head dim 72 3.58 -> 3.52, 256 5.53 -> 5.38.  The halves of a product by separate
+// instructions, which alone have less latency than the wide multiply, changed nothing here.)
 // c[n][0..1]: counter in, words 0 and 1 out; c[n][2..3]: words 2 and 3 out.
 template <int N>
 __device__ __forceinline__ void philox4x32_10_lockstep(uint64_t seed, uint32_t (&c)[N][4]) {
@@ -254,12 +246,10 @@ __device__ __forceinline__ void philox4x32_10_lockstep(uint64_t seed, uint32_t (
   for (int i = 0; i < 10; ++i) {
 #pragma unroll
     for (int n = 0; n < N; ++n) {
-      uint32_t ah, al, bh = 0u, bl = 0u;
-      mul_hi_lo(kA, c[n][0], ah, al);
-      if (i > 0) mul_hi_lo(kB, c[n][2], bh, bl);
-      const uint32_t n0 = bh ^ c[n][1] ^ k0;
-      const uint32_t n2 = ah ^ c[n][3] ^ k1;
-      c[n][1] = bl; c[n][3] = al; c[n][0] = n0; c[n][2] = n2;
+      const uint64_t pa = (uint64_t)kA * c[n][0], pb = (uint64_t)kB * c[n][2];
+      const uint32_t n0 = (uint32_t)(pb >> 32) ^ c[n][1] ^ k0;
+      const uint32_t n2 = (uint32_t)(pa >> 32) ^ c[n][3] ^ k1;
+      c[n][1] = (uint32_t)pb; c[n][3] = (uint32_t)pa; c[n][0] = n0; c[n][2] = n2;
     }
     k0 += kKA; k1 += kKB;
   }

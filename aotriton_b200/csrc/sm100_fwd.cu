@@ -393,7 +393,7 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
     // With one tile per CTA these warps have nothing else to do, and Philox is the one thing that neither the tensor
     // pipe, the special-function unit nor the softmax warps' chain has a part in: it runs beside them, a thread
     // drawing the 128 bits of its row up to two blocks ahead.  Measured, training step with bias
-    // and dropout 0.2, 8 x 16 heads x 2048: 5.38 -> 5.03 ms.
+    // and dropout 0.2, 8 x 16 heads x 2048: 5.38 -> 4.99 ms.
     // (With two tiles it does not pay: a warpgroup more leaves its threads 56 registers, too few for the independent
     // counters that one warp per scheduler needs: 16 packed sequences 23.3 -> 26.1 ms.)
     if constexpr (!PLAIN) {
