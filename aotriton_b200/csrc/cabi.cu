@@ -74,10 +74,50 @@ cudaError_t h_set_device(int dev) {
   if (fake()) return cudaSuccess;
   return cudaSetDevice(dev);
 }
+// The driver's context queries (none of them an operation on a stream).
+struct DriverContexts {
+  CUresult (*of_stream)(CUstream, CUcontext*) = nullptr;
+  CUresult (*current)(CUcontext*) = nullptr;
+  CUresult (*push)(CUcontext) = nullptr;
+  CUresult (*pop)(CUcontext*) = nullptr;
+  CUresult (*device)(CUdevice*) = nullptr;
+  bool known = false;
+  template <typename F>
+  static bool find(const char* name, F* fn) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    // (by the version that introduced this form: newer ones of the same name take more arguments)
+    const bool ok = cudaGetDriverEntryPointByVersion(name, &p, 9020, cudaEnableDefault, &q) == cudaSuccess &&
+                    q == cudaDriverEntryPointSuccess && p != nullptr;
+    *fn = ok ? reinterpret_cast<F>(p) : nullptr;
+    return ok;
+  }
+  DriverContexts() {
+    known = find("cuStreamGetCtx", &of_stream) && find("cuCtxGetCurrent", &current) && find("cuCtxPushCurrent", &push) &&
+            find("cuCtxPopCurrent", &pop) && find("cuCtxGetDevice", &device);
+    (void)cudaGetLastError();
+  }
+};
+
+// The stream's device by way of its context: cudaStreamGetDevice refuses a stream that is being captured into a
+// graph, and the refusal invalidates the capture.
+bool device_by_context(cudaStream_t st, int* dev) {
+  static const DriverContexts d;
+  CUcontext of = nullptr, cur = nullptr;
+  if (!d.known || d.of_stream(st, &of) != CUDA_SUCCESS || of == nullptr || d.current(&cur) != CUDA_SUCCESS) return false;
+  if (of == cur) return cudaGetDevice(dev) == cudaSuccess;
+  CUdevice cd = -1;
+  if (d.push(of) != CUDA_SUCCESS) return false;
+  const bool ok = d.device(&cd) == CUDA_SUCCESS;
+  d.pop(&of);
+  *dev = cd;
+  return ok;
+}
 cudaError_t h_stream_device(cudaStream_t st, int* dev) {
   cudaError_t c;
   if (injected(kCallStreamDevice, &c)) return c;
   if (fake()) { *dev = 0; return cudaSuccess; }
+  if (device_by_context(st, dev)) return cudaSuccess;
 #if CUDART_VERSION >= 12080
   return cudaStreamGetDevice(st, dev);
 #else
