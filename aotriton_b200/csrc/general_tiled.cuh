@@ -90,31 +90,55 @@ __device__ __forceinline__ void tile_dots(float (&s)[4][Tiled<DP>::kNC], const f
   }
 }
 
-// acc[i][j] += P[ty*4 + i][0..BN) x X[0..BN)[tx*4 + 64 j ..]
+// The part [k0, k1) of the block of BN columns at `col0` that some row of the warp's eight sees (columns lo..hi), k0
+// rounded down to eight.  The accumulations stop there.  A masked pair's weight is zero, but zero times a non-finite row
+// of X is not: a row must not depend on rows that neither it nor its neighbours in the warp see.  (The 16x16-tile
+// kernels keep the same distance with their tiles.)
 template <int DP>
-__device__ __forceinline__ void tile_accumulate(float4 (&acc)[4][Tiled<DP>::kND], const float* P, const float* X, int ty, int tx) {
+__device__ __forceinline__ void seen_columns(int lo, int hi, int col0, int& k0, int& k1) {
+  k0 = max(lo - col0, 0) & ~7;
+  k1 = min(hi - col0 + 1, Tiled<DP>::kBN);
+}
+constexpr int kWarpRows = 8;      // rows of a tile whose weights one warp writes and reads
+
+// acc[i][j] += P[ty*4 + i][k..k + 4) x X[k..k + 4)[tx*4 + 64 j ..]
+template <int DP>
+__device__ __forceinline__ void accumulate4(float4 (&acc)[4][Tiled<DP>::kND], const float* p0, const float* x0, int k) {
   using C = Tiled<DP>;
-  const float* p0 = P + ty * 4 * C::kLdP;
-  const float* x0 = X + tx * 4;
-#pragma unroll 2
-  for (int k = 0; k < C::kBN; k += 4) {
-    float4 a[4];
+  float4 a[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(p0 + i * C::kLdP + k);
+  for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(p0 + i * C::kLdP + k);
 #pragma unroll
-    for (int kk = 0; kk < 4; ++kk)
+  for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-      for (int j = 0; j < C::kND; ++j) {
-        const float4 x = *reinterpret_cast<const float4*>(x0 + (k + kk) * C::kLd + 64 * j);
+    for (int j = 0; j < C::kND; ++j) {
+      const float4 x = *reinterpret_cast<const float4*>(x0 + (k + kk) * C::kLd + 64 * j);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float w = kk == 0 ? a[i].x : (kk == 1 ? a[i].y : (kk == 2 ? a[i].z : a[i].w));
-          acc[i][j].x = fmaf(w, x.x, acc[i][j].x);
-          acc[i][j].y = fmaf(w, x.y, acc[i][j].y);
-          acc[i][j].z = fmaf(w, x.z, acc[i][j].z);
-          acc[i][j].w = fmaf(w, x.w, acc[i][j].w);
-        }
+      for (int i = 0; i < 4; ++i) {
+        const float w = kk == 0 ? a[i].x : (kk == 1 ? a[i].y : (kk == 2 ? a[i].z : a[i].w));
+        acc[i][j].x = fmaf(w, x.x, acc[i][j].x);
+        acc[i][j].y = fmaf(w, x.y, acc[i][j].y);
+        acc[i][j].z = fmaf(w, x.z, acc[i][j].z);
+        acc[i][j].w = fmaf(w, x.w, acc[i][j].w);
       }
+    }
+}
+
+// The same over [k0, k1); k0 is a multiple of eight, k1 is rounded up to one.  (Pointers that advance, eight columns an
+// iteration: measured like a loop over the whole block.  Indexed by k, or four columns at a time, the forward took up to
+// 24 % more and the backward up to 4 %.)
+template <int DP>
+__device__ __forceinline__ void tile_accumulate(float4 (&acc)[4][Tiled<DP>::kND], const float* P, const float* X, int k0, int k1, int ty, int tx) {
+  using C = Tiled<DP>;
+  static_assert(C::kBN % 8 == 0, "a rounded-up k1 stays inside the block");
+  const float* p0 = P + ty * 4 * C::kLdP + k0;
+  const float* x0 = X + k0 * C::kLd + tx * 4;
+#pragma unroll 1
+  for (int n = (k1 - k0 + 7) >> 3; n > 0; --n) {
+    accumulate4<DP>(acc, p0, x0, 0);
+    accumulate4<DP>(acc, p0, x0, 4);
+    p0 += 8;
+    x0 += 8 * C::kLd;
   }
 }
 
@@ -186,8 +210,10 @@ __global__ void __launch_bounds__(128) tiled_fwd_kernel(const __grid_constant__ 
 #pragma unroll
     for (int j = 0; j < C::kND; ++j) acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  int n_lo, n_hi;
+  int n_lo, n_hi, w_lo = 1, w_hi = 0;
   key_range(p, sq, m0, min(m0 + C::kBM, sq.sq) - 1, n_lo, n_hi);
+  const int wm = m0 + (threadIdx.x >> 5) * kWarpRows;
+  if (wm < sq.sq) key_range(p, sq, wm, min(wm + kWarpRows, sq.sq) - 1, w_lo, w_hi);
   const int d4 = (p.dqk + 3) >> 2;
   for (int n0 = n_lo / C::kBN * C::kBN; n0 <= n_hi; n0 += C::kBN) {
     __syncthreads();   // the previous block's tiles have been read
@@ -228,7 +254,9 @@ __global__ void __launch_bounds__(128) tiled_fwd_kernel(const __grid_constant__ 
       }
     }
     __syncwarp();
-    tile_accumulate<DP>(acc, Ps, Vs, ty, tx);
+    int k0, k1;
+    seen_columns<DP>(w_lo, w_hi, n0, k0, k1);
+    tile_accumulate<DP>(acc, Ps, Vs, k0, k1, ty, tx);
     __syncwarp();
   }
 #pragma unroll
@@ -265,8 +293,10 @@ __device__ __forceinline__ void tiled_bwd_dkdv(const Params& p, float* smem, int
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < C::kND; ++j) adv[i][j] = adk[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
-  int m_lo, m_hi;
+  int m_lo, m_hi, w_lo = 1, w_hi = 0;
   query_range(p, sq, n0, min(n0 + C::kBM, sq.sk) - 1, m_lo, m_hi);
+  const int wn = n0 + (threadIdx.x >> 5) * kWarpRows;
+  if (wn < sq.sk) query_range(p, sq, wn, min(wn + kWarpRows, sq.sk) - 1, w_lo, w_hi);
   const int dq4 = (p.dqk + 3) >> 2, dv4 = (p.dvo + 3) >> 2;
   for (int g = 0; g < p.group; ++g) {
     const int h = hk * p.group + g;
@@ -309,8 +339,10 @@ __device__ __forceinline__ void tiled_bwd_dkdv(const Params& p, float* smem, int
         }
       }
       __syncwarp();
-      tile_accumulate<DP>(adv, Ps, dOs, ty, tx);
-      tile_accumulate<DP>(adk, dSs, Qs, ty, tx);
+      int k0, k1;
+      seen_columns<DP>(w_lo, w_hi, m0, k0, k1);
+      tile_accumulate<DP>(adv, Ps, dOs, k0, k1, ty, tx);
+      tile_accumulate<DP>(adk, dSs, Qs, k0, k1, ty, tx);
       __syncwarp();
     }
   }
@@ -351,8 +383,10 @@ __device__ __forceinline__ void tiled_bwd_dq(const Params& p, float* smem, int z
 #pragma unroll
     for (int j = 0; j < C::kND; ++j) adq[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  int n_lo, n_hi;
+  int n_lo, n_hi, w_lo = 1, w_hi = 0;
   key_range(p, sq, m0, min(m0 + C::kBM, sq.sq) - 1, n_lo, n_hi);
+  const int wm = m0 + (threadIdx.x >> 5) * kWarpRows;
+  if (wm < sq.sq) key_range(p, sq, wm, min(wm + kWarpRows, sq.sq) - 1, w_lo, w_hi);
   if (n_hi >= n_lo) zero_dbias_outside<T>(p, sq, h, m0, C::kBM, n_lo / C::kBN * C::kBN, (n_hi / C::kBN + 1) * C::kBN);
   else zero_dbias_outside<T>(p, sq, h, m0, C::kBM, 0, 0);
   const int dq4 = (p.dqk + 3) >> 2, dv4 = (p.dvo + 3) >> 2;
@@ -387,7 +421,9 @@ __device__ __forceinline__ void tiled_bwd_dq(const Params& p, float* smem, int z
       }
     }
     __syncwarp();
-    tile_accumulate<DP>(adq, dSs, Ks, ty, tx);
+    int k0, k1;
+    seen_columns<DP>(w_lo, w_hi, n0, k0, k1);
+    tile_accumulate<DP>(adq, dSs, Ks, k0, k1, ty, tx);
     __syncwarp();
   }
 #pragma unroll
