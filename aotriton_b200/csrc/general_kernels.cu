@@ -531,9 +531,26 @@ cudaError_t launch_general_T(int which, const Params& p, cudaStream_t st) {
   return e;
 }
 
+// dK/dV and dQ in one launch, or in two.  Together they fill the chip where one alone does not, and share its last
+// wave.  What they lose is occupancy: a CTA of the joint launch asks for the shared memory of dK/dV (77 KB at head dims
+// above 64, two CTAs an SM) where dQ alone has room for three.  16-bit types there lose from 4096 working CTAs on.
+// Measured, whole backward, joint against two launches, us: fp32 2x8x8x500x64 causal 143 / 197, 4x16x16x2048x64 8312 / 9232,
+// 4x8x8x1024x128 2683 / 2997, 4x16x16x2048x128 20174 / 20928; fp16 4x16x16x2048x60 8373 / 9064, 4x8x8x1024x124 2713 / 2957,
+// 4x12x12x1024x124 (3072 CTAs) 4092 / 4129, 4x16x16x1024x124 (4096) 5344 / 5140, 4x16x16x2048x124 20705 / 20357.
+template <typename T, int DP>
+bool joint_backward(const Params& p) {
+  if (sizeof(T) != 2 || DP <= 64) return true;
+  auto blocks = [](int n) { return (int64_t)((n + Tiled<DP>::kBM - 1) / Tiled<DP>::kBM); };
+  return p.batch * (p.hq * blocks(p.max_sq) + p.hk * blocks(p.max_sk)) < 4096;
+}
+
 template <typename T, int DP>
 cudaError_t launch_tiled_T(int which, const Params& p, cudaStream_t st) {
   using C = Tiled<DP>;
+  if (which == 3 && !joint_backward<T, DP>(p)) {
+    const cudaError_t e = launch_tiled_T<T, DP>(1, p, st);
+    return e != cudaSuccess ? e : launch_tiled_T<T, DP>(2, p, st);
+  }
   const size_t rows = which == 0 ? C::kBM + 2 * C::kBN : 2 * C::kBM + 2 * C::kBN;      // staged rows of DP + 4 floats
   const size_t tiles = which & 1 ? 2 : 1;                                              // P and dS, or one of them
   const size_t sm = (rows * C::kLd + tiles * C::kBM * C::kLdP + (which & 1 ? 2 * C::kBN : 0)) * sizeof(float);

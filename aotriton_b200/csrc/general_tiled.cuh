@@ -435,7 +435,7 @@ __device__ __forceinline__ void tiled_bwd_dq(const Params& p, float* smem, int z
 
 // The backward.  WHICH 1: dK / dV, grid = (cdiv(max_sk, 32), Hk, batch).  2: dQ (+ dBias), grid = (cdiv(max_sq, 32),
 // Hq, batch), last rows first.  3: both in one launch, x alternating between the two (neither reads what the other
-// writes).  At the sizes single precision is used at, each of the two alone leaves most of the chip idle: 2 x 8
+// writes); joint_backward() says when.  At the sizes single precision is used at, each of the two alone leaves most of the chip idle: 2 x 8
 // heads x 500 tokens are 256 CTAs of four warps, 7 warps an SM, waiting for their own loads and barriers.
 // Measured there (fp32, head dim 64, causal): the whole training step 273 -> 213 us, together with a shorter host path.
 template <typename T, int DP, int WHICH>

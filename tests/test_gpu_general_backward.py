@@ -24,9 +24,12 @@ def test_equal_to_separate_stages(B, Hq, Hk, Sq, Sk, D, bias, in_place):
     def backward(dq, do, *stages):
         dk, dv, db = torch.full_like(k, float("nan")), torch.full_like(v, float("nan")), torch.full_like(b, float("nan")) if bias else None
         delta = torch.empty_like(lse)
+        n0 = cabi.lib().ab200_launch_count()
         for stage in stages:
             assert cabi.attn_bwd(q, k, v, out, do, dq, dk, dv, lse, delta, dbias=db, stage=stage, **kw) == 0
         assert cabi.lib().ab200_last_bwd_family() == 1
+        one = stages == ("all",) and D <= 128 and dq.data_ptr() != do.data_ptr()
+        assert cabi.lib().ab200_launch_count() - n0 == (2 if one else 3)
         return [dq, dk, dv] + ([db] if bias else [])
 
     want = backward(torch.full_like(q, float("nan")), do, "preprocess", "dkdv", "dq")
