@@ -675,9 +675,20 @@ int ab200_attn_bwd(const ab200_attn_bwd_args* a, void* stream) {
   return run_dq(a, stream, true);
 }
 
+// Whether ab200_attn_bwd would run the two-kernel tcgen05 backward, the device apart: 1, 0, or a negative error.
+static int two_kernel_bwd(const ab200_attn_bwd_args* a, const Params& p) {
+  const bool fused = a->dq_acc != nullptr && !a->deterministic && want_fused(g_family);
+  const int sel = ab200_select_variant(kOpBwd, a->prob.dtype, p.dqk, p.dvo,
+                                       family_flags(g_family) | (sm100_bwd_shape(a->prob.dtype, p) ? AB200_SELECT_ALIGNED : 0) |
+                                           (fused ? AB200_SELECT_FUSED_REQUESTED : 0) | (p.has_dbias ? AB200_SELECT_DBIAS : 0));
+  return sel < 0 ? sel : (sel & 0xff) == kVarTcgen05;
+}
+
 int ab200_debug_keep_tiles(const ab200_attn_bwd_args* a) {
   Params p{};
   if (int e = fill_bwd(a, p, true)) return -e;
+  const int tc = two_kernel_bwd(a, p);
+  if (tc <= 0) return tc;
   keep_share_setup(p);
   return p.keep_tiles;
 }

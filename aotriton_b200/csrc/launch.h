@@ -74,9 +74,10 @@ cudaError_t launch_dropout_sign(int dtype, const View4& r, int batch, int heads,
                                 const uint64_t* seed, const uint64_t* off1, uint64_t off2, cudaStream_t st);
 
 // tcgen05 kernels (sm100_fwd.cu / sm100_bwd.cu).  *_supported say whether the shape is
-// inside the kernel's range; the launchers assume it is.
+// inside the kernel's range (and tile maps can be encoded here); the launchers assume it is.  *_shape: the shape alone.
 bool sm100_fwd_supported(int dtype, const Params& p);
 cudaError_t launch_sm100_fwd(int dtype, const Params& p, cudaStream_t st);
+bool sm100_bwd_shape(int dtype, const Params& p);
 bool sm100_bwd_supported(int dtype, const Params& p);
 cudaError_t launch_sm100_bwd_dkdv(int dtype, const Params& p, cudaStream_t st);
 cudaError_t launch_sm100_bwd_dq(int dtype, const Params& p, cudaStream_t st);

@@ -1461,7 +1461,7 @@ cudaError_t launch_bwd(int which, int dtype, const Params& p, cudaStream_t st, f
 
 }  // namespace
 
-bool sm100_bwd_supported(int dtype, const Params& p) {
+bool sm100_bwd_shape(int dtype, const Params& p) {
   if (dtype != 2 && dtype != 3) return false;
   if (p.dqk > 256 || p.dvo > 256 || p.dqk % 8 != 0 || p.dvo % 8 != 0) return false;
   if (p.max_sq <= 0 || p.max_sk <= 0 || p.batch <= 0) return false;
@@ -1471,8 +1471,9 @@ bool sm100_bwd_supported(int dtype, const Params& p) {
   if (p.dq.ptr && !vector_store_friendly(p.dq)) return false;
   if (p.dk.ptr && !vector_store_friendly(p.dk)) return false;
   if (p.dv.ptr && !vector_store_friendly(p.dv)) return false;
-  return host().have_encoder();
+  return true;
 }
+bool sm100_bwd_supported(int dtype, const Params& p) { return sm100_bwd_shape(dtype, p) && host().have_encoder(); }
 
 cudaError_t launch_sm100_bwd_dkdv(int dtype, const Params& p, cudaStream_t st) { return launch_bwd(1, dtype, p, st, nullptr); }
 cudaError_t launch_sm100_bwd_dq(int dtype, const Params& p, cudaStream_t st) { return launch_bwd(2, dtype, p, st, nullptr); }

@@ -55,6 +55,37 @@ def test_rule():
     assert _keep_tiles(q, k, v, mk(2, 4, 300, 132)[..., :128]) == 0           # rows off a 16-byte boundary
 
 
+def test_rule_follows_the_kernels_that_run():
+    """No bits are handed on where the general kernels or the fused backward take the call."""
+    from aotriton_b200 import cabi
+    L = cabi.lib()
+
+    def ask(dt, d, dq_acc=None, family=0, **kw):
+        mk = lambda h: torch.empty(2, h, 300, d, dtype=dt)
+        q, k, v, out, do, dq, dk, dv = mk(4), mk(2), mk(2), mk(4), mk(4), mk(4), mk(2), mk(2)
+        lse = torch.empty(8, 300)
+        a = cabi.make_bwd_args(q, k, v, out, do, dq, dk, dv, lse, torch.empty_like(lse), sm_scale=1.0, dropout_p=0.1, **kw)
+        if dq_acc:
+            a.dq_acc = lse.data_ptr()
+        old = L.ab200_set_kernel_family(family)
+        try:
+            return L.ab200_debug_keep_tiles(C.byref(a))
+        finally:
+            L.ab200_set_kernel_family(old)
+
+    h = torch.bfloat16
+    assert ask(h, 128) == 10 and ask(h, 128, family=2) == 10
+    assert ask(torch.float32, 128) == 0                              # general kernels: single precision,
+    assert ask(h, 100) == 0 and ask(h, 264) == 0                     # head dims outside the tcgen05 kernels',
+    assert ask(h, 128, family=1) == 0                                # or by force
+    assert ask(h, 100, family=2) == -801                             # refused
+    assert ask(h, 128, dq_acc=True, family=3) == 0                   # fused
+    assert ask(h, 128, dq_acc=True, family=3, deterministic=True) == 10
+    assert ask(h, 128, dq_acc=True) == 10 and ask(h, 128, family=3) == 10
+    assert ask(h, 64, dq_acc=True, family=3) == 10                   # no fused form for 64 and above 128
+    assert ask(h, 256, dq_acc=True, family=3) == 10
+
+
 CASES = [
     # B, Hq, Hk, Sq, Sk, D, causal (type, left, right), bias, packed lengths
     (2, 4, 4, 128, 128, 64, (0, 0, 0), False, None),
