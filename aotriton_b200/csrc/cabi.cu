@@ -478,7 +478,7 @@ uint64_t ab200_debug_host_call_count(int call) {
 }
 
 void ab200_debug_bounded_wait_test(int drop_copy, unsigned int wait_limit_kcycles) {
-  t_drop_copy = (drop_copy >= 0 && drop_copy <= 3) ? drop_copy : 0;
+  t_drop_copy = (drop_copy >= 0 && drop_copy <= 4) ? drop_copy : 0;
   t_wait_limit_kcycles = wait_limit_kcycles;
 }
 uint64_t ab200_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }

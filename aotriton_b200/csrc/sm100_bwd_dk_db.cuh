@@ -83,6 +83,7 @@ sm100_bwd_dk_db_kernel(const __grid_constant__ Params p, const __grid_constant__
         const int h = hk * p.group + hg, row = (mb_lo + mb) * L::kRows;
         if (++mb == nmb) { mb = 0; ++hg; }
         if (!mbar_wait(&bars[L::bEmpty + s], ((uint32_t)(i / L::kStages) & 1u) ^ 1u, abort_flag, status, 0x4000)) break;
+        if (p.drop_copy == 4 && i == 0) continue;      // (test hook: the first stage never arrives)
         uint8_t* a = smem + s * L::kStage;
         mbar_expect_tx(&bars[L::bFull + s], L::kA + qboxes * L::kBox);
         for (int b = 0; b < 2; ++b) tma_load_4d(a + b * L::kBox, &tm_db, &bars[L::bFull + s], n0 + b * 64, row, h, sq.bidx);
@@ -91,7 +92,7 @@ sm100_bwd_dk_db_kernel(const __grid_constant__ Params p, const __grid_constant__
         issued = i + 1;
       }
       if (*abort_flag) {      // copies still in flight land before the CTA gives its shared memory back
-        for (int i = max(0, issued - L::kStages); i < issued; ++i)
+        for (int i = max(p.drop_copy == 4 ? 1 : 0, issued - L::kStages); i < issued; ++i)
           mbar_wait_quiet(&bars[L::bFull + i % L::kStages], (uint32_t)(i / L::kStages) & 1u, abort_flag);
       }
     }

@@ -400,22 +400,17 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
       if (drop_on) {
         const int r = (warp & 3) * 32 + lane;
         const DropoutCtx dctx = dropout_ctx(p, z, h);
-        bool ok = true;
-        for (int j = 0; ok && j < nblk; ++j) {
-          {
-            const int buf = j & 1;
-            if (!mbar_wait_relaxed(&bars[L::bKeepEmpty + buf], ((uint32_t)(j >> 1) & 1u) ^ 1u, abort_flag, status, 0xA00 + j)) {
-              ok = false;
-              break;
-            }
-            const int mm = min(m0 + r, p.max_sq - 1);
-            const uint64_t offset = dctx.base + (uint64_t)mm * dctx.stride + (uint64_t)((jb_lo + j) * (kBN / 4));
-            uint32_t* dst = reinterpret_cast<uint32_t*>(smem + L::kKeep + buf * L::kKeepTile) + r * 4;
+        for (int j = 0; j < nblk; ++j) {
+          const int buf = j & 1;
+          if (!__all_sync(0xffffffffu, mbar_wait_relaxed(&bars[L::bKeepEmpty + buf], ((uint32_t)(j >> 1) & 1u) ^ 1u, abort_flag, status, 0xA00 + j)))
+            break;
+          const int mm = min(m0 + r, p.max_sq - 1);
+          const uint64_t offset = dctx.base + (uint64_t)mm * dctx.stride + (uint64_t)((jb_lo + j) * (kBN / 4));
+          uint32_t* dst = reinterpret_cast<uint32_t*>(smem + L::kKeep + buf * L::kKeepTile) + r * 4;
 #pragma unroll 1
-            for (int u = 0; u < 4; ++u) dst[u] = draw_keep_word(dctx.seed, offset + (uint64_t)(8 * u), dctx.threshold);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars[L::bKeepFull + buf]);
-          }
+          for (int u = 0; u < 4; ++u) dst[u] = draw_keep_word(dctx.seed, offset + (uint64_t)(8 * u), dctx.threshold);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars[L::bKeepFull + buf]);
         }
       }
     }

@@ -17,6 +17,9 @@
 // The products are 16 rows high, where the 128-row tensor-memory MMA would compute padding and add its
 // read-out latency to every tile: they run as warp-level m16n8k16 MMAs from registers and ldmatrix.
 //
+// Every wait inside a CTA is bounded.  A CTA whose wait ran out, or that starts after a failure, still takes both
+// cluster barriers, so its peers do not wait for it.
+//
 // Arithmetic as in the tile kernel: scores scaled by sm_scale*log2(e) in fp32, masked scores -inf, P cast to
 // the value type before P V, fp32 sums, rows without a key give O = 0, LSE = +inf.
 
@@ -140,8 +143,8 @@ sm100_fwd_decode_kernel(const __grid_constant__ Params p, const __grid_constant_
       int issued = 0;
       for (int i = 0, s = 0, ph = 1; i < n; ++i) {      // s, ph: ring stage and the parity that frees it
         const int krow = (int)(sq.k0 + (int64_t)(t_lo + first + i) * kDecKeys);
-        if (!mbar_wait(&bars[L::bEmpty + s], (uint32_t)ph, abort_flag, status, 0xA00)) break;
-        if (!(p.drop_copy == 1 && i == 0)) {      // (test hook: the first tile never arrives)
+        if (!mbar_wait(&bars[L::bEmpty + s], (uint32_t)ph, abort_flag, status, 0x5000)) break;
+        if (!(p.drop_copy == 1 && i == 0 && rank == 0)) {      // (test hook: the cluster's first tile never arrives)
           uint8_t* kt = smem + L::kRing + s * (2 * L::kTile);
           mbar_expect_tx(&bars[L::bFull + s], 2 * L::kTile);
           for (int b = 0; b < kBoxes; ++b)
@@ -153,7 +156,7 @@ sm100_fwd_decode_kernel(const __grid_constant__ Params p, const __grid_constant_
         if (++s == stages) { s = 0; ph ^= 1; }
       }
       if (*abort_flag) {      // let copies that are still in flight land before the memory is used again
-        for (int i = max(p.drop_copy == 1 ? 1 : 0, issued - stages); i < issued; ++i)
+        for (int i = max(p.drop_copy == 1 && rank == 0 ? 1 : 0, issued - stages); i < issued; ++i)
           mbar_wait_quiet(&bars[L::bFull + i % stages], (uint32_t)(i / stages) & 1u, abort_flag);
       }
     }
@@ -209,7 +212,7 @@ sm100_fwd_decode_kernel(const __grid_constant__ Params p, const __grid_constant_
     const int krow = (warp & 3) * 16 + (lane & 7) + ((lane >> 4) << 3), kchunk = (lane >> 3) & 1;
     const int vrow = (warp & 3) * 16 + (lane & 7) + (((lane >> 3) & 1) << 3), vchunk = lane >> 4;
     for (int i = warp >> 2, s = warp >> 2, ph = 0; i < n; i += W / 4) {
-      if (!__all_sync(0xffffffffu, mbar_wait(&bars[L::bFull + s], (uint32_t)ph, abort_flag, status, 0xA10))) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(&bars[L::bFull + s], (uint32_t)ph, abort_flag, status, 0x5100))) break;
       const int key0 = (t_lo + first + i) * kDecKeys + (warp & 3) * 16;      // first key of this warp's 16
       const uint32_t kt = smem_s + L::kRing + s * (2 * L::kTile) + krow * 128;
       const uint32_t vt = smem_s + L::kRing + s * (2 * L::kTile) + L::kTile + vrow * 128;

@@ -248,9 +248,13 @@ AB200_API int ab200_stream_check(void* stream);
  * wait (units of 1024 SM cycles, 0 = the default of about a second) and `drop_copy` makes
  * the producer leave out one tile copy (1 = the forward's first V block, 2 = the dK/dV
  * kernel's first Q/dO block, 3 = the dQ kernel's first V block, 0 = none; for head dims above
- * 128: 2 = the first block's Q of the dV and dO of the dK kernel, 3 = its V), so that a wait
- * runs out, the kernel records which one and returns normally.  Nothing faults or hangs:
- * the kernel takes a few limits to drain.  Call with (0, 0) to restore normal operation. */
+ * 128: 2 = the first block's Q of the dV and dO of the dK kernel, 3 = its V, 4 = the first stage of
+ * dK formed from dBias; few queries: 1 = the first tile of each cluster of the split-key forward),
+ * so that a wait runs out, the kernel records which one and returns normally.  Nothing faults or hangs:
+ * the kernel takes a few limits to drain.  Call with (0, 0) to restore normal operation.
+ * The word ab200_kernel_status returns names the kernel: 0x100 to 0xFFF forward, 0x1xxx dK/dV, 0x2xxx
+ * dQ, 0x3xxx the wide kernels, 0x4xxx dK from dBias, 0x5xxx the split-key forward.  (Some waits add the
+ * number of their block, which in sequences beyond 100000 tokens runs into the next range.) */
 AB200_API void ab200_debug_bounded_wait_test(int drop_copy, unsigned int wait_limit_kcycles);
 
 /* Number of 32-key tiles whose dropout keep bits ab200_attn_bwd hands from the dK/dV kernel to the dQ kernel
