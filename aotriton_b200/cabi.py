@@ -25,6 +25,7 @@ SYMBOLS = [
     "ab200_debug_simulate_encoded_softmax", "ab200_check_gpu", "ab200_multiprocessor_count",
     "ab200_set_kernel_family", "ab200_select_variant", "ab200_last_fwd_family", "ab200_last_bwd_family",
     "ab200_kernel_status", "ab200_stream_check", "ab200_debug_bounded_wait_test", "ab200_debug_keep_tiles",
+    "ab200_debug_dk_from_dbias", "ab200_debug_split_keys",
     "ab200_debug_host_calls", "ab200_debug_host_call_count", "ab200_launch_count", "ab200_version",
 ]
 
@@ -90,7 +91,8 @@ def lib() -> C.CDLL:
         L.ab200_stream_check.argtypes = [C.c_void_p]
         L.ab200_debug_bounded_wait_test.argtypes = [C.c_int, C.c_uint]
         L.ab200_debug_bounded_wait_test.restype = None
-        L.ab200_debug_keep_tiles.argtypes = [C.POINTER(BwdArgs)]
+        L.ab200_debug_keep_tiles.argtypes = L.ab200_debug_dk_from_dbias.argtypes = [C.POINTER(BwdArgs)]
+        L.ab200_debug_split_keys.argtypes = [C.POINTER(FwdArgs), C.c_void_p]
         L.ab200_debug_host_calls.argtypes = [C.c_int] * 4
         L.ab200_debug_host_calls.restype = None
         L.ab200_debug_host_call_count.argtypes = [C.c_int]
@@ -153,8 +155,8 @@ def make_problem(q, k, v, *, sm_scale, causal_type=0, window_left=0, window_righ
     return p
 
 
-def attn_fwd(q, k, v, out, lse, *, bias=None, philox_seed_output=None, philox_offset_output=None,
-             encoded_softmax=None, stream=None, **problem) -> int:
+def make_fwd_args(q, k, v, out, lse, *, bias=None, philox_seed_output=None, philox_offset_output=None,
+                  encoded_softmax=None, **problem) -> FwdArgs:
     a = FwdArgs()
     a.prob = make_problem(q, k, v, **problem)
     a.q, a.k, a.v, a.bias, a.out = view4(q), view4(k), view4(v), view4(bias), view4(out)
@@ -163,6 +165,11 @@ def attn_fwd(q, k, v, out, lse, *, bias=None, philox_seed_output=None, philox_of
     a.encoded_softmax = view4(encoded_softmax)
     if encoded_softmax is not None:
         a.encoded_softmax_rows, a.encoded_softmax_cols = encoded_softmax.shape[2], encoded_softmax.shape[3]
+    return a
+
+
+def attn_fwd(q, k, v, out, lse, *, stream=None, **kw) -> int:
+    a = make_fwd_args(q, k, v, out, lse, **kw)
     return lib().ab200_attn_fwd(C.byref(a), stream if stream is not None else current_stream_handle())
 
 

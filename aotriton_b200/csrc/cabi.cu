@@ -496,25 +496,31 @@ int ab200_debug_simulate_encoded_softmax(const ab200_view4* r, int32_t dtype, in
                                   philox_offset1, philox_offset2, st);
 }
 
-int ab200_attn_fwd(const ab200_attn_fwd_args* a, void* stream) {
+static int fill_fwd(const ab200_attn_fwd_args* a, Params& p) {
   if (a == nullptr) return kErrInvalidValue;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  Params p{};
   if (int e = fill_common(a->prob, p)) return e;
   if (!a->q.ptr || !a->k.ptr || !a->v.ptr || !a->out.ptr) return kErrInvalidValue;
   if (!inner_contiguous(a->q) || !inner_contiguous(a->k) || !inner_contiguous(a->v) || !inner_contiguous(a->out))
     return kErrInvalidValue;
-  if (int e = check_device(st)) return e;
-  DeviceGuard guard(st);
   p.q = to_view(a->q); p.k = to_view(a->k); p.v = to_view(a->v); p.out = to_view(a->out);
   p.bias = to_view(a->bias); p.has_bias = a->bias.ptr != nullptr; p.bias_vec = rows_16byte(a->bias.ptr, a->bias.stride);
   p.lse = a->lse;
   p.seed_out = a->philox_seed_output; p.off_out = a->philox_offset_output;
+  return 0;
+}
+static int select_fwd(const ab200_attn_fwd_args* a, const Params& p) {
+  return ab200_select_variant(kOpFwd, a->prob.dtype, p.dqk, p.dvo,
+                              family_flags(g_family) | (sm100_fwd_supported(a->prob.dtype, p) ? AB200_SELECT_ALIGNED : 0));
+}
 
-  const int family = g_family;
+int ab200_attn_fwd(const ab200_attn_fwd_args* a, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  Params p{};
+  if (int e = fill_fwd(a, p)) return e;
+  if (int e = check_device(st)) return e;
+  DeviceGuard guard(st);
   cudaError_t err;
-  const int sel = ab200_select_variant(kOpFwd, a->prob.dtype, p.dqk, p.dvo,
-                                       family_flags(family) | (sm100_fwd_supported(a->prob.dtype, p) ? AB200_SELECT_ALIGNED : 0));
+  const int sel = select_fwd(a, p);
   if (sel < 0) return -sel;
   if ((sel & 0xff) >= kVarTcgen05) {
     err = launch_sm100_fwd(a->prob.dtype, p, st);
@@ -532,6 +538,16 @@ int ab200_attn_fwd(const ab200_attn_fwd_args* a, void* stream) {
                               p.off1_ptr, p.off2, st);
   }
   return (int)err;
+}
+
+int ab200_debug_split_keys(const ab200_attn_fwd_args* a, void* stream) {
+  Params p{};
+  if (int e = fill_fwd(a, p)) return -e;
+  const int sel = select_fwd(a, p);
+  SplitPlan s;
+  if (sel < 0) return sel;
+  if ((sel & 0xff) < kVarTcgen05 || !sm100_fwd_split(p, ab200_multiprocessor_count(stream), &s)) return 0;
+  return s.pieces | s.warps << 8 | s.stages << 16;
 }
 
 static int fill_bwd(const ab200_attn_bwd_args* a, Params& p, bool need_outputs) {
@@ -691,6 +707,13 @@ int ab200_debug_keep_tiles(const ab200_attn_bwd_args* a) {
   if (tc <= 0) return tc;
   keep_share_setup(p);
   return p.keep_tiles;
+}
+
+int ab200_debug_dk_from_dbias(const ab200_attn_bwd_args* a) {
+  Params p{};
+  if (int e = fill_bwd(a, p, true)) return -e;
+  const int tc = two_kernel_bwd(a, p);
+  return tc <= 0 ? tc : dk_from_db_possible(p);
 }
 
 // --- backward with the delta scratch inside the library image -----------------------------

@@ -77,6 +77,9 @@ cudaError_t launch_dropout_sign(int dtype, const View4& r, int batch, int heads,
 // inside the kernel's range (and tile maps can be encoded here); the launchers assume it is.  *_shape: the shape alone.
 bool sm100_fwd_supported(int dtype, const Params& p);
 cudaError_t launch_sm100_fwd(int dtype, const Params& p, cudaStream_t st);
+// Whether the split-key kernel takes a forward that the tcgen05 family runs, and how it cuts it.
+struct SplitPlan { int pieces, warps, stages, chunks; };
+bool sm100_fwd_split(const Params& p, int sms, SplitPlan* plan);
 bool sm100_bwd_shape(int dtype, const Params& p);
 bool sm100_bwd_supported(int dtype, const Params& p);
 cudaError_t launch_sm100_bwd_dkdv(int dtype, const Params& p, cudaStream_t st);

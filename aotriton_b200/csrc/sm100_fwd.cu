@@ -780,6 +780,12 @@ bool sm100_fwd_supported(int dtype, const Params& p) {
   return host().have_encoder();
 }
 
+bool sm100_fwd_split(const Params& p, int sms, SplitPlan* plan) {
+  if (!decode_shape(p)) return false;
+  *plan = with_decode_tile(p, [&]<int HD, int MT>() { return split_plan<HD, MT>(p, sms); });
+  return true;
+}
+
 cudaError_t launch_sm100_fwd(int dtype, const Params& p, cudaStream_t st) {
   if (decode_shape(p)) return dtype == 2 ? launch_decode_T<__half>(p, st) : launch_decode_T<__nv_bfloat16>(p, st);
   const int dmax = p.dqk > p.dvo ? p.dqk : p.dvo;

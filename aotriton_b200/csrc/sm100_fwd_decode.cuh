@@ -407,9 +407,29 @@ cudaError_t launch_decode_CS(const Params& p, int chunks, const CUtensorMap& tk,
   return e;
 }
 
+// How a call is cut: pieces of the keys (CTAs of a cluster), consumer warps of a CTA, ring stages, row chunks.
+template <int HD, int MT>
+SplitPlan split_plan(const Params& p, int sms) {
+  using L = DecSmem<HD, MT, 4>;
+  const int chunks = (p.group * p.max_sq + L::kRows - 1) / L::kRows;
+  const int64_t clusters = (int64_t)p.hk * chunks * p.batch;
+  const int tiles = (p.max_sk + kDecKeys - 1) / kDecKeys;
+  // Cut the keys until the CTAs fill the chip once or a piece would fall below two tiles.  (More pieces than
+  // that only add CTAs that wait for a slot: 2 x 8192 keys, 64:8 heads, 5 queries: 37 us with 4 pieces, 58 us with 8.)
+  // The rule counts SMs; a cluster of eight also needs its SMs in one GPC, so a few counts just below the line leave
+  // clusters for a second round (6007 keys, 8 heads of 128 per kv head: 15 clusters 12.4 us, 16 to 18 21 us, 19, with
+  // four pieces, 16.5; 32 clusters 17.1, 34 to 37 30).
+  int cs = 1;
+  while (cs < 8 && clusters * cs * 2 <= (int64_t)L::kCtasPerSm * sms && tiles >= 4 * cs) cs *= 2;
+  // With no more CTAs than SMs each gets the whole ring, and eight warps if its rows fit one tile: four warps
+  // spend 1100 clocks on a tile of 64 keys, which is less than a CTA alone on its SM could be fed
+  // (32768 keys, 32:8 heads of 128: 31 us with eight warps, 41 us with four).
+  const bool alone = clusters * cs <= sms;
+  return {cs, MT == 1 && alone && cs == 8 ? 8 : 4, alone ? L::kMaxStages : L::kMaxStages / L::kCtasPerSm, chunks};
+}
+
 template <typename T, int HD, int MT>
 cudaError_t launch_decode_MT(const Params& p, cudaStream_t st) {
-  using L = DecSmem<HD, MT, 4>;
   CUtensorMap tk, tv;
   if (!make_tile_map_16bit(&tk, p.k, p.dqk, p.k.n[2], kDecKeys) || !make_tile_map_16bit(&tv, p.v, p.dvo, p.v.n[2], kDecKeys))
     return cudaErrorInvalidValue;
@@ -418,27 +438,15 @@ cudaError_t launch_decode_MT(const Params& p, cudaStream_t st) {
   bool remember = false;
   cudaError_t e = fwd_device_facts(&dev, &status, &sms, &remember);
   if (e != cudaSuccess) return e;
-  const int chunks = (p.group * p.max_sq + L::kRows - 1) / L::kRows;
-  const int64_t clusters = (int64_t)p.hk * chunks * p.batch;
-  const int tiles = (p.max_sk + kDecKeys - 1) / kDecKeys;
-  // Cut the keys until the CTAs fill the chip once or a piece would fall below two tiles.  (More pieces than
-  // that only add CTAs that wait for a slot: 2 x 8192 keys, 64:8 heads, 5 queries: 37 us with 4 pieces, 58 us with 8.)
-  int cs = 1;
-  while (cs < 8 && clusters * cs * 2 <= (int64_t)L::kCtasPerSm * sms && tiles >= 4 * cs) cs *= 2;
-  // With no more CTAs than SMs each gets the whole ring, and eight warps if its rows fit one tile: four warps
-  // spend 1100 clocks on a tile of 64 keys, which is less than a CTA alone on its SM could be fed
-  // (32768 keys, 32:8 heads of 128: 31 us with eight warps, 41 us with four).
-  const bool alone = clusters * cs <= sms;
+  const SplitPlan s = split_plan<HD, MT>(p, sms);
   if constexpr (MT == 1) {
-    if (alone && cs == 8)
-      return launch_decode_CS<T, HD, 1, 8, 8>(p, chunks, tk, tv, status, dev, remember, L::kMaxStages, st);
+    if (s.warps == 8) return launch_decode_CS<T, HD, 1, 8, 8>(p, s.chunks, tk, tv, status, dev, remember, s.stages, st);
   }
-  const int stages = alone ? L::kMaxStages : L::kMaxStages / L::kCtasPerSm;
-  switch (cs) {
-    case 1: return launch_decode_CS<T, HD, MT, 1, 4>(p, chunks, tk, tv, status, dev, remember, stages, st);
-    case 2: return launch_decode_CS<T, HD, MT, 2, 4>(p, chunks, tk, tv, status, dev, remember, stages, st);
-    case 4: return launch_decode_CS<T, HD, MT, 4, 4>(p, chunks, tk, tv, status, dev, remember, stages, st);
-    default: return launch_decode_CS<T, HD, MT, 8, 4>(p, chunks, tk, tv, status, dev, remember, stages, st);
+  switch (s.pieces) {
+    case 1: return launch_decode_CS<T, HD, MT, 1, 4>(p, s.chunks, tk, tv, status, dev, remember, s.stages, st);
+    case 2: return launch_decode_CS<T, HD, MT, 2, 4>(p, s.chunks, tk, tv, status, dev, remember, s.stages, st);
+    case 4: return launch_decode_CS<T, HD, MT, 4, 4>(p, s.chunks, tk, tv, status, dev, remember, s.stages, st);
+    default: return launch_decode_CS<T, HD, MT, 8, 4>(p, s.chunks, tk, tv, status, dev, remember, s.stages, st);
   }
 }
 
@@ -446,9 +454,15 @@ inline bool decode_shape(const Params& p) {
   return p.max_sq <= kDecodeMaxQueries && p.dqk <= 128 && p.dvo <= 128 && !p.has_bias && !p.dropout_on;
 }
 
+// f<HD, MT>() of the instantiation that takes the call
+template <typename F>
+auto with_decode_tile(const Params& p, F f) {
+  const bool small = p.dqk <= 64 && p.dvo <= 64, one = p.group * p.max_sq <= 16;
+  if (small) return one ? f.template operator()<64, 1>() : f.template operator()<64, 2>();
+  return one ? f.template operator()<128, 1>() : f.template operator()<128, 2>();
+}
+
 template <typename T>
 cudaError_t launch_decode_T(const Params& p, cudaStream_t st) {
-  const bool small = p.dqk <= 64 && p.dvo <= 64, one = p.group * p.max_sq <= 16;
-  if (small) return one ? launch_decode_MT<T, 64, 1>(p, st) : launch_decode_MT<T, 64, 2>(p, st);
-  return one ? launch_decode_MT<T, 128, 1>(p, st) : launch_decode_MT<T, 128, 2>(p, st);
+  return with_decode_tile(p, [&]<int HD, int MT>() { return launch_decode_MT<T, HD, MT>(p, st); });
 }

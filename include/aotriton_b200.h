@@ -261,6 +261,14 @@ AB200_API void ab200_debug_bounded_wait_test(int drop_copy, unsigned int wait_li
  * through rows of dQ (0: each draws its own); negative: error.  Launches nothing. */
 AB200_API int ab200_debug_keep_tiles(const ab200_attn_bwd_args* args);
 
+/* 1 when ab200_attn_bwd forms dK from dBias (head dims above 128), 0 when a kernel of its own forms it; negative: error.
+ * Launches nothing. */
+AB200_API int ab200_debug_dk_from_dbias(const ab200_attn_bwd_args* args);
+
+/* How ab200_attn_fwd cuts a call that the split-key kernel takes: pieces of the keys | consumer warps of a CTA << 8 |
+ * ring stages << 16.  0: another kernel takes it; negative: error.  Launches nothing. */
+AB200_API int ab200_debug_split_keys(const ab200_attn_fwd_args* args, void* stream);
+
 /* Test hooks for the host side of the launch path; no counterpart in the reference.  Every CUDA
  * call the library makes on that path goes through one table.  fake_device != 0 makes the table
  * pretend an sm_100 device (148 SMs): device queries answer, symbol look-ups, attribute settings

@@ -5,6 +5,8 @@ dQ in the place of Q.
 The 16-bit dS values and the order of the sums (16 query rows at a time) are the same, so the results are equal
 bit for bit.
 """
+import ctypes as C
+
 import pytest
 import torch
 
@@ -45,10 +47,12 @@ def test_equal_to_separate_stages(B, Hq, Hk, Sq, Sk, D, causal, how, p, dt):
         grads = [dq] + [torch.full_like(t, float("nan")) for t in (k, v)]
         db, delta = torch.full_like(bias, float("nan")), torch.empty_like(lse)
         n0 = cabi.lib().ab200_launch_count()
+        if stages == ("all",):
+            args = cabi.make_bwd_args(q, k, v, out, do, *grads, lse, delta, dbias=db, **kw)
+            assert cabi.lib().ab200_debug_dk_from_dbias(C.byref(args)) == (how in ("", "bshd"))
         for stage in stages:
             assert cabi.attn_bwd(q, k, v, out, do, *grads, lse, delta, dbias=db, stage=stage, **kw) == 0
-        # (preprocess, dQ, and dV and dK in one launch or two)
-        assert cabi.lib().ab200_launch_count() - n0 == (4 if D > 128 or (stages[0] == "all" and how in ("", "bshd")) else 3)
+        assert cabi.lib().ab200_launch_count() - n0 == 4      # preprocess, dV, dQ, and dK by either kernel
         return grads + [db]
 
     nan = torch.full_like(q, float("nan"))
