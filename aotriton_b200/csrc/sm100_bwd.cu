@@ -278,11 +278,12 @@ __device__ __forceinline__ DkdvItem dkdv_item(const Params& p, int w) {
 // HD: every tile is full, so the instantiation carries no tail handling and fixed GEMM shapes (the
 // MMA issuer's loop is latency-critical: even untaken branches and call sites in it cost several
 // per cent of the kernel's time).
-// PLAIN: no dropout, no bias, no bias gradient.  At 96 registers a thread the compute warps' loop spills, and
-// what it keeps for these (Philox round keys, row pointers, strides) is most of it: with them 176 bytes stored in dK/dV
-// and 28 in dQ, without 52 and none.  Measured, forward + backward: dense causal 4 x 32 heads x 4096, head dim 128,
-// 2.85 -> 2.72 ms; 64:8 heads x 16384, window 4096, 8.90 -> 8.48.
-template <typename T, int HD, bool FUSED, bool EXACT, bool PLAIN>
+// FEAT (features()): at 96 registers a thread the compute warps' loop spills, and what dropout and bias keep there
+// (generator state, row pointers, strides) is most of it: at head dim 128 dK/dV stores 156 bytes with dropout, 100 with bias,
+// 52 with neither, dQ 44, 28 and none.  Measured, whole backward, us, dropout's instantiation against the call's own:
+// neither, dense causal 4 x 32 heads x 4096 of 128 1875 -> 1768, 64:8 heads x 16384, window 4096, 6530 -> 6200; bias,
+// 4 x 8 heads x 1024 of 64 131.5 -> 113.1, 4 x 8:2 heads x 1024 of 128 with dBias 228 -> 207.
+template <typename T, int HD, bool FUSED, bool EXACT, int FEAT>
 __global__ void __launch_bounds__(FUSED ? kFusedThreads : kBwdThreads, 1)
 sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm_q,
                       const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -300,8 +301,8 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
   volatile int* sched = reinterpret_cast<volatile int*>(smem + L::kSched);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // (constants where PLAIN: nothing of dropout, bias or its gradient is compiled in)
-  const bool drop_on = !PLAIN && p.dropout_on != 0, bias_on = !PLAIN && p.has_bias != 0;
+  // (constants where FEAT leaves them out: nothing of theirs is compiled in)
+  const bool drop_on = FEAT == kDropout && p.dropout_on != 0, bias_on = FEAT == kBias || (FEAT == kDropout && p.has_bias != 0);
   // An earlier CTA timed out: the whole CTA leaves (one read, one CTA-wide decision).
   if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile unsigned int*>(status) != 0u)) return;
   if ((int)(smem - smem_raw) + L::kUsed > L::kDynamic) {      // the alignment padding did not fit
@@ -787,7 +788,7 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
             mine |= dropout_keep_nibbles<4>(dctx.seed, dctx.threshold, [&](int u) {
                       return dctx.base + (uint64_t)min(mbase + q4 + 4 * (k + u), p.max_sq - 1) * dctx.stride + (uint64_t)(n >> 2);
                     }) << (4 * k);
-          if (drop_on && keep_shared(p, sq, mbase, it.n0 + quarter * 32))
+          if (keep_shared(p, sq, mbase, it.n0 + quarter * 32))
             *keep_share_word(p, sq, h, mbase, it.n0 + quarter * 32, lane) = keep_rows_from_quads(mine, lane);
           keep = 0u;
 #pragma unroll
@@ -951,7 +952,7 @@ struct DqSmem {
 
 // =========================================================================================
 // dQ (+ dBias).  grid = (cdiv(max_sq, 128), Hq, batch)
-template <typename T, int HD, bool EXACT, bool PLAIN>
+template <typename T, int HD, bool EXACT, int FEAT>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm_q,
                     const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -964,8 +965,8 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + L::kAbort);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // (constants where PLAIN: nothing of dropout, bias or its gradient is compiled in)
-  const bool drop_on = !PLAIN && p.dropout_on != 0, bias_on = !PLAIN && p.has_bias != 0, dbias_on = !PLAIN && p.has_dbias != 0;
+  // (constants where FEAT leaves them out: nothing of theirs is compiled in)
+  const bool drop_on = FEAT == kDropout && p.dropout_on != 0, bias_on = FEAT == kBias || (FEAT == kDropout && p.has_bias != 0), dbias_on = FEAT != kPlain && p.has_dbias != 0;
   // Order of the CTAs (the hardware starts them by linear block index): (batch, head) pairs in groups
   // of kHeadGroup, inside a group the query-block index slowest, from the block with the most key
   // blocks of a causal problem to the one with the fewest.  The heavy blocks of a group start
@@ -1380,9 +1381,9 @@ cudaError_t launch_bwd_T(int which, const Params& p, cudaStream_t st, float* dq_
   // make the stream's device, and remembered.
   struct PerDevice { std::atomic<unsigned int*> status{nullptr}, tickets{nullptr}; std::atomic<int> sms{0}; };
   static PerDevice per_device[64];
-  static std::atomic<bool> attr_set[64][10];
+  static std::atomic<bool> attr_set[64][15];
   const bool exact = p.varlen_mode == 0 && p.max_sq % 128 == 0 && p.max_sk % 128 == 0 && p.dqk == HD && p.dvo == HD;
-  const bool plain = !p.dropout_on && !p.has_bias && !p.has_dbias;
+  const int feat = features(p);
   int dev = 0;
   cudaError_t e = host().get_device(&dev);
   if (e != cudaSuccess) return e;
@@ -1405,11 +1406,17 @@ cudaError_t launch_bwd_T(int which, const Params& p, cudaStream_t st, float* dq_
   if (which == 1 || which == 3) {
     const bool fused = which == 3;
     if (fused && HD != 128) return cudaErrorInvalidValue;
-    auto kern_split = plain ? (exact ? sm100_bwd_dkdv_kernel<T, HD, false, true, true> : sm100_bwd_dkdv_kernel<T, HD, false, false, true>)
-                            : (exact ? sm100_bwd_dkdv_kernel<T, HD, false, true, false> : sm100_bwd_dkdv_kernel<T, HD, false, false, false>);
-    auto kern_fused = sm100_bwd_dkdv_kernel<T, 128, true, false, false>;
-    e = fused ? set_smem(2, reinterpret_cast<const void*>(kern_fused), BwdSmem<128>::kDynamic)
-              : set_smem((exact ? 3 : 0) + (plain ? 5 : 0), reinterpret_cast<const void*>(kern_split), L::kDynamic);
+    using Kernel = decltype(&sm100_bwd_dkdv_kernel<T, HD, false, true, kPlain>);
+    static constexpr Kernel kSplit[2][3] = {
+        {sm100_bwd_dkdv_kernel<T, HD, false, false, kPlain>, sm100_bwd_dkdv_kernel<T, HD, false, false, kBias>,
+         sm100_bwd_dkdv_kernel<T, HD, false, false, kDropout>},
+        {sm100_bwd_dkdv_kernel<T, HD, false, true, kPlain>, sm100_bwd_dkdv_kernel<T, HD, false, true, kBias>,
+         sm100_bwd_dkdv_kernel<T, HD, false, true, kDropout>}};
+    static constexpr Kernel kFused[3] = {sm100_bwd_dkdv_kernel<T, 128, true, false, kPlain>, sm100_bwd_dkdv_kernel<T, 128, true, false, kBias>,
+                                         sm100_bwd_dkdv_kernel<T, 128, true, false, kDropout>};
+    const Kernel kern_split = kSplit[exact][feat], kern_fused = kFused[feat];
+    e = fused ? set_smem(12 + feat, reinterpret_cast<const void*>(kern_fused), BwdSmem<128>::kDynamic)
+              : set_smem(2 * feat + exact, reinterpret_cast<const void*>(kern_split), L::kDynamic);
     if (e != cudaSuccess) return e;
     const int nitems = ((p.max_sk + kBlk - 1) / kBlk) * ((p.hk * p.batch + 7) / 8) * 8;
     int sms = pd.sms.load(std::memory_order_acquire);
@@ -1434,9 +1441,12 @@ cudaError_t launch_bwd_T(int which, const Params& p, cudaStream_t st, float* dq_
       e = launch_kernel(kern_split, grid, dim3(kBwdThreads), L::kDynamic, st, p, tq, tk, tv, tdo, status, nitems, ticket,
                         static_cast<float*>(nullptr));
   } else {
-    auto kern_dq = plain ? (exact ? sm100_bwd_dq_kernel<T, HD, true, true> : sm100_bwd_dq_kernel<T, HD, false, true>)
-                         : (exact ? sm100_bwd_dq_kernel<T, HD, true, false> : sm100_bwd_dq_kernel<T, HD, false, false>);
-    e = set_smem((exact ? 4 : 1) + (plain ? 5 : 0), reinterpret_cast<const void*>(kern_dq), DqSmem<HD>::kDynamic);
+    using Kernel = decltype(&sm100_bwd_dq_kernel<T, HD, true, kPlain>);
+    static constexpr Kernel kDq[2][3] = {
+        {sm100_bwd_dq_kernel<T, HD, false, kPlain>, sm100_bwd_dq_kernel<T, HD, false, kBias>, sm100_bwd_dq_kernel<T, HD, false, kDropout>},
+        {sm100_bwd_dq_kernel<T, HD, true, kPlain>, sm100_bwd_dq_kernel<T, HD, true, kBias>, sm100_bwd_dq_kernel<T, HD, true, kDropout>}};
+    const Kernel kern_dq = kDq[exact][feat];
+    e = set_smem(6 + 2 * feat + exact, reinterpret_cast<const void*>(kern_dq), DqSmem<HD>::kDynamic);
     if (e != cudaSuccess) return e;
     dim3 grid((p.max_sq + kBlk - 1) / kBlk, p.hq, p.batch);
     e = launch_kernel(kern_dq, grid, dim3(kBwdThreads), DqSmem<HD>::kDynamic, st, p, tq, tk, tv, tdo, status);

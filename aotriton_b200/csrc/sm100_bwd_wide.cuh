@@ -62,7 +62,7 @@ static __device__ __noinline__ void zero_tail_rows_streamed(uint8_t* tile, int v
 }
 
 // grid = (cdiv(rows, 128), heads, batch): rows/heads are keys/kv heads (dV, dK) or queries/q heads (dQ)
-template <typename T, int MODE, bool PLAIN>
+template <typename T, int MODE, int FEAT>
 __global__ void __launch_bounds__(kWideThreads, 1)
 sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm_r1,
                       const __grid_constant__ CUtensorMap tm_r2, const __grid_constant__ CUtensorMap tm_late,
@@ -84,8 +84,8 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
   volatile uint32_t* aux_flag = reinterpret_cast<volatile uint32_t*>(smem + L::kAuxFlag);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // (constants where PLAIN: nothing of dropout, bias or its gradient is compiled in)
-  const bool drop_on = !PLAIN && p.dropout_on != 0, bias_on = !PLAIN && p.has_bias != 0, dbias_on = !PLAIN && p.has_dbias != 0;
+  // (constants where FEAT leaves them out: nothing of theirs is compiled in)
+  const bool drop_on = FEAT == kDropout && p.dropout_on != 0, bias_on = FEAT == kBias || (FEAT == kDropout && p.has_bias != 0), dbias_on = FEAT != kPlain && p.has_dbias != 0;
   if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile unsigned int*>(status) != 0u)) return;
   if ((int)(smem - smem_raw) + L::kUsed > L::kDynamic) {      // the alignment padding did not fit
     if (threadIdx.x == 0) atomicCAS(status, 0u, 0x3F00u);
@@ -450,7 +450,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
                       return dctx.base + (uint64_t)min(mbase + q4 + 4 * (k + u), p.max_sq - 1) * dctx.stride + (uint64_t)(n >> 2);
                     }) << (4 * k);
           if constexpr (MODE == kWideDV) {
-            if (drop_on && keep_shared(p, sq, mbase, r0 + quarter * 32))
+            if (keep_shared(p, sq, mbase, r0 + quarter * 32))
               *keep_share_word(p, sq, h, mbase, r0 + quarter * 32, lane) = keep_rows_from_quads(mine, lane);
           }
           keep = 0u;
@@ -686,8 +686,8 @@ cudaError_t launch_bwd_wide_T(int which, const Params& p, cudaStream_t st) {
       return cudaErrorInvalidValue;
   }
   static std::atomic<unsigned int*> status_of[64];
-  static std::atomic<bool> attr_set[64][7];
-  const bool plain = !p.dropout_on && !p.has_bias && !p.has_dbias;
+  static std::atomic<bool> attr_set[64][10];
+  const int feat = features(p);
   int dev = 0;
   cudaError_t e = host().get_device(&dev);
   if (e != cudaSuccess) return e;
@@ -704,11 +704,15 @@ cudaError_t launch_bwd_wide_T(int which, const Params& p, cudaStream_t st) {
     if (r == cudaSuccess && !pretend) attr_set[dev][slot].store(true, std::memory_order_release);
     return r;
   };
+  using Kernel = decltype(&sm100_bwd_wide_kernel<T, kWideDV, kPlain>);
+  static constexpr Kernel kKernels[3][3] = {      // [kWide*][features]
+      {sm100_bwd_wide_kernel<T, 0, kPlain>, sm100_bwd_wide_kernel<T, 0, kBias>, sm100_bwd_wide_kernel<T, 0, kDropout>},
+      {sm100_bwd_wide_kernel<T, 1, kPlain>, sm100_bwd_wide_kernel<T, 1, kBias>, sm100_bwd_wide_kernel<T, 1, kDropout>},
+      {sm100_bwd_wide_kernel<T, 2, kPlain>, sm100_bwd_wide_kernel<T, 2, kBias>, sm100_bwd_wide_kernel<T, 2, kDropout>}};
   if (which == 1) {
-    auto kern_dv = plain ? sm100_bwd_wide_kernel<T, kWideDV, true> : sm100_bwd_wide_kernel<T, kWideDV, false>;
-    auto kern_dk = plain ? sm100_bwd_wide_kernel<T, kWideDK, true> : sm100_bwd_wide_kernel<T, kWideDK, false>;
-    if ((e = set_smem(0 + (plain ? 3 : 0), reinterpret_cast<const void*>(kern_dv))) != cudaSuccess) return e;
-    if ((e = set_smem(1 + (plain ? 3 : 0), reinterpret_cast<const void*>(kern_dk))) != cudaSuccess) return e;
+    const Kernel kern_dv = kKernels[kWideDV][feat], kern_dk = kKernels[kWideDK][feat];
+    if ((e = set_smem(3 * kWideDV + feat, reinterpret_cast<const void*>(kern_dv))) != cudaSuccess) return e;
+    if ((e = set_smem(3 * kWideDK + feat, reinterpret_cast<const void*>(kern_dk))) != cudaSuccess) return e;
     dim3 grid((p.max_sk + kBlk - 1) / kBlk, p.hk, p.batch);
     e = launch_kernel(kern_dv, grid, dim3(kWideThreads), L::kDynamic, st, p, k128, k128, do64, q64, status);
     if (e != cudaSuccess) return e;
@@ -717,14 +721,14 @@ cudaError_t launch_bwd_wide_T(int which, const Params& p, cudaStream_t st) {
       e = launch_kernel(kern_dk, grid, dim3(kWideThreads), L::kDynamic, st, p, k128, v128, q64, do64, status);
     }
   } else {
-    auto kern_dq = plain ? sm100_bwd_wide_kernel<T, kWideDQ, true> : sm100_bwd_wide_kernel<T, kWideDQ, false>;
-    if ((e = set_smem(2 + (plain ? 3 : 0), reinterpret_cast<const void*>(kern_dq))) != cudaSuccess) return e;
+    const Kernel kern_dq = kKernels[kWideDQ][feat];
+    if ((e = set_smem(3 * kWideDQ + feat, reinterpret_cast<const void*>(kern_dq))) != cudaSuccess) return e;
     dim3 grid((p.max_sq + kBlk - 1) / kBlk, p.hq, p.batch);
     e = launch_kernel(kern_dq, grid, dim3(kWideThreads), L::kDynamic, st, p, q128, do128, k64, v64, status);
     if (e == cudaSuccess && p.dk_from_db) {
       count_launch();
       auto kern_db = sm100_bwd_dk_db_kernel<T>;
-      if ((e = set_smem(6, reinterpret_cast<const void*>(kern_db), DkDbSmem::kDynamic)) != cudaSuccess) return e;
+      if ((e = set_smem(9, reinterpret_cast<const void*>(kern_db), DkDbSmem::kDynamic)) != cudaSuccess) return e;
       dim3 grid_k((p.max_sk + kBlk - 1) / kBlk, p.hk, p.batch);
       e = launch_kernel(kern_db, grid_k, dim3(kDkDbThreads), DkDbSmem::kDynamic, st, p, db64, q64, status);
     }

@@ -147,10 +147,12 @@ __device__ void write_dead_rows(const Params& p, const Seq& sq, int h, int m0, i
 // HD.  Every tile is then full, so the instantiation carries no tail handling and fixed GEMM shapes:
 // the MMA issuer's loop is latency-critical, and even untaken branches and a call site in it cost
 // several per cent of the kernel's time (measured: 3 to 10 % over the three tcgen05 kernels).
-// PLAIN: no dropout and no bias.  The compute warps' loop is short of registers, and what it keeps for these
-// (Philox round keys, row pointers) is spilled around every block even where it is never used.  Measured: 24 packed
-// prompts of 32 to 2048 tokens, 32:8 heads of 128, 418 -> 399 us; one of 3001 tokens 105 -> 104.
-template <typename T, int HD, bool EXACT, bool PLAIN>
+// FEAT (features()): with code for dropout in the loop a call with bias alone, and with code for either a call with
+// neither, spills around every block.  Measured, us, dropout's instantiation against the call's own, neither: 4 x 32 heads
+// x 4096 of 128, causal, 583 -> 571; 8 x 16 heads x 2048 of 64 260 -> 241; bias, 4 x 8 heads x 1024 of 64 41.6 -> 40.8.
+// (That bias is there stays a test at run time: with it known, whole tiles gain 10 to 20 %, but unaligned rows
+// and the last, partial block, whose loads then wait one by one, lose as much or more.)
+template <typename T, int HD, bool EXACT, int FEAT>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -164,8 +166,8 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + L::kAbort);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // (constants where PLAIN: nothing of dropout, bias or its gradient is compiled in)
-  const bool drop_on = !PLAIN && p.dropout_on != 0, bias_on = !PLAIN && p.has_bias != 0;
+  // (constants where FEAT leaves them out: nothing of theirs is compiled in)
+  const bool drop_on = FEAT == kDropout && p.dropout_on != 0, bias_on = FEAT != kPlain && p.has_bias != 0;
   // Order of the CTAs (the hardware starts them by linear block index): (batch, head) pairs are taken
   // in groups of kHeadGroup; inside a group the row-tile index runs slowest, from the tile with the
   // most key blocks of a causal problem to the one with the fewest.  The heavy tiles of a group so
@@ -393,10 +395,10 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
     // With one tile per CTA these warps have nothing else to do, and Philox is the one thing that neither the tensor
     // pipe, the special-function unit nor the softmax warps' chain has a part in: it runs beside them, a thread
     // drawing the 128 bits of its row up to two blocks ahead.  Measured, training step with bias
-    // and dropout 0.2, 8 x 16 heads x 2048: 5.38 -> 4.99 ms.
+    // and dropout 0.2, 8 x 16 heads x 2048: 5.38 -> 5.0 ms.
     // (With two tiles it does not pay: a warpgroup more leaves its threads 56 registers, too few for the independent
     // counters that one warp per scheduler needs: 16 packed sequences 23.3 -> 26.1 ms.)
-    if constexpr (!PLAIN) {
+    if constexpr (FEAT == kDropout) {
       if (drop_on) {
         const int r = (warp & 3) * 32 + lane;
         const DropoutCtx dctx = dropout_ctx(p, z, h);
@@ -732,7 +734,7 @@ inline bool exact_tiles(const Params& p, int hd) {
   return p.varlen_mode == 0 && p.max_sq % 128 == 0 && p.max_sk % 128 == 0 && p.dqk == hd && p.dvo == hd;
 }
 
-template <typename T, int HD, bool EXACT, bool PLAIN>
+template <typename T, int HD, bool EXACT, int FEAT>
 cudaError_t launch_fwd_TE(const Params& p, cudaStream_t st) {
   using L = FwdSmem<HD>;
   CUtensorMap tq, tk, tv;
@@ -746,7 +748,7 @@ cudaError_t launch_fwd_TE(const Params& p, cudaStream_t st) {
   cudaError_t e = fwd_device_facts(&dev, &status, nullptr, &remember);
   if (e != cudaSuccess) return e;
   if (!remember || !attr_set[dev].load(std::memory_order_acquire)) {
-    e = host().func_set_smem(reinterpret_cast<const void*>(sm100_fwd_kernel<T, HD, EXACT, PLAIN>), L::kDynamic);
+    e = host().func_set_smem(reinterpret_cast<const void*>(sm100_fwd_kernel<T, HD, EXACT, FEAT>), L::kDynamic);
     if (e != cudaSuccess) return e;
     if (remember) attr_set[dev].store(true, std::memory_order_release);
   }
@@ -754,7 +756,7 @@ cudaError_t launch_fwd_TE(const Params& p, cudaStream_t st) {
   Params pp = p;
   pp.packed_tiles = packed_tiles_bound(p, L::kCtaRows);
   if (pp.packed_tiles > 0) grid = dim3(pp.packed_tiles * p.hq);
-  e = launch_kernel(sm100_fwd_kernel<T, HD, EXACT, PLAIN>, grid, dim3(kFwdThreads), L::kDynamic, st, pp, tq, tk, tv, status);
+  e = launch_kernel(sm100_fwd_kernel<T, HD, EXACT, FEAT>, grid, dim3(kFwdThreads), L::kDynamic, st, pp, tq, tk, tv, status);
   if (e == cudaSuccess) count_launch();
   return e;
 }
@@ -762,9 +764,14 @@ cudaError_t launch_fwd_TE(const Params& p, cudaStream_t st) {
 template <typename T, int HD>
 cudaError_t launch_fwd_T(const Params& p, cudaStream_t st) {
   const bool exact = exact_tiles(p, HD);
-  if (!p.dropout_on && !p.has_bias)
-    return exact ? launch_fwd_TE<T, HD, true, true>(p, st) : launch_fwd_TE<T, HD, false, true>(p, st);
-  return exact ? launch_fwd_TE<T, HD, true, false>(p, st) : launch_fwd_TE<T, HD, false, false>(p, st);
+  switch (features(p)) {
+    case kPlain:
+      // (Whole tiles of 256 columns: ptxas spills 320 bytes in the instantiation without bias, 268 in the one with it.
+      // Measured, 8 x 16 heads x 2048, not causal: 642 us against 628.)
+      return exact ? launch_fwd_TE<T, HD, true, HD == 256 ? kBias : kPlain>(p, st) : launch_fwd_TE<T, HD, false, kPlain>(p, st);
+    case kBias: return exact ? launch_fwd_TE<T, HD, true, kBias>(p, st) : launch_fwd_TE<T, HD, false, kBias>(p, st);
+    default: return exact ? launch_fwd_TE<T, HD, true, kDropout>(p, st) : launch_fwd_TE<T, HD, false, kDropout>(p, st);
+  }
 }
 
 }  // namespace
