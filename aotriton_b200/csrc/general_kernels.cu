@@ -376,9 +376,9 @@ __global__ void __launch_bounds__(kThreads) general_bwd_dq_kernel(const __grid_c
 // ---------------------------------------------------------------------------
 // delta[m] = sum_d O[m,d] * dO[m,d] in fp32, written with the LSE layout.  HBM-bound.
 // grid = (cdiv(max_sq, 128), Hq, batch); a CTA of 8 warps owns 128 rows of one (sequence, head).
-// Fast path (16-bit types, D in {64,128,256}, 16-byte aligned rows): D/8 lanes share a row with
-// one 16-byte load each from O and dO, four rows in flight per lane group.  Otherwise one warp
-// per row with scalar loads.
+// Fast path (16-bit types, D a multiple of 8 up to 256, 16-byte aligned rows): the smallest power of two of
+// at least D/8 lanes shares a row with one 16-byte load each from O and dO, four rows in flight per lane
+// group.  Otherwise one warp per row with scalar loads.
 template <typename T>
 __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_constant__ Params p) {
   const int z = blockIdx.z, h = blockIdx.y;
