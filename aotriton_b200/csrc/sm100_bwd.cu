@@ -633,11 +633,14 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
       }
       int col_lo = 0, col_hi = sq.sq - 1;     // valid query rows for this key
       if (p.causal) {
-        int64_t lo = (int64_t)n - sq.wr, hi = (int64_t)n + sq.wl;
+        // (keys beyond the sequence's end take the last key's bounds: their rows of dV and dK are not stored, and
+        // bounds of their own would make every block of their warps a masked one.  The fused form sums over keys.)
+        const int nb = FUSED ? n : min(n, sq.sk - 1);
+        int64_t lo = (int64_t)nb - sq.wr, hi = (int64_t)nb + sq.wl;
         if (lo > col_lo) col_lo = (int)(lo > 0x7fffffffLL ? 0x7fffffffLL : lo);
         if (hi < col_hi) col_hi = (int)(hi < -1 ? -1 : hi);
       }
-      if (n >= sq.sk) { col_lo = 1; col_hi = 0; }
+      if (FUSED && n >= sq.sk) { col_lo = 1; col_hi = 0; }
       // the tightest bounds over the warp's rows: a block needs masking iff it is not inside them
       const int warp_lo = __reduce_max_sync(0xffffffffu, col_lo), warp_hi = __reduce_min_sync(0xffffffffu, col_hi);
       // Fused form: the dQ^T partial of iteration g (head dim x queries, in the S columns) is taken
@@ -1194,11 +1197,11 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
     const int cbase = kWgCols * wg;
     int row_lo = 0, row_hi = sq.sk - 1;     // valid keys for this query row
     if (p.causal) {
-      int64_t lo = (int64_t)m - sq.wl, hi = (int64_t)m + sq.wr;
+      const int mb = min(m, sq.sq - 1);      // (rows beyond the sequence's end take the last row's bounds: they are not stored)
+      int64_t lo = (int64_t)mb - sq.wl, hi = (int64_t)mb + sq.wr;
       if (lo > row_lo) row_lo = (int)(lo > 0x7fffffffLL ? 0x7fffffffLL : lo);
       if (hi < row_hi) row_hi = (int)(hi < -1 ? -1 : hi);
     }
-    if (m >= sq.sq) { row_lo = 1; row_hi = 0; }
     // the tightest bounds over the warp's rows: a block needs masking iff it is not inside them
     const int warp_lo = __reduce_max_sync(0xffffffffu, row_lo), warp_hi = __reduce_min_sync(0xffffffffu, row_hi);
     const int64_t lrow = lse_offset(p, sq, h);

@@ -349,11 +349,11 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
     // columns this row may see
     int v_lo = 0, v_hi = cols_total - 1;
     if (p.causal) {
-      const int64_t lo = (int64_t)row - (kKeys ? sq.wr : sq.wl), hi = (int64_t)row + (kKeys ? sq.wl : sq.wr);
+      const int rb = min(row, rows_total - 1);      // (rows beyond the sequence's end take the last row's bounds: they are not stored)
+      const int64_t lo = (int64_t)rb - (kKeys ? sq.wr : sq.wl), hi = (int64_t)rb + (kKeys ? sq.wl : sq.wr);
       if (lo > v_lo) v_lo = (int)(lo > 0x7fffffffLL ? 0x7fffffffLL : lo);
       if (hi < v_hi) v_hi = (int)(hi < -1 ? -1 : hi);
     }
-    if (row >= rows_total) { v_lo = 1; v_hi = 0; }
     // the tightest bounds over the warp's rows: a block needs masking iff it is not inside them
     const int warp_lo = __reduce_max_sync(0xffffffffu, v_lo), warp_hi = __reduce_min_sync(0xffffffffu, v_hi);
     bool ok = true;

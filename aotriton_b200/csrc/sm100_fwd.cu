@@ -427,13 +427,17 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const uint32_t s_addr = tmem_base + lane_addr + (uint32_t)t * 128u;
     const uint32_t o_addr = tmem_base + lane_addr + 256u + (uint32_t)t * 128u;
+    // Rows beyond the sequence's end take the last row's bounds: nothing of theirs is stored, a row of the products
+    // depends on no other one, and bounds of their own (none) would make every block of their warps a masked one.
+    // Measured, forward on the device, us: 24 packed prompts of 32 to 2048 tokens, 32:8 heads of 128, 379 -> 360; a prompt of
+    // 3001 108.5 -> 106.5; training step of 16 x 12 heads x 391 of 64 with dropout (the backward likewise) 342 -> 331.
+    const int mb = min(m, sq.sq - 1);
     int row_lo = 0, row_hi = sq.sk - 1;
     if (p.causal) {
-      int64_t lo = (int64_t)m - sq.wl, hi = (int64_t)m + sq.wr;
+      int64_t lo = (int64_t)mb - sq.wl, hi = (int64_t)mb + sq.wr;
       if (lo > row_lo) row_lo = (int)(lo > 0x7fffffffLL ? 0x7fffffffLL : lo);
       if (hi < row_hi) row_hi = (int)(hi < -1 ? -1 : hi);
     }
-    if (m >= sq.sq) { row_lo = 1; row_hi = 0; }
     // the tightest bounds over the warp's rows: a block needs masking iff it is not inside them
     const int warp_lo = __reduce_max_sync(0xffffffffu, row_lo), warp_hi = __reduce_min_sync(0xffffffffu, row_hi);
     DropoutCtx dctx;
@@ -485,7 +489,7 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
         for (int c = 16; c < 128; c += 2) m8[(c >> 1) & 7] = fmax3(m8[(c >> 1) & 7], sc[c], sc[c + 1]);
         mx = fmaxf(fmax3(m8[0], m8[1], m8[2]), fmaxf(fmax3(m8[3], m8[4], m8[5]), fmaxf(m8[6], m8[7])));
         mx *= p.qk_scale;
-        const bool huge = fabsf(mx) > 1.0e6f && mx != -INFINITY;
+        const bool huge = fabsf(mx) > 1.0e6f && mx != -INFINITY && m < sq.sq;      // (rows that are not stored decide nothing)
         if (__any_sync(0xffffffffu, huge)) simple = false;
       }
       if (!simple) {
