@@ -18,6 +18,7 @@
 // bwd_preprocess.py:118-133 and dropout_rng.py:86-126.
 #include "common.cuh"
 #include "launch.h"
+#include "sm100_ptx.cuh"
 
 namespace ab200 {
 
@@ -375,40 +376,40 @@ __global__ void __launch_bounds__(kThreads) general_bwd_dq_kernel(const __grid_c
 
 // ---------------------------------------------------------------------------
 // delta[m] = sum_d O[m,d] * dO[m,d] in fp32, written with the LSE layout.  HBM-bound.
-// grid = (cdiv(max_sq, 128), Hq, batch); a CTA of 8 warps owns 128 rows of one (sequence, head).
-// Fast path (16-bit types, D a multiple of 8 up to 256, 16-byte aligned rows): the smallest power of two of
-// at least D/8 lanes shares a row with one 16-byte load each from O and dO, four rows in flight per lane
-// group.  Otherwise one warp per row with scalar loads.
+// grid = (cdiv(max_sq, 128), Hq, batch); a CTA of 8 warps owns 128 rows of one (sequence, head), 16 of them a warp's.  (32
+// rows a CTA for small grids: 2.7 -> 2.9 us at 2 x 4 heads x 128, 6.0 -> 6.9 at 4 x 8 x 1024 of 80.)
+// Fast path (rows of 16-byte pieces, at most 32 of them, 16-byte aligned): the smallest power of two of lanes that covers a
+// row has one 16-byte load each from O and dO, four rows in flight per lane group.  Otherwise one warp per row with scalar loads
+// (which fp32 used to take: 2 x 8 heads x 500 rows of 64, with nothing in L2, 20.6 -> 3.7 us).
 template <typename T>
 __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_constant__ Params p) {
+  constexpr int kWarpRows = 16, kPer = 16 / (int)sizeof(T);      // elements of a 16-byte load
   const int z = blockIdx.z, h = blockIdx.y;
   const Seq sq = resolve_seq(p, z);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int d = p.dvo;
-  const int row0 = blockIdx.x * 128;
-  if (row0 >= sq.sq) return;
+  const int wrow0 = ((int)blockIdx.x * 8 + warp) * kWarpRows;
+  if (wrow0 >= sq.sq) return;
   const int64_t lrow = lse_offset(p, sq, h);
-  // 16-byte loads wherever rows allow them: a row goes to the smallest power of two of lanes that
-  // covers its d / 8 loads.
-  const bool vec_ok = (sizeof(T) == 2) && d % 8 == 0 && d <= 256 &&
+  const bool vec_ok = d % kPer == 0 && d <= 32 * kPer &&
                       ((reinterpret_cast<uintptr_t>(p.out.ptr) | reinterpret_cast<uintptr_t>(p.dout.ptr)) % 16 == 0) &&
-                      (p.out.s[0] % 8 == 0) && (p.out.s[1] % 8 == 0) && (p.out.s[2] % 8 == 0) &&
-                      (p.dout.s[0] % 8 == 0) && (p.dout.s[1] % 8 == 0) && (p.dout.s[2] % 8 == 0);
+                      (p.out.s[0] % kPer == 0) && (p.out.s[1] % kPer == 0) && (p.out.s[2] % kPer == 0) &&
+                      (p.dout.s[0] % kPer == 0) && (p.dout.s[1] % kPer == 0) && (p.dout.s[2] % kPer == 0);
   if (vec_ok) {
-    const int loads = d >> 3;
+    const int loads = d / kPer;
     const int lpr = loads <= 4 ? 4 : (loads <= 8 ? 8 : (loads <= 16 ? 16 : 32));      // lanes per row
     const int rpw = 32 / lpr;               // rows per warp pass
-    const int sub = lane / lpr, col = (lane % lpr) * 8;
-    // warp w covers rows row0 + 16w .. +15 in passes of rpw rows, four passes in flight
-    const int wrow0 = row0 + warp * 16;
-    for (int pass = 0; pass < 16 / rpw; pass += 4) {
+    const int sub = lane / lpr, col = (lane % lpr) * kPer;
+    for (int pass = 0; pass * rpw < kWarpRows; pass += 4) {
       uint4 a[4], b[4];
       int rows[4];
+      bool in[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        rows[u] = wrow0 + (pass + u) * rpw + sub;
-        const bool in = (pass + u) * rpw < 16 && rows[u] < sq.sq && col < d;
-        if (in) {
+        const int r = (pass + u) * rpw + sub;
+        rows[u] = wrow0 + r;
+        in[u] = r < kWarpRows && rows[u] < sq.sq;
+        if (in[u] && col < d) {
           a[u] = *reinterpret_cast<const uint4*>(row_ptr<T>(p.out, sq.bidx, h, sq.q0 + rows[u]) + col);
           b[u] = *reinterpret_cast<const uint4*>(row_ptr<T>(p.dout, sq.bidx, h, sq.q0 + rows[u]) + col);
         } else {
@@ -422,14 +423,14 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
         const T* be = reinterpret_cast<const T*>(&b[u]);
         float acc = 0.f;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc = fmaf(to_f32<T>(ae[e]), to_f32<T>(be[e]), acc);
+        for (int e = 0; e < kPer; ++e) acc = fmaf(to_f32<T>(ae[e]), to_f32<T>(be[e]), acc);
         for (int o = lpr >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if ((lane % lpr) == 0 && (pass + u) * rpw < 16 && rows[u] < sq.sq) p.delta[lrow + rows[u]] = acc;
+        if ((lane % lpr) == 0 && in[u]) p.delta[lrow + rows[u]] = acc;
       }
     }
     return;
   }
-  for (int m = row0 + warp; m < min(sq.sq, row0 + 128); m += 8) {
+  for (int m = wrow0; m < min(sq.sq, wrow0 + kWarpRows); ++m) {
     const T* op = row_ptr<T>(p.out, sq.bidx, h, sq.q0 + m);
     const T* gp = row_ptr<T>(p.dout, sq.bidx, h, sq.q0 + m);
     float acc = 0.f;
@@ -551,8 +552,8 @@ cudaError_t launch_tiled_T(int which, const Params& p, cudaStream_t st) {
     const cudaError_t e = launch_tiled_T<T, DP>(1, p, st);
     return e != cudaSuccess ? e : launch_tiled_T<T, DP>(2, p, st);
   }
-  const size_t rows = which == 0 ? C::kBM + 2 * C::kBN : 2 * C::kBM + 2 * C::kBN;      // staged rows of DP + 4 floats
-  const size_t tiles = which & 1 ? 2 : 1;                                              // P and dS, or one of them
+  const size_t rows = which == 0 ? C::kBM + kFwdGroups * 2 * C::kBN : 2 * C::kBM + 2 * C::kBN;      // staged rows of DP + 4 floats
+  const size_t tiles = which == 0 ? kFwdGroups : (which & 1 ? 2 : 1);                              // P and dS, or one of them
   const size_t sm = (rows * C::kLd + tiles * C::kBM * C::kLdP + (which & 1 ? 2 * C::kBN : 0)) * sizeof(float);
   auto kern = which == 0   ? tiled_fwd_kernel<T, DP>
               : which == 1 ? tiled_bwd_kernel<T, DP, 1>
@@ -563,7 +564,7 @@ cudaError_t launch_tiled_T(int which, const Params& p, cudaStream_t st) {
   const int rows_total = which == 1 ? p.max_sk : (which == 3 && p.max_sk > p.max_sq ? p.max_sk : p.max_sq);
   const int blocks = (rows_total + C::kBM - 1) / C::kBM;
   dim3 grid(which == 3 ? 2 * blocks : blocks, which == 1 ? p.hk : p.hq, p.batch);
-  e = launch_kernel(kern, grid, dim3(C::kThreads), sm, st, p);
+  e = launch_kernel(kern, grid, dim3(which == 0 ? kFwdGroups * C::kThreads : C::kThreads), sm, st, p);
   if (e == cudaSuccess) count_launch();
   return e;
 }

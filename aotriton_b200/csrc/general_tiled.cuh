@@ -4,13 +4,13 @@
 // What bounds them: 16-byte shared-memory reads (an 8-read step feeds 64 multiply-adds per thread) where the
 // grid fills the chip, the latency of a block's chain -- stage, scores, softmax, accumulate -- where it does
 // not.  The 16x16-tile kernels (kept for head dims above 128) compute one dot product per thread, two
-// reads for every four multiply-adds.  Here a CTA of 128 threads owns 32 rows (queries; keys for
-// dK / dV) and walks the other sequence dimension in blocks of BN columns; a thread holds a 4 x BN/16
+// reads for every four multiply-adds.  Here 128 threads own 32 rows (queries; keys for
+// dK / dV) and walk the other sequence dimension in blocks of BN columns; a thread holds a 4 x BN/16
 // tile of scores (rows ty*4.., columns tx + 16 j) and a 4 x DP/16 tile of each accumulator (columns tx*4.. + 64 j),
 // so that a 16-byte read feeds 8 or more multiply-adds.  32 rows and not 64: at the sizes single precision is
-// used at, the number of CTAs is what is short.  Measured, fp32: 2 x 8 heads x 500 tokens, head dim 64, causal:
-// forward 114 -> 68 us, dK/dV 176 -> 101, dQ 141 -> 86; 4 x 8 x 1024, head dim 128: 1471 -> 719, 2684 -> 1820,
-// 2038 -> 1244.
+// used at, the number of CTAs is what is short.  fp32 tiles are copied asynchronously, a block ahead of their use
+// where a tile's last reader is known early.  Measured, fp32, 2 x 8 heads x 500 tokens, head dim 64, causal, nothing in L2,
+// against loads through registers with one group of warps a tile: forward 98 -> 35 us, backward 139 -> 110.
 //
 // All tiles are row-major fp32 with four floats of padding: (DP + 4) / 4 is odd, so the 16 lanes that
 // read 16 different rows at one column hit different banks.  The P / dS rows that a warp writes are read
@@ -31,20 +31,23 @@ __device__ __forceinline__ bool rows_vec4(const View4& v, int d) {
 
 // Rows row0.. of one head into dst[ROWS][DP + 4]; rows at or beyond nrows and columns at or beyond d
 // are zero (columns up to the next multiple of four: the contractions stop there, the accumulators' ones
-// are never stored).
-template <typename T, int DP, int ROWS>
-__device__ __forceinline__ void stage_tile(float* dst, const View4& v, int b, int h, int64_t tok0, int row0, int nrows, int d, bool vec) {
-  constexpr int kThreadsT = Tiled<DP>::kThreads, kLd = Tiled<DP>::kLd, kC4 = DP / 4;
+// are never stored).  `tid` of THREADS threads.  fp32 rows that allow it are copied asynchronously, all of a tile in flight at
+// once: stage_wait() and a barrier come before their use.  (Through registers four loads were in flight, and half of the
+// forward's time went by waiting for them.)
+template <typename T, int DP, int ROWS, int THREADS>
+__device__ __forceinline__ void stage_tile(float* dst, const View4& v, int b, int h, int64_t tok0, int row0, int nrows, int d, bool vec, int tid) {
+  constexpr int kLd = Tiled<DP>::kLd, kC4 = DP / 4;
   const T* base = row_ptr<T>(v, b, h, tok0 + row0);
-#pragma unroll 4
-  for (int idx = threadIdx.x; idx < ROWS * kC4; idx += kThreadsT) {
+#pragma unroll 8
+  for (int idx = tid; idx < ROWS * kC4; idx += THREADS) {
     const int r = idx / kC4, c = (idx - r * kC4) * 4;
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
     if (row0 + r < nrows && c < d) {
       const T* src = base + (int64_t)r * v.s[2] + c;
       if (vec) {
         if constexpr (sizeof(T) == 4) {
-          x = __ldg(reinterpret_cast<const float4*>(src));
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ptx::smem_u32(dst + r * kLd + c)), "l"(src) : "memory");
+          continue;
         } else {
           const uint2 w = __ldg(reinterpret_cast<const uint2*>(src));
           const T* e = reinterpret_cast<const T*>(&w);
@@ -59,16 +62,22 @@ __device__ __forceinline__ void stage_tile(float* dst, const View4& v, int b, in
     }
     *reinterpret_cast<float4*>(dst + r * kLd + c) = x;
   }
+  asm volatile("cp.async.commit_group;" ::: "memory");
 }
+// This thread's copies have landed, all but those of its last PENDING stage_tile calls.
+template <int PENDING>
+__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
 
-// s[i][j] = A[ty*4 + i] . B[tx + 16 j] over d4 groups of four columns
+// s[i][j] = A[ty*4 + i] . B[tx + 16 j] over d4 groups of four columns, even and odd columns in the two halves of a packed
+// sum (two multiply-adds an instruction: the issue slots, not the arithmetic, are what a block of few warps is short of)
 template <int DP>
 __device__ __forceinline__ void tile_dots(float (&s)[4][Tiled<DP>::kNC], const float* A, const float* B, int d4, int ty, int tx) {
   using C = Tiled<DP>;
+  float2 t[4][C::kNC];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < C::kNC; ++j) s[i][j] = 0.f;
+    for (int j = 0; j < C::kNC; ++j) t[i][j] = make_float2(0.f, 0.f);
   const float* a0 = A + ty * 4 * C::kLd;
   const float* b0 = B + tx * C::kLd;
 #pragma unroll 2
@@ -82,12 +91,14 @@ __device__ __forceinline__ void tile_dots(float (&s)[4][Tiled<DP>::kNC], const f
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < C::kNC; ++j) {
-        s[i][j] = fmaf(a[i].x, b[j].x, s[i][j]);
-        s[i][j] = fmaf(a[i].y, b[j].y, s[i][j]);
-        s[i][j] = fmaf(a[i].z, b[j].z, s[i][j]);
-        s[i][j] = fmaf(a[i].w, b[j].w, s[i][j]);
+        t[i][j] = ptx::fma2(make_float2(a[i].x, a[i].y), make_float2(b[j].x, b[j].y), t[i][j]);
+        t[i][j] = ptx::fma2(make_float2(a[i].z, a[i].w), make_float2(b[j].z, b[j].w), t[i][j]);
       }
   }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < C::kNC; ++j) s[i][j] = t[i][j].x + t[i][j].y;
 }
 
 // The part [k0, k1) of the block of BN columns at `col0` that some row of the warp's eight sees (columns lo..hi), k0
@@ -178,29 +189,57 @@ __device__ __forceinline__ const T* bias_at(const Params& p, const Seq& sq, int 
          (int64_t)m * p.bias.s[2] + (int64_t)n * p.bias.s[3];
 }
 
-// Forward.  grid = (cdiv(max_sq, 32), Hq, batch); the last rows of a causal problem see the most keys and start first.
+// Which (row tile counted from the last, head, batch) a CTA takes: heads in groups of 32, inside a group the row tiles
+// slowest, so that the long tiles of a causal problem start together and first.
+__device__ __forceinline__ void tile_of_block(int nx, int nh, int nz, int& x, int& h, int& z) {
+  constexpr int kHeadGroup = 32;
+  const int lin = (int)blockIdx.x + nx * ((int)blockIdx.y + nh * (int)blockIdx.z);
+  const int grp = lin / (kHeadGroup * nx), r = lin - grp * (kHeadGroup * nx), gsize = min(kHeadGroup, nh * nz - grp * kHeadGroup);
+  x = r / gsize;
+  const int hz = grp * kHeadGroup + (r - x * gsize);
+  z = hz / nh;
+  h = hz - z * nh;
+}
+
+// Forward.  grid = (cdiv(max_sq, 32), Hq, batch).  Two groups of four warps take every other block of the keys, each with
+// tiles of its own, and merge at the end: a row tile's chain of blocks, which is what a small grid waits for, is half
+// as long, and an SM has 16 warps instead of 12.  Within a group the copy of V runs under the scores, that of the next K
+// under the accumulation.
+constexpr int kFwdGroups = 2;
 template <typename T, int DP>
-__global__ void __launch_bounds__(128) tiled_fwd_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(kFwdGroups * 128, 2) tiled_fwd_kernel(const __grid_constant__ Params p) {
   using C = Tiled<DP>;
+  constexpr int kGroupFloats = 2 * C::kBN * C::kLd + C::kBM * C::kLdP;
   extern __shared__ float smem[];
-  float* Qs = smem;                       // [32][LD]
-  float* Ks = Qs + C::kBM * C::kLd;       // [BN][LD]
-  float* Vs = Ks + C::kBN * C::kLd;       // [BN][LD]
-  float* Ps = Vs + C::kBN * C::kLd;       // [32][BN + 4]
-  const int z = blockIdx.z, h = blockIdx.y, m0 = (int)(gridDim.x - 1 - blockIdx.x) * C::kBM;
+  const int grp = threadIdx.x >> 7, tid = threadIdx.x & 127;
+  float* Qs = smem;                                              // [32][LD]
+  float* Ks = Qs + C::kBM * C::kLd + grp * kGroupFloats;         // [BN][LD]
+  float* Vs = Ks + C::kBN * C::kLd;                              // [BN][LD]
+  float* Ps = Vs + C::kBN * C::kLd;                              // [32][BN + 4]
   // One thread of the grid reports the seed and offset actually used, before any early exit
   // (the first sequence of a varlen batch may be empty).
   if (p.dropout_on && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) {
     if (p.seed_out) *p.seed_out = p.seed_ptr ? *p.seed_ptr : 0ull;
     if (p.off_out) *p.off_out = p.off2 + (p.off1_ptr ? *p.off1_ptr : 0ull);
   }
+  int x, h, z;
+  tile_of_block((int)gridDim.x, (int)gridDim.y, (int)gridDim.z, x, h, z);
+  const int m0 = ((int)gridDim.x - 1 - x) * C::kBM;
   const Seq sq = resolve_seq(p, z);
   if (m0 >= sq.sq) return;
-  const int hk = h / p.group, ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const int hk = h / p.group, ty = tid >> 4, tx = tid & 15;
   const bool kvec = rows_vec4<T>(p.k, p.dqk), vvec = rows_vec4<T>(p.v, p.dvo);
+  auto group_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory"); };
   DropoutCtx dctx;
   if (p.dropout_on) dctx = dropout_ctx(p, z, h);
-  stage_tile<T, DP, C::kBM>(Qs, p.q, sq.bidx, h, sq.q0, m0, sq.sq, p.dqk, rows_vec4<T>(p.q, p.dqk));
+  int n_lo, n_hi, w_lo = 1, w_hi = 0;
+  key_range(p, sq, m0, min(m0 + C::kBM, sq.sq) - 1, n_lo, n_hi);
+  const int wm = m0 + (tid >> 5) * kWarpRows;
+  if (wm < sq.sq) key_range(p, sq, wm, min(wm + kWarpRows, sq.sq) - 1, w_lo, w_hi);
+  const int d4 = (p.dqk + 3) >> 2;
+  int n0 = n_lo / C::kBN * C::kBN + grp * C::kBN;
+  stage_tile<T, DP, C::kBM, kFwdGroups * 128>(Qs, p.q, sq.bidx, h, sq.q0, m0, sq.sq, p.dqk, rows_vec4<T>(p.q, p.dqk), threadIdx.x);
+  if (n0 <= n_hi) stage_tile<T, DP, C::kBN, 128>(Ks, p.k, sq.bidx, hk, sq.k0, n0, sq.sk, p.dqk, kvec, tid);
   float m_i[4], l_i[4];
   float4 acc[4][C::kND];
 #pragma unroll
@@ -210,16 +249,12 @@ __global__ void __launch_bounds__(128) tiled_fwd_kernel(const __grid_constant__ 
 #pragma unroll
     for (int j = 0; j < C::kND; ++j) acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  int n_lo, n_hi, w_lo = 1, w_hi = 0;
-  key_range(p, sq, m0, min(m0 + C::kBM, sq.sq) - 1, n_lo, n_hi);
-  const int wm = m0 + (threadIdx.x >> 5) * kWarpRows;
-  if (wm < sq.sq) key_range(p, sq, wm, min(wm + kWarpRows, sq.sq) - 1, w_lo, w_hi);
-  const int d4 = (p.dqk + 3) >> 2;
-  for (int n0 = n_lo / C::kBN * C::kBN; n0 <= n_hi; n0 += C::kBN) {
-    __syncthreads();   // the previous block's tiles have been read
-    stage_tile<T, DP, C::kBN>(Ks, p.k, sq.bidx, hk, sq.k0, n0, sq.sk, p.dqk, kvec);
-    stage_tile<T, DP, C::kBN>(Vs, p.v, sq.bidx, hk, sq.k0, n0, sq.sk, p.dvo, vvec);
-    __syncthreads();
+  stage_wait<0>();
+  __syncthreads();      // (Q is staged by both groups)
+  for (; n0 <= n_hi; n0 += kFwdGroups * C::kBN) {
+    stage_wait<0>();
+    group_sync();       // K has landed, the previous block's V has been read
+    stage_tile<T, DP, C::kBN, 128>(Vs, p.v, sq.bidx, hk, sq.k0, n0, sq.sk, p.dvo, vvec, tid);
     float s[4][C::kNC];
     tile_dots<DP>(s, Qs, Ks, d4, ty, tx);
     const uint32_t keep = p.dropout_on ? tile_keep_bits<C::kNC>(dctx, m0 + ty * 4, n0, tx) : 0xffffffffu;
@@ -253,27 +288,59 @@ __global__ void __launch_bounds__(128) tiled_fwd_kernel(const __grid_constant__ 
         acc[i][j].x *= alpha; acc[i][j].y *= alpha; acc[i][j].z *= alpha; acc[i][j].w *= alpha;
       }
     }
-    __syncwarp();
+    stage_wait<0>();
+    group_sync();       // V has landed, K has been read
+    if (n0 + kFwdGroups * C::kBN <= n_hi)
+      stage_tile<T, DP, C::kBN, 128>(Ks, p.k, sq.bidx, hk, sq.k0, n0 + kFwdGroups * C::kBN, sq.sk, p.dqk, kvec, tid);
     int k0, k1;
     seen_columns<DP>(w_lo, w_hi, n0, k0, k1);
     tile_accumulate<DP>(acc, Ps, Vs, k0, k1, ty, tx);
     __syncwarp();
   }
 #pragma unroll
+  for (int i = 0; i < 4; ++i) l_i[i] = half_warp_sum(l_i[i]);
+  // The second group's sums reach the first through the second's own K tile (every warp of the group has read the last
+  // one), a row's maximum and sum in the padding behind it.
+  float* theirs = Qs + C::kBM * C::kLd + kGroupFloats;
+  if (grp == 1) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = ty * 4 + i;
+#pragma unroll
+      for (int j = 0; j < C::kND; ++j) *reinterpret_cast<float4*>(theirs + r * C::kLd + tx * 4 + 64 * j) = acc[i][j];
+      if (tx == 0) *reinterpret_cast<float2*>(theirs + r * C::kLd + DP) = make_float2(m_i[i], l_i[i]);
+    }
+  }
+  __syncthreads();
+  if (grp == 1) return;
+#pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    const float l = half_warp_sum(l_i[i]);
+    const int r = ty * 4 + i, m = m0 + r;
+    const float2 o = *reinterpret_cast<const float2*>(theirs + r * C::kLd + DP);
+    const float mx = fmaxf(m_i[i], o.x), ms = mx == -INFINITY ? 0.f : mx;
+    const float mine = exp2f(m_i[i] - ms), other = exp2f(o.x - ms);      // (-inf: no key in that half -> 0)
+    const float l = l_i[i] * mine + o.y * other;
     if (m >= sq.sq) continue;
+#pragma unroll
+    for (int j = 0; j < C::kND; ++j) {
+      const float4 t = *reinterpret_cast<const float4*>(theirs + r * C::kLd + tx * 4 + 64 * j);
+      acc[i][j].x = acc[i][j].x * mine + t.x * other;
+      acc[i][j].y = acc[i][j].y * mine + t.y * other;
+      acc[i][j].z = acc[i][j].z * mine + t.z * other;
+      acc[i][j].w = acc[i][j].w * mine + t.w * other;
+    }
     // natural-log LSE of the scaled, biased logits; rows without any valid key get O = 0, LSE = +inf
-    if (tx == 0 && p.lse != nullptr) p.lse[lse_offset(p, sq, h) + m] = l > 0.f ? (m_i[i] + log2f(l)) * kLn2 : INFINITY;
+    if (tx == 0 && p.lse != nullptr) p.lse[lse_offset(p, sq, h) + m] = l > 0.f ? (mx + log2f(l)) * kLn2 : INFINITY;
     store_acc_row<T, DP>(row_ptr_mut<T>(p.out, sq.bidx, h, sq.q0 + m), acc[i], l > 0.f ? (1.f / l) * p.dropout_scale : 0.f, p.dvo, tx);
   }
 }
 
-// dK / dV of 32 keys of one kv head
+// dK / dV of 32 keys of one kv head.  The scores of dO V^T come first: its tile is the first to be free again, so that the
+// next block's dO is on its way under the accumulation of dK, Q behind it.
 template <typename T, int DP>
 __device__ __forceinline__ void tiled_bwd_dkdv(const Params& p, float* smem, int z, int hk, int n0) {
   using C = Tiled<DP>;
+  constexpr int kThr = C::kThreads;
   float* Ks = smem;                       // [32][LD]
   float* Vs = Ks + C::kBM * C::kLd;
   float* Qs = Vs + C::kBM * C::kLd;       // [BN][LD]
@@ -284,10 +351,8 @@ __device__ __forceinline__ void tiled_bwd_dkdv(const Params& p, float* smem, int
   float* dl_s = lse_s + C::kBN;
   const Seq sq = resolve_seq(p, z);
   if (n0 >= sq.sk) return;
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
   const bool qvec = rows_vec4<T>(p.q, p.dqk), dovec = rows_vec4<T>(p.dout, p.dvo);
-  stage_tile<T, DP, C::kBM>(Ks, p.k, sq.bidx, hk, sq.k0, n0, sq.sk, p.dqk, rows_vec4<T>(p.k, p.dqk));
-  stage_tile<T, DP, C::kBM>(Vs, p.v, sq.bidx, hk, sq.k0, n0, sq.sk, p.dvo, rows_vec4<T>(p.v, p.dvo));
   float4 adv[4][C::kND], adk[4][C::kND];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
@@ -295,27 +360,42 @@ __device__ __forceinline__ void tiled_bwd_dkdv(const Params& p, float* smem, int
     for (int j = 0; j < C::kND; ++j) adv[i][j] = adk[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
   int m_lo, m_hi, w_lo = 1, w_hi = 0;
   query_range(p, sq, n0, min(n0 + C::kBM, sq.sk) - 1, m_lo, m_hi);
-  const int wn = n0 + (threadIdx.x >> 5) * kWarpRows;
+  const int wn = n0 + (tid >> 5) * kWarpRows;
   if (wn < sq.sk) query_range(p, sq, wn, min(wn + kWarpRows, sq.sk) - 1, w_lo, w_hi);
   const int dq4 = (p.dqk + 3) >> 2, dv4 = (p.dvo + 3) >> 2;
+  const int first = m_lo / C::kBN * C::kBN;
+  auto stage_q = [&](int h, int m0) {      // Q, and the rows' logsumexp and delta
+    stage_tile<T, DP, C::kBN, kThr>(Qs, p.q, sq.bidx, h, sq.q0, m0, sq.sq, p.dqk, qvec, tid);
+    if (tid < C::kBN) {
+      const int m = m0 + tid;
+      const int64_t lrow = lse_offset(p, sq, h);
+      lse_s[tid] = m < sq.sq ? p.lse[lrow + m] * kLog2e : INFINITY;
+      dl_s[tid] = m < sq.sq ? p.delta[lrow + m] : 0.f;
+    }
+  };
+  auto stage_do = [&](int h, int m0) {
+    stage_tile<T, DP, C::kBN, kThr>(dOs, p.dout, sq.bidx, h, sq.q0, m0, sq.sq, p.dvo, dovec, tid);
+  };
+  if (m_lo <= m_hi) {
+    stage_tile<T, DP, C::kBM, kThr>(Vs, p.v, sq.bidx, hk, sq.k0, n0, sq.sk, p.dvo, rows_vec4<T>(p.v, p.dvo), tid);
+    stage_do(hk * p.group, first);
+    stage_tile<T, DP, C::kBM, kThr>(Ks, p.k, sq.bidx, hk, sq.k0, n0, sq.sk, p.dqk, rows_vec4<T>(p.k, p.dqk), tid);
+    stage_wait<1>();      // V and dO
+    __syncthreads();
+    stage_q(hk * p.group, first);
+  }
   for (int g = 0; g < p.group; ++g) {
     const int h = hk * p.group + g;
     DropoutCtx dctx;
     if (p.dropout_on) dctx = dropout_ctx(p, z, h);
-    const int64_t lrow = lse_offset(p, sq, h);
-    for (int m0 = m_lo / C::kBN * C::kBN; m0 <= m_hi; m0 += C::kBN) {
-      __syncthreads();
-      stage_tile<T, DP, C::kBN>(Qs, p.q, sq.bidx, h, sq.q0, m0, sq.sq, p.dqk, qvec);
-      stage_tile<T, DP, C::kBN>(dOs, p.dout, sq.bidx, h, sq.q0, m0, sq.sq, p.dvo, dovec);
-      if (threadIdx.x < C::kBN) {
-        const int m = m0 + threadIdx.x;
-        lse_s[threadIdx.x] = m < sq.sq ? p.lse[lrow + m] * kLog2e : INFINITY;
-        dl_s[threadIdx.x] = m < sq.sq ? p.delta[lrow + m] : 0.f;
-      }
-      __syncthreads();
+    for (int m0 = first; m0 <= m_hi; m0 += C::kBN) {
+      const bool last_of_head = m0 + C::kBN > m_hi, more = !last_of_head || g + 1 < p.group;
+      const int next_h = last_of_head ? h + 1 : h, next_m0 = last_of_head ? first : m0 + C::kBN;
       float s[4][C::kNC], dp[4][C::kNC];
-      tile_dots<DP>(s, Ks, Qs, dq4, ty, tx);
       tile_dots<DP>(dp, Vs, dOs, dv4, ty, tx);
+      stage_wait<0>();
+      __syncthreads();      // K, Q, logsumexp and delta are there
+      tile_dots<DP>(s, Ks, Qs, dq4, ty, tx);
 #pragma unroll
       for (int j = 0; j < C::kNC; ++j) {
         const int c = tx + 16 * j, m = m0 + c;
@@ -342,8 +422,12 @@ __device__ __forceinline__ void tiled_bwd_dkdv(const Params& p, float* smem, int
       int k0, k1;
       seen_columns<DP>(w_lo, w_hi, m0, k0, k1);
       tile_accumulate<DP>(adv, Ps, dOs, k0, k1, ty, tx);
+      __syncthreads();      // dO has been read
+      if (more) stage_do(next_h, next_m0);
       tile_accumulate<DP>(adk, dSs, Qs, k0, k1, ty, tx);
-      __syncwarp();
+      stage_wait<0>();
+      __syncthreads();      // Q has been read, the next dO is there
+      if (more) stage_q(next_h, next_m0);
     }
   }
 #pragma unroll
@@ -355,10 +439,12 @@ __device__ __forceinline__ void tiled_bwd_dkdv(const Params& p, float* smem, int
   }
 }
 
-// dQ (+ dBias) of 32 query rows of one head
+// dQ (+ dBias) of 32 query rows of one head.  V is read by the scores only: the next block's is on its way for the rest
+// of a block.
 template <typename T, int DP>
 __device__ __forceinline__ void tiled_bwd_dq(const Params& p, float* smem, int z, int h, int m0) {
   using C = Tiled<DP>;
+  constexpr int kThr = C::kThreads;
   float* Qs = smem;                       // [32][LD]
   float* dOs = Qs + C::kBM * C::kLd;
   float* Ks = dOs + C::kBM * C::kLd;      // [BN][LD]
@@ -366,12 +452,21 @@ __device__ __forceinline__ void tiled_bwd_dq(const Params& p, float* smem, int z
   float* dSs = Vs + C::kBN * C::kLd;      // [32][BN + 4]
   const Seq sq = resolve_seq(p, z);
   if (m0 >= sq.sq) return;
-  const int hk = h / p.group, ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const int tid = threadIdx.x, hk = h / p.group, ty = tid >> 4, tx = tid & 15;
   const bool kvec = rows_vec4<T>(p.k, p.dqk), vvec = rows_vec4<T>(p.v, p.dvo);
   DropoutCtx dctx;
   if (p.dropout_on) dctx = dropout_ctx(p, z, h);
-  stage_tile<T, DP, C::kBM>(Qs, p.q, sq.bidx, h, sq.q0, m0, sq.sq, p.dqk, rows_vec4<T>(p.q, p.dqk));
-  stage_tile<T, DP, C::kBM>(dOs, p.dout, sq.bidx, h, sq.q0, m0, sq.sq, p.dvo, rows_vec4<T>(p.dout, p.dvo));
+  int n_lo, n_hi, w_lo = 1, w_hi = 0;
+  key_range(p, sq, m0, min(m0 + C::kBM, sq.sq) - 1, n_lo, n_hi);
+  const int first = n_lo / C::kBN * C::kBN;
+  auto stage_k = [&](int n0) { stage_tile<T, DP, C::kBN, kThr>(Ks, p.k, sq.bidx, hk, sq.k0, n0, sq.sk, p.dqk, kvec, tid); };
+  auto stage_v = [&](int n0) { stage_tile<T, DP, C::kBN, kThr>(Vs, p.v, sq.bidx, hk, sq.k0, n0, sq.sk, p.dvo, vvec, tid); };
+  if (n_lo <= n_hi) {
+    stage_tile<T, DP, C::kBM, kThr>(dOs, p.dout, sq.bidx, h, sq.q0, m0, sq.sq, p.dvo, rows_vec4<T>(p.dout, p.dvo), tid);
+    stage_v(first);
+    stage_tile<T, DP, C::kBM, kThr>(Qs, p.q, sq.bidx, h, sq.q0, m0, sq.sq, p.dqk, rows_vec4<T>(p.q, p.dqk), tid);
+    stage_k(first);
+  }
   const int64_t lrow = lse_offset(p, sq, h);
   float lse[4], dl[4];
   float4 adq[4][C::kND];
@@ -383,21 +478,21 @@ __device__ __forceinline__ void tiled_bwd_dq(const Params& p, float* smem, int z
 #pragma unroll
     for (int j = 0; j < C::kND; ++j) adq[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  int n_lo, n_hi, w_lo = 1, w_hi = 0;
-  key_range(p, sq, m0, min(m0 + C::kBM, sq.sq) - 1, n_lo, n_hi);
-  const int wm = m0 + (threadIdx.x >> 5) * kWarpRows;
+  const int wm = m0 + (tid >> 5) * kWarpRows;
   if (wm < sq.sq) key_range(p, sq, wm, min(wm + kWarpRows, sq.sq) - 1, w_lo, w_hi);
   if (n_hi >= n_lo) zero_dbias_outside<T>(p, sq, h, m0, C::kBM, n_lo / C::kBN * C::kBN, (n_hi / C::kBN + 1) * C::kBN);
   else zero_dbias_outside<T>(p, sq, h, m0, C::kBM, 0, 0);
   const int dq4 = (p.dqk + 3) >> 2, dv4 = (p.dvo + 3) >> 2;
-  for (int n0 = n_lo / C::kBN * C::kBN; n0 <= n_hi; n0 += C::kBN) {
-    __syncthreads();
-    stage_tile<T, DP, C::kBN>(Ks, p.k, sq.bidx, hk, sq.k0, n0, sq.sk, p.dqk, kvec);
-    stage_tile<T, DP, C::kBN>(Vs, p.v, sq.bidx, hk, sq.k0, n0, sq.sk, p.dvo, vvec);
-    __syncthreads();
+  stage_wait<2>();      // dO and V
+  __syncthreads();
+  for (int n0 = first; n0 <= n_hi; n0 += C::kBN) {
+    const bool more = n0 + C::kBN <= n_hi;
     float s[4][C::kNC], dp[4][C::kNC];
-    tile_dots<DP>(s, Qs, Ks, dq4, ty, tx);
     tile_dots<DP>(dp, dOs, Vs, dv4, ty, tx);
+    stage_wait<0>();
+    __syncthreads();      // V has been read, K (and Q) is there
+    if (more) stage_v(n0 + C::kBN);
+    tile_dots<DP>(s, Qs, Ks, dq4, ty, tx);
     const uint32_t keep = p.dropout_on ? tile_keep_bits<C::kNC>(dctx, m0 + ty * 4, n0, tx) : 0xffffffffu;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -424,7 +519,9 @@ __device__ __forceinline__ void tiled_bwd_dq(const Params& p, float* smem, int z
     int k0, k1;
     seen_columns<DP>(w_lo, w_hi, n0, k0, k1);
     tile_accumulate<DP>(adq, dSs, Ks, k0, k1, ty, tx);
-    __syncwarp();
+    stage_wait<0>();
+    __syncthreads();      // K has been read, the next V is there
+    if (more) stage_k(n0 + C::kBN);
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -437,12 +534,12 @@ __device__ __forceinline__ void tiled_bwd_dq(const Params& p, float* smem, int z
 // Hq, batch), last rows first.  3: both in one launch, x alternating between the two (neither reads what the other
 // writes); joint_backward() says when.  At the sizes single precision is used at, each of the two alone leaves most of the chip idle: 2 x 8
 // heads x 500 tokens are 256 CTAs of four warps, 7 warps an SM, waiting for their own loads and barriers.
-// Measured there (fp32, head dim 64, causal): the whole training step 273 -> 213 us, together with a shorter host path.
 template <typename T, int DP, int WHICH>
-__global__ void __launch_bounds__(128) tiled_bwd_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(128, DP <= 64 || WHICH == 2 ? 3 : 2) tiled_bwd_kernel(const __grid_constant__ Params p) {
   extern __shared__ float smem[];
   constexpr int kBM = Tiled<DP>::kBM;
-  const int z = blockIdx.z, h = blockIdx.y, x = blockIdx.x;
+  int x, h, z;
+  tile_of_block((int)gridDim.x, (int)gridDim.y, (int)gridDim.z, x, h, z);
   if constexpr (WHICH == 1) {
     tiled_bwd_dkdv<T, DP>(p, smem, z, h, x * kBM);
   } else if constexpr (WHICH == 2) {
