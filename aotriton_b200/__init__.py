@@ -29,4 +29,16 @@ def load_pyaotriton():
     return pyaotriton
 
 
-__all__ = ["PKG_DIR", "load_pyaotriton"]
+def load_torch_ops():
+    """Import the in-tree `_torch_ops` extension module (raises if it has not been built)."""
+    import torch  # noqa: F401  (its libraries are what the module links)
+    if str(PKG_DIR) not in sys.path:
+        sys.path.insert(0, str(PKG_DIR))
+    try:
+        import _torch_ops
+    except ImportError as e:
+        raise ImportError("_torch_ops extension not built; run `python -m aotriton_b200.build`") from e
+    return _torch_ops
+
+
+__all__ = ["PKG_DIR", "load_pyaotriton", "load_torch_ops"]

@@ -9,8 +9,10 @@ from __future__ import annotations
 
 import torch
 
-from . import flash
+from . import flash, load_torch_ops
 from .flash import hipError_t
+
+_native = load_torch_ops()
 
 DEFAULT_PHILOX_SEED = 0x1BF52
 DEFAULT_PHILOX_OFFSET_1 = 0x1D4000
@@ -46,15 +48,25 @@ def _philox_tensors(device, dropout_p, seed, offset1):
     return _device_u64(device, seed), _device_u64(device, (offset1 + DEFAULT_PHILOX_OFFSET_2) % (1 << 64))
 
 
-# Kernel family of the most recent backward (the library keeps it per thread, and autograd runs
-# backward on a thread of its own): 1 = general, 2 = tcgen05, 0 = none yet.
-last_bwd_family = 0
+def __getattr__(name):
+    # Kernel family of the most recent backward (the library keeps it per thread, and autograd runs
+    # backward on a thread of its own): 1 = general, 2 = tcgen05, 0 = none yet.
+    if name == "last_bwd_family":
+        return _native.last_bwd_family()
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
-def _note_bwd_family():
-    global last_bwd_family
-    from . import cabi
-    last_bwd_family = int(cabi.lib().ab200_last_bwd_family())
+def _attend(q, k, v, b, cu_q, cu_k, max_q, max_k, sm_scale, dropout_p, causal, return_lse, seed, offset1, op):
+    """The native route (csrc/torch_ops.cc): the result, or None where the call is not an ordinary one -- other tensors, modes
+    or argument types, graph capture by torch.compile.  Those go by the Function or the operators below."""
+    if torch.compiler.is_compiling():
+        return None
+    ct, wl, wr = flash.translate_causal(causal)
+    if type(offset1) is int and 0 <= offset1 < 1 << 64:
+        offset1 = (offset1 + DEFAULT_PHILOX_OFFSET_2) % (1 << 64)
+    elif dropout_p > 0.0:
+        return None
+    return _native.attend(q, k, v, b, cu_q, cu_k, max_q, max_k, sm_scale, dropout_p, ct, wl, wr, return_lse, seed, offset1, op)
 
 
 class _Attention(torch.autograd.Function):
@@ -80,7 +92,7 @@ class _Attention(torch.autograd.Function):
         delta = torch.empty_like(L)
         _check(flash.attn_bwd(q, k, v, b, ctx.sm_scale, o, do, dq, dk, dv, db, None, L, flash.eager_delta(delta),
                               ctx.dropout_p, ctx.philox_seed, ctx.philox_offset, 0, ctx.causal), "attn_bwd")
-        _note_bwd_family()
+        _native.note_bwd_family()
         return dq, dk, dv, db, None, None, None, None, None, None
 
 
@@ -89,7 +101,8 @@ def attention(q, k, v, b=None, causal=False, sm_scale=None, dropout_p=0.0, retur
     """O = dropout(softmax(Q K^T * sm_scale + b, mask)) V for (B, H, S, D) tensors (any strides with
     unit innermost stride).  `causal` is a bool, a (left, right) window or a flash.CausalType."""
     sm_scale = q.shape[-1] ** -0.5 if sm_scale is None else sm_scale
-    return _Attention.apply(q, k, v, b, causal, sm_scale, dropout_p, return_lse, philox_seed, philox_offset1)
+    r = _attend(q, k, v, b, None, None, 0, 0, sm_scale, dropout_p, causal, return_lse, philox_seed, philox_offset1, False)
+    return r if r is not None else _Attention.apply(q, k, v, b, causal, sm_scale, dropout_p, return_lse, philox_seed, philox_offset1)
 
 
 class _VarlenAttention(torch.autograd.Function):
@@ -120,14 +133,16 @@ class _VarlenAttention(torch.autograd.Function):
                                      ctx.sm_scale, o, do, dq, dk, dv, None, None, L, flash.eager_delta(delta),
                                      ctx.dropout_p, ctx.philox_seed, ctx.philox_offset, 0, ctx.causal,
                                      "compact"), "attn_bwd (varlen)")
-        _note_bwd_family()
+        _native.note_bwd_family()
         return (dq, dk, dv) + (None,) * 10
 
 
 def varlen_attention(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, causal=False,
                      sm_scale=None, dropout_p=0.0, return_lse=False):
     sm_scale = q.shape[-1] ** -0.5 if sm_scale is None else sm_scale
-    return _VarlenAttention.apply(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, causal,
+    r = _attend(q, k, v, None, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, sm_scale, dropout_p, causal, return_lse,
+                DEFAULT_PHILOX_SEED, DEFAULT_PHILOX_OFFSET_1, False)
+    return r if r is not None else _VarlenAttention.apply(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, causal,
                                   sm_scale, dropout_p, return_lse)
 
 
@@ -181,7 +196,7 @@ def op_attn_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, bias: torch.T
     _check(flash.attn_bwd(q, k, v, bias, sm_scale, out, dout, dq, dk, dv, db, flash.lazy_dq_acc(dq), lse,
                           flash.lazy_delta(lse), dropout_p, philox_seed if dropout_p > 0 else _NULL_SCALAR,
                           philox_offset if dropout_p > 0 else _NULL_SCALAR, 0, causal, opts), "attn_bwd")
-    _note_bwd_family()
+    _native.note_bwd_family()
     return dq, dk, dv, db if db is not None else q.new_empty([0])
 
 
@@ -228,6 +243,10 @@ def scaled_dot_product_attention(query, key, value, attn_mask=None, dropout_p=0.
     if not enable_gqa and query.shape[1] != key.shape[1]:
         raise ValueError("query and key head counts differ; pass enable_gqa=True")
     scale = query.shape[-1] ** -0.5 if scale is None else scale
+    r = _attend(query, key, value, attn_mask, None, None, 0, 0, float(scale), float(dropout_p), bool(is_causal), False, philox_seed,
+                philox_offset1, True)
+    if r is not None:
+        return r
     ct, wl, wr = flash.translate_causal(bool(is_causal))
     return op_attn_fwd(query, key, value, attn_mask, float(scale), float(dropout_p), ct, wl, wr, philox_seed,
                        philox_offset1)[0]

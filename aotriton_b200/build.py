@@ -6,6 +6,7 @@ Products, all written next to this file so that they are found without installat
                                (include/aotriton/*.h); the name follows the reference's
                                library (v3src/CMakeLists.txt:383-387)
   pyaotriton.<abi>.so          pybind11 module with the reference's Python surface
+  _torch_ops.<abi>.so          the autograd entry points' native route (links libtorch)
 
 `python -m aotriton_b200.build` rebuilds what is out of date.  Set AOTRITON_NAME_SUFFIX
 to compile namespace aotriton<suffix> the way the reference's cmake option does.
@@ -132,12 +133,40 @@ def build_pymodule() -> Path:
     return out
 
 
+def torch_ops_path() -> Path:
+    return PKG / ("_torch_ops" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def build_torch_ops() -> Path:
+    import torch
+    from torch.utils.cpp_extension import include_paths
+
+    OBJ.mkdir(exist_ok=True)
+    out = torch_ops_path()
+    src = CSRC / "torch_ops.cc"
+    cuda = Path(_nvcc()).resolve().parent.parent
+    lib = Path(torch.__file__).resolve().parent / "lib"
+    # (torch is in the process before the module is imported, so its libraries need no run path)
+    cmd = ["g++", "-O2", "-std=c++20", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           f"-I{ROOT / 'include'}", *(f"-isystem{p}" for p in include_paths()), f"-I{sysconfig.get_paths()['include']}",
+           f"-I{cuda / 'include'}", *_suffix_flags(), str(src), "-o", str(out), f"-L{PKG}", "-l:libaotriton_v2.so", f"-L{lib}",
+           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10_cuda", "-lc10", "-Wl,-rpath,$ORIGIN"]
+    stamp = OBJ / "torch_ops.stamp"
+    want = _digest([src, *HEADERS], " ".join(cmd) + torch.__version__)
+    if out.exists() and stamp.exists() and stamp.read_text() == want:
+        return out
+    _run(cmd)
+    stamp.write_text(want)
+    return out
+
+
 def build_all(verbose_ptxas: bool = False) -> None:
     build_library(verbose_ptxas)
-    build_pymodule()
+    with ThreadPoolExecutor(max_workers=2) as ex:
+        list(ex.map(lambda f: f(), (build_pymodule, build_torch_ops)))
 
 
 if __name__ == "__main__":
     os.environ.setdefault("AB200_BUILD_VERBOSE", "1")
     build_all(verbose_ptxas="-v" in sys.argv)
-    print("built", LIB, "and", pymodule_path())
+    print("built", LIB, pymodule_path(), "and", torch_ops_path())
