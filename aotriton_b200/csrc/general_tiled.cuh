@@ -36,31 +36,42 @@ __device__ __forceinline__ bool rows_vec4(const View4& v, int d) {
 // forward's time went by waiting for them.)
 template <typename T, int DP, int ROWS, int THREADS>
 __device__ __forceinline__ void stage_tile(float* dst, const View4& v, int b, int h, int64_t tok0, int row0, int nrows, int d, bool vec, int tid) {
-  constexpr int kLd = Tiled<DP>::kLd, kC4 = DP / 4;
-  const T* base = row_ptr<T>(v, b, h, tok0 + row0);
-#pragma unroll 8
-  for (int idx = tid; idx < ROWS * kC4; idx += THREADS) {
-    const int r = idx / kC4, c = (idx - r * kC4) * 4;
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (row0 + r < nrows && c < d) {
-      const T* src = base + (int64_t)r * v.s[2] + c;
-      if (vec) {
-        if constexpr (sizeof(T) == 4) {
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ptx::smem_u32(dst + r * kLd + c)), "l"(src) : "memory");
-          continue;
-        } else {
-          const uint2 w = __ldg(reinterpret_cast<const uint2*>(src));
+  constexpr int kLd = Tiled<DP>::kLd, kC4 = DP / 4, kStep = THREADS / kC4;      // a thread's column, rows kStep apart
+  static_assert(THREADS % kC4 == 0 && ROWS % kStep == 0, "whole rows a pass");
+  const int r0 = tid / kC4, c = (tid - r0 * kC4) * 4;
+  const T* src = row_ptr<T>(v, b, h, tok0 + row0 + r0) + c;
+  dst += r0 * kLd + c;
+  // (rolled up where nothing is gained: the unrolled forms of all a kernel's tiles together did not fit the instruction cache)
+  if constexpr (sizeof(T) == 4) {
+    if (vec) {
+      const int in = c < d ? nrows - row0 - r0 : 0;      // rows to copy from here on
+      uint32_t to = ptx::smem_u32(dst);
+      const int64_t step = kStep * v.s[2];
+#pragma unroll 2
+      for (int i = 0; i < ROWS; i += kStep, to += kStep * kLd * 4, src += step)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                     ::"r"(to), "l"(i < in ? src : reinterpret_cast<const T*>(v.ptr)), "r"(i < in ? 16 : 0) : "memory");
+    }
+  }
+  if (sizeof(T) != 4 || !vec) {
+#pragma unroll (sizeof(T) == 4 ? 1 : 4)
+    for (int i = 0; i < ROWS / kStep; ++i) {
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (row0 + r0 + i * kStep < nrows && c < d) {
+        const T* s = src + (int64_t)(i * kStep) * v.s[2];
+        if (vec) {
+          const uint2 w = __ldg(reinterpret_cast<const uint2*>(s));
           const T* e = reinterpret_cast<const T*>(&w);
           x = make_float4(to_f32<T>(e[0]), to_f32<T>(e[1]), to_f32<T>(e[2]), to_f32<T>(e[3]));
+        } else {
+          x.x = to_f32<T>(s[0]);
+          if (c + 1 < d) x.y = to_f32<T>(s[1]);
+          if (c + 2 < d) x.z = to_f32<T>(s[2]);
+          if (c + 3 < d) x.w = to_f32<T>(s[3]);
         }
-      } else {
-        x.x = to_f32<T>(src[0]);
-        if (c + 1 < d) x.y = to_f32<T>(src[1]);
-        if (c + 2 < d) x.z = to_f32<T>(src[2]);
-        if (c + 3 < d) x.w = to_f32<T>(src[3]);
       }
+      *reinterpret_cast<float4*>(dst + i * kStep * kLd) = x;
     }
-    *reinterpret_cast<float4*>(dst + r * kLd + c) = x;
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
