@@ -263,9 +263,15 @@ __device__ __forceinline__ void philox4x32_10_lockstep(uint64_t seed, uint32_t (
   }
 }
 
-// Keep bits of N counters as nibbles (nibble n, bit j = column 4c+j of counter n).  `offset(n)`: the n-th counter.
+// Keep bits of one row (or key) and 32 columns: the bit of column 4a + b is bit 8b + 7 - a, so that the word shifted left by a
+// has the bits of columns 4a..4a+3 as the signs of its bytes, which one byte permute spreads over a pair of 16-bit halves
+// (keep_mask).  In the natural order a column took a test and a select of its own, for P and again for dP.  Measured, dK/dV and dQ on
+// the device, ms (with the reads of dP in two halves, sm100_bwd.cu): 16 packed sequences of 64 to 8192 tokens, 32:8 heads of 128, 9.93 ->
+// 8.98 and 5.54 -> 5.45; 8 x 16 heads x 2048 of 72 with bias 1.42 -> 1.31 and 1.145 -> 1.139; head dim 256, dV, 1.92 -> 1.79.
+// keep_bits(): the bits of counters `first`..`first` + N - 1 of such a word, counter a being columns 4a..4a+3.  `offset(n)`: the
+// n-th of them.
 template <int N, typename F>
-__device__ __forceinline__ uint32_t dropout_keep_nibbles(uint64_t seed, int32_t threshold, F offset) {
+__device__ __forceinline__ uint32_t keep_bits(uint64_t seed, int32_t threshold, int first, F offset) {
   uint32_t c[N][4], k = 0u;
 #pragma unroll
   for (int n = 0; n < N; ++n) {
@@ -276,12 +282,21 @@ __device__ __forceinline__ uint32_t dropout_keep_nibbles(uint64_t seed, int32_t 
   philox4x32_10_lockstep<N>(seed, c);
 #pragma unroll
   for (int n = 0; n < N; ++n) {
-    k |= ((int32_t)c[n][0] > threshold) ? 1u << (4 * n) : 0u;
-    k |= ((int32_t)c[n][2] > threshold) ? 2u << (4 * n) : 0u;
-    k |= ((int32_t)c[n][1] > threshold) ? 4u << (4 * n) : 0u;
-    k |= ((int32_t)c[n][3] > threshold) ? 8u << (4 * n) : 0u;
+    k |= ((int32_t)c[n][0] > threshold) ? 1u << (7 - first - n) : 0u;
+    k |= ((int32_t)c[n][2] > threshold) ? 1u << (15 - first - n) : 0u;
+    k |= ((int32_t)c[n][1] > threshold) ? 1u << (23 - first - n) : 0u;
+    k |= ((int32_t)c[n][3] > threshold) ? 1u << (31 - first - n) : 0u;
   }
   return k;
+}
+__device__ __forceinline__ int keep_bit_of(int column) { return 8 * (column & 3) + 7 - (column >> 2); }
+__device__ __forceinline__ int keep_column_of(int bit) { return 4 * (7 - (bit & 7)) + (bit >> 3); }
+// Columns 2 * pair and 2 * pair + 1 of a keep word: all ones in the halves of those that are kept.
+__device__ __forceinline__ uint32_t keep_mask(uint32_t w, int pair) {
+  uint32_t m;
+  if (pair & 1) asm("prmt.b32 %0, %1, 0, 0xbbaa;" : "=r"(m) : "r"(w << (pair >> 1)));
+  else asm("prmt.b32 %0, %1, 0, 0x9988;" : "=r"(m) : "r"(w << (pair >> 1)));
+  return m;
 }
 
 // ---------------------------------------------------------------------------
@@ -289,8 +304,7 @@ __device__ __forceinline__ uint32_t dropout_keep_nibbles(uint64_t seed, int32_t 
 // per four scores), and dK/dV and dQ need the same bits.  When both run in one call, the kernel that
 // runs first (dK/dV; dV for wide heads) leaves the bits it drew in rows of dQ that only the last kernel
 // writes, and the later ones read them: one bit per score moved instead of ten Philox rounds per four.
-// Unit: 32 query rows (aligned to 32 in the sequence) x 32 keys = 32 words, one per query row, bit c =
-// key c of the tile.  The words of a tile are 128 contiguous bytes (one coalesced access of a warp) in one
+// Unit: 32 query rows (aligned to 32 in the sequence) x 32 keys = 32 words, one per query row (keep_bits()).  The words of a tile are 128 contiguous bytes (one coalesced access of a warp) in one
 // of the same 32 rows of dQ; a row takes 2^keep_shift tiles (its 2 * dqk bytes allow no more), so the 32 rows
 // hold 32 << keep_shift key tiles: 1024 keys at head dims 64 to 127, 2048 up to 255, 4096 at 256.  Tiles
 // further right, partial row groups and all other launches draw their bits.
@@ -315,14 +329,25 @@ __device__ __forceinline__ bool keep_shared(const Params& p, const Seq& sq, int 
   return !p.causal || ((int64_t)row32 + 31 + sq.wr >= key0 && (int64_t)row32 - sq.wl <= (int64_t)key0 + 31);
 }
 
-// The writer's side.  Lane 4a + q of a warp holds in nibble k the bits of keys 4a..4a+3 for query row q + 4k;
-// an 8 x 8 transpose of nibbles over the lanes with the same q gives lane l the 32 bits of query row l.
+// Key-per-thread kernels: a counter serves four consecutive keys of one query row, and the four lanes of a quad own exactly such
+// keys.  Lane 4a + q of a warp draws for query rows q + 4k (k = 0..7): byte j, bit 7 - k of `x` is key 4a + j.
+
+// The bits of this lane's own key over the 32 query rows, as a keep word.
+__device__ __forceinline__ uint32_t keep_word_of_key(uint32_t x, int lane) {
+  const uint32_t sel = (uint32_t)(lane & 3) | (uint32_t)(4 + (lane & 3)) << 4;      // (the byte of this lane's key in either word)
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) w[i] = __shfl_sync(0xffffffffu, x, (lane & ~3) | i);
+  return __byte_perm(__byte_perm(w[0], w[1], sel), __byte_perm(w[2], w[3], sel), 0x5410);
+}
+// The writer's side: an 8 x 8 transpose of bits over the lanes with the same q, in each byte, gives lane l the keep word of query
+// row l.  (Lane bit against bit index, which counts down: lane 4a + q, bit 7 - k goes to lane 4k + q, bit 7 - a.)
 __device__ __forceinline__ uint32_t keep_rows_from_quads(uint32_t x, int lane) {
 #pragma unroll
   for (int b = 1; b < 8; b <<= 1) {
-    const uint32_t m = b == 1 ? 0x0f0f0f0fu : (b == 2 ? 0x00ff00ffu : 0x0000ffffu);
+    const uint32_t m = b == 1 ? 0xaaaaaaaau : (b == 2 ? 0xccccccccu : 0xf0f0f0f0u);
     const uint32_t y = __shfl_xor_sync(0xffffffffu, x, 4 * b);
-    x = (lane & (4 * b)) ? ((x & ~m) | ((y >> (4 * b)) & m)) : ((x & m) | ((y << (4 * b)) & ~m));
+    x = (lane & (4 * b)) ? ((x & ~m) | ((y & ~m) << b)) : ((x & m) | ((y & m) >> b));
   }
   return x;
 }
@@ -336,6 +361,11 @@ __device__ __forceinline__ uint32_t transpose_bits32(uint32_t x, int lane) {
     x = (lane & b) ? ((x & ~m) | ((y >> b) & m)) : ((x & m) | ((y << b) & ~m));
   }
   return x;
+}
+// A reader whose lanes are keys: lane l has the keep word of query row l and gets that of key l.
+__device__ __forceinline__ uint32_t keep_keys_from_rows(uint32_t x, int lane) {
+  x = __shfl_sync(0xffffffffu, x, keep_column_of(lane));      // (rows in the order of their bits)
+  return __shfl_sync(0xffffffffu, transpose_bits32(x, lane), keep_bit_of(lane));
 }
 
 // ---------------------------------------------------------------------------

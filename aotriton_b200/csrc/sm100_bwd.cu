@@ -279,8 +279,8 @@ __device__ __forceinline__ DkdvItem dkdv_item(const Params& p, int w) {
 // MMA issuer's loop is latency-critical: even untaken branches and call sites in it cost several
 // per cent of the kernel's time).
 // FEAT (features()): at 96 registers a thread the compute warps' loop spills, and what dropout and bias keep there
-// (generator state, row pointers, strides) is most of it: at head dim 128 dK/dV stores 156 bytes with dropout, 100 with bias,
-// 52 with neither, dQ 44, 28 and none.  Measured, whole backward, us, dropout's instantiation against the call's own:
+// (generator state, row pointers, strides) is most of it: at head dim 128 dK/dV stores 148 bytes with dropout, 92 with bias,
+// none with neither, dQ 44, 28 and none.  Measured, whole backward, us, dropout's instantiation against the call's own:
 // neither, dense causal 4 x 32 heads x 4096 of 128 1875 -> 1768, 64:8 heads x 16384, window 4096, 6530 -> 6200; bias,
 // 4 x 8 heads x 1024 of 64 131.5 -> 113.1, 4 x 8:2 heads x 1024 of 128 with dBias 228 -> 207.
 template <typename T, int HD, bool FUSED, bool EXACT, int FEAT>
@@ -780,65 +780,61 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         if (threadIdx.x == AB200_TRACE_TID) AB200_STAMP(G, 7);
         uint32_t keep = 0xffffffffu;
         if (drop_on) {
-          // One Philox counter serves four consecutive keys of one query row, and the four lanes of
-          // a quad own exactly such keys (same n >> 2): lane q4 of the quad draws the counters of
-          // query rows mbase + q4 + 4k (k = 0..7) for all four keys, then the quad exchanges them.
+          // lane q4 of a quad draws the counters of query rows mbase + q4 + 4k (k = 0..7) for all four keys
           const DropoutCtx dctx = dropout_ctx_from(p, ph_seed, ph_off, z, h);
           const int q4 = lane & 3;
-          uint32_t mine = 0u;            // nibble k: keep bits of keys 4a..4a+3 for query row mbase + q4 + 4k
+          uint32_t mine = 0u;
 #pragma unroll
           for (int k = 0; k < 8; k += 4)
-            mine |= dropout_keep_nibbles<4>(dctx.seed, dctx.threshold, [&](int u) {
-                      return dctx.base + (uint64_t)min(mbase + q4 + 4 * (k + u), p.max_sq - 1) * dctx.stride + (uint64_t)(n >> 2);
-                    }) << (4 * k);
+            mine |= keep_bits<4>(dctx.seed, dctx.threshold, k, [&](int u) {
+              return dctx.base + (uint64_t)min(mbase + q4 + 4 * (k + u), p.max_sq - 1) * dctx.stride + (uint64_t)(n >> 2);
+            });
           if (keep_shared(p, sq, mbase, it.n0 + quarter * 32))
             *keep_share_word(p, sq, h, mbase, it.n0 + quarter * 32, lane) = keep_rows_from_quads(mine, lane);
-          keep = 0u;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const uint32_t w = __shfl_sync(0xffffffffu, mine, (lane & ~3) | i);
-            keep |= ((w >> q4) & 0x11111111u) << i;      // this lane's key, query rows mbase + i + 4k -> bit 4k + i
-          }
+          keep = keep_word_of_key(mine, lane);
         }
         if (threadIdx.x == AB200_TRACE_TID) AB200_STAMP(G, 1);
         if (!mbar_wait(&bars[L::bDpFull], par, abort_flag, status, 0x1900)) { ok = false; break; }
         if (threadIdx.x == AB200_TRACE_TID) AB200_STAMP(G, 2);
         tc_fence_after();
         {
-          float dp[32];
-          tmem_ld32f(tmem_base + lane_addr + kColDP + cbase, dp);
+          // P^T goes over the first half of this thread's 32 columns of dP once that half has been read; the second half follows
+          // under the first one's arithmetic and makes room for dS^T.  (All 32 at once are 16 more registers at the point where
+          // the fewest are free: 52 bytes spilled without dropout and bias, 220 with dropout.  Dense causal 4 x 32 heads x 4096 982 -> 960 us.)
+          const uint32_t dp_col = tmem_base + lane_addr + kColDP + cbase;
+          float dp[2][16];
+          uint32_t pk[16];
+          tmem_ld16f(dp_col, dp[0]);
           tmem_wait_ld();
           if (threadIdx.x == AB200_TRACE_TID) AB200_STAMP(G, 10);
-          // This thread has now read its 32 columns of dP: they can take P^T (packed, 16 columns)
-          // followed by dS^T (packed, 16 columns).
-          uint32_t pk[16];
 #pragma unroll
           for (int c = 0; c < 16; ++c) {
-            float a = pr[2 * c], b = pr[2 * c + 1];
-            if (drop_on) {
-              a = ((keep >> (2 * c)) & 1u) ? a * p.dropout_scale : 0.f;
-              b = ((keep >> (2 * c + 1)) & 1u) ? b * p.dropout_scale : 0.f;
-            }
-            pk[c] = pack2<T>(a, b);
+            pk[c] = pack2<T>(pr[2 * c], pr[2 * c + 1]);
+            if constexpr (FEAT == kDropout) pk[c] &= keep_mask(keep, c);      // (1 / (1 - p) follows at the write-out of dV)
           }
-          tmem_st16(tmem_base + lane_addr + kColDP + cbase, pk);
+          tmem_st16(dp_col, pk);
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars[L::bPFull]);
-          if (drop_on) {
-#pragma unroll
-            for (int c = 0; c < 32; ++c) dp[c] = ((keep >> c) & 1u) ? dp[c] * p.dropout_scale : 0.f;
-          }
+          tmem_ld16f(dp_col + 16, dp[1]);
+          const float2 ds2 = make_float2(p.dropout_scale, p.dropout_scale);
 #pragma unroll
           for (int c4 = 0; c4 < 8; ++c4) {
+            if (c4 == 4) tmem_wait_ld();
+            const float* d = &dp[c4 >> 2][4 * (c4 & 3)];
             const float4 d4 = lds128(dlt + 16u * c4);
-            const float2 a = mul2(make_float2(pr[4 * c4], pr[4 * c4 + 1]),
-                                  add2(make_float2(dp[4 * c4], dp[4 * c4 + 1]), make_float2(d4.x, d4.y)));
-            const float2 b = mul2(make_float2(pr[4 * c4 + 2], pr[4 * c4 + 3]),
-                                  add2(make_float2(dp[4 * c4 + 2], dp[4 * c4 + 3]), make_float2(d4.z, d4.w)));
-            pk[2 * c4] = pack2<T>(a.x, a.y);
-            pk[2 * c4 + 1] = pack2<T>(b.x, b.y);
+            const float2 p0 = make_float2(pr[4 * c4], pr[4 * c4 + 1]), p1 = make_float2(pr[4 * c4 + 2], pr[4 * c4 + 3]);
+            const float2 dp0 = make_float2(d[0], d[1]), dp1 = make_float2(d[2], d[3]);
+            const float2 nd0 = make_float2(d4.x, d4.y), nd1 = make_float2(d4.z, d4.w);
+            if constexpr (FEAT == kDropout) {
+              pk[2 * c4] = dropout_ds_pair<T>(p0, dp0, ds2, nd0, keep_mask(keep, 2 * c4));
+              pk[2 * c4 + 1] = dropout_ds_pair<T>(p1, dp1, ds2, nd1, keep_mask(keep, 2 * c4 + 1));
+            } else {
+              const float2 a = mul2(p0, add2(dp0, nd0)), b = mul2(p1, add2(dp1, nd1));
+              pk[2 * c4] = pack2<T>(a.x, a.y);
+              pk[2 * c4 + 1] = pack2<T>(b.x, b.y);
+            }
           }
           tmem_st16(tmem_base + lane_addr + kColDP + cbase + 16, pk);
           if constexpr (FUSED) {
@@ -900,7 +896,7 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         tc_fence_after();
         tmem_ld32f(tmem_base + lane_addr + kColAcc0 + d0, v);
         tmem_wait_ld();
-        stage_put32<T>(stage, r, d0, v, 1.0f, HD * 2);
+        stage_put32<T>(stage, r, d0, v, FEAT == kDropout ? p.dropout_scale : 1.0f, HD * 2);
         __syncwarp();
         warp_copy_out<T, 4>(stage, reinterpret_cast<T*>(p.dv.ptr) + (int64_t)sq.bidx * p.dv.s[0] + (int64_t)hk * p.dv.s[1] +
                                        (sq.k0 + it.n0) * p.dv.s[2],
@@ -1292,9 +1288,9 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
         const int md = min(m, p.max_sq - 1);
 #pragma unroll
         for (int c4 = 0; c4 < 8; c4 += 4)
-          keep |= dropout_keep_nibbles<4>(dctx.seed, dctx.threshold, [&](int u) {
-                    return dctx.base + (uint64_t)md * dctx.stride + (uint64_t)((nbase >> 2) + c4 + u);
-                  }) << (4 * c4);
+          keep |= keep_bits<4>(dctx.seed, dctx.threshold, c4, [&](int u) {
+            return dctx.base + (uint64_t)md * dctx.stride + (uint64_t)((nbase >> 2) + c4 + u);
+          });
       }
       const uint32_t dp_col = tmem_base + lane_addr + kColDP + (uint32_t)(i & 1) * 128u + cbase;
       if (threadIdx.x == AB200_TRACE_TID) AB200_STAMPQ(i, 7);
@@ -1306,16 +1302,17 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
         tmem_ld32f(dp_col, dp);
         tmem_wait_ld();
         if (threadIdx.x == AB200_TRACE_TID) AB200_STAMPQ(i, 10);
-        if (drop_on) {
-#pragma unroll
-          for (int c = 0; c < 32; ++c) dp[c] = ((keep >> c) & 1u) ? dp[c] * p.dropout_scale : 0.f;
-        }
         uint32_t pk[16];
-        const float2 dl2 = make_float2(dlt, dlt);
+        const float2 dl2 = make_float2(dlt, dlt), nd2 = make_float2(-dlt, -dlt), ds2 = make_float2(p.dropout_scale, p.dropout_scale);
 #pragma unroll
         for (int c = 0; c < 16; ++c) {
-          const float2 a = mul2(make_float2(pr[2 * c], pr[2 * c + 1]), sub2(make_float2(dp[2 * c], dp[2 * c + 1]), dl2));
-          pk[c] = pack2<T>(a.x, a.y);
+          const float2 p2 = make_float2(pr[2 * c], pr[2 * c + 1]), dp2 = make_float2(dp[2 * c], dp[2 * c + 1]);
+          if constexpr (FEAT == kDropout) {
+            pk[c] = dropout_ds_pair<T>(p2, dp2, ds2, nd2, keep_mask(keep, c));
+          } else {
+            const float2 a = mul2(p2, sub2(dp2, dl2));
+            pk[c] = pack2<T>(a.x, a.y);
+          }
         }
         tmem_st16(dp_col, pk);
         if (dbias_on && m < sq.sq) {

@@ -436,29 +436,22 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         }
         uint32_t keep = 0xffffffffu;
         if (shared) {
-          keep = transpose_bits32(shared_bits, lane);      // (this lane's key, query rows in the bits)
+          keep = keep_keys_from_rows(shared_bits, lane);
         } else if (drop_on) {
-          // One Philox counter serves four consecutive keys of one query row, and the four lanes of
-          // a quad own exactly such keys: lane q4 of the quad draws the counters of query rows
-          // mbase + q4 + 4k (k = 0..7) for all four keys, then the quad exchanges them.
+          // lane q4 of a quad draws the counters of query rows mbase + q4 + 4k (k = 0..7) for all four keys
           const DropoutCtx dctx = dropout_ctx_from(p, ph_seed, ph_off, z, h);
           const int q4 = lane & 3;
           uint32_t mine = 0u;
 #pragma unroll
           for (int k = 0; k < 8; k += 4)
-            mine |= dropout_keep_nibbles<4>(dctx.seed, dctx.threshold, [&](int u) {
-                      return dctx.base + (uint64_t)min(mbase + q4 + 4 * (k + u), p.max_sq - 1) * dctx.stride + (uint64_t)(n >> 2);
-                    }) << (4 * k);
+            mine |= keep_bits<4>(dctx.seed, dctx.threshold, k, [&](int u) {
+              return dctx.base + (uint64_t)min(mbase + q4 + 4 * (k + u), p.max_sq - 1) * dctx.stride + (uint64_t)(n >> 2);
+            });
           if constexpr (MODE == kWideDV) {
             if (keep_shared(p, sq, mbase, r0 + quarter * 32))
               *keep_share_word(p, sq, h, mbase, r0 + quarter * 32, lane) = keep_rows_from_quads(mine, lane);
           }
-          keep = 0u;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint32_t w = __shfl_sync(0xffffffffu, mine, (lane & ~3) | j);
-            keep |= ((w >> q4) & 0x11111111u) << j;      // this lane's key, query rows mbase + j + 4k -> bit 4k + j
-          }
+          keep = keep_word_of_key(mine, lane);
         }
         // dP' of this block is there (dK); for dV the same barrier says that the buffer's previous
         // P' has been consumed
@@ -469,30 +462,28 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         if constexpr (MODE == kWideDV) {
 #pragma unroll
           for (int c = 0; c < 16; ++c) {
-            float a = pr[2 * c], b = pr[2 * c + 1];
-            if (drop_on) {
-              a = ((keep >> (2 * c)) & 1u) ? a * p.dropout_scale : 0.f;
-              b = ((keep >> (2 * c + 1)) & 1u) ? b * p.dropout_scale : 0.f;
-            }
-            pk[c] = pack2<T>(a, b);
+            pk[c] = pack2<T>(pr[2 * c], pr[2 * c + 1]);
+            if constexpr (FEAT == kDropout) pk[c] &= keep_mask(keep, c);      // (1 / (1 - p) follows at the write-out)
           }
         } else {
           float dp[32];
           tmem_ld32f(a_col, dp);
           tmem_wait_ld();
-          if (drop_on) {
-#pragma unroll
-            for (int c = 0; c < 32; ++c) dp[c] = ((keep >> c) & 1u) ? dp[c] * p.dropout_scale : 0.f;
-          }
+          const float2 ds2 = make_float2(p.dropout_scale, p.dropout_scale);
 #pragma unroll
           for (int c4 = 0; c4 < 8; ++c4) {
             const float4 d4 = lds128(dlt + 16u * c4);
-            const float2 a = mul2(make_float2(pr[4 * c4], pr[4 * c4 + 1]),
-                                  add2(make_float2(dp[4 * c4], dp[4 * c4 + 1]), make_float2(d4.x, d4.y)));
-            const float2 b = mul2(make_float2(pr[4 * c4 + 2], pr[4 * c4 + 3]),
-                                  add2(make_float2(dp[4 * c4 + 2], dp[4 * c4 + 3]), make_float2(d4.z, d4.w)));
-            pk[2 * c4] = pack2<T>(a.x, a.y);
-            pk[2 * c4 + 1] = pack2<T>(b.x, b.y);
+            const float2 p0 = make_float2(pr[4 * c4], pr[4 * c4 + 1]), p1 = make_float2(pr[4 * c4 + 2], pr[4 * c4 + 3]);
+            const float2 dp0 = make_float2(dp[4 * c4], dp[4 * c4 + 1]), dp1 = make_float2(dp[4 * c4 + 2], dp[4 * c4 + 3]);
+            const float2 nd0 = make_float2(d4.x, d4.y), nd1 = make_float2(d4.z, d4.w);
+            if constexpr (FEAT == kDropout) {
+              pk[2 * c4] = dropout_ds_pair<T>(p0, dp0, ds2, nd0, keep_mask(keep, 2 * c4));
+              pk[2 * c4 + 1] = dropout_ds_pair<T>(p1, dp1, ds2, nd1, keep_mask(keep, 2 * c4 + 1));
+            } else {
+              const float2 a = mul2(p0, add2(dp0, nd0)), b = mul2(p1, add2(dp1, nd1));
+              pk[2 * c4] = pack2<T>(a.x, a.y);
+              pk[2 * c4 + 1] = pack2<T>(b.x, b.y);
+            }
           }
         }
         tmem_st16(a_col, pk);
@@ -586,9 +577,9 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           const int md = min(m, p.max_sq - 1);
 #pragma unroll
           for (int c4 = 0; c4 < 8; c4 += 4)
-          keep |= dropout_keep_nibbles<4>(dctx.seed, dctx.threshold, [&](int u) {
-                    return dctx.base + (uint64_t)md * dctx.stride + (uint64_t)((nbase >> 2) + c4 + u);
-                  }) << (4 * c4);
+            keep |= keep_bits<4>(dctx.seed, dctx.threshold, c4, [&](int u) {
+              return dctx.base + (uint64_t)md * dctx.stride + (uint64_t)((nbase >> 2) + c4 + u);
+            });
         }
         const uint32_t a_col = tmem_base + lane_addr + kWColDP + (uint32_t)s * 64u + cbase;
         if (!mbar_wait(&bars[L::bDpFull + s], par2, abort_flag, status, 0x3D00)) { ok = false; break; }
@@ -597,16 +588,17 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           float dp[32];
           tmem_ld32f(a_col, dp);
           tmem_wait_ld();
-          if (drop_on) {
-#pragma unroll
-            for (int c = 0; c < 32; ++c) dp[c] = ((keep >> c) & 1u) ? dp[c] * p.dropout_scale : 0.f;
-          }
           uint32_t pk[16];
-          const float2 dl2 = make_float2(dlt, dlt);
+          const float2 dl2 = make_float2(dlt, dlt), nd2 = make_float2(-dlt, -dlt), ds2 = make_float2(p.dropout_scale, p.dropout_scale);
 #pragma unroll
           for (int c = 0; c < 16; ++c) {
-            const float2 a = mul2(make_float2(pr[2 * c], pr[2 * c + 1]), sub2(make_float2(dp[2 * c], dp[2 * c + 1]), dl2));
-            pk[c] = pack2<T>(a.x, a.y);
+            const float2 p2 = make_float2(pr[2 * c], pr[2 * c + 1]), dp2 = make_float2(dp[2 * c], dp[2 * c + 1]);
+            if constexpr (FEAT == kDropout) {
+              pk[c] = dropout_ds_pair<T>(p2, dp2, ds2, nd2, keep_mask(keep, c));
+            } else {
+              const float2 a = mul2(p2, sub2(dp2, dl2));
+              pk[c] = pack2<T>(a.x, a.y);
+            }
           }
           tmem_st16(a_col, pk);
           if (dbias_on && m < sq.sq) {
@@ -644,7 +636,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
       const int nrows = min(kBlk, rows_total - r0);
       T* dst = reinterpret_cast<T*>(outv.ptr) + (int64_t)sq.bidx * outv.s[0] + (int64_t)hrow * outv.s[1] +
                (row_tok0 + r0) * outv.s[2];
-      const float scale = MODE == kWideDV ? 1.0f : p.sm_scale;
+      const float scale = MODE != kWideDV ? p.sm_scale : (FEAT == kDropout ? p.dropout_scale : 1.0f);
       for (int c = wg; c * 32 < d_out; c += 2) {
         float v[32];
         tmem_ld32f(tmem_base + lane_addr + kWColAcc + c * 32, v);

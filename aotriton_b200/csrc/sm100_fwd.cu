@@ -95,41 +95,6 @@ struct FwdSmem {
   static constexpr int kDynamic = kTotal + 1024;             // slack for manual 1024-byte alignment
 };
 
-// Keep bits of one row and 32 keys, in the order in which the softmax warps use them: the bit of key 4c + i is
-// bit 8i + 7 - c, so that the word shifted left by c has the bits of keys 4c..4c+3 as the signs of its bytes.
-__device__ __forceinline__ uint32_t draw_keep_word(uint64_t seed, uint64_t offset, int32_t threshold) {
-  uint32_t w = 0u;
-#pragma unroll
-  for (int h = 0; h < 8; h += 4) {
-    uint32_t c[4][4];
-#pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      c[n][0] = (uint32_t)(offset + (uint64_t)(h + n));
-      c[n][1] = (uint32_t)((offset + (uint64_t)(h + n)) >> 32);
-    }
-    philox4x32_10_lockstep<4>(seed, c);
-#pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      w |= ((int32_t)c[n][0] > threshold) ? 1u << (7 - h - n) : 0u;
-      w |= ((int32_t)c[n][2] > threshold) ? 1u << (15 - h - n) : 0u;
-      w |= ((int32_t)c[n][1] > threshold) ? 1u << (23 - h - n) : 0u;
-      w |= ((int32_t)c[n][3] > threshold) ? 1u << (31 - h - n) : 0u;
-    }
-  }
-  return w;
-}
-// 16 packed pairs of 16-bit probabilities (32 keys): the dropped ones become zero.
-__device__ __forceinline__ void apply_keep_word(uint32_t* pk, uint32_t w) {
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    uint32_t lo, hi;      // byte signs spread over halves: keys 4c, 4c+1 and 4c+2, 4c+3
-    asm("prmt.b32 %0, %1, 0, 0x9988;" : "=r"(lo) : "r"(w << c));
-    asm("prmt.b32 %0, %1, 0, 0xbbaa;" : "=r"(hi) : "r"(w << c));
-    pk[2 * c] &= lo;
-    pk[2 * c + 1] &= hi;
-  }
-}
-
 // Rows [m0, m0+rows) of the output that have no key at all: O = 0, LSE = +inf.
 template <typename T>
 __device__ void write_dead_rows(const Params& p, const Seq& sq, int h, int m0, int rows) {
@@ -410,7 +375,11 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
           const uint64_t offset = dctx.base + (uint64_t)mm * dctx.stride + (uint64_t)((jb_lo + j) * (kBN / 4));
           uint32_t* dst = reinterpret_cast<uint32_t*>(smem + L::kKeep + buf * L::kKeepTile) + r * 4;
 #pragma unroll 1
-          for (int u = 0; u < 4; ++u) dst[u] = draw_keep_word(dctx.seed, offset + (uint64_t)(8 * u), dctx.threshold);
+          for (int u = 0; u < 4; ++u) {
+            auto counter = [&](int n) { return offset + (uint64_t)(8 * u + n); };
+            dst[u] = keep_bits<4>(dctx.seed, dctx.threshold, 0, counter) |
+                     keep_bits<4>(dctx.seed, dctx.threshold, 4, [&](int n) { return counter(4 + n); });
+          }
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars[L::bKeepFull + buf]);
         }
@@ -647,8 +616,8 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
               __syncwarp();
               if (lane == 0) mbar_arrive(&bars[L::bKeepEmpty + buf]);
             }
-            apply_keep_word(pk, half == 0 ? keep.x : keep.z);
-            apply_keep_word(pk + 16, half == 0 ? keep.y : keep.w);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) pk[i] &= keep_mask(half == 0 ? (i < 16 ? keep.x : keep.y) : (i < 16 ? keep.z : keep.w), i & 15);
           }
           tmem_st32(s_addr + half * 32, pk);
         }

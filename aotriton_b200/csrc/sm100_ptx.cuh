@@ -372,6 +372,11 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
       "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -407,6 +412,15 @@ template <>
 __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
+}
+
+// Score gradients of two neighbouring columns, packed: P * (keep ? dP / (1 - p) : 0  -  delta), `nd` = -delta, `mask` from keep_mask().
+// Both outcomes are formed and the packed words selected by the mask, so that a dropped dP, finite or not, has no part.
+template <typename T>
+__device__ __forceinline__ uint32_t dropout_ds_pair(float2 pr, float2 dp, float2 scale, float2 nd, uint32_t mask) {
+  const float2 kept = ptx::mul2(pr, ptx::fma2(dp, scale, nd)), dropped = ptx::mul2(pr, nd);
+  const uint32_t a = pack2<T>(kept.x, kept.y), b = pack2<T>(dropped.x, dropped.y);
+  return (mask & a) | (~mask & b);
 }
 
 inline bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; }
