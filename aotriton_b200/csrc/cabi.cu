@@ -246,10 +246,13 @@ struct DeviceGuard {
   ~DeviceGuard() { if (switched_) { (void)host().set_device(old_); } }
 };
 
-bool rows_16byte(const void* ptr, const int64_t* stride) {
-  return ptr != nullptr && (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0 && stride[3] == 1 && stride[0] % 8 == 0 &&
-         stride[1] % 8 == 0 && stride[2] % 8 == 0;
+bool rows_aligned(const void* ptr, const int64_t* stride, int elements) {      // unit-stride rows of 16-bit elements
+  return ptr != nullptr && (reinterpret_cast<uintptr_t>(ptr) & (2 * elements - 1)) == 0 && stride[3] == 1 && stride[0] % elements == 0 &&
+         stride[1] % elements == 0 && stride[2] % elements == 0;
 }
+bool rows_16byte(const void* ptr, const int64_t* stride) { return rows_aligned(ptr, stride, 8); }
+// The widest accesses rows allow: 2 for 32 bytes, 1 for 16, 0 for single elements.
+int row_vec(const void* ptr, const int64_t* stride) { return rows_aligned(ptr, stride, 16) ? 2 : rows_aligned(ptr, stride, 8); }
 
 View4 to_view(const ab200_view4& v) {
   View4 r; r.ptr = v.ptr;
@@ -503,7 +506,7 @@ static int fill_fwd(const ab200_attn_fwd_args* a, Params& p) {
   if (!inner_contiguous(a->q) || !inner_contiguous(a->k) || !inner_contiguous(a->v) || !inner_contiguous(a->out))
     return kErrInvalidValue;
   p.q = to_view(a->q); p.k = to_view(a->k); p.v = to_view(a->v); p.out = to_view(a->out);
-  p.bias = to_view(a->bias); p.has_bias = a->bias.ptr != nullptr; p.bias_vec = rows_16byte(a->bias.ptr, a->bias.stride);
+  p.bias = to_view(a->bias); p.has_bias = a->bias.ptr != nullptr; p.bias_vec = row_vec(a->bias.ptr, a->bias.stride);
   p.lse = a->lse;
   p.seed_out = a->philox_seed_output; p.off_out = a->philox_offset_output;
   return 0;
@@ -564,12 +567,13 @@ static int fill_bwd(const ab200_attn_bwd_args* a, Params& p, bool need_outputs) 
       return kErrInvalidValue;
   }
   p.q = to_view(a->q); p.k = to_view(a->k); p.v = to_view(a->v);
-  p.bias = to_view(a->bias); p.has_bias = a->bias.ptr != nullptr; p.bias_vec = rows_16byte(a->bias.ptr, a->bias.stride);
+  p.bias = to_view(a->bias); p.has_bias = a->bias.ptr != nullptr; p.bias_vec = row_vec(a->bias.ptr, a->bias.stride);
   p.dq = to_view(a->dq); p.dk = to_view(a->dk); p.dv = to_view(a->dv); p.dbias = to_view(a->dbias);
   // dBias is skipped when absent or when all its strides are zero
   // (modules/flash/kernel/bwd_kernel_dq.py:265-266).
   p.has_dbias = a->dbias.ptr != nullptr &&
                 (a->dbias.stride[0] | a->dbias.stride[1] | a->dbias.stride[2] | a->dbias.stride[3]) != 0;
+  p.dbias_vec = row_vec(a->dbias.ptr, a->dbias.stride);
   return 0;
 }
 

@@ -47,7 +47,7 @@ struct Params {
   uint64_t *seed_out, *off_out;
   int32_t philox_head_offset, philox_hq;
   int32_t has_bias, has_dbias;
-  int32_t bias_vec;               // bias rows are 16-byte aligned and unit-stride: read eight values per load
+  int32_t bias_vec, dbias_vec;    // bias (dBias) rows are unit-stride and 16-byte (1), 32-byte (2) aligned, or not (0)
   uint32_t wait_limit_kcycles;    // bound of every in-kernel wait, in units of 1024 SM cycles (0 = about a second)
   int32_t drop_copy;              // test hook of the bounded waits: the producer leaves out one tile copy
                                   // (1 = first V block of the forward, 2 = first Q/dO block of dK/dV, 3 = first V block of dQ)
@@ -58,10 +58,14 @@ struct Params {
 
 // Geometry of one (sequence z) slice.
 // What a tcgen05 kernel is compiled with.  At most 96 to 216 registers a thread go to the compute warps; what
-// dropout (generator state, keep bits) and bias (row pointers, strides) need is spilled around every block even where a
-// call uses neither, so each has instantiations without them.
-enum : int { kPlain = 0, kBias = 1, kDropout = 2 };      // neither; bias, and its gradient or not; anything
-inline int features(const Params& p) { return p.dropout_on || (p.has_dbias && !p.has_bias) ? kDropout : (p.has_bias ? kBias : kPlain); }
+// dropout (generator state, keep bits) and bias (its tile, pointers, strides) need is spilled around every block even where a
+// call uses neither, so each combination has instantiations of its own.  kAll leaves everything to the run time (dBias without
+// bias too).
+enum : int { kPlain = 0, kBias = 1, kDropout = 2, kAll = 3 };      // bias, and its gradient or not; dropout; anything
+inline int features(const Params& p) {
+  if (p.has_dbias && !p.has_bias) return kAll;
+  return (p.has_bias ? kBias : 0) | (p.dropout_on ? kDropout : 0);
+}
 
 struct Seq {
   int32_t sq, sk;        // actual lengths

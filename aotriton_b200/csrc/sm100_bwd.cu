@@ -57,6 +57,7 @@
 #include <atomic>
 #include "launch.h"
 #include "sm100_ptx.cuh"
+#include "tile32.cuh"
 
 namespace ab200 {
 
@@ -156,51 +157,6 @@ __device__ __forceinline__ void store_row_chunk32(T* dst, const float* v, float 
   }
 }
 
-// Bias of a key-per-thread kernel.  A warp owns 32 keys (one per lane) x 32 query rows of the score
-// tile, i.e. a 32 x 32 tile of the bias matrix whose rows (queries) are 64 contiguous bytes.  A
-// thread needs a COLUMN of it; reading that directly takes 32 two-byte loads per thread at a row
-// stride.  Instead the warp reads the tile with four 16-byte loads per thread (load t: lane 8q+e
-// reads keys 8q..8q+7 of query row 8t+e) and transposes it in registers: within each group of
-// eight lanes an 8 x 8 transpose of 16-bit values, three exchange steps (lane bit <-> position bit).
-// Adds bias * log2(e) to pr[c] (c = query row in the tile).  `tile` points at (first query row,
-// first key of the warp); rows are `row_stride` elements apart and 16-byte aligned.
-template <typename T>
-__device__ __forceinline__ void add_bias_column32(float* pr, const T* tile, int64_t row_stride, int lane) {
-  const int q = lane >> 3, e = lane & 7;
-  uint4 raw[4];
-#pragma unroll
-  for (int t = 0; t < 4; ++t) raw[t] = __ldg(reinterpret_cast<const uint4*>(tile + (int64_t)(8 * t + e) * row_stride + 8 * q));
-#pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    uint32_t w[4] = {raw[t].x, raw[t].y, raw[t].z, raw[t].w};
-    // lane bit 0 <-> low/high half
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint32_t o = __shfl_xor_sync(0xffffffffu, w[k], 1);
-      w[k] = (lane & 1) ? __byte_perm(w[k], o, 0x3276) : __byte_perm(w[k], o, 0x5410);
-    }
-    // lane bit 1 <-> register index bit 0, lane bit 2 <-> register index bit 1
-#pragma unroll
-    for (int k = 0; k < 4; k += 2) {
-      const bool up = (lane & 2) != 0;
-      const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? w[k] : w[k + 1], 2);
-      if (up) w[k] = got; else w[k + 1] = got;
-    }
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const bool up = (lane & 4) != 0;
-      const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? w[k] : w[k + 2], 4);
-      if (up) w[k] = got; else w[k + 2] = got;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const T* h = reinterpret_cast<const T*>(&w[k]);
-      pr[8 * t + 2 * k] = fmaf(to_f32<T>(h[0]), kLog2e, pr[8 * t + 2 * k]);
-      pr[8 * t + 2 * k + 1] = fmaf(to_f32<T>(h[1]), kLog2e, pr[8 * t + 2 * k + 1]);
-    }
-  }
-}
-
 template <typename T>
 __device__ void zero_rows(const View4& v, int b, int h, int64_t tok0, int row0, int nrows, int d) {
   for (int r = threadIdx.x; r < kBlk; r += blockDim.x) {
@@ -279,10 +235,11 @@ __device__ __forceinline__ DkdvItem dkdv_item(const Params& p, int w) {
 // MMA issuer's loop is latency-critical: even untaken branches and call sites in it cost several
 // per cent of the kernel's time).
 // FEAT (features()): at 96 registers a thread the compute warps' loop spills, and what dropout and bias keep there
-// (generator state, row pointers, strides) is most of it: at head dim 128 dK/dV stores 148 bytes with dropout, 92 with bias,
-// none with neither, dQ 44, 28 and none.  Measured, whole backward, us, dropout's instantiation against the call's own:
-// neither, dense causal 4 x 32 heads x 4096 of 128 1875 -> 1768, 64:8 heads x 16384, window 4096, 6530 -> 6200; bias,
-// 4 x 8 heads x 1024 of 64 131.5 -> 113.1, 4 x 8:2 heads x 1024 of 128 with dBias 228 -> 207.
+// (generator state, bias tile, pointers, strides) is most of it: at head dim 128 dK/dV stores 148 bytes with both, 124 with
+// dropout, 84 with bias, none with neither; dQ 28 with both, else none.  Measured, whole backward, us, the instantiation for both against the
+// call's own: neither, dense causal 4 x 32 heads x 4096 of 128 1875 -> 1768, 64:8 heads x 16384, window 4096, 6530 -> 6200; bias,
+// 4 x 8 heads x 1024 of 64 131.5 -> 113.1, 4 x 8:2 heads x 1024 of 128 with dBias 228 -> 207; dropout, 16 packed sequences of 64 to 8192
+// tokens, 32:8 heads of 128, dK/dV 8980 -> 8713, dQ 5450 -> 4960; 16 x 12 x 391 of 64, training step, 324 -> 303.
 template <typename T, int HD, bool FUSED, bool EXACT, int FEAT>
 __global__ void __launch_bounds__(FUSED ? kFusedThreads : kBwdThreads, 1)
 sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm_q,
@@ -302,7 +259,7 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // (constants where FEAT leaves them out: nothing of theirs is compiled in)
-  const bool drop_on = FEAT == kDropout && p.dropout_on != 0, bias_on = FEAT == kBias || (FEAT == kDropout && p.has_bias != 0);
+  const bool drop_on = (FEAT & kDropout) && p.dropout_on != 0, bias_on = FEAT == kBias || (FEAT == kAll && p.has_bias != 0);
   // An earlier CTA timed out: the whole CTA leaves (one read, one CTA-wide decision).
   if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile unsigned int*>(status) != 0u)) return;
   if ((int)(smem - smem_raw) + L::kUsed > L::kDynamic) {      // the alignment padding did not fit
@@ -668,11 +625,23 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         const uint32_t lse2 = aux_s + (uint32_t)(s * 256 + cbase) * 4u;      // shared-space addresses
         const uint32_t dlt = lse2 + 128u * 4u;
         if (threadIdx.x == AB200_TRACE_TID) AB200_STAMP(G, 4);
-        // (the warp's 32 x 32 bias tile, one 64-byte row per lane: on its way to L2 meanwhile)
-        if (bias_on && p.bias_vec)
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
-                                                       (int64_t)h * p.bias.s[1] + (int64_t)min(mbase + lane, sq.sq - 1) * p.bias.s[2] +
-                                                       (it.n0 + quarter * 32)));
+        // the warp's 32 x 32 bias tile: on its way while the tensor pipe computes the scores, unless the generator's state is to find
+        // room as well (then 240 bytes are spilled instead of 148: head dim 72 with dropout 1.40 ms instead of 1.31)
+        const T* bias_tile = nullptr;
+        if (bias_on)
+          bias_tile = reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] + (int64_t)h * p.bias.s[1] +
+                      (int64_t)mbase * p.bias.s[2] + (int64_t)(it.n0 + quarter * 32) * p.bias.s[3];
+        uint4 braw[4];
+        auto load_bias = [&] {
+          tile32_load<T>(braw, bias_tile, p.bias.s[2], p.bias.s[3], p.bias_vec != 0, sq.sq - mbase, sq.sk - (it.n0 + quarter * 32), lane);
+        };
+        if constexpr (FEAT == kBias) load_bias();
+        if (bias_on && i + 1 < it.niter) {      // (hg, mb: the next block's by now)
+          const int mnext = (it.mb_lo + mb) * kBlk + cbase;
+          tile32_prefetch(reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] + (int64_t)(hk * p.group + hg) * p.bias.s[1] +
+                              (int64_t)mnext * p.bias.s[2] + (int64_t)(it.n0 + quarter * 32) * p.bias.s[3],
+                          p.bias.s[2], p.bias.s[3], sq.sq - mnext, sq.sk - (it.n0 + quarter * 32), lane);
+        }
         // S^T of this block and its logsumexp/delta stage (two arrivals on one barrier)
         if (!mbar_wait(&bars[L::bSFull + s], (G >> 1) & 1u, abort_flag, status, 0x1800)) { ok = false; break; }
         if (threadIdx.x == AB200_TRACE_TID) AB200_STAMP(G, 0);
@@ -744,23 +713,13 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars[L::bDqRead]);
           }
+          if (bias_on) {
+            if constexpr (FEAT != kBias) load_bias();
+            add_bias_column32<T>(pr, braw, p.qk_scale, lane);
+          } else {
 #pragma unroll
-          for (int c = 0; c < 32; ++c) pr[c] *= p.qk_scale;
-          if (bias_on && p.bias_vec && mbase + 32 <= sq.sq && it.n0 + quarter * 32 + 32 <= sq.sk) {
-            // the warp's whole 32 x 32 bias tile is inside the sequence: vector loads and a transpose
-            add_bias_column32<T>(pr, reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
-                                         (int64_t)h * p.bias.s[1] + (int64_t)mbase * p.bias.s[2] + (it.n0 + quarter * 32),
-                                 p.bias.s[2], lane);
-          } else if (bias_on && n < sq.sk) {
-            const T* bcol = reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
-                            (int64_t)h * p.bias.s[1] + (int64_t)n * p.bias.s[3];
-#pragma unroll
-            for (int c = 0; c < 32; ++c) {
-              const int m = mbase + c;
-              if (m < sq.sq) pr[c] = fmaf(to_f32<T>(bcol[(int64_t)m * p.bias.s[2]]), kLog2e, pr[c]);
-            }
+            for (int c = 0; c < 32; ++c) pr[c] *= p.qk_scale;
           }
-          __syncwarp();   // lanes beyond the sequence skipped the loads
 #pragma unroll
           for (int c4 = 0; c4 < 8; ++c4) {
             const float4 l4 = lds128(lse2 + 16u * c4);
@@ -810,7 +769,7 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
 #pragma unroll
           for (int c = 0; c < 16; ++c) {
             pk[c] = pack2<T>(pr[2 * c], pr[2 * c + 1]);
-            if constexpr (FEAT == kDropout) pk[c] &= keep_mask(keep, c);      // (1 / (1 - p) follows at the write-out of dV)
+            if constexpr ((FEAT & kDropout) != 0) pk[c] &= keep_mask(keep, c);      // (1 / (1 - p) follows at the write-out of dV)
           }
           tmem_st16(dp_col, pk);
           tmem_wait_st();
@@ -827,7 +786,7 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
             const float2 p0 = make_float2(pr[4 * c4], pr[4 * c4 + 1]), p1 = make_float2(pr[4 * c4 + 2], pr[4 * c4 + 3]);
             const float2 dp0 = make_float2(d[0], d[1]), dp1 = make_float2(d[2], d[3]);
             const float2 nd0 = make_float2(d4.x, d4.y), nd1 = make_float2(d4.z, d4.w);
-            if constexpr (FEAT == kDropout) {
+            if constexpr ((FEAT & kDropout) != 0) {
               pk[2 * c4] = dropout_ds_pair<T>(p0, dp0, ds2, nd0, keep_mask(keep, 2 * c4));
               pk[2 * c4 + 1] = dropout_ds_pair<T>(p1, dp1, ds2, nd1, keep_mask(keep, 2 * c4 + 1));
             } else {
@@ -896,7 +855,7 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         tc_fence_after();
         tmem_ld32f(tmem_base + lane_addr + kColAcc0 + d0, v);
         tmem_wait_ld();
-        stage_put32<T>(stage, r, d0, v, FEAT == kDropout ? p.dropout_scale : 1.0f, HD * 2);
+        stage_put32<T>(stage, r, d0, v, (FEAT & kDropout) ? p.dropout_scale : 1.0f, HD * 2);
         __syncwarp();
         warp_copy_out<T, 4>(stage, reinterpret_cast<T*>(p.dv.ptr) + (int64_t)sq.bidx * p.dv.s[0] + (int64_t)hk * p.dv.s[1] +
                                        (sq.k0 + it.n0) * p.dv.s[2],
@@ -965,7 +924,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // (constants where FEAT leaves them out: nothing of theirs is compiled in)
-  const bool drop_on = FEAT == kDropout && p.dropout_on != 0, bias_on = FEAT == kBias || (FEAT == kDropout && p.has_bias != 0), dbias_on = FEAT != kPlain && p.has_dbias != 0;
+  const bool drop_on = (FEAT & kDropout) && p.dropout_on != 0, bias_on = FEAT == kBias || (FEAT == kAll && p.has_bias != 0), dbias_on = (FEAT & kBias) && p.has_dbias != 0;
   // Order of the CTAs (the hardware starts them by linear block index): (batch, head) pairs in groups
   // of kHeadGroup, inside a group the query-block index slowest, from the block with the most key
   // blocks of a causal problem to the one with the fewest.  The heavy blocks of a group start
@@ -1208,12 +1167,12 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
     const bool simple = !bias_on && !__any_sync(0xffffffffu, fabsf(lse2) > 1.0e6f && lse2 != INFINITY);
     DropoutCtx dctx;
     if (drop_on) dctx = dropout_ctx(p, z, h);
-    const int mm = min(m, sq.sq - 1);
-    const T* bias_row = bias_on ? reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
-                                         (int64_t)h * p.bias.s[1] + (int64_t)mm * p.bias.s[2]
+    const int row0 = m0 + quarter * 32, rows_left = sq.sq - row0;      // the warp's tiles of bias and dBias start in this row
+    const T* bias_tile = bias_on ? reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
+                                         (int64_t)h * p.bias.s[1] + (int64_t)row0 * p.bias.s[2]
                                    : nullptr;
-    T* db_row = dbias_on ? reinterpret_cast<T*>(p.dbias.ptr) + (int64_t)sq.bidx * p.dbias.s[0] +
-                                  (int64_t)h * p.dbias.s[1] + (int64_t)mm * p.dbias.s[2]
+    T* db_tile = dbias_on ? reinterpret_cast<T*>(p.dbias.ptr) + (int64_t)sq.bidx * p.dbias.s[0] +
+                                  (int64_t)h * p.dbias.s[1] + (int64_t)row0 * p.dbias.s[2]
                             : nullptr;
     bool ok = true;
     for (int i = 0; i < niter; ++i) {
@@ -1224,8 +1183,14 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
       const bool shared = drop_on && keep_shared(p, sq, m0 + quarter * 32, nbase);
       uint32_t shared_bits = 0u;
       if (shared) shared_bits = *keep_share_word(p, sq, h, m0 + quarter * 32, nbase, lane);
-      // (the thread's 64 bytes of bias for this block: on their way to L2 while the tensor pipe computes S)
-      if (bias_on && p.bias_vec) asm volatile("prefetch.global.L2 [%0];" ::"l"(bias_row + nbase));
+      // the warp's 32 x 32 bias tile: on its way while the tensor pipe computes S, unless the generator's state is to find room as well
+      uint4 braw[4];
+      auto load_bias = [&] {
+        row32_load<T>(braw, bias_tile + (int64_t)nbase * p.bias.s[3], p.bias.s[2], p.bias.s[3], p.bias_vec, rows_left, sq.sk - nbase, lane);
+      };
+      if constexpr (FEAT == kBias) load_bias();
+      if (bias_on && i + 1 < niter)
+        tile32_prefetch(bias_tile + (int64_t)(nbase + kBlk) * p.bias.s[3], p.bias.s[2], p.bias.s[3], rows_left, sq.sk - (nbase + kBlk), lane);
       if (!mbar_wait(&bars[L::bSFull], par, abort_flag, status, 0x2600 + i)) { ok = false; break; }
       if (threadIdx.x == AB200_TRACE_TID) AB200_STAMPQ(i, 0);
       tc_fence_after();
@@ -1247,28 +1212,12 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
           pr[c + 1] = ex2(a.y);
         }
       } else {
-#pragma unroll
-        for (int c = 0; c < 32; ++c) pr[c] *= p.qk_scale;
         if (bias_on) {
-          if (p.bias_vec && nbase + kWgCols <= sq.sk) {
-            // the thread's 32 bias values are 64 contiguous bytes: four 16-byte loads
-            const uint4* bp = reinterpret_cast<const uint4*>(bias_row + nbase);
-            uint4 w[4];
+          if constexpr (FEAT != kBias) load_bias();
+          add_bias_row32<T>(pr, braw, p.qk_scale);
+        } else {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) w[u] = __ldg(bp + u);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const T* e = reinterpret_cast<const T*>(&w[u]);
-#pragma unroll
-              for (int i = 0; i < 8; ++i) pr[u * 8 + i] = fmaf(to_f32<T>(e[i]), kLog2e, pr[u * 8 + i]);
-            }
-          } else {
-#pragma unroll
-            for (int c = 0; c < 32; ++c) {
-              const int n = nbase + c;
-              if (n < sq.sk) pr[c] = fmaf(to_f32<T>(bias_row[(int64_t)n * p.bias.s[3]]), kLog2e, pr[c]);
-            }
-          }
+          for (int c = 0; c < 32; ++c) pr[c] *= p.qk_scale;
         }
 #pragma unroll
         for (int c = 0; c < 32; ++c) pr[c] = ex2(pr[c] - lse2);
@@ -1307,7 +1256,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
 #pragma unroll
         for (int c = 0; c < 16; ++c) {
           const float2 p2 = make_float2(pr[2 * c], pr[2 * c + 1]), dp2 = make_float2(dp[2 * c], dp[2 * c + 1]);
-          if constexpr (FEAT == kDropout) {
+          if constexpr ((FEAT & kDropout) != 0) {
             pk[c] = dropout_ds_pair<T>(p2, dp2, ds2, nd2, keep_mask(keep, c));
           } else {
             const float2 a = mul2(p2, sub2(dp2, dl2));
@@ -1315,23 +1264,12 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
           }
         }
         tmem_st16(dp_col, pk);
-        if (dbias_on && m < sq.sq) {
+        if (dbias_on) {
           // dB = cast(dS): the packed pairs are exactly the values to store
-          if (p.dbias.s[3] == 1 && nbase + 32 <= sq.sk && (reinterpret_cast<uintptr_t>(db_row + nbase) & 15u) == 0) {
+          uint4 w[4];
 #pragma unroll
-            for (int v4 = 0; v4 < 4; ++v4)
-              *reinterpret_cast<uint4*>(db_row + nbase + v4 * 8) =
-                  make_uint4(pk[v4 * 4], pk[v4 * 4 + 1], pk[v4 * 4 + 2], pk[v4 * 4 + 3]);
-          } else {
-#pragma unroll
-            for (int c = 0; c < 32; ++c) {
-              const int n = nbase + c;
-              if (n < sq.sk) {
-                const uint16_t bits = (uint16_t)((pk[c >> 1] >> ((c & 1) * 16)) & 0xffffu);
-                reinterpret_cast<uint16_t*>(db_row)[(int64_t)n * p.dbias.s[3]] = bits;
-              }
-            }
-          }
+          for (int v4 = 0; v4 < 4; ++v4) w[v4] = make_uint4(pk[v4 * 4], pk[v4 * 4 + 1], pk[v4 * 4 + 2], pk[v4 * 4 + 3]);
+          row32_store<T>(w, db_tile + (int64_t)nbase * p.dbias.s[3], p.dbias.s[2], p.dbias.s[3], p.dbias_vec, rows_left, sq.sk - nbase, lane);
         }
       }
       __syncwarp();   // the dB stores diverge; TMEM instructions are warp-collective
@@ -1381,7 +1319,7 @@ cudaError_t launch_bwd_T(int which, const Params& p, cudaStream_t st, float* dq_
   // make the stream's device, and remembered.
   struct PerDevice { std::atomic<unsigned int*> status{nullptr}, tickets{nullptr}; std::atomic<int> sms{0}; };
   static PerDevice per_device[64];
-  static std::atomic<bool> attr_set[64][15];
+  static std::atomic<bool> attr_set[64][20];
   const bool exact = p.varlen_mode == 0 && p.max_sq % 128 == 0 && p.max_sk % 128 == 0 && p.dqk == HD && p.dvo == HD;
   const int feat = features(p);
   int dev = 0;
@@ -1407,15 +1345,15 @@ cudaError_t launch_bwd_T(int which, const Params& p, cudaStream_t st, float* dq_
     const bool fused = which == 3;
     if (fused && HD != 128) return cudaErrorInvalidValue;
     using Kernel = decltype(&sm100_bwd_dkdv_kernel<T, HD, false, true, kPlain>);
-    static constexpr Kernel kSplit[2][3] = {
+    static constexpr Kernel kSplit[2][4] = {
         {sm100_bwd_dkdv_kernel<T, HD, false, false, kPlain>, sm100_bwd_dkdv_kernel<T, HD, false, false, kBias>,
-         sm100_bwd_dkdv_kernel<T, HD, false, false, kDropout>},
+         sm100_bwd_dkdv_kernel<T, HD, false, false, kDropout>, sm100_bwd_dkdv_kernel<T, HD, false, false, kAll>},
         {sm100_bwd_dkdv_kernel<T, HD, false, true, kPlain>, sm100_bwd_dkdv_kernel<T, HD, false, true, kBias>,
-         sm100_bwd_dkdv_kernel<T, HD, false, true, kDropout>}};
-    static constexpr Kernel kFused[3] = {sm100_bwd_dkdv_kernel<T, 128, true, false, kPlain>, sm100_bwd_dkdv_kernel<T, 128, true, false, kBias>,
-                                         sm100_bwd_dkdv_kernel<T, 128, true, false, kDropout>};
+         sm100_bwd_dkdv_kernel<T, HD, false, true, kDropout>, sm100_bwd_dkdv_kernel<T, HD, false, true, kAll>}};
+    static constexpr Kernel kFused[4] = {sm100_bwd_dkdv_kernel<T, 128, true, false, kPlain>, sm100_bwd_dkdv_kernel<T, 128, true, false, kBias>,
+                                         sm100_bwd_dkdv_kernel<T, 128, true, false, kDropout>, sm100_bwd_dkdv_kernel<T, 128, true, false, kAll>};
     const Kernel kern_split = kSplit[exact][feat], kern_fused = kFused[feat];
-    e = fused ? set_smem(12 + feat, reinterpret_cast<const void*>(kern_fused), BwdSmem<128>::kDynamic)
+    e = fused ? set_smem(16 + feat, reinterpret_cast<const void*>(kern_fused), BwdSmem<128>::kDynamic)
               : set_smem(2 * feat + exact, reinterpret_cast<const void*>(kern_split), L::kDynamic);
     if (e != cudaSuccess) return e;
     const int nitems = ((p.max_sk + kBlk - 1) / kBlk) * ((p.hk * p.batch + 7) / 8) * 8;
@@ -1442,11 +1380,13 @@ cudaError_t launch_bwd_T(int which, const Params& p, cudaStream_t st, float* dq_
                         static_cast<float*>(nullptr));
   } else {
     using Kernel = decltype(&sm100_bwd_dq_kernel<T, HD, true, kPlain>);
-    static constexpr Kernel kDq[2][3] = {
-        {sm100_bwd_dq_kernel<T, HD, false, kPlain>, sm100_bwd_dq_kernel<T, HD, false, kBias>, sm100_bwd_dq_kernel<T, HD, false, kDropout>},
-        {sm100_bwd_dq_kernel<T, HD, true, kPlain>, sm100_bwd_dq_kernel<T, HD, true, kBias>, sm100_bwd_dq_kernel<T, HD, true, kDropout>}};
+    static constexpr Kernel kDq[2][4] = {
+        {sm100_bwd_dq_kernel<T, HD, false, kPlain>, sm100_bwd_dq_kernel<T, HD, false, kBias>,
+         sm100_bwd_dq_kernel<T, HD, false, kDropout>, sm100_bwd_dq_kernel<T, HD, false, kAll>},
+        {sm100_bwd_dq_kernel<T, HD, true, kPlain>, sm100_bwd_dq_kernel<T, HD, true, kBias>,
+         sm100_bwd_dq_kernel<T, HD, true, kDropout>, sm100_bwd_dq_kernel<T, HD, true, kAll>}};
     const Kernel kern_dq = kDq[exact][feat];
-    e = set_smem(6 + 2 * feat + exact, reinterpret_cast<const void*>(kern_dq), DqSmem<HD>::kDynamic);
+    e = set_smem(8 + 2 * feat + exact, reinterpret_cast<const void*>(kern_dq), DqSmem<HD>::kDynamic);
     if (e != cudaSuccess) return e;
     dim3 grid((p.max_sq + kBlk - 1) / kBlk, p.hq, p.batch);
     e = launch_kernel(kern_dq, grid, dim3(kBwdThreads), DqSmem<HD>::kDynamic, st, p, tq, tk, tv, tdo, status);

@@ -85,7 +85,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // (constants where FEAT leaves them out: nothing of theirs is compiled in)
-  const bool drop_on = FEAT == kDropout && p.dropout_on != 0, bias_on = FEAT == kBias || (FEAT == kDropout && p.has_bias != 0), dbias_on = FEAT != kPlain && p.has_dbias != 0;
+  const bool drop_on = (FEAT & kDropout) && p.dropout_on != 0, bias_on = FEAT == kBias || (FEAT == kAll && p.has_bias != 0), dbias_on = (FEAT & kBias) && p.has_dbias != 0;
   if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile unsigned int*>(status) != 0u)) return;
   if ((int)(smem - smem_raw) + L::kUsed > L::kDynamic) {      // the alignment padding did not fit
     if (threadIdx.x == 0) atomicCAS(status, 0u, 0x3F00u);
@@ -374,10 +374,17 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         const bool shared = MODE == kWideDK && drop_on && keep_shared(p, sq, mbase, r0 + quarter * 32);
         uint32_t shared_bits = 0u;
         if (shared) shared_bits = *keep_share_word(p, sq, h, mbase, r0 + quarter * 32, lane);
-        if (bias_on && p.bias_vec)      // the warp's 32 x 32 bias tile, one 64-byte row per lane, towards L2
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
-                                                       (int64_t)h * p.bias.s[1] + (int64_t)min(mbase + lane, sq.sq - 1) * p.bias.s[2] +
-                                                       (r0 + quarter * 32)));
+        uint4 braw[4];      // the warp's 32 x 32 bias tile: on its way while the tensor pipe computes S'
+        if (bias_on)
+          tile32_load<T>(braw, reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] + (int64_t)h * p.bias.s[1] +
+                                   (int64_t)mbase * p.bias.s[2] + (int64_t)(r0 + quarter * 32) * p.bias.s[3],
+                         p.bias.s[2], p.bias.s[3], p.bias_vec != 0, sq.sq - mbase, sq.sk - (r0 + quarter * 32), lane);
+        if (bias_on && i + 1 < niter) {      // (hg, cb: the next block's by now)
+          const int mnext = (cb_lo + cb) * kNB + cbase;
+          tile32_prefetch(reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] + (int64_t)(hk * p.group + hg) * p.bias.s[1] +
+                              (int64_t)mnext * p.bias.s[2] + (int64_t)(r0 + quarter * 32) * p.bias.s[3],
+                          p.bias.s[2], p.bias.s[3], sq.sq - mnext, sq.sk - (r0 + quarter * 32), lane);
+        }
         if (!mbar_wait(&bars[L::bSFull], (uint32_t)i & 1u, abort_flag, status, 0x3A00)) { ok = false; break; }
         if (!mbar_wait(&bars[L::bAuxFull + s], par2, abort_flag, status, 0x3A80)) { ok = false; break; }
         tc_fence_after();
@@ -401,23 +408,12 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
             pr[4 * c4 + 3] = ex2(b.y);
           }
         } else {
+          if (bias_on) {
+            add_bias_column32<T>(pr, braw, p.qk_scale, lane);
+          } else {
 #pragma unroll
-          for (int c = 0; c < 32; ++c) pr[c] *= p.qk_scale;
-          if (bias_on && p.bias_vec && mbase + 32 <= sq.sq && r0 + quarter * 32 + 32 <= sq.sk) {
-            // the warp's whole 32 x 32 bias tile is inside the sequence: vector loads and a transpose
-            add_bias_column32<T>(pr, reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
-                                         (int64_t)h * p.bias.s[1] + (int64_t)mbase * p.bias.s[2] + (r0 + quarter * 32),
-                                 p.bias.s[2], lane);
-          } else if (bias_on && n < sq.sk) {
-            const T* bcol = reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
-                            (int64_t)h * p.bias.s[1] + (int64_t)n * p.bias.s[3];
-#pragma unroll
-            for (int c = 0; c < 32; ++c) {
-              const int m = mbase + c;
-              if (m < sq.sq) pr[c] = fmaf(to_f32<T>(bcol[(int64_t)m * p.bias.s[2]]), kLog2e, pr[c]);
-            }
+            for (int c = 0; c < 32; ++c) pr[c] *= p.qk_scale;
           }
-          __syncwarp();   // lanes beyond the sequence skipped the loads
 #pragma unroll
           for (int c4 = 0; c4 < 8; ++c4) {
             const float4 l4 = lds128(lse2 + 16u * c4);
@@ -463,7 +459,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
 #pragma unroll
           for (int c = 0; c < 16; ++c) {
             pk[c] = pack2<T>(pr[2 * c], pr[2 * c + 1]);
-            if constexpr (FEAT == kDropout) pk[c] &= keep_mask(keep, c);      // (1 / (1 - p) follows at the write-out)
+            if constexpr ((FEAT & kDropout) != 0) pk[c] &= keep_mask(keep, c);      // (1 / (1 - p) follows at the write-out)
           }
         } else {
           float dp[32];
@@ -476,7 +472,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
             const float2 p0 = make_float2(pr[4 * c4], pr[4 * c4 + 1]), p1 = make_float2(pr[4 * c4 + 2], pr[4 * c4 + 3]);
             const float2 dp0 = make_float2(dp[4 * c4], dp[4 * c4 + 1]), dp1 = make_float2(dp[4 * c4 + 2], dp[4 * c4 + 3]);
             const float2 nd0 = make_float2(d4.x, d4.y), nd1 = make_float2(d4.z, d4.w);
-            if constexpr (FEAT == kDropout) {
+            if constexpr ((FEAT & kDropout) != 0) {
               pk[2 * c4] = dropout_ds_pair<T>(p0, dp0, ds2, nd0, keep_mask(keep, 2 * c4));
               pk[2 * c4 + 1] = dropout_ds_pair<T>(p1, dp1, ds2, nd1, keep_mask(keep, 2 * c4 + 1));
             } else {
@@ -503,12 +499,12 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
       const bool simple = !bias_on && !__any_sync(0xffffffffu, fabsf(lse2) > 1.0e6f && lse2 != INFINITY);
       DropoutCtx dctx;
       if (drop_on) dctx = dropout_ctx_from(p, ph_seed, ph_off, z, hrow);
-      const int mm = min(m, sq.sq - 1);
-      const T* bias_row = bias_on ? reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
-                                           (int64_t)hrow * p.bias.s[1] + (int64_t)mm * p.bias.s[2]
+      const int row0 = r0 + quarter * 32, rows_left = sq.sq - row0;      // the warp's tiles of bias and dBias start in this row
+      const T* bias_tile = bias_on ? reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] +
+                                           (int64_t)hrow * p.bias.s[1] + (int64_t)row0 * p.bias.s[2]
                                      : nullptr;
-      T* db_row = dbias_on ? reinterpret_cast<T*>(p.dbias.ptr) + (int64_t)sq.bidx * p.dbias.s[0] +
-                                    (int64_t)hrow * p.dbias.s[1] + (int64_t)mm * p.dbias.s[2]
+      T* db_tile = dbias_on ? reinterpret_cast<T*>(p.dbias.ptr) + (int64_t)sq.bidx * p.dbias.s[0] +
+                                    (int64_t)hrow * p.dbias.s[1] + (int64_t)row0 * p.dbias.s[2]
                               : nullptr;
       for (int i = 0; i < niter; ++i) {
         const int s = i & 1;
@@ -517,7 +513,11 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         const bool shared = drop_on && keep_shared(p, sq, r0 + quarter * 32, nbase);
         uint32_t shared_bits = 0u;
         if (shared) shared_bits = *keep_share_word(p, sq, hrow, r0 + quarter * 32, nbase, lane);
-        if (bias_on && p.bias_vec) asm volatile("prefetch.global.L2 [%0];" ::"l"(bias_row + nbase));
+        uint4 braw[4];      // the warp's 32 x 32 bias tile: on its way while the tensor pipe computes S'
+        if (bias_on)
+          row32_load<T>(braw, bias_tile + (int64_t)nbase * p.bias.s[3], p.bias.s[2], p.bias.s[3], p.bias_vec, rows_left, sq.sk - nbase, lane);
+        if (bias_on && i + 1 < niter)
+          tile32_prefetch(bias_tile + (int64_t)(nbase + kNB) * p.bias.s[3], p.bias.s[2], p.bias.s[3], rows_left, sq.sk - (nbase + kNB), lane);
         if (!mbar_wait(&bars[L::bSFull], (uint32_t)i & 1u, abort_flag, status, 0x3C00)) { ok = false; break; }
         tc_fence_after();
         float pr[32];
@@ -536,28 +536,11 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
             pr[c + 1] = ex2(a.y);
           }
         } else {
-#pragma unroll
-          for (int c = 0; c < 32; ++c) pr[c] *= p.qk_scale;
           if (bias_on) {
-            if (p.bias_vec && nbase + kWgCols <= sq.sk) {
-              // the thread's 32 bias values are 64 contiguous bytes: four 16-byte loads
-              const uint4* bp = reinterpret_cast<const uint4*>(bias_row + nbase);
-              uint4 w[4];
+            add_bias_row32<T>(pr, braw, p.qk_scale);
+          } else {
 #pragma unroll
-              for (int u = 0; u < 4; ++u) w[u] = __ldg(bp + u);
-#pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                const T* e = reinterpret_cast<const T*>(&w[u]);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) pr[u * 8 + j] = fmaf(to_f32<T>(e[j]), kLog2e, pr[u * 8 + j]);
-              }
-            } else {
-#pragma unroll
-              for (int c = 0; c < 32; ++c) {
-                const int n = nbase + c;
-                if (n < sq.sk) pr[c] = fmaf(to_f32<T>(bias_row[(int64_t)n * p.bias.s[3]]), kLog2e, pr[c]);
-              }
-            }
+            for (int c = 0; c < 32; ++c) pr[c] *= p.qk_scale;
           }
 #pragma unroll
           for (int c = 0; c < 32; ++c) pr[c] = ex2(pr[c] - lse2);
@@ -593,7 +576,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
 #pragma unroll
           for (int c = 0; c < 16; ++c) {
             const float2 p2 = make_float2(pr[2 * c], pr[2 * c + 1]), dp2 = make_float2(dp[2 * c], dp[2 * c + 1]);
-            if constexpr (FEAT == kDropout) {
+            if constexpr ((FEAT & kDropout) != 0) {
               pk[c] = dropout_ds_pair<T>(p2, dp2, ds2, nd2, keep_mask(keep, c));
             } else {
               const float2 a = mul2(p2, sub2(dp2, dl2));
@@ -601,23 +584,12 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
             }
           }
           tmem_st16(a_col, pk);
-          if (dbias_on && m < sq.sq) {
+          if (dbias_on) {
             // dB = cast(dS): the packed pairs are exactly the values to store
-            if (p.dbias.s[3] == 1 && nbase + 32 <= sq.sk && (reinterpret_cast<uintptr_t>(db_row + nbase) & 15u) == 0) {
+            uint4 w[4];
 #pragma unroll
-              for (int v4 = 0; v4 < 4; ++v4)
-                *reinterpret_cast<uint4*>(db_row + nbase + v4 * 8) =
-                    make_uint4(pk[v4 * 4], pk[v4 * 4 + 1], pk[v4 * 4 + 2], pk[v4 * 4 + 3]);
-            } else {
-#pragma unroll
-              for (int c = 0; c < 32; ++c) {
-                const int n = nbase + c;
-                if (n < sq.sk) {
-                  const uint16_t bits = (uint16_t)((pk[c >> 1] >> ((c & 1) * 16)) & 0xffffu);
-                  reinterpret_cast<uint16_t*>(db_row)[(int64_t)n * p.dbias.s[3]] = bits;
-                }
-              }
-            }
+            for (int v4 = 0; v4 < 4; ++v4) w[v4] = make_uint4(pk[v4 * 4], pk[v4 * 4 + 1], pk[v4 * 4 + 2], pk[v4 * 4 + 3]);
+            row32_store<T>(w, db_tile + (int64_t)nbase * p.dbias.s[3], p.dbias.s[2], p.dbias.s[3], p.dbias_vec, rows_left, sq.sk - nbase, lane);
           }
         }
         __syncwarp();   // the dB stores diverge; TMEM instructions are warp-collective
@@ -636,7 +608,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
       const int nrows = min(kBlk, rows_total - r0);
       T* dst = reinterpret_cast<T*>(outv.ptr) + (int64_t)sq.bidx * outv.s[0] + (int64_t)hrow * outv.s[1] +
                (row_tok0 + r0) * outv.s[2];
-      const float scale = MODE != kWideDV ? p.sm_scale : (FEAT == kDropout ? p.dropout_scale : 1.0f);
+      const float scale = MODE != kWideDV ? p.sm_scale : ((FEAT & kDropout) ? p.dropout_scale : 1.0f);
       for (int c = wg; c * 32 < d_out; c += 2) {
         float v[32];
         tmem_ld32f(tmem_base + lane_addr + kWColAcc + c * 32, v);
@@ -678,7 +650,7 @@ cudaError_t launch_bwd_wide_T(int which, const Params& p, cudaStream_t st) {
       return cudaErrorInvalidValue;
   }
   static std::atomic<unsigned int*> status_of[64];
-  static std::atomic<bool> attr_set[64][10];
+  static std::atomic<bool> attr_set[64][13];
   const int feat = features(p);
   int dev = 0;
   cudaError_t e = host().get_device(&dev);
@@ -697,14 +669,14 @@ cudaError_t launch_bwd_wide_T(int which, const Params& p, cudaStream_t st) {
     return r;
   };
   using Kernel = decltype(&sm100_bwd_wide_kernel<T, kWideDV, kPlain>);
-  static constexpr Kernel kKernels[3][3] = {      // [kWide*][features]
-      {sm100_bwd_wide_kernel<T, 0, kPlain>, sm100_bwd_wide_kernel<T, 0, kBias>, sm100_bwd_wide_kernel<T, 0, kDropout>},
-      {sm100_bwd_wide_kernel<T, 1, kPlain>, sm100_bwd_wide_kernel<T, 1, kBias>, sm100_bwd_wide_kernel<T, 1, kDropout>},
-      {sm100_bwd_wide_kernel<T, 2, kPlain>, sm100_bwd_wide_kernel<T, 2, kBias>, sm100_bwd_wide_kernel<T, 2, kDropout>}};
+  static constexpr Kernel kKernels[3][4] = {      // [kWide*][features]
+      {sm100_bwd_wide_kernel<T, 0, kPlain>, sm100_bwd_wide_kernel<T, 0, kBias>, sm100_bwd_wide_kernel<T, 0, kDropout>, sm100_bwd_wide_kernel<T, 0, kAll>},
+      {sm100_bwd_wide_kernel<T, 1, kPlain>, sm100_bwd_wide_kernel<T, 1, kBias>, sm100_bwd_wide_kernel<T, 1, kDropout>, sm100_bwd_wide_kernel<T, 1, kAll>},
+      {sm100_bwd_wide_kernel<T, 2, kPlain>, sm100_bwd_wide_kernel<T, 2, kBias>, sm100_bwd_wide_kernel<T, 2, kDropout>, sm100_bwd_wide_kernel<T, 2, kAll>}};
   if (which == 1) {
     const Kernel kern_dv = kKernels[kWideDV][feat], kern_dk = kKernels[kWideDK][feat];
-    if ((e = set_smem(3 * kWideDV + feat, reinterpret_cast<const void*>(kern_dv))) != cudaSuccess) return e;
-    if ((e = set_smem(3 * kWideDK + feat, reinterpret_cast<const void*>(kern_dk))) != cudaSuccess) return e;
+    if ((e = set_smem(4 * kWideDV + feat, reinterpret_cast<const void*>(kern_dv))) != cudaSuccess) return e;
+    if ((e = set_smem(4 * kWideDK + feat, reinterpret_cast<const void*>(kern_dk))) != cudaSuccess) return e;
     dim3 grid((p.max_sk + kBlk - 1) / kBlk, p.hk, p.batch);
     e = launch_kernel(kern_dv, grid, dim3(kWideThreads), L::kDynamic, st, p, k128, k128, do64, q64, status);
     if (e != cudaSuccess) return e;
@@ -714,13 +686,13 @@ cudaError_t launch_bwd_wide_T(int which, const Params& p, cudaStream_t st) {
     }
   } else {
     const Kernel kern_dq = kKernels[kWideDQ][feat];
-    if ((e = set_smem(3 * kWideDQ + feat, reinterpret_cast<const void*>(kern_dq))) != cudaSuccess) return e;
+    if ((e = set_smem(4 * kWideDQ + feat, reinterpret_cast<const void*>(kern_dq))) != cudaSuccess) return e;
     dim3 grid((p.max_sq + kBlk - 1) / kBlk, p.hq, p.batch);
     e = launch_kernel(kern_dq, grid, dim3(kWideThreads), L::kDynamic, st, p, q128, do128, k64, v64, status);
     if (e == cudaSuccess && p.dk_from_db) {
       count_launch();
       auto kern_db = sm100_bwd_dk_db_kernel<T>;
-      if ((e = set_smem(9, reinterpret_cast<const void*>(kern_db), DkDbSmem::kDynamic)) != cudaSuccess) return e;
+      if ((e = set_smem(12, reinterpret_cast<const void*>(kern_db), DkDbSmem::kDynamic)) != cudaSuccess) return e;
       dim3 grid_k((p.max_sk + kBlk - 1) / kBlk, p.hk, p.batch);
       e = launch_kernel(kern_db, grid_k, dim3(kDkDbThreads), DkDbSmem::kDynamic, st, p, db64, q64, status);
     }

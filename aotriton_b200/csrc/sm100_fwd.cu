@@ -38,6 +38,7 @@
 #include <atomic>
 #include "launch.h"
 #include "sm100_ptx.cuh"
+#include "tile32.cuh"
 
 namespace ab200 {
 
@@ -115,8 +116,6 @@ __device__ void write_dead_rows(const Params& p, const Seq& sq, int h, int m0, i
 // FEAT (features()): with code for dropout in the loop a call with bias alone, and with code for either a call with
 // neither, spills around every block.  Measured, us, dropout's instantiation against the call's own, neither: 4 x 32 heads
 // x 4096 of 128, causal, 583 -> 571; 8 x 16 heads x 2048 of 64 260 -> 241; bias, 4 x 8 heads x 1024 of 64 41.6 -> 40.8.
-// (That bias is there stays a test at run time: with it known, whole tiles gain 10 to 20 %, but unaligned rows
-// and the last, partial block, whose loads then wait one by one, lose as much or more.)
 template <typename T, int HD, bool EXACT, int FEAT>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm_q,
@@ -132,7 +131,7 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // (constants where FEAT leaves them out: nothing of theirs is compiled in)
-  const bool drop_on = FEAT == kDropout && p.dropout_on != 0, bias_on = FEAT != kPlain && p.has_bias != 0;
+  const bool drop_on = (FEAT & kDropout) && p.dropout_on != 0, bias_on = (FEAT & kBias) && p.has_bias != 0;
   // Order of the CTAs (the hardware starts them by linear block index): (batch, head) pairs are taken
   // in groups of kHeadGroup; inside a group the row-tile index runs slowest, from the tile with the
   // most key blocks of a causal problem to the one with the fewest.  The heavy tiles of a group so
@@ -363,7 +362,7 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
     // and dropout 0.2, 8 x 16 heads x 2048: 5.38 -> 5.0 ms.
     // (With two tiles it does not pay: a warpgroup more leaves its threads 56 registers, too few for the independent
     // counters that one warp per scheduler needs: 16 packed sequences 23.3 -> 26.1 ms.)
-    if constexpr (FEAT == kDropout) {
+    if constexpr ((FEAT & kDropout) != 0) {
       if (drop_on) {
         const int r = (warp & 3) * 32 + lane;
         const DropoutCtx dctx = dropout_ctx(p, z, h);
@@ -411,29 +410,50 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
     const int warp_lo = __reduce_max_sync(0xffffffffu, row_lo), warp_hi = __reduce_min_sync(0xffffffffu, row_hi);
     DropoutCtx dctx;
     if (L::kTiles == 2 && drop_on) dctx = dropout_ctx(p, z, h);
-    const T* bias_row = nullptr;
+    const int row0 = m0 + t * kBM + quarter * 32;      // the warp's tiles of bias start in this row
+    const T* bias_tile = nullptr;
     if (bias_on)
-      bias_row = reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] + (int64_t)h * p.bias.s[1] +
-                 (int64_t)min(m, sq.sq - 1) * p.bias.s[2];
+      bias_tile = reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] + (int64_t)h * p.bias.s[1] +
+                  (int64_t)row0 * p.bias.s[2];
 
     float m_used = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < nblk; ++j) {
       const int n0 = (jb_lo + j) * kBN;
       const uint32_t par = (uint32_t)j & 1u;
-      if (bias_on && p.bias_vec) {
-        // the thread's 256 bytes of bias for this block: on their way to L2 while the tensor pipe computes S
-        const char* bp = reinterpret_cast<const char*>(bias_row + n0);
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(bp));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(bp + 128));
+      // The warp's four 32 x 32 tiles of bias: two on their way while the tensor pipe computes S, the others as these are used.
+      // (All four are 64 registers beside 128 scores: 264 bytes spilled, head dim 72 877 -> 1231 us with the exchange.)
+      uint4 braw[2][4];
+      if (bias_on) {
+#pragma unroll
+        for (int g = 0; g < 2; ++g)
+          row32_load<T>(braw[g], bias_tile + (int64_t)(n0 + 32 * g) * p.bias.s[3], p.bias.s[2], p.bias.s[3], p.bias_vec, sq.sq - row0,
+                         sq.sk - (n0 + 32 * g), lane);
+        if (j + 1 < nblk) {
+          // (256 bytes of a row: two lines)
+          tile32_prefetch(bias_tile + (int64_t)(n0 + kBN) * p.bias.s[3], p.bias.s[2], p.bias.s[3], sq.sq - row0, sq.sk - (n0 + kBN), lane);
+          tile32_prefetch(bias_tile + (int64_t)(n0 + kBN + 64) * p.bias.s[3], p.bias.s[2], p.bias.s[3], sq.sq - row0, sq.sk - (n0 + kBN + 64), lane);
+        }
       }
       if (!mbar_wait(&bars[L::bSFull + t], par, abort_flag, status, 0x700 + 2 * j + t)) { ok = false; break; }
       AB200_FSTAMP(j, 0);
       tc_fence_after();
       float sc[128];
+      if (bias_on) {      // (a tile at a time: bias and scores of the whole block are more registers than there are)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld32f(s_addr + c * 32, &sc[c * 32]);
-      tmem_wait_ld();
+        for (int g = 0; g < 4; ++g) {
+          tmem_ld32f(s_addr + g * 32, &sc[g * 32]);
+          tmem_wait_ld();
+          add_bias_row32<T>(&sc[g * 32], braw[g & 1], p.qk_scale);
+          if (g < 2)
+            row32_load<T>(braw[g], bias_tile + (int64_t)(n0 + 32 * (g + 2)) * p.bias.s[3], p.bias.s[2], p.bias.s[3], p.bias_vec, sq.sq - row0,
+                           sq.sk - (n0 + 32 * (g + 2)), lane);
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tmem_ld32f(s_addr + c * 32, &sc[c * 32]);
+        tmem_wait_ld();
+      }
       AB200_FSTAMP(j, 1);
       // Scores -> exponent arguments.  The common case (no bias, positive scale, ordinary
       // magnitudes) keeps the raw scores and folds scale and maximum into one FMA per element
@@ -462,30 +482,9 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
         if (__any_sync(0xffffffffu, huge)) simple = false;
       }
       if (!simple) {
+        if (!bias_on) {      // (else scaled above)
 #pragma unroll
-        for (int c = 0; c < 128; ++c) sc[c] *= p.qk_scale;
-        if (bias_on) {
-          const int nmax = sq.sk - n0;
-          if (p.bias_vec && nmax >= kBN) {
-            // the thread's 128 bias values are 256 contiguous bytes: sixteen 16-byte loads, four in flight
-            const uint4* bp = reinterpret_cast<const uint4*>(bias_row + n0);
-#pragma unroll
-            for (int g = 0; g < 16; g += 4) {
-              uint4 w[4];
-#pragma unroll
-              for (int u = 0; u < 4; ++u) w[u] = __ldg(bp + g + u);
-#pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                const T* e = reinterpret_cast<const T*>(&w[u]);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) sc[(g + u) * 8 + i] = fmaf(to_f32<T>(e[i]), kLog2e, sc[(g + u) * 8 + i]);
-              }
-            }
-          } else {
-#pragma unroll
-            for (int c = 0; c < 128; ++c)
-              if (c < nmax) sc[c] = fmaf(to_f32<T>(bias_row[(int64_t)(n0 + c) * p.bias.s[3]]), kLog2e, sc[c]);
-          }
+          for (int c = 0; c < 128; ++c) sc[c] *= p.qk_scale;
         }
         if (any_mask) {
 #pragma unroll
@@ -743,7 +742,8 @@ cudaError_t launch_fwd_T(const Params& p, cudaStream_t st) {
       // Measured, 8 x 16 heads x 2048, not causal: 642 us against 628.)
       return exact ? launch_fwd_TE<T, HD, true, HD == 256 ? kBias : kPlain>(p, st) : launch_fwd_TE<T, HD, false, kPlain>(p, st);
     case kBias: return exact ? launch_fwd_TE<T, HD, true, kBias>(p, st) : launch_fwd_TE<T, HD, false, kBias>(p, st);
-    default: return exact ? launch_fwd_TE<T, HD, true, kDropout>(p, st) : launch_fwd_TE<T, HD, false, kDropout>(p, st);
+    case kDropout: return exact ? launch_fwd_TE<T, HD, true, kDropout>(p, st) : launch_fwd_TE<T, HD, false, kDropout>(p, st);
+    default: return exact ? launch_fwd_TE<T, HD, true, kAll>(p, st) : launch_fwd_TE<T, HD, false, kAll>(p, st);
   }
 }
 
