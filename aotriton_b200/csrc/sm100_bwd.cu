@@ -848,7 +848,7 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
       if (wg < HD / 32) {
         // Each warp transposes its 32 rows x 32 columns through the staging tile, so that the global
         // stores are 64-byte row segments instead of 16 bytes per row.
-        uint8_t* stage = smem + L::kStage;
+        const uint32_t stage = smem_u32(smem + L::kStage);
         const int nrows = min(kBlk, sq.sk - it.n0);
         const int d0 = wg * 32;
         float v[32];
@@ -945,7 +945,9 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
     h = hz - z * nh;
     m0 = (nx - 1 - xi) * kBlk;
   }
-  if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile unsigned int*>(status) != 0u)) return;
+  // Whether an earlier CTA timed out: read here, decided on behind the set-up, which then runs under the read.
+  const unsigned int failed_before = threadIdx.x == 0 ? *reinterpret_cast<volatile unsigned int*>(status) : 0u;
+  if (warp == 2 && lane == 0) { prefetch_tmap(&tm_q); prefetch_tmap(&tm_do); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); }
   const Seq sq = resolve_seq(p, z);
   if (m0 >= sq.sq) return;
   const int hk = h / p.group;
@@ -999,9 +1001,21 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  const bool leave = __syncthreads_or(failed_before != 0u) != 0;      // (one read, one CTA-wide decision)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (leave) {
+    if (threadIdx.x == 0) {      // the copies requested above land before the CTA gives its shared memory back
+      mbar_wait_quiet(&bars[L::bResFull], 0, abort_flag);
+      for (int i = 0; i < min(2, niter); ++i) {
+        mbar_wait_quiet(&bars[L::bKFull + i], 0, abort_flag);
+        if (!(p.drop_copy == 3 && i == 0)) mbar_wait_quiet(&bars[L::bVFull + i], 0, abort_flag);
+      }
+    }
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
+    return;
+  }
 
   if (warp == 0) {
     if (lane == 0) {
@@ -1283,7 +1297,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
     if (ok && wg < HD / 32) {
       // Each warp transposes its 32 rows x 32 columns of dQ through the (now idle) Q tile, so that
       // the global stores are 64-byte row segments instead of 16 bytes per row.
-      uint8_t* stage = smem + L::kResA;
+      const uint32_t stage = smem_u32(smem + L::kResA);
       tc_fence_after();
       float v[32];
       const int d0 = wg * 32;

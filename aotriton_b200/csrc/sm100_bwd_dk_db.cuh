@@ -129,9 +129,9 @@ sm100_bwd_dk_db_kernel(const __grid_constant__ Params p, const __grid_constant__
         float v[32];
         tmem_ld32f(tmem_base + ((uint32_t)(quarter * 32) << 16) + c * 32, v);
         tmem_wait_ld();
-        stage_put32<T>(smem, r, c * 32, v, p.sm_scale, 512);
+        stage_put32<T>(smem_u32(smem), r, c * 32, v, p.sm_scale, 512);
         __syncwarp();
-        warp_copy_out<T, 4>(smem, dst, p.dk.s[2], min(kBlk, sq.sk - n0), p.dqk, quarter * 32, c * 4, lane, 512);
+        warp_copy_out<T, 4>(smem_u32(smem), dst, p.dk.s[2], min(kBlk, sq.sk - n0), p.dqk, quarter * 32, c * 4, lane, 512);
         __syncwarp();
       }
     }

@@ -604,7 +604,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
     if (ok) ok = mbar_wait(&bars[L::bAccDone], 0, abort_flag, status, 0x3E00);
     if (ok) {
       tc_fence_after();
-      uint8_t* stage = smem + L::kResA;
+      const uint32_t stage = smem_u32(smem + L::kResA);
       const int nrows = min(kBlk, rows_total - r0);
       T* dst = reinterpret_cast<T*>(outv.ptr) + (int64_t)sq.bidx * outv.s[0] + (int64_t)hrow * outv.s[1] +
                (row_tok0 + r0) * outv.s[2];

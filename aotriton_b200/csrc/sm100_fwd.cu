@@ -152,8 +152,9 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
     h = hz - z * nh;
     m0 = (nx - 1 - xi) * kCtaRows;
   }
-  // An earlier CTA timed out: the whole CTA leaves (one read, one CTA-wide decision).
-  if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile unsigned int*>(status) != 0u)) return;
+  // Whether an earlier CTA timed out: read here, decided on behind the set-up, which then runs under the read.
+  const unsigned int failed_before = threadIdx.x == 0 ? *reinterpret_cast<volatile unsigned int*>(status) : 0u;
+  if (warp == 2 && lane == 0) { prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); }
   // One thread of the grid reports the seed and offset actually used, before any early exit.
   if (drop_on && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) {
     uint64_t seed = p.seed_ptr ? *p.seed_ptr : 0ull;
@@ -161,12 +162,15 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
     if (p.seed_out) *p.seed_out = seed;
     if (p.off_out) *p.off_out = base;
   }
+  int4 ends;
   if (!EXACT && p.packed_tiles > 0) {      // one-dimensional grid: the heads of a tile next to each other
     const int tile = (int)blockIdx.x / p.hq;
     h = (int)blockIdx.x - tile * p.hq;
-    if (!packed_tile<kCtaRows>(p, tile, lane, z, m0)) return;
+    if (!packed_tile<kCtaRows>(p, tile, lane, z, m0, ends)) return;
+  } else if (p.varlen_mode != 0) {
+    ends = make_int4(p.cu_q[z], p.cu_q[z + 1], p.cu_k[z], p.cu_k[z + 1]);
   }
-  const Seq sq = resolve_seq(p, z);
+  const Seq sq = seq_from_ends(p, z, ends);
   if (m0 >= sq.sq) return;
   const int hk = h / p.group;
   const int ntile = (L::kTiles == 2 && m0 + kBM < sq.sq) ? 2 : 1;   // the second tile may lie beyond the sequence
@@ -225,9 +229,21 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  const bool leave = __syncthreads_or(failed_before != 0u) != 0;      // (one read, one CTA-wide decision)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (leave) {
+    if (threadIdx.x == 0) {      // the copies requested above land before the CTA gives its shared memory back
+      for (int t = 0; t < ntile; ++t) mbar_wait_quiet(&bars[L::bQFull + t], 0, abort_flag);
+      for (int j = 0; j < min(kStages, nblk); ++j) {
+        mbar_wait_quiet(&bars[L::bKFull + j], 0, abort_flag);
+        if (!(p.drop_copy == 1 && j == 0)) mbar_wait_quiet(&bars[L::bVFull + j], 0, abort_flag);
+      }
+    }
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
+    return;
+  }
 
   if (warp < 4) {
     reg_dealloc<56>();
@@ -647,14 +663,17 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
       const float inv = (l > 0.f) ? p.dropout_scale / l : 0.f;
       // Each warp transposes its 32 rows through the tile's (now idle) Q buffer, so that the global
       // stores are whole rows instead of 16 bytes per row.
-      uint8_t* stage = smem + L::kQ + t * L::kTileBytes;
+      // (Two 32-column pieces of O at a time, so that a piece is on its way while the one before it is packed.)
+      const uint32_t stage = smem_u32(smem + L::kQ + t * L::kTileBytes);
 #pragma unroll
-      for (int c = 0; c < HD / 32; ++c) {
+      for (int c = 0; c < HD / 32; c += 2) {
         if (c * 32 >= p.dvo) break;
-        float o[32];
-        tmem_ld32f(o_addr + c * 32, o);
+        float o[2][32];
+        tmem_ld32f(o_addr + c * 32, o[0]);
+        tmem_ld32f(o_addr + c * 32 + 32, o[1]);
         tmem_wait_ld();
-        stage_put32<T>(stage, r, c * 32, o, inv, HD * 2);
+        stage_put32<T>(stage, r, c * 32, o[0], inv, HD * 2);
+        if (c * 32 + 32 < p.dvo) stage_put32<T>(stage, r, c * 32 + 32, o[1], inv, HD * 2);
       }
       __syncwarp();
       warp_copy_out<T, HD / 8>(stage, reinterpret_cast<T*>(p.out.ptr) + (int64_t)sq.bidx * p.out.s[0] +
