@@ -374,14 +374,23 @@ bool rows_disjoint(const View4& v, int64_t inner) {
 }
 
 // ---- keep bits shared between the kernels of one backward (KeepShare in common.cuh) ---------
-// Decides whether (and for how many 32-key tiles) dQ's rows carry keep bits from the dK/dV kernel to the dQ
-// kernel.  dQ must be a tensor in which no two rows share memory, shaped like q, and apart from everything
+// Decides whether (and for how many 32-key tiles) dQ's rows, or dBias, carry keep bits from the dK/dV kernel to the dQ
+// kernel.  dBias must be dense, with 16-byte aligned rows, every element in a place of its own, and apart from everything the
+// kernels still read when the bits are written (dQ included: wide heads read them once more).  dQ must be a tensor in which no two rows share memory, shaped like q, and apart from everything
 // the kernels still read when the bits are written.  Head dims below 64 have no room for a tile (128 bytes)
 // in a row.
 void keep_share_setup(Params& p) {
   p.keep_tiles = 0;
   p.keep_shift = 0;
-  if (!p.dropout_on || p.dqk < 64 || p.dq.s[3] != 1 || (reinterpret_cast<uintptr_t>(p.dq.ptr) & 15u) != 0) return;
+  if (!p.dropout_on) return;
+  const View4& d = p.dbias;
+  if (p.has_dbias && p.varlen_mode == 0 && p.dbias_vec != 0 && d.n[0] == p.batch && d.n[1] == p.hq && d.n[2] == p.max_sq &&
+      d.n[3] == p.max_sk && rows_disjoint(d, p.max_sk) && apart_from_inputs(d, p, 2)) {
+    p.keep_shift = kKeepInDbias;
+    p.keep_tiles = p.max_sk / 32;
+    return;
+  }
+  if (p.dqk < 64 || p.dq.s[3] != 1 || (reinterpret_cast<uintptr_t>(p.dq.ptr) & 15u) != 0) return;
   for (int i = 0; i < 3; ++i)
     if (p.dq.n[i] != p.q.n[i] || p.dq.s[i] % 8 != 0) return;
   if (p.dq.n[3] != p.dqk) return;

@@ -53,7 +53,8 @@ struct Params {
                                   // (1 = first V block of the forward, 2 = first Q/dO block of dK/dV, 3 = first V block of dQ)
   int32_t packed_tiles;           // token-packed: the grid counts row tiles of all sequences instead of max_sq's per sequence
   int32_t dk_from_db;             // dK = sm_scale * dBias^T Q, after the dQ kernel has written dBias (sm100_bwd_dk_db.cuh)
-  int32_t keep_tiles, keep_shift; // keep bits of the first keep_tiles 32-key tiles pass through dQ's rows (0: none); see KeepShare
+  int32_t keep_tiles, keep_shift; // keep bits of the first keep_tiles 32-key tiles pass through dQ's rows (0: none), or, with
+                                  // keep_shift kKeepInDbias, through dBias; see KeepShare
 };
 
 // Geometry of one (sequence z) slice.
@@ -330,8 +331,18 @@ __device__ __forceinline__ uint32_t keep_mask(uint32_t w, int pair) {
 // Measured, forward + backward before and after: head dim 256, bias, dropout 0.2, 8 x 16 heads x 2048 tokens 7.43 ->
 // 6.74 ms (two of three draws gone); head dim 72 3.82 -> 3.77 (half of the keys have room); 16 packed sequences of
 // 64 to 8192 tokens, 32:8 heads of 128, 23.41 -> 23.09; 16 x 12 heads x 391, head dim 64, 0.66 -> 0.65.
-// `row32`: first of the 32 query rows; `key0`: first key of the tile (both multiples of 32).
+// Where dBias is written, each tile's words go into its own 32 x 32 of it, 64 bytes into the first row and 64 into the second:
+// there is room for every whole tile of keys, and the warp of the dQ kernel that reads them is the one that then writes these
+// 32 x 32.  Measured, 8 x 16 heads x 2048 of 72 with bias, dropout 0.2 (half of the keys have room in dQ): dQ 948 -> 832 us, dK/dV 1312 -> 1343 (all of its bits are stored).
+// `row32`: first of the 32 query rows; `key0`: first key of the tile (both multiples of 32).  IN_DBIAS: compiled with dBias.
+constexpr int kKeepInDbias = -1;
+template <bool IN_DBIAS>
 __device__ __forceinline__ uint32_t* keep_share_word(const Params& p, const Seq& sq, int h, int row32, int key0, int lane) {
+  if (IN_DBIAS && p.keep_shift == kKeepInDbias) {
+    char* base = reinterpret_cast<char*>(p.dbias.ptr) +
+                 2 * ((int64_t)sq.bidx * p.dbias.s[0] + (int64_t)h * p.dbias.s[1] + (int64_t)(row32 + (lane >> 4)) * p.dbias.s[2] + key0);
+    return reinterpret_cast<uint32_t*>(base) + (lane & 15);
+  }
   const int t = key0 >> 5;
   const int64_t row = sq.q0 + row32 + (t >> p.keep_shift);
   char* base = reinterpret_cast<char*>(p.dq.ptr) +

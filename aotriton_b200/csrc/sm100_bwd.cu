@@ -749,7 +749,7 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
               return dctx.base + (uint64_t)min(mbase + q4 + 4 * (k + u), p.max_sq - 1) * dctx.stride + (uint64_t)(n >> 2);
             });
           if (keep_shared(p, sq, mbase, it.n0 + quarter * 32))
-            *keep_share_word(p, sq, h, mbase, it.n0 + quarter * 32, lane) = keep_rows_from_quads(mine, lane);
+            *keep_share_word<(FEAT & kBias) != 0>(p, sq, h, mbase, it.n0 + quarter * 32, lane) = keep_rows_from_quads(mine, lane);
           keep = keep_word_of_key(mine, lane);
         }
         if (threadIdx.x == AB200_TRACE_TID) AB200_STAMP(G, 1);
@@ -1196,7 +1196,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
       // keep bits the dK/dV kernel left behind: on their way while the tensor pipe computes S
       const bool shared = drop_on && keep_shared(p, sq, m0 + quarter * 32, nbase);
       uint32_t shared_bits = 0u;
-      if (shared) shared_bits = *keep_share_word(p, sq, h, m0 + quarter * 32, nbase, lane);
+      if (shared) shared_bits = *keep_share_word<(FEAT & kBias) != 0>(p, sq, h, m0 + quarter * 32, nbase, lane);
       // the warp's 32 x 32 bias tile: on its way while the tensor pipe computes S, unless the generator's state is to find room as well
       uint4 braw[4];
       auto load_bias = [&] {

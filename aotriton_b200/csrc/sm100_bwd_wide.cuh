@@ -373,7 +373,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         // dK: keep bits the dV launch left behind, on their way while the tensor pipe computes S'
         const bool shared = MODE == kWideDK && drop_on && keep_shared(p, sq, mbase, r0 + quarter * 32);
         uint32_t shared_bits = 0u;
-        if (shared) shared_bits = *keep_share_word(p, sq, h, mbase, r0 + quarter * 32, lane);
+        if (shared) shared_bits = *keep_share_word<(FEAT & kBias) != 0>(p, sq, h, mbase, r0 + quarter * 32, lane);
         uint4 braw[4];      // the warp's 32 x 32 bias tile: on its way while the tensor pipe computes S'
         if (bias_on)
           tile32_load<T>(braw, reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] + (int64_t)h * p.bias.s[1] +
@@ -445,7 +445,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
             });
           if constexpr (MODE == kWideDV) {
             if (keep_shared(p, sq, mbase, r0 + quarter * 32))
-              *keep_share_word(p, sq, h, mbase, r0 + quarter * 32, lane) = keep_rows_from_quads(mine, lane);
+              *keep_share_word<(FEAT & kBias) != 0>(p, sq, h, mbase, r0 + quarter * 32, lane) = keep_rows_from_quads(mine, lane);
           }
           keep = keep_word_of_key(mine, lane);
         }
@@ -512,7 +512,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         const int nbase = (cb_lo + i) * kNB + cbase;     // first key of this thread's columns
         const bool shared = drop_on && keep_shared(p, sq, r0 + quarter * 32, nbase);
         uint32_t shared_bits = 0u;
-        if (shared) shared_bits = *keep_share_word(p, sq, hrow, r0 + quarter * 32, nbase, lane);
+        if (shared) shared_bits = *keep_share_word<(FEAT & kBias) != 0>(p, sq, hrow, r0 + quarter * 32, nbase, lane);
         uint4 braw[4];      // the warp's 32 x 32 bias tile: on its way while the tensor pipe computes S'
         if (bias_on)
           row32_load<T>(braw, bias_tile + (int64_t)nbase * p.bias.s[3], p.bias.s[2], p.bias.s[3], p.bias_vec, rows_left, sq.sk - nbase, lane);
