@@ -20,15 +20,21 @@
 // then take the packed 16-bit P' / dS' (the A operand of the accumulating GEMM), [256,512) the
 // accumulator.  Twelve warps: TMA producer, MMA issuer, logsumexp/delta stager (dV, dK), one idle,
 // eight compute warps (thread = one row of the 128 x 64 score tile, two warpgroups split its columns
-// 32 apiece).  The arithmetic is that of the 128-wide kernels (see the head of sm100_bwd.cu); dK and dV
+// 32 apiece); dV with bias and dropout has eight more and two S' buffers (wide_groups).  The arithmetic is that of the 128-wide kernels (see the head of sm100_bwd.cu); dK and dV
 // recompute the probabilities separately, which is the price of the one-accumulator form.
 // Every wait is bounded.
 
-constexpr int kWideThreads = 384;
-constexpr int kWideCompute = 8;        // warps 4..11
+constexpr int kWideCompute = 8;        // warps of a compute group: 4..11, and 12..19 where there are two
 constexpr int kNB = 64;                // rows of a streamed block
 constexpr uint32_t kWColS = 0, kWColDP = 64, kWColAcc = 256;
 constexpr int kWideDV = 0, kWideDK = 1, kWideDQ = 2;
+// Compute groups.  dV with dropout and bias is bound by its compute warps (they read the bias and draw the bits that the later
+// kernels get from it): two groups take every other streamed block, with a buffer of S' each, so that one's loads and
+// generator run beside the other's.  Measured, 8 x 16 heads x 2048 of 256, bias, dropout 0.2: 1448 -> 1237 us.  Elsewhere it
+// gains nothing (dropout alone, 4 x 16 x 1000: 158 us either way) or the tensor pipe or the memory is the bound and 96 registers a thread
+// instead of 168 only cost (bias alone, 2 x 4 x 300 of 160: 15 -> 18; causal, 2 x 16:8 heads x 4096: dK 485 -> 523, dQ 436 -> 464).
+constexpr int wide_groups(int mode, int feat) { return mode == kWideDV && feat == kAll ? 2 : 1; }
+constexpr int wide_threads(int mode, int feat) { return 128 + 32 * kWideCompute * wide_groups(mode, feat); }
 
 struct WideSmem {
   static constexpr int kBoxes = 4;                       // 64-column boxes per 256-wide tile
@@ -41,7 +47,7 @@ struct WideSmem {
   static constexpr int kAuxFlag = kAux + 2 * 2 * kNB * 4;
   static constexpr int kBars = kAuxFlag + 16;
   static constexpr int bResFull = 0, bLateFull = 1, bLateEmpty = 3, bEarlyFull = 5, bEarlyEmpty = 7, bSFull = 9,
-                       bSRead = 10, bDpFull = 11, bDsFull = 13, bAccDone = 15, bAuxFull = 16, bAuxEmpty = 18, bCount = 20;
+                       bSRead = 11, bDpFull = 13, bDsFull = 15, bAccDone = 17, bAuxFull = 18, bAuxEmpty = 20, bCount = 22;
   static constexpr int kTmemSlot = kBars + bCount * 8;
   static constexpr int kAbort = kTmemSlot + 8;
   static constexpr int kUsed = kAbort + 8;
@@ -63,13 +69,15 @@ static __device__ __noinline__ void zero_tail_rows_streamed(uint8_t* tile, int v
 
 // grid = (cdiv(rows, 128), heads, batch): rows/heads are keys/kv heads (dV, dK) or queries/q heads (dQ)
 template <typename T, int MODE, int FEAT>
-__global__ void __launch_bounds__(kWideThreads, 1)
+__global__ void __launch_bounds__(wide_threads(MODE, FEAT), 1)
 sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm_r1,
                       const __grid_constant__ CUtensorMap tm_r2, const __grid_constant__ CUtensorMap tm_late,
                       const __grid_constant__ CUtensorMap tm_early, unsigned int* status) {
   using L = WideSmem;
   constexpr bool kKeys = MODE != kWideDQ;      // the CTA's rows are keys
   constexpr bool kHasDp = MODE != kWideDV;
+  constexpr int kGroups = wide_groups(MODE, FEAT);
+  constexpr uint32_t kColDPW = kGroups == 2 ? 128 : kWColDP;      // (behind two S' buffers)
   // The early tile has one stage; dV, which keeps only K resident, gives it two in the second
   // resident tile's place.
   constexpr int kEarlyStages = MODE == kWideDV ? 2 : 1;
@@ -129,9 +137,9 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
     for (int s = 0; s < 2; ++s) {
       mbar_init(&bars[L::bEarlyFull + s], 1);
       mbar_init(&bars[L::bEarlyEmpty + s], 1);
+      mbar_init(&bars[L::bSFull + s], 1);
+      mbar_init(&bars[L::bSRead + s], kWideCompute);
     }
-    mbar_init(&bars[L::bSFull], 1);
-    mbar_init(&bars[L::bSRead], kWideCompute);
     mbar_init(&bars[L::bAccDone], 1);
     fence_barrier_init();
     prefetch_tmap(&tm_r1); prefetch_tmap(&tm_r2); prefetch_tmap(&tm_late); prefetch_tmap(&tm_early);
@@ -230,16 +238,17 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
     auto issue_early = [&](int i) -> bool {
       const uint32_t s = (uint32_t)i & 1u;
       const uint32_t es = (uint32_t)(i % kEarlyStages), epar = (uint32_t)(i / kEarlyStages) & 1u;
+      const uint32_t sb = kGroups == 2 ? s : 0u;      // S' buffer
       if constexpr (MODE == kWideDV) {
-        if (i > 0 && !wait(L::bSRead, (uint32_t)(i - 1) & 1u, 0x3800)) return false;
+        if (i >= kGroups && !wait(L::bSRead + sb, (uint32_t)(kGroups == 2 ? (i >> 1) - 1 : i - 1) & 1u, 0x3800)) return false;
         if (!wait(L::bEarlyFull + es, epar, 0x3200)) return false;
         tc_fence_after();
         const uint64_t ea = early_km + (uint64_t)(es * kStageStep);
         if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < 16; ++kk)
-            if (kk < ksteps_qk) mma_ss(tmem_base + kWColS, r1_km + res_step(kk), ea + str_step(kk), kIdescS, kk > 0 ? 1u : 0u);
-          mma_commit(&bars[L::bSFull]);
+            if (kk < ksteps_qk) mma_ss(tmem_base + kWColS + sb * 64u, r1_km + res_step(kk), ea + str_step(kk), kIdescS, kk > 0 ? 1u : 0u);
+          mma_commit(&bars[L::bSFull + sb]);
           mma_commit(&bars[L::bEarlyEmpty + es]);
           // the accumulating GEMM of block i-2 has run: its P' buffer can be written again
           mma_commit(&bars[L::bDpFull + s]);
@@ -255,7 +264,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
 #pragma unroll
           for (int kk = 0; kk < 16; ++kk)
             if (kk < ksteps_vo)
-              mma_ss(tmem_base + kWColDP + s * 64u, r2_km + res_step(kk), ea + str_step(kk), kIdescS, kk > 0 ? 1u : 0u);
+              mma_ss(tmem_base + kColDPW + s * 64u, r2_km + res_step(kk), ea + str_step(kk), kIdescS, kk > 0 ? 1u : 0u);
           mma_commit(&bars[L::bDpFull + s]);
           mma_commit(&bars[L::bEarlyEmpty + es]);
         }
@@ -286,7 +295,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
       }
       tc_fence_after();
       const uint64_t lb = late_mn + (uint64_t)(s * kStageStep);
-      const uint32_t a_col = tmem_base + kWColDP + s * 64u;
+      const uint32_t a_col = tmem_base + kColDPW + s * 64u;
       const uint32_t first = i > 0 ? 1u : 0u;
       if (elect_one()) {
 #pragma unroll
@@ -302,9 +311,17 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
     // compute warps' copy of S'_i into registers; dP'_{i+1} takes the buffer acc_{i-1} has read)
     bool ok = wait(L::bResFull, 0, 0x3700);
     if (ok) ok = issue_early(0);
-    for (int i = 0; ok && i < niter; ++i) {
-      if (i + 1 < niter && !(ok = issue_early(i + 1))) break;
-      ok = issue_acc(i);
+    if constexpr (kGroups == 2) {      // (acc_i | S'_{i+2}: a group's next block follows its last one's accumulation)
+      if (ok && niter > 1) ok = issue_early(1);
+      for (int i = 0; ok && i < niter; ++i) {
+        ok = issue_acc(i);
+        if (ok && i + 2 < niter) ok = issue_early(i + 2);
+      }
+    } else {
+      for (int i = 0; ok && i < niter; ++i) {
+        if (i + 1 < niter && !(ok = issue_early(i + 1))) break;
+        ok = issue_acc(i);
+      }
     }
   } else if (warp == 2) {
     // logsumexp (in log2 units) and delta of the streamed query blocks (dV, dK), staged negated
@@ -341,7 +358,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
     }
   } else if (warp >= 4) {
     // ================================== compute ======================================
-    const int quarter = warp & 3, wg = (warp - 4) >> 2;
+    const int quarter = warp & 3, wg = ((warp - 4) >> 2) & 1, group = (warp - 4) >> 3;
     const int r = quarter * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const int cbase = kWgCols * wg;
@@ -362,12 +379,17 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
     const uint64_t ph_off = p.off2 + ((drop_on && p.off1_ptr) ? *p.off1_ptr : 0ull);
     if constexpr (kKeys) {
       const int n = row;
-      for (int i = 0, hg = 0, cb = 0; i < niter; ++i) {
+      int hg = 0, cb = 0;      // i / ncb, i % ncb
+      auto advance = [&] { if (++cb == ncb) { cb = 0; ++hg; } };
+      if (kGroups == 2 && group == 1) advance();
+      for (int i = kGroups == 2 ? group : 0; i < niter; i += kGroups) {
         const int s = i & 1;
         const uint32_t par2 = (uint32_t)(i >> 1) & 1u;
+        const uint32_t sb = kGroups == 2 ? (uint32_t)s : 0u, spar = kGroups == 2 ? par2 : (uint32_t)i & 1u;      // S' buffer and phase
         const int h = hk * p.group + hg;
         const int mbase = (cb_lo + cb) * kNB + cbase;      // first query row of this thread's columns
-        if (++cb == ncb) { cb = 0; ++hg; }
+        advance();
+        if constexpr (kGroups == 2) advance();
         const uint32_t lse2 = aux_s + (uint32_t)(s * 2 * kNB + cbase) * 4u;      // shared-space addresses
         const uint32_t dlt = lse2 + (uint32_t)kNB * 4u;
         // dK: keep bits the dV launch left behind, on their way while the tensor pipe computes S'
@@ -379,21 +401,21 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           tile32_load<T>(braw, reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] + (int64_t)h * p.bias.s[1] +
                                    (int64_t)mbase * p.bias.s[2] + (int64_t)(r0 + quarter * 32) * p.bias.s[3],
                          p.bias.s[2], p.bias.s[3], p.bias_vec != 0, sq.sq - mbase, sq.sk - (r0 + quarter * 32), lane);
-        if (bias_on && i + 1 < niter) {      // (hg, cb: the next block's by now)
+        if (bias_on && i + kGroups < niter) {      // (hg, cb: the group's next block's by now)
           const int mnext = (cb_lo + cb) * kNB + cbase;
           tile32_prefetch(reinterpret_cast<const T*>(p.bias.ptr) + (int64_t)sq.bidx * p.bias.s[0] + (int64_t)(hk * p.group + hg) * p.bias.s[1] +
                               (int64_t)mnext * p.bias.s[2] + (int64_t)(r0 + quarter * 32) * p.bias.s[3],
                           p.bias.s[2], p.bias.s[3], sq.sq - mnext, sq.sk - (r0 + quarter * 32), lane);
         }
-        if (!mbar_wait(&bars[L::bSFull], (uint32_t)i & 1u, abort_flag, status, 0x3A00)) { ok = false; break; }
+        if (!mbar_wait(&bars[L::bSFull + sb], spar, abort_flag, status, 0x3A00)) { ok = false; break; }
         if (!mbar_wait(&bars[L::bAuxFull + s], par2, abort_flag, status, 0x3A80)) { ok = false; break; }
         tc_fence_after();
         float pr[32];
-        tmem_ld32f(tmem_base + lane_addr + kWColS + cbase, pr);
+        tmem_ld32f(tmem_base + lane_addr + kWColS + sb * 64u + cbase, pr);
         tmem_wait_ld();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[L::bSRead]);
+        if (lane == 0) mbar_arrive(&bars[L::bSRead + sb]);
         const bool any_mask = !(mbase >= warp_lo && mbase + kWgCols - 1 <= warp_hi);
         if (!bias_on && aux_flag[s] == 0) {
           const float2 sc2 = make_float2(p.qk_scale, p.qk_scale);
@@ -453,7 +475,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         // P' has been consumed
         if (!mbar_wait(&bars[L::bDpFull + s], par2, abort_flag, status, 0x3B00)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t a_col = tmem_base + lane_addr + kWColDP + (uint32_t)s * 64u + cbase;
+        const uint32_t a_col = tmem_base + lane_addr + kColDPW + (uint32_t)s * 64u + cbase;
         uint32_t pk[16];
         if constexpr (MODE == kWideDV) {
 #pragma unroll
@@ -564,7 +586,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
               return dctx.base + (uint64_t)md * dctx.stride + (uint64_t)((nbase >> 2) + c4 + u);
             });
         }
-        const uint32_t a_col = tmem_base + lane_addr + kWColDP + (uint32_t)s * 64u + cbase;
+        const uint32_t a_col = tmem_base + lane_addr + kColDPW + (uint32_t)s * 64u + cbase;
         if (!mbar_wait(&bars[L::bDpFull + s], par2, abort_flag, status, 0x3D00)) { ok = false; break; }
         tc_fence_after();
         {
@@ -609,7 +631,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
       T* dst = reinterpret_cast<T*>(outv.ptr) + (int64_t)sq.bidx * outv.s[0] + (int64_t)hrow * outv.s[1] +
                (row_tok0 + r0) * outv.s[2];
       const float scale = MODE != kWideDV ? p.sm_scale : ((FEAT & kDropout) ? p.dropout_scale : 1.0f);
-      for (int c = wg; c * 32 < d_out; c += 2) {
+      for (int c = (warp - 4) >> 2; c * 32 < d_out; c += 2 * kGroups) {
         float v[32];
         tmem_ld32f(tmem_base + lane_addr + kWColAcc + c * 32, v);
         tmem_wait_ld();
@@ -678,17 +700,17 @@ cudaError_t launch_bwd_wide_T(int which, const Params& p, cudaStream_t st) {
     if ((e = set_smem(4 * kWideDV + feat, reinterpret_cast<const void*>(kern_dv))) != cudaSuccess) return e;
     if ((e = set_smem(4 * kWideDK + feat, reinterpret_cast<const void*>(kern_dk))) != cudaSuccess) return e;
     dim3 grid((p.max_sk + kBlk - 1) / kBlk, p.hk, p.batch);
-    e = launch_kernel(kern_dv, grid, dim3(kWideThreads), L::kDynamic, st, p, k128, k128, do64, q64, status);
+    e = launch_kernel(kern_dv, grid, dim3(wide_threads(kWideDV, feat)), L::kDynamic, st, p, k128, k128, do64, q64, status);
     if (e != cudaSuccess) return e;
     if (!p.dk_from_db) {
       count_launch();
-      e = launch_kernel(kern_dk, grid, dim3(kWideThreads), L::kDynamic, st, p, k128, v128, q64, do64, status);
+      e = launch_kernel(kern_dk, grid, dim3(wide_threads(kWideDK, feat)), L::kDynamic, st, p, k128, v128, q64, do64, status);
     }
   } else {
     const Kernel kern_dq = kKernels[kWideDQ][feat];
     if ((e = set_smem(4 * kWideDQ + feat, reinterpret_cast<const void*>(kern_dq))) != cudaSuccess) return e;
     dim3 grid((p.max_sq + kBlk - 1) / kBlk, p.hq, p.batch);
-    e = launch_kernel(kern_dq, grid, dim3(kWideThreads), L::kDynamic, st, p, q128, do128, k64, v64, status);
+    e = launch_kernel(kern_dq, grid, dim3(wide_threads(kWideDQ, feat)), L::kDynamic, st, p, q128, do128, k64, v64, status);
     if (e == cudaSuccess && p.dk_from_db) {
       count_launch();
       auto kern_db = sm100_bwd_dk_db_kernel<T>;
