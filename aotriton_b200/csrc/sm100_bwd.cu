@@ -210,9 +210,9 @@ __device__ __forceinline__ DkdvItem dkdv_item(const Params& p, int w) {
   DkdvItem it;
   const int per = p.batch * p.hk;
   const int nkb = (p.max_sk + kBlk - 1) / kBlk;
-  const int grp = w / (nkb * 8), r = w - grp * (nkb * 8);
+  const int grp = quick_div(w, nkb * 8), r = w - grp * (nkb * 8);
   const int kb = r >> 3, rem = grp * 8 + (r & 7);
-  it.z = min(rem, per - 1) / p.hk;
+  it.z = quick_div(min(rem, per - 1), p.hk);
   it.hk = min(rem, per - 1) - it.z * p.hk;
   it.n0 = kb * kBlk;
   it.sq = resolve_seq(p, it.z);
@@ -945,12 +945,13 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
     h = hz - z * nh;
     m0 = (nx - 1 - xi) * kBlk;
   }
-  // Whether an earlier CTA timed out: read here, decided on behind the set-up, which then runs under the read.
-  const unsigned int failed_before = threadIdx.x == 0 ? *reinterpret_cast<volatile unsigned int*>(status) : 0u;
+  // Whether an earlier CTA timed out: read here, by every thread (in a branch the read would be waited for at its end), decided
+  // on behind the set-up, which so runs under the read.
+  const unsigned int failed_before = *reinterpret_cast<volatile unsigned int*>(status);
   if (warp == 2 && lane == 0) { prefetch_tmap(&tm_q); prefetch_tmap(&tm_do); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); }
   const Seq sq = resolve_seq(p, z);
   if (m0 >= sq.sq) return;
-  const int hk = h / p.group;
+  const int hk = quick_div(h, p.group);
   int n_lo, n_hi;
   key_range(p, sq, m0, min(m0 + kBlk, sq.sq) - 1, n_lo, n_hi);
   if (n_hi < n_lo) {
@@ -976,24 +977,23 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
     mbar_init(&bars[L::bSRead], kComputeWarps);
     mbar_init(&bars[L::bAccDone], 1);
     fence_barrier_init();
-    // This thread is also the TMA producer: Q, dO and the first two K and V blocks (all ring stages
-    // are free) are requested right away, before the CTA-wide synchronisation and the tensor-memory
-    // allocation, which then overlap with the copies' latency.
+    // This thread is also the TMA producer: Q, dO and the first block of K and V are requested right away, before the
+    // CTA-wide synchronisation and the tensor-memory allocation, which then overlap with the copies' latency.  (A request takes
+    // this thread 100 clocks: the others follow behind the synchronisation.)
     const int qrow = (int)(sq.q0 + m0);
     mbar_expect_tx(&bars[L::bResFull], 2 * L::kTile);
     for (int hf = 0; hf < L::kHalves; ++hf) {
       tma_load_4d(smem + L::kResA + hf * 16384, &tm_q, &bars[L::bResFull], hf * 64, qrow, h, sq.bidx);
       tma_load_4d(smem + L::kResB + hf * 16384, &tm_do, &bars[L::bResFull], hf * 64, qrow, h, sq.bidx);
     }
-    for (int i = 0; i < min(2, niter); ++i) {
-      const int krow = (int)(sq.k0 + (int64_t)(jb_lo + i) * kBlk);
-      mbar_expect_tx(&bars[L::bKFull + i], L::kTile);
+    const int krow = (int)(sq.k0 + (int64_t)jb_lo * kBlk);
+    mbar_expect_tx(&bars[L::bKFull], L::kTile);
+    for (int hf = 0; hf < L::kHalves; ++hf)
+      tma_load_4d(smem + L::kK + hf * 16384, &tm_k, &bars[L::bKFull], hf * 64, krow, hk, sq.bidx);
+    if (p.drop_copy != 3) {   // (test hook: the first block's V never arrives)
+      mbar_expect_tx(&bars[L::bVFull], L::kTile);
       for (int hf = 0; hf < L::kHalves; ++hf)
-        tma_load_4d(smem + L::kK + i * L::kTile + hf * 16384, &tm_k, &bars[L::bKFull + i], hf * 64, krow, hk, sq.bidx);
-      if (p.drop_copy == 3 && i == 0) continue;   // test hook: this block's V never arrives
-      mbar_expect_tx(&bars[L::bVFull + i], L::kTile);
-      for (int hf = 0; hf < L::kHalves; ++hf)
-        tma_load_4d(smem + L::kV + i * L::kTile + hf * 16384, &tm_v, &bars[L::bVFull + i], hf * 64, krow, hk, sq.bidx);
+        tma_load_4d(smem + L::kV + hf * 16384, &tm_v, &bars[L::bVFull], hf * 64, krow, hk, sq.bidx);
     }
   }
   if (warp == 1) {
@@ -1001,16 +1001,14 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
     tmem_relinquish();
   }
   tc_fence_before();
-  const bool leave = __syncthreads_or(failed_before != 0u) != 0;      // (one read, one CTA-wide decision)
+  const bool leave = __syncthreads_or(failed_before != 0u) != 0;      // (one CTA-wide decision)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   if (leave) {
     if (threadIdx.x == 0) {      // the copies requested above land before the CTA gives its shared memory back
       mbar_wait_quiet(&bars[L::bResFull], 0, abort_flag);
-      for (int i = 0; i < min(2, niter); ++i) {
-        mbar_wait_quiet(&bars[L::bKFull + i], 0, abort_flag);
-        if (!(p.drop_copy == 3 && i == 0)) mbar_wait_quiet(&bars[L::bVFull + i], 0, abort_flag);
-      }
+      mbar_wait_quiet(&bars[L::bKFull], 0, abort_flag);
+      if (p.drop_copy != 3) mbar_wait_quiet(&bars[L::bVFull], 0, abort_flag);
     }
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
@@ -1019,9 +1017,9 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
 
   if (warp == 0) {
     if (lane == 0) {
-      // (Q, dO and the first two K and V blocks were requested during set-up)
-      int issued_k = min(2, niter), issued_v = min(2, niter);
-      for (int i = min(2, niter); i < niter; ++i) {
+      // (Q, dO and the first K and V block were requested during set-up; waits for the first use of a stage pass at once)
+      int issued_k = 1, issued_v = 1;
+      for (int i = 1; i < niter; ++i) {
         const int sv = i & 1, sk = i % L::kKStages;
         const int krow = (int)(sq.k0 + (int64_t)(jb_lo + i) * kBlk);
         if (!mbar_wait(&bars[L::bKEmpty + sk], ((uint32_t)(i / L::kKStages) & 1u) ^ 1u, abort_flag, status, 0x2180 + i)) break;

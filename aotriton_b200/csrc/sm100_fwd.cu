@@ -145,15 +145,16 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
     constexpr int kHeadGroup = AB200_FWD_HEAD_GROUP > 0 ? AB200_FWD_HEAD_GROUP : 1;
     const int nx = (int)gridDim.x, nh = (int)gridDim.y, nhz = nh * (int)gridDim.z;
     const int lin = (int)blockIdx.x + nx * ((int)blockIdx.y + nh * (int)blockIdx.z);
-    const int grp = lin / (kHeadGroup * nx), r = lin - grp * (kHeadGroup * nx);
+    const int grp = quick_div(lin, kHeadGroup * nx), r = lin - grp * (kHeadGroup * nx);
     const int gsize = min(kHeadGroup, nhz - grp * kHeadGroup);
-    const int xi = r / gsize, hz = grp * kHeadGroup + (r - xi * gsize);
-    z = hz / nh;
+    const int xi = quick_div(r, gsize), hz = grp * kHeadGroup + (r - xi * gsize);
+    z = quick_div(hz, nh);
     h = hz - z * nh;
     m0 = (nx - 1 - xi) * kCtaRows;
   }
-  // Whether an earlier CTA timed out: read here, decided on behind the set-up, which then runs under the read.
-  const unsigned int failed_before = threadIdx.x == 0 ? *reinterpret_cast<volatile unsigned int*>(status) : 0u;
+  // Whether an earlier CTA timed out: read here, by every thread (in a branch the read would be waited for at its end), decided
+  // on behind the set-up, which so runs under the read.
+  const unsigned int failed_before = *reinterpret_cast<volatile unsigned int*>(status);
   if (warp == 2 && lane == 0) { prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); }
   // One thread of the grid reports the seed and offset actually used, before any early exit.
   if (drop_on && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) {
@@ -164,7 +165,7 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
   }
   int4 ends;
   if (!EXACT && p.packed_tiles > 0) {      // one-dimensional grid: the heads of a tile next to each other
-    const int tile = (int)blockIdx.x / p.hq;
+    const int tile = quick_div((int)blockIdx.x, p.hq);
     h = (int)blockIdx.x - tile * p.hq;
     if (!packed_tile<kCtaRows>(p, tile, lane, z, m0, ends)) return;
   } else if (p.varlen_mode != 0) {
@@ -172,7 +173,7 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
   }
   const Seq sq = seq_from_ends(p, z, ends);
   if (m0 >= sq.sq) return;
-  const int hk = h / p.group;
+  const int hk = quick_div(h, p.group);
   const int ntile = (L::kTiles == 2 && m0 + kBM < sq.sq) ? 2 : 1;   // the second tile may lie beyond the sequence
 
   // Block range: the union over the CTA's rows; a tile simply sees fully masked blocks outside its own.
@@ -204,41 +205,32 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
       mbar_init(&bars[L::bKeepEmpty + s], 4);     // one per softmax warp of the tile
     }
     fence_barrier_init();
-    // This thread is also the TMA producer: both Q tiles and the first blocks of K and V (the ring
-    // stages are all free) are requested right away, before the CTA-wide synchronisation and the
-    // tensor-memory allocation, which then overlap with the copies' latency.
+    // This thread is also the TMA producer: what the first products need, both Q tiles and the first block of K, is
+    // requested right away, before the CTA-wide synchronisation and the tensor-memory allocation, which then overlap with
+    // the copies' latency.  (A request takes this thread 100 clocks: the other blocks that the rings have room for follow behind the
+    // synchronisation.)
     for (int t = 0; t < ntile; ++t) {
       const int qrow = (int)(sq.q0 + m0 + t * kBM);
       mbar_expect_tx(&bars[L::bQFull + t], L::kTileBytes);
       for (int hf = 0; hf < L::kHalves; ++hf)
         tma_load_4d(smem + L::kQ + t * L::kTileBytes + hf * 16384, &tm_q, &bars[L::bQFull + t], hf * 64, qrow, h, sq.bidx);
     }
-    for (int j = 0; j < min(kStages, nblk); ++j) {
-      const int krow = (int)(sq.k0 + (int64_t)(jb_lo + j) * kBN);
-      mbar_expect_tx(&bars[L::bKFull + j], L::kTileBytes);
-      for (int hf = 0; hf < L::kHalves; ++hf)
-        tma_load_4d(smem + L::kK + j * L::kTileBytes + hf * 16384, &tm_k, &bars[L::bKFull + j], hf * 64, krow, hk, sq.bidx);
-      if (p.drop_copy == 1 && j == 0) continue;   // test hook: this block's V never arrives
-      mbar_expect_tx(&bars[L::bVFull + j], L::kTileBytes);
-      for (int hf = 0; hf < L::kHalves; ++hf)
-        tma_load_4d(smem + L::kV + j * L::kTileBytes + hf * 16384, &tm_v, &bars[L::bVFull + j], hf * 64, krow, hk, sq.bidx);
-    }
+    mbar_expect_tx(&bars[L::bKFull], L::kTileBytes);
+    for (int hf = 0; hf < L::kHalves; ++hf)
+      tma_load_4d(smem + L::kK + hf * 16384, &tm_k, &bars[L::bKFull], hf * 64, (int)(sq.k0 + (int64_t)jb_lo * kBN), hk, sq.bidx);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before();
-  const bool leave = __syncthreads_or(failed_before != 0u) != 0;      // (one read, one CTA-wide decision)
+  const bool leave = __syncthreads_or(failed_before != 0u) != 0;      // (one CTA-wide decision)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   if (leave) {
     if (threadIdx.x == 0) {      // the copies requested above land before the CTA gives its shared memory back
       for (int t = 0; t < ntile; ++t) mbar_wait_quiet(&bars[L::bQFull + t], 0, abort_flag);
-      for (int j = 0; j < min(kStages, nblk); ++j) {
-        mbar_wait_quiet(&bars[L::bKFull + j], 0, abort_flag);
-        if (!(p.drop_copy == 1 && j == 0)) mbar_wait_quiet(&bars[L::bVFull + j], 0, abort_flag);
-      }
+      mbar_wait_quiet(&bars[L::bKFull], 0, abort_flag);
     }
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
@@ -250,18 +242,21 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
     if (warp == 0) {
       // =============================== TMA producer ===================================
       if (lane == 0) {
-        // (the Q tiles and the first kStages blocks were requested during set-up)
-        int issued = 2 * min(kStages, nblk);
-        for (int j = min(kStages, nblk); j < nblk; ++j) {
+        // (the Q tiles and the first block of K were requested during set-up; waits for the first use of a stage pass at once)
+        int issued = 1;
+        for (int j = 0; j < nblk; ++j) {
           const int s = j % kStages;
           const uint32_t ph = (uint32_t)(j / kStages) & 1u;
           const int krow = (int)(sq.k0 + (int64_t)(jb_lo + j) * kBN);
-          if (!mbar_wait(&bars[L::bKEmpty + s], ph ^ 1u, abort_flag, status, 0x100 + j)) break;
-          mbar_expect_tx(&bars[L::bKFull + s], L::kTileBytes);
-          for (int hf = 0; hf < L::kHalves; ++hf)
-            tma_load_4d(smem + L::kK + s * L::kTileBytes + hf * 16384, &tm_k, &bars[L::bKFull + s], hf * 64, krow, hk,
-                        sq.bidx);
+          if (j > 0) {
+            if (!mbar_wait(&bars[L::bKEmpty + s], ph ^ 1u, abort_flag, status, 0x100 + j)) break;
+            mbar_expect_tx(&bars[L::bKFull + s], L::kTileBytes);
+            for (int hf = 0; hf < L::kHalves; ++hf)
+              tma_load_4d(smem + L::kK + s * L::kTileBytes + hf * 16384, &tm_k, &bars[L::bKFull + s], hf * 64, krow, hk,
+                          sq.bidx);
+          }
           if (!mbar_wait(&bars[L::bVEmpty + s], ph ^ 1u, abort_flag, status, 0x200 + j)) { issued = j * 2 + 1; break; }
+          if (p.drop_copy == 1 && j == 0) { issued = 2; continue; }   // test hook: this block's V never arrives
           mbar_expect_tx(&bars[L::bVFull + s], L::kTileBytes);
           for (int hf = 0; hf < L::kHalves; ++hf)
             tma_load_4d(smem + L::kV + s * L::kTileBytes + hf * 16384, &tm_v, &bars[L::bVFull + s], hf * 64, krow, hk,
