@@ -595,12 +595,12 @@ int ab200_bwd_preprocess(const ab200_attn_bwd_args* a, void* stream) {
   return (int)launch_preprocess(a->prob.dtype, p, st);
 }
 
-// `share`: dK/dV and dQ run in one call, so that keep bits may pass from one to the other, and dK come out of the second.
-static int run_dkdv(const ab200_attn_bwd_args* a, void* stream, bool share) {
+// One stage by itself (which: 1 dK/dV, 2 dQ): nothing passes from one kernel to another.
+static int run_stage(int which, const ab200_attn_bwd_args* a, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   Params p{};
   if (int e = fill_bwd(a, p, true)) return e;
-  if (!a->dk.ptr || !a->dv.ptr) return kErrInvalidValue;
+  if (which == 1 ? !a->dk.ptr || !a->dv.ptr : !a->dq.ptr) return kErrInvalidValue;
   if (int e = check_device(st)) return e;
   DeviceGuard guard(st);
   const int sel = ab200_select_variant(kOpBwd, a->prob.dtype, p.dqk, p.dvo,
@@ -608,52 +608,14 @@ static int run_dkdv(const ab200_attn_bwd_args* a, void* stream, bool share) {
   if (sel < 0) return -sel;
   if ((sel & 0xff) >= kVarTcgen05) {
     t_last_bwd = 2;
-    if (share) { keep_share_setup(p); p.dk_from_db = dk_from_db_possible(p); }
-    return (int)launch_sm100_bwd_dkdv(a->prob.dtype, p, st);
+    return (int)(which == 1 ? launch_sm100_bwd_dkdv(a->prob.dtype, p, st) : launch_sm100_bwd_dq(a->prob.dtype, p, st));
   }
   t_last_bwd = 1;
-  return (int)launch_general(1, a->prob.dtype, p, st);
+  return (int)launch_general(which, a->prob.dtype, p, st);
 }
 
-static int run_dq(const ab200_attn_bwd_args* a, void* stream, bool share) {
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  Params p{};
-  if (int e = fill_bwd(a, p, true)) return e;
-  if (!a->dq.ptr) return kErrInvalidValue;
-  if (int e = check_device(st)) return e;
-  DeviceGuard guard(st);
-  const int sel = ab200_select_variant(kOpBwd, a->prob.dtype, p.dqk, p.dvo,
-                                       family_flags(g_family) | (sm100_bwd_supported(a->prob.dtype, p) ? AB200_SELECT_ALIGNED : 0));
-  if (sel < 0) return -sel;
-  if ((sel & 0xff) >= kVarTcgen05) {
-    t_last_bwd = 2;
-    if (share) { keep_share_setup(p); p.dk_from_db = dk_from_db_possible(p); }
-    return (int)launch_sm100_bwd_dq(a->prob.dtype, p, st);
-  }
-  t_last_bwd = 1;
-  return (int)launch_general(2, a->prob.dtype, p, st);
-}
-
-// dK/dV and dQ of the general kernels in one launch.  -1: done; 0: not a case for it; else an error.
-static int run_general_bwd(const ab200_attn_bwd_args* a, void* stream) {
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  Params p{};
-  if (int e = fill_bwd(a, p, true)) return e;
-  if (int e = check_device(st)) return e;
-  DeviceGuard guard(st);
-  const int sel = ab200_select_variant(kOpBwd, a->prob.dtype, p.dqk, p.dvo,
-                                       family_flags(g_family) | (sm100_bwd_supported(a->prob.dtype, p) ? AB200_SELECT_ALIGNED : 0));
-  if (sel < 0) return -sel;
-  const int elt = a->prob.dtype == AB200_DTYPE_FP32 ? 4 : 2;
-  if ((sel & 0xff) != kVarGeneral || !apart_from_inputs(p.dq, p, elt) || (p.has_dbias && !apart_from_inputs(p.dbias, p, elt)))
-    return 0;
-  t_last_bwd = 1;
-  const int e = (int)launch_general(3, a->prob.dtype, p, st);
-  return e ? e : -1;
-}
-
-int ab200_bwd_dkdv(const ab200_attn_bwd_args* a, void* stream) { return run_dkdv(a, stream, false); }
-int ab200_bwd_dq(const ab200_attn_bwd_args* a, void* stream) { return run_dq(a, stream, false); }
+int ab200_bwd_dkdv(const ab200_attn_bwd_args* a, void* stream) { return run_stage(1, a, stream); }
+int ab200_bwd_dq(const ab200_attn_bwd_args* a, void* stream) { return run_stage(2, a, stream); }
 
 int ab200_bwd_uses_dq_acc(const ab200_attn_bwd_args* a, void* stream) {
   if (a == nullptr || a->deterministic || !want_fused(g_family)) return 0;
@@ -694,14 +656,43 @@ int ab200_bwd_postprocess(const ab200_attn_bwd_args* a, void* stream) {
 int ab200_attn_bwd(const ab200_attn_bwd_args* a, void* stream) {
   if (a == nullptr) return kErrInvalidValue;
   if (!a->dq.ptr || !a->dk.ptr || !a->dv.ptr) return kErrInvalidValue;
-  if (int e = ab200_bwd_preprocess(a, stream)) return e;
   if (a->dq_acc != nullptr && ab200_bwd_uses_dq_acc(a, stream)) {
+    if (int e = ab200_bwd_preprocess(a, stream)) return e;
     if (int e = ab200_bwd_fused(a, stream)) return e;
     return ab200_bwd_postprocess(a, stream);
   }
-  if (int e = run_general_bwd(a, stream)) return e > 0 ? e : 0;
-  if (int e = run_dkdv(a, stream, true)) return e;
-  return run_dq(a, stream, true);
+  // The stages in one: validated, and the device looked up, once (a call of the smallest size is bound by the host, and each
+  // stage by itself costs about a microsecond of it beyond its launch).
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int dtype = a->prob.dtype;
+  Params p{};
+  // (a problem the preprocess stage takes and the others do not: delta is written before the refusal, as stage by stage)
+  const int refused = fill_bwd(a, p, true);
+  if (refused) {
+    const int e = ab200_bwd_preprocess(a, stream);
+    return e ? e : refused;
+  }
+  if (int e = check_device(st)) return e;
+  DeviceGuard guard(st);
+  const int sel = ab200_select_variant(kOpBwd, dtype, p.dqk, p.dvo,
+                                       family_flags(g_family) | (sm100_bwd_supported(dtype, p) ? AB200_SELECT_ALIGNED : 0));
+  const bool tc = sel > 0 && (sel & 0xff) >= kVarTcgen05;
+  cudaError_t e = cudaSuccess;
+  if (tc && p.dqk <= 128 && p.dvo <= 128 && p.max_sq > 0 && p.batch > 0 && (e = sm100_bwd_ticket(&p.ticket)) != cudaSuccess) return (int)e;
+  if ((e = launch_preprocess(dtype, p, st)) != cudaSuccess) return (int)e;
+  if (sel < 0) return -sel;
+  t_last_bwd = tc ? 2 : 1;
+  if (tc) {
+    keep_share_setup(p);
+    p.dk_from_db = dk_from_db_possible(p);
+    if ((e = launch_sm100_bwd_dkdv(dtype, p, st)) != cudaSuccess) return (int)e;
+    return (int)launch_sm100_bwd_dq(dtype, p, st);
+  }
+  const int elt = dtype == AB200_DTYPE_FP32 ? 4 : 2;
+  if (apart_from_inputs(p.dq, p, elt) && (!p.has_dbias || apart_from_inputs(p.dbias, p, elt)))
+    return (int)launch_general(3, dtype, p, st);      // dK/dV and dQ in one launch
+  if ((e = launch_general(1, dtype, p, st)) != cudaSuccess) return (int)e;
+  return (int)launch_general(2, dtype, p, st);
 }
 
 // Whether ab200_attn_bwd would run the two-kernel tcgen05 backward, the device apart: 1, 0, or a negative error.

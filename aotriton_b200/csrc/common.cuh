@@ -52,6 +52,7 @@ struct Params {
   int32_t drop_copy;              // test hook of the bounded waits: the producer leaves out one tile copy
                                   // (1 = first V block of the forward, 2 = first Q/dO block of dK/dV, 3 = first V block of dQ)
   int32_t packed_tiles;           // token-packed: the grid counts row tiles of all sequences instead of max_sq's per sequence
+  unsigned int* ticket;           // dK/dV's ticket counter, zeroed by the preprocess kernel of the same call (null: by the launch itself)
   int32_t dk_from_db;             // dK = sm_scale * dBias^T Q, after the dQ kernel has written dBias (sm100_bwd_dk_db.cuh)
   int32_t keep_tiles, keep_shift; // keep bits of the first keep_tiles 32-key tiles pass through dQ's rows (0: none), or, with
                                   // keep_shift kKeepInDbias, through dBias; see KeepShare

@@ -385,6 +385,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_constant__ Params p) {
   constexpr int kWarpRows = 16, kPer = 16 / (int)sizeof(T);      // elements of a 16-byte load
   const int z = blockIdx.z, h = blockIdx.y;
+  if (p.ticket != nullptr && blockIdx.x == 0 && h == 0 && z == 0 && threadIdx.x == 0) *p.ticket = 0u;
   const Seq sq = resolve_seq(p, z);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int d = p.dvo;

@@ -89,6 +89,8 @@ cudaError_t launch_sm100_bwd_dq(int dtype, const Params& p, cudaStream_t st);
 bool sm100_bwd_fused_supported(int dtype, const Params& p);
 cudaError_t launch_sm100_bwd_fused(int dtype, const Params& p, float* dq_acc, cudaStream_t st);
 cudaError_t launch_postprocess(int dtype, const View4& dq, const float* acc, float scale, cudaStream_t st);
+// The ticket counter of the next dK/dV launch on the current device (head dims up to 128), to be zeroed ahead of it in stream order.
+cudaError_t sm100_bwd_ticket(unsigned int** ticket);
 // Words the tcgen05 kernels of the current device set when a bounded wait ran out (0 = none).
 // Reading synchronises the device.
 unsigned int sm100_fwd_status(bool reset);

@@ -63,8 +63,8 @@ namespace ab200 {
 
 __device__ unsigned int g_sm100_bwd_status = 0;
 
-// Ticket counters of the persistent dK/dV kernel.  Each launch takes the next one of the pool and
-// zeroes it in stream order, so launches on different streams do not share a counter unless more
+// Ticket counters of the persistent dK/dV kernel.  Each launch takes the next one of the pool, zeroed
+// ahead of it in stream order, so launches on different streams do not share a counter unless more
 // than kTicketPool of them are in flight at once.
 constexpr unsigned int kTicketPool = 256;
 __device__ unsigned int g_dkdv_ticket[kTicketPool];
@@ -1317,6 +1317,27 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
   }
 }
 
+}  // namespace
+
+cudaError_t sm100_bwd_ticket(unsigned int** ticket) {
+  static std::atomic<unsigned int> launch_seq{0};
+  static std::atomic<unsigned int*> pool_of[64];
+  int dev = 0;
+  cudaError_t e = host().get_device(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  const bool pretend = host_pretends();      // (a pretended device's address is not remembered)
+  unsigned int* pool = pretend ? nullptr : pool_of[dev].load(std::memory_order_acquire);
+  if (pool == nullptr) {
+    if ((e = host().symbol_address(reinterpret_cast<void**>(&pool), reinterpret_cast<const void*>(&g_dkdv_ticket))) != cudaSuccess) return e;
+    if (!pretend) pool_of[dev].store(pool, std::memory_order_release);
+  }
+  *ticket = pool + (launch_seq.fetch_add(1) % kTicketPool);
+  return cudaSuccess;
+}
+
+namespace {
+
 // which: 1 dK/dV, 2 dQ(+dBias), 3 dK/dV fused with dQ accumulation into `dq_acc` (HD == 128 only)
 template <typename T, int HD>
 cudaError_t launch_bwd_T(int which, const Params& p, cudaStream_t st, float* dq_acc) {
@@ -1326,10 +1347,10 @@ cudaError_t launch_bwd_T(int which, const Params& p, cudaStream_t st, float* dq_
       !make_tile_map_16bit(&tv, p.v, p.dvo, p.v.n[2], kBlk) ||
       !make_tile_map_16bit(&tdo, p.dout, p.dvo, p.dout.n[2], kBlk))
     return cudaErrorInvalidValue;
-  // Per-device facts (addresses of the status word and the ticket pool, SM count, the shared-memory
+  // Per-device facts (address of the status word, SM count, the shared-memory
   // attribute of each kernel) are looked up once for the current device, which the entry points
   // make the stream's device, and remembered.
-  struct PerDevice { std::atomic<unsigned int*> status{nullptr}, tickets{nullptr}; std::atomic<int> sms{0}; };
+  struct PerDevice { std::atomic<unsigned int*> status{nullptr}; std::atomic<int> sms{0}; };
   static PerDevice per_device[64];
   static std::atomic<bool> attr_set[64][20];
   const bool exact = p.varlen_mode == 0 && p.max_sq % 128 == 0 && p.max_sk % 128 == 0 && p.dqk == HD && p.dvo == HD;
@@ -1375,15 +1396,12 @@ cudaError_t launch_bwd_T(int which, const Params& p, cudaStream_t st, float* dq_
       pd.sms.store(sms, std::memory_order_release);
     }
     dim3 grid(nitems < sms ? nitems : sms, 1, 1);     // persistent: one CTA per SM
-    // ticket counter of this launch: one of a small pool, zeroed in stream order
-    static std::atomic<unsigned int> launch_seq{0};
-    unsigned int* tickets = pd.tickets.load(std::memory_order_acquire);
-    if (tickets == nullptr) {
-      if ((e = host().symbol_address(reinterpret_cast<void**>(&tickets), reinterpret_cast<const void*>(&g_dkdv_ticket))) != cudaSuccess) return e;
-      pd.tickets.store(tickets, std::memory_order_release);
+    // ticket counter of this launch: one of a small pool, zeroed in stream order, by the preprocess kernel of the same call or here
+    unsigned int* ticket = p.ticket;
+    if (ticket == nullptr) {
+      if ((e = sm100_bwd_ticket(&ticket)) != cudaSuccess) return e;
+      if ((e = host().memset_async(ticket, 0, sizeof(unsigned int), st)) != cudaSuccess) return e;
     }
-    unsigned int* ticket = tickets + (launch_seq.fetch_add(1) % kTicketPool);
-    if ((e = host().memset_async(ticket, 0, sizeof(unsigned int), st)) != cudaSuccess) return e;
     if (fused)
       e = launch_kernel(kern_fused, grid, dim3(kFusedThreads), BwdSmem<128>::kDynamic, st, p, tq, tk, tv, tdo, status, nitems,
                         ticket, dq_acc);
