@@ -152,11 +152,23 @@ cudaError_t h_memset_async(void* ptr, int value, size_t bytes, cudaStream_t st) 
   if (fake()) return cudaSuccess;
   return cudaMemsetAsync(ptr, value, bytes, st);
 }
-cudaError_t h_launch(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t st) {
+cudaError_t h_launch(const void* fn, dim3 grid, dim3 block, void** args, size_t smem, cudaStream_t st, bool early) {
   cudaError_t c;
   if (injected(kCallLaunch, &c)) return c;
   if (fake()) return cudaSuccess;
-  return cudaLaunchKernel(fn, grid, block, args, smem, st);
+  // `early`: the grid may be set up while the one before it in the stream still runs, which saves the launch's latency between
+  // the two; every kernel waits for the earlier grids first thing (wait_for_earlier_grids).
+  cudaLaunchAttribute overlap{};
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = st;
+  config.attrs = &overlap;
+  config.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelExC(&config, fn, args);
 }
 int h_encode_tiled(CUtensorMap* map, CUtensorMapDataType type, cuuint32_t rank, void* base, const cuuint64_t* dims,
                    const cuuint64_t* strides, const cuuint32_t* box, const cuuint32_t* estr, CUtensorMapInterleave il,

@@ -21,6 +21,15 @@ namespace ab200 {
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471824645996f;
 
+// Every kernel's first statement.  Kernels are launched so that a grid may be set up while the one before it in the stream
+// still runs (h_launch, cabi.cu): nothing may be read or written before this wait, which ends when all earlier grids have
+// completed and their writes can be seen, and no thread may leave without it, or a later grid could overtake an earlier one.  The
+// second instruction lets the next grid in the stream be set up in turn.
+__device__ __forceinline__ void wait_for_earlier_grids() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 struct View4 {
   void* ptr;
   int64_t n[4];   // extents

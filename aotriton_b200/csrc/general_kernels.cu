@@ -77,6 +77,7 @@ __device__ __forceinline__ float half_warp_sum(float x) {
 // Forward.  grid = (cdiv(max_sq, 16), Hq, batch)
 template <typename T, int DJ>
 __global__ void __launch_bounds__(kThreads) general_fwd_kernel(const __grid_constant__ Params p) {
+  wait_for_earlier_grids();
   extern __shared__ float smem[];
   constexpr int DPAD = DJ * 32;
   constexpr int LD = DPAD + kPad;
@@ -211,6 +212,7 @@ __device__ __forceinline__ void bwd_pair(const Params& p, const Seq& sq, const D
 // dK / dV.  grid = (cdiv(max_sk, 16), Hk, batch)
 template <typename T, int DJ>
 __global__ void __launch_bounds__(kThreads) general_bwd_dkdv_kernel(const __grid_constant__ Params p) {
+  wait_for_earlier_grids();
   extern __shared__ float smem[];
   constexpr int DPAD = DJ * 32;
   constexpr int LD = DPAD + kPad;
@@ -293,6 +295,7 @@ __global__ void __launch_bounds__(kThreads) general_bwd_dkdv_kernel(const __grid
 // dQ (+ dBias).  grid = (cdiv(max_sq, 16), Hq, batch)
 template <typename T, int DJ>
 __global__ void __launch_bounds__(kThreads) general_bwd_dq_kernel(const __grid_constant__ Params p) {
+  wait_for_earlier_grids();
   extern __shared__ float smem[];
   constexpr int DPAD = DJ * 32;
   constexpr int LD = DPAD + kPad;
@@ -383,6 +386,7 @@ __global__ void __launch_bounds__(kThreads) general_bwd_dq_kernel(const __grid_c
 // (which fp32 used to take: 2 x 8 heads x 500 rows of 64, with nothing in L2, 20.6 -> 3.7 us).
 template <typename T>
 __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_constant__ Params p) {
+  wait_for_earlier_grids();
   constexpr int kWarpRows = 16, kPer = 16 / (int)sizeof(T);      // elements of a 16-byte load
   const int z = blockIdx.z, h = blockIdx.y;
   if (p.ticket != nullptr && blockIdx.x == 0 && h == 0 && z == 0 && threadIdx.x == 0) *p.ticket = 0u;
@@ -451,6 +455,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
 template <typename T>
 __global__ void __launch_bounds__(256) bwd_postprocess_kernel(View4 dq, const float* __restrict__ acc, float scale,
                                                               int vec) {
+  wait_for_earlier_grids();
   const int64_t tokens = dq.n[2], d = dq.n[3];
   const int b = blockIdx.z, h = blockIdx.y;
   const float* src = acc + ((int64_t)b * dq.n[1] + h) * tokens * d;
@@ -481,6 +486,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) dropout_sign_kernel(View4 r, int rows, int cols, int num_head, DropoutCtx base,
                                                            const uint64_t* seed_ptr, const uint64_t* off1_ptr,
                                                            uint64_t off2) {
+  wait_for_earlier_grids();
   const int z = blockIdx.z, h = blockIdx.y;
   const uint32_t stride = (uint32_t)((cols + 3) / 4);
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -517,17 +523,17 @@ cudaError_t launch_general_T(int which, const Params& p, cudaStream_t st) {
     size_t sm = fwd_smem<T, DJ>();
     if ((e = set_smem(general_fwd_kernel<T, DJ>, sm)) != cudaSuccess) return e;
     dim3 grid((p.max_sq + kTile - 1) / kTile, p.hq, p.batch);
-    e = launch_kernel(general_fwd_kernel<T, DJ>, dim3(grid), dim3(kThreads), sm, st, p);
+    e = launch_kernel_as<false>(general_fwd_kernel<T, DJ>, dim3(grid), dim3(kThreads), sm, st, p);
   } else if (which == 1) {
     size_t sm = bwd_smem<T, DJ>();
     if ((e = set_smem(general_bwd_dkdv_kernel<T, DJ>, sm)) != cudaSuccess) return e;
     dim3 grid((p.max_sk + kTile - 1) / kTile, p.hk, p.batch);
-    e = launch_kernel(general_bwd_dkdv_kernel<T, DJ>, dim3(grid), dim3(kThreads), sm, st, p);
+    e = launch_kernel_as<false>(general_bwd_dkdv_kernel<T, DJ>, dim3(grid), dim3(kThreads), sm, st, p);
   } else {
     size_t sm = bwd_smem<T, DJ>();
     if ((e = set_smem(general_bwd_dq_kernel<T, DJ>, sm)) != cudaSuccess) return e;
     dim3 grid((p.max_sq + kTile - 1) / kTile, p.hq, p.batch);
-    e = launch_kernel(general_bwd_dq_kernel<T, DJ>, dim3(grid), dim3(kThreads), sm, st, p);
+    e = launch_kernel_as<false>(general_bwd_dq_kernel<T, DJ>, dim3(grid), dim3(kThreads), sm, st, p);
   }
   if (e == cudaSuccess) count_launch();
   return e;
@@ -565,7 +571,7 @@ cudaError_t launch_tiled_T(int which, const Params& p, cudaStream_t st) {
   const int rows_total = which == 1 ? p.max_sk : (which == 3 && p.max_sk > p.max_sq ? p.max_sk : p.max_sq);
   const int blocks = (rows_total + C::kBM - 1) / C::kBM;
   dim3 grid(which == 3 ? 2 * blocks : blocks, which == 1 ? p.hk : p.hq, p.batch);
-  e = launch_kernel(kern, grid, dim3(which == 0 ? kFwdGroups * C::kThreads : C::kThreads), sm, st, p);
+  e = launch_kernel_as<false>(kern, grid, dim3(which == 0 ? kFwdGroups * C::kThreads : C::kThreads), sm, st, p);
   if (e == cudaSuccess) count_launch();
   return e;
 }

@@ -219,6 +219,7 @@ __device__ __forceinline__ void tile_of_block(int nx, int nh, int nz, int& x, in
 constexpr int kFwdGroups = 2;
 template <typename T, int DP>
 __global__ void __launch_bounds__(kFwdGroups * 128, 2) tiled_fwd_kernel(const __grid_constant__ Params p) {
+  wait_for_earlier_grids();
   using C = Tiled<DP>;
   constexpr int kGroupFloats = 2 * C::kBN * C::kLd + C::kBM * C::kLdP;
   extern __shared__ float smem[];
@@ -547,6 +548,7 @@ __device__ __forceinline__ void tiled_bwd_dq(const Params& p, float* smem, int z
 // heads x 500 tokens are 256 CTAs of four warps, 7 warps an SM, waiting for their own loads and barriers.
 template <typename T, int DP, int WHICH>
 __global__ void __launch_bounds__(128, DP <= 64 || WHICH == 2 ? 3 : 2) tiled_bwd_kernel(const __grid_constant__ Params p) {
+  wait_for_earlier_grids();
   extern __shared__ float smem[];
   constexpr int kBM = Tiled<DP>::kBM;
   int x, h, z;

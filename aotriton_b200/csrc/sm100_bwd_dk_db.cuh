@@ -33,6 +33,7 @@ template <typename T>
 __global__ void __launch_bounds__(kDkDbThreads, 2)
 sm100_bwd_dk_db_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm_db,
                        const __grid_constant__ CUtensorMap tm_q, unsigned int* status) {
+  wait_for_earlier_grids();
   using L = DkDbSmem;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));

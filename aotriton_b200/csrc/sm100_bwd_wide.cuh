@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(wide_threads(MODE, FEAT), 1)
 sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm_r1,
                       const __grid_constant__ CUtensorMap tm_r2, const __grid_constant__ CUtensorMap tm_late,
                       const __grid_constant__ CUtensorMap tm_early, unsigned int* status) {
+  wait_for_earlier_grids();
   using L = WideSmem;
   constexpr bool kKeys = MODE != kWideDQ;      // the CTA's rows are keys
   constexpr bool kHasDp = MODE != kWideDV;

@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
 sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                  unsigned int* status) {
+  wait_for_earlier_grids();
   using L = FwdSmem<HD>;
   constexpr int kStages = L::kStages, kCtaRows = L::kCtaRows;
   extern __shared__ uint8_t smem_raw[];

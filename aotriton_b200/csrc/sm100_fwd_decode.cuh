@@ -96,6 +96,7 @@ template <typename T, int HD, int MT, int CS, int W>
 __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(DecSmem<HD, MT, W>::kThreads, DecSmem<HD, MT, W>::kCtasPerSm)
 sm100_fwd_decode_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm_k,
                         const __grid_constant__ CUtensorMap tm_v, unsigned int* status, int stages) {
+  wait_for_earlier_grids();
   using L = DecSmem<HD, MT, W>;
   constexpr int kBoxes = HD / 64, kKsteps = HD / 16;
   extern __shared__ uint8_t smem_raw[];
