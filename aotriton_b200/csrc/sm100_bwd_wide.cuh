@@ -447,11 +447,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           }
         }
         if (any_mask) {
-#pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            const int m = mbase + c;
-            pr[c] = (m >= v_lo && m <= v_hi) ? pr[c] : 0.f;
-          }
+          mask_columns<32>(pr, v_lo - mbase, v_hi - mbase, mbase >= warp_lo, 0.f);
         }
         uint32_t keep = 0xffffffffu;
         if (shared) {
@@ -569,11 +565,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           for (int c = 0; c < 32; ++c) pr[c] = ex2(pr[c] - lse2);
         }
         if (any_mask) {
-#pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            const int n = nbase + c;
-            pr[c] = (n >= v_lo && n <= v_hi) ? pr[c] : 0.f;
-          }
+          mask_columns<32>(pr, v_lo - nbase, v_hi - nbase, nbase >= warp_lo, 0.f);
         }
         uint32_t keep = 0xffffffffu;
         if (shared) {
