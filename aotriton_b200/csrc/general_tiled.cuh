@@ -10,7 +10,7 @@
 // so that a 16-byte read feeds 8 or more multiply-adds.  32 rows and not 64: at the sizes single precision is
 // used at, the number of CTAs is what is short.  fp32 tiles are copied asynchronously, a block ahead of their use
 // where a tile's last reader is known early.  Measured, fp32, 2 x 8 heads x 500 tokens, head dim 64, causal, nothing in L2,
-// against loads through registers with one group of warps a tile: forward 98 -> 35 us, backward 139 -> 110.
+// against loads through registers with one group of warps a tile: forward 98 -> 35 us, backward 139 -> 110 (97 once the copy loops fit the instruction cache).
 //
 // All tiles are row-major fp32 with four floats of padding: (DP + 4) / 4 is odd, so the 16 lanes that
 // read 16 different rows at one column hit different banks.  The P / dS rows that a warp writes are read
@@ -27,6 +27,35 @@ template <int DP> struct Tiled {
 template <typename T>
 __device__ __forceinline__ bool rows_vec4(const View4& v, int d) {
   return ((reinterpret_cast<uintptr_t>(v.ptr) & (4 * sizeof(T) - 1)) == 0) && ((v.s[0] | v.s[1] | v.s[2]) & 3) == 0 && (d & 3) == 0;
+}
+
+// A thread's part of a tile through registers: rows `kStep` apart, `rows` of them (from the first) in the tensor, `cols` of its four
+// columns.
+template <typename T, int DP, int ROWS, int kStep, int kUnroll>
+__device__ __forceinline__ void stage_loaded(float* dst, const T* src, int64_t stride, int rows, int cols, bool vec) {
+#pragma unroll kUnroll
+  for (int i = 0; i < ROWS / kStep; ++i) {
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i * kStep < rows && cols > 0) {
+      const T* s = src + (int64_t)(i * kStep) * stride;
+      if (sizeof(T) == 2 && vec) {
+        const uint2 w = __ldg(reinterpret_cast<const uint2*>(s));
+        const T* e = reinterpret_cast<const T*>(&w);
+        x = make_float4(to_f32<T>(e[0]), to_f32<T>(e[1]), to_f32<T>(e[2]), to_f32<T>(e[3]));
+      } else {
+        x.x = to_f32<T>(s[0]);
+        if (cols > 1) x.y = to_f32<T>(s[1]);
+        if (cols > 2) x.z = to_f32<T>(s[2]);
+        if (cols > 3) x.w = to_f32<T>(s[3]);
+      }
+    }
+    *reinterpret_cast<float4*>(dst + i * kStep * Tiled<DP>::kLd) = x;
+  }
+}
+// fp32 rows that cannot be copied 16 bytes at a time; out of line, so that the copies of aligned rows are all that the kernels' loops hold.
+template <typename T, int DP, int ROWS, int kStep>
+static __device__ __noinline__ void stage_elements(float* dst, const T* src, int64_t stride, int rows, int cols) {
+  stage_loaded<T, DP, ROWS, kStep, 4>(dst, src, stride, rows, cols, false);
 }
 
 // Rows row0.. of one head into dst[ROWS][DP + 4]; rows at or beyond nrows and columns at or beyond d
@@ -53,25 +82,10 @@ __device__ __forceinline__ void stage_tile(float* dst, const View4& v, int b, in
                      ::"r"(to), "l"(i < in ? src : reinterpret_cast<const T*>(v.ptr)), "r"(i < in ? 16 : 0) : "memory");
     }
   }
-  if (sizeof(T) != 4 || !vec) {
-#pragma unroll (sizeof(T) == 4 ? 1 : 4)
-    for (int i = 0; i < ROWS / kStep; ++i) {
-      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (row0 + r0 + i * kStep < nrows && c < d) {
-        const T* s = src + (int64_t)(i * kStep) * v.s[2];
-        if (vec) {
-          const uint2 w = __ldg(reinterpret_cast<const uint2*>(s));
-          const T* e = reinterpret_cast<const T*>(&w);
-          x = make_float4(to_f32<T>(e[0]), to_f32<T>(e[1]), to_f32<T>(e[2]), to_f32<T>(e[3]));
-        } else {
-          x.x = to_f32<T>(s[0]);
-          if (c + 1 < d) x.y = to_f32<T>(s[1]);
-          if (c + 2 < d) x.z = to_f32<T>(s[2]);
-          if (c + 3 < d) x.w = to_f32<T>(s[3]);
-        }
-      }
-      *reinterpret_cast<float4*>(dst + i * kStep * kLd) = x;
-    }
+  if (sizeof(T) != 4) {
+    stage_loaded<T, DP, ROWS, kStep, 4>(dst, src, v.s[2], nrows - row0 - r0, c < d ? d - c : 0, vec);
+  } else if (!vec) {
+    stage_elements<T, DP, ROWS, kStep>(dst, src, v.s[2], nrows - row0 - r0, c < d ? d - c : 0);
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
@@ -201,10 +215,18 @@ __device__ __forceinline__ const T* bias_at(const Params& p, const Seq& sq, int 
 }
 
 // Which (row tile counted from the last, head, batch) a CTA takes: heads in groups of 32, inside a group the row tiles
-// slowest, so that the long tiles of a causal problem start together and first.
+// slowest, so that the long tiles of a causal problem start together and first.  SNAKE: the CTAs that find room at once are dealt out
+// a round of all SMs at a time, so every other round runs from the short tiles to the long ones; in the same order the SM with the
+// longest first tile also had the longest second one.  Measured, forward, fp32, 2 x 8 x 500 x 64 causal: 35 -> 31 us.  (The backward's
+// time is its longest CTA's, whichever SM that is on.)
+template <bool SNAKE>
 __device__ __forceinline__ void tile_of_block(int nx, int nh, int nz, int& x, int& h, int& z) {
-  constexpr int kHeadGroup = 32;
-  const int lin = (int)blockIdx.x + nx * ((int)blockIdx.y + nh * (int)blockIdx.z);
+  constexpr int kHeadGroup = 32, kSms = 148;
+  int lin = (int)blockIdx.x + nx * ((int)blockIdx.y + nh * (int)blockIdx.z);
+  if constexpr (SNAKE) {
+    const int round = lin / kSms, round0 = round * kSms;
+    if (round & 1) lin = round0 + min(kSms, nx * nh * nz - round0) - 1 - (lin - round0);
+  }
   const int grp = lin / (kHeadGroup * nx), r = lin - grp * (kHeadGroup * nx), gsize = min(kHeadGroup, nh * nz - grp * kHeadGroup);
   x = r / gsize;
   const int hz = grp * kHeadGroup + (r - x * gsize);
@@ -235,7 +257,7 @@ __global__ void __launch_bounds__(kFwdGroups * 128, 2) tiled_fwd_kernel(const __
     if (p.off_out) *p.off_out = p.off2 + (p.off1_ptr ? *p.off1_ptr : 0ull);
   }
   int x, h, z;
-  tile_of_block((int)gridDim.x, (int)gridDim.y, (int)gridDim.z, x, h, z);
+  tile_of_block<true>((int)gridDim.x, (int)gridDim.y, (int)gridDim.z, x, h, z);
   const int m0 = ((int)gridDim.x - 1 - x) * C::kBM;
   const Seq sq = resolve_seq(p, z);
   if (m0 >= sq.sq) return;
@@ -552,7 +574,7 @@ __global__ void __launch_bounds__(128, DP <= 64 || WHICH == 2 ? 3 : 2) tiled_bwd
   extern __shared__ float smem[];
   constexpr int kBM = Tiled<DP>::kBM;
   int x, h, z;
-  tile_of_block((int)gridDim.x, (int)gridDim.y, (int)gridDim.z, x, h, z);
+  tile_of_block<false>((int)gridDim.x, (int)gridDim.y, (int)gridDim.z, x, h, z);
   if constexpr (WHICH == 1) {
     tiled_bwd_dkdv<T, DP>(p, smem, z, h, x * kBM);
   } else if constexpr (WHICH == 2) {
