@@ -539,18 +539,28 @@ cudaError_t launch_general_T(int which, const Params& p, cudaStream_t st) {
   return e;
 }
 
+template <int DP>
+int64_t row_tiles(const Params& p) {      // of dQ, dK and dV together
+  auto blocks = [](int n) { return (int64_t)((n + Tiled<DP>::kBM - 1) / Tiled<DP>::kBM); };
+  return p.batch * (p.hq * blocks(p.max_sq) + p.hk * blocks(p.max_sk));
+}
 // dK/dV and dQ in one launch, or in two.  Together they fill the chip where one alone does not, and share its last
 // wave.  What they lose is occupancy: a CTA of the joint launch asks for the shared memory of dK/dV (77 KB at head dims
-// above 64, two CTAs an SM) where dQ alone has room for three.  16-bit types there lose from 4096 working CTAs on.
-// Measured, whole backward, joint against two launches, us: fp32 2x8x8x500x64 causal 143 / 197, 4x16x16x2048x64 8312 / 9232,
-// 4x8x8x1024x128 2683 / 2997, 4x16x16x2048x128 20174 / 20928; fp16 4x16x16x2048x60 8373 / 9064, 4x8x8x1024x124 2713 / 2957,
-// 4x12x12x1024x124 (3072 CTAs) 4092 / 4129, 4x16x16x1024x124 (4096) 5344 / 5140, 4x16x16x2048x124 20705 / 20357.
+// above 64, two CTAs an SM) where dQ alone has room for three.  16-bit types there lose from 4096 row tiles on; single
+// precision is small as a rule, and keeps the one launch.
+// Measured, dK/dV and dQ, joint against two launches, us (row tiles): fp32 2x8x8x500x64 causal (512) 74 / 81, 4x8x8x1024x128 (2048)
+// 1941 / 1971, 4x16x16x2048x64 (8192) 6535 / 6469, 4x16x16x2048x128 (8192) 14910 / 14062; fp16 4x16x16x2048x60 (8192) 7799 / 7759,
+// 4x8x8x1024x124 (2048) 2560 / 2624, 4x12x12x1024x124 (3072) 3844 / 3780, 4x16x16x1024x124 (4096) 4738 / 4712.
 template <typename T, int DP>
-bool joint_backward(const Params& p) {
-  if (sizeof(T) != 2 || DP <= 64) return true;
-  auto blocks = [](int n) { return (int64_t)((n + Tiled<DP>::kBM - 1) / Tiled<DP>::kBM); };
-  return p.batch * (p.hq * blocks(p.max_sq) + p.hk * blocks(p.max_sk)) < 4096;
-}
+bool joint_backward(const Params& p) { return sizeof(T) != 2 || DP <= 64 || row_tiles<DP>(p) < 4096; }
+
+// Whether two CTAs share the blocks of a row tile: where the grid fills the chip's slots (444 at head dims up to 64, 296 above) a few times
+// over, each CTA's own start and end only cost.  By the problem alone, so that the stages by themselves sum in the same order.
+// Measured, training step, us, without and with: fp32 2 x 8 x 500 x 64 causal (512 tiles) 137 / 117, 1 x 8 x 300 x 64 (160) 88 / 74,
+// 2 x 4 x 500 x 128 causal (256) 197 / 148, 4 x 8 x 500 x 64 (1024) 342 / 322, 2 x 8 x 2000 x 64 causal (2016) 1098 / 1121, 4 x 8 x 1000 x 64
+// causal (2048) 596 / 625, 4 x 8 x 1024 x 128 (2048) 2487 / 2479; fp16 2 x 8 x 500 x 60 causal 192 / 173, 4 x 16 x 1024 x 124 (4096) 6076 / 6133.
+template <int DP>
+bool split_backward(const Params& p) { return row_tiles<DP>(p) < 1536; }
 
 template <typename T, int DP>
 cudaError_t launch_tiled_T(int which, const Params& p, cudaStream_t st) {
@@ -559,18 +569,19 @@ cudaError_t launch_tiled_T(int which, const Params& p, cudaStream_t st) {
     const cudaError_t e = launch_tiled_T<T, DP>(1, p, st);
     return e != cudaSuccess ? e : launch_tiled_T<T, DP>(2, p, st);
   }
+  const bool split = which != 0 && split_backward<DP>(p);
   const size_t rows = which == 0 ? C::kBM + kFwdGroups * 2 * C::kBN : 2 * C::kBM + 2 * C::kBN;      // staged rows of DP + 4 floats
   const size_t tiles = which == 0 ? kFwdGroups : (which & 1 ? 2 : 1);                              // P and dS, or one of them
   const size_t sm = (rows * C::kLd + tiles * C::kBM * C::kLdP + (which & 1 ? 2 * C::kBN : 0)) * sizeof(float);
   auto kern = which == 0   ? tiled_fwd_kernel<T, DP>
-              : which == 1 ? tiled_bwd_kernel<T, DP, 1>
-              : which == 2 ? tiled_bwd_kernel<T, DP, 2>
-                           : tiled_bwd_kernel<T, DP, 3>;
+              : which == 1 ? (split ? tiled_bwd_kernel<T, DP, 1, 2> : tiled_bwd_kernel<T, DP, 1, 1>)
+              : which == 2 ? (split ? tiled_bwd_kernel<T, DP, 2, 2> : tiled_bwd_kernel<T, DP, 2, 1>)
+                           : (split ? tiled_bwd_kernel<T, DP, 3, 2> : tiled_bwd_kernel<T, DP, 3, 1>);
   cudaError_t e = set_smem(kern, sm);
   if (e != cudaSuccess) return e;
   const int rows_total = which == 1 ? p.max_sk : (which == 3 && p.max_sk > p.max_sq ? p.max_sk : p.max_sq);
   const int blocks = (rows_total + C::kBM - 1) / C::kBM;
-  dim3 grid(which == 3 ? 2 * blocks : blocks, which == 1 ? p.hk : p.hq, p.batch);
+  dim3 grid((which == 3 ? 2 : 1) * (split ? 2 : 1) * blocks, which == 1 ? p.hk : p.hq, p.batch);
   e = launch_kernel_as<false>(kern, grid, dim3(which == 0 ? kFwdGroups * C::kThreads : C::kThreads), sm, st, p);
   if (e == cudaSuccess) count_launch();
   return e;

@@ -220,9 +220,9 @@ __device__ __forceinline__ const T* bias_at(const Params& p, const Seq& sq, int 
 // longest first tile also had the longest second one.  Measured, forward, fp32, 2 x 8 x 500 x 64 causal: 35 -> 31 us.  (The backward's
 // time is its longest CTA's, whichever SM that is on.)
 template <bool SNAKE>
-__device__ __forceinline__ void tile_of_block(int nx, int nh, int nz, int& x, int& h, int& z) {
+__device__ __forceinline__ void tile_of_block(int bx, int nx, int nh, int nz, int& x, int& h, int& z) {
   constexpr int kHeadGroup = 32, kSms = 148;
-  int lin = (int)blockIdx.x + nx * ((int)blockIdx.y + nh * (int)blockIdx.z);
+  int lin = bx + nx * ((int)blockIdx.y + nh * (int)blockIdx.z);
   if constexpr (SNAKE) {
     const int round = lin / kSms, round0 = round * kSms;
     if (round & 1) lin = round0 + min(kSms, nx * nh * nz - round0) - 1 - (lin - round0);
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(kFwdGroups * 128, 2) tiled_fwd_kernel(const __
     if (p.off_out) *p.off_out = p.off2 + (p.off1_ptr ? *p.off1_ptr : 0ull);
   }
   int x, h, z;
-  tile_of_block<true>((int)gridDim.x, (int)gridDim.y, (int)gridDim.z, x, h, z);
+  tile_of_block<true>((int)blockIdx.x, (int)gridDim.x, (int)gridDim.y, (int)gridDim.z, x, h, z);
   const int m0 = ((int)gridDim.x - 1 - x) * C::kBM;
   const Seq sq = resolve_seq(p, z);
   if (m0 >= sq.sq) return;
@@ -369,9 +369,38 @@ __global__ void __launch_bounds__(kFwdGroups * 128, 2) tiled_fwd_kernel(const __
   }
 }
 
+// SPLIT 2: two CTAs of a cluster take every other block of the other sequence dimension and exchange their sums at the end, each
+// finishing one half of the result.  A row tile's chain of blocks is then half as long: where the grid does not fill the
+// chip several times over, the longest chain is the launch's time (split_backward()).
+__device__ __forceinline__ uint32_t pair_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void pair_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// This thread's N float4 of `give` go to the same thread of the other CTA, whose are added to `keep`.  `buf`: 128 * N float4 that nobody
+// reads or copies to any more.
+template <int N>
+__device__ __forceinline__ void pair_exchange(float* buf, float4 (&keep)[N], const float4 (&give)[N], uint32_t rank) {
+#pragma unroll
+  for (int n = 0; n < N; ++n) *reinterpret_cast<float4*>(buf + 4 * (n * 128 + (int)threadIdx.x)) = give[n];
+  pair_sync();
+  const uint32_t addr = ptx::smem_u32(buf + 4 * threadIdx.x);
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    float4 v;
+    asm volatile("{\n\t.reg .u32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\tld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [a];\n\t}"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr + 2048 * n), "r"(rank ^ 1u) : "memory");
+    keep[n].x += v.x; keep[n].y += v.y; keep[n].z += v.z; keep[n].w += v.w;
+  }
+  pair_sync();      // (the other CTA may still be reading)
+}
+
 // dK / dV of 32 keys of one kv head.  The scores of dO V^T come first: its tile is the first to be free again, so that the
 // next block's dO is on its way under the accumulation of dK, Q behind it.
-template <typename T, int DP>
+template <typename T, int DP, int SPLIT>
 __device__ __forceinline__ void tiled_bwd_dkdv(const Params& p, float* smem, int z, int hk, int n0) {
   using C = Tiled<DP>;
   constexpr int kThr = C::kThreads;
@@ -410,21 +439,28 @@ __device__ __forceinline__ void tiled_bwd_dkdv(const Params& p, float* smem, int
   auto stage_do = [&](int h, int m0) {
     stage_tile<T, DP, C::kBN, kThr>(dOs, p.dout, sq.bidx, h, sq.q0, m0, sq.sq, p.dvo, dovec, tid);
   };
-  if (m_lo <= m_hi) {
+  const uint32_t rank = SPLIT == 2 ? pair_rank() : 0u;
+  const int nblk = m_lo <= m_hi ? m_hi / C::kBN - m_lo / C::kBN + 1 : 0, total = nblk * p.group;
+  int g = 0, mb = 0;      // head of the group and block of it
+  auto advance = [&] { if (++mb == nblk) { mb = 0; ++g; } };
+  if (rank == 1) advance();
+  if ((int)rank < total) {
     stage_tile<T, DP, C::kBM, kThr>(Vs, p.v, sq.bidx, hk, sq.k0, n0, sq.sk, p.dvo, rows_vec4<T>(p.v, p.dvo), tid);
-    stage_do(hk * p.group, first);
+    stage_do(hk * p.group + g, first + mb * C::kBN);
     stage_tile<T, DP, C::kBM, kThr>(Ks, p.k, sq.bidx, hk, sq.k0, n0, sq.sk, p.dqk, rows_vec4<T>(p.k, p.dqk), tid);
     stage_wait<1>();      // V and dO
     __syncthreads();
-    stage_q(hk * p.group, first);
+    stage_q(hk * p.group + g, first + mb * C::kBN);
   }
-  for (int g = 0; g < p.group; ++g) {
-    const int h = hk * p.group + g;
-    DropoutCtx dctx;
-    if (p.dropout_on) dctx = dropout_ctx(p, z, h);
-    for (int m0 = first; m0 <= m_hi; m0 += C::kBN) {
-      const bool last_of_head = m0 + C::kBN > m_hi, more = !last_of_head || g + 1 < p.group;
-      const int next_h = last_of_head ? h + 1 : h, next_m0 = last_of_head ? first : m0 + C::kBN;
+  for (int i = (int)rank; i < total; i += SPLIT) {
+    {
+      const int h = hk * p.group + g, m0 = first + mb * C::kBN;
+      DropoutCtx dctx;
+      if (p.dropout_on) dctx = dropout_ctx(p, z, h);
+#pragma unroll
+      for (int u = 0; u < SPLIT; ++u) advance();
+      const bool more = i + SPLIT < total;
+      const int next_h = hk * p.group + g, next_m0 = first + mb * C::kBN;
       float s[4][C::kNC], dp[4][C::kNC];
       tile_dots<DP>(dp, Vs, dOs, dv4, ty, tx);
       stage_wait<0>();
@@ -464,6 +500,27 @@ __device__ __forceinline__ void tiled_bwd_dkdv(const Params& p, float* smem, int
       if (more) stage_q(next_h, next_m0);
     }
   }
+  if constexpr (SPLIT == 2) {      // the first CTA finishes dK, the second dV (Q's and dO's tiles are free)
+    float4 mine[4 * C::kND], theirs[4 * C::kND];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < C::kND; ++j) {
+        mine[i * C::kND + j] = rank == 0 ? adk[i][j] : adv[i][j];
+        theirs[i * C::kND + j] = rank == 0 ? adv[i][j] : adk[i][j];
+      }
+    pair_exchange<4 * C::kND>(Qs, mine, theirs, rank);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int n = n0 + ty * 4 + i;
+      if (n >= sq.sk) continue;
+      float4 row[C::kND];
+#pragma unroll
+      for (int j = 0; j < C::kND; ++j) row[j] = mine[i * C::kND + j];
+      store_acc_row<T, DP>(row_ptr_mut<T>(rank == 0 ? p.dk : p.dv, sq.bidx, hk, sq.k0 + n), row, rank == 0 ? p.sm_scale : 1.f, rank == 0 ? p.dqk : p.dvo, tx);
+    }
+    return;
+  }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int n = n0 + ty * 4 + i;
@@ -475,7 +532,7 @@ __device__ __forceinline__ void tiled_bwd_dkdv(const Params& p, float* smem, int
 
 // dQ (+ dBias) of 32 query rows of one head.  V is read by the scores only: the next block's is on its way for the rest
 // of a block.
-template <typename T, int DP>
+template <typename T, int DP, int SPLIT>
 __device__ __forceinline__ void tiled_bwd_dq(const Params& p, float* smem, int z, int h, int m0) {
   using C = Tiled<DP>;
   constexpr int kThr = C::kThreads;
@@ -492,10 +549,11 @@ __device__ __forceinline__ void tiled_bwd_dq(const Params& p, float* smem, int z
   if (p.dropout_on) dctx = dropout_ctx(p, z, h);
   int n_lo, n_hi, w_lo = 1, w_hi = 0;
   key_range(p, sq, m0, min(m0 + C::kBM, sq.sq) - 1, n_lo, n_hi);
-  const int first = n_lo / C::kBN * C::kBN;
+  const uint32_t rank = SPLIT == 2 ? pair_rank() : 0u;
+  const int first = n_lo / C::kBN * C::kBN + (int)rank * C::kBN;      // (this CTA's)
   auto stage_k = [&](int n0) { stage_tile<T, DP, C::kBN, kThr>(Ks, p.k, sq.bidx, hk, sq.k0, n0, sq.sk, p.dqk, kvec, tid); };
   auto stage_v = [&](int n0) { stage_tile<T, DP, C::kBN, kThr>(Vs, p.v, sq.bidx, hk, sq.k0, n0, sq.sk, p.dvo, vvec, tid); };
-  if (n_lo <= n_hi) {
+  if (first <= n_hi) {
     stage_tile<T, DP, C::kBM, kThr>(dOs, p.dout, sq.bidx, h, sq.q0, m0, sq.sq, p.dvo, rows_vec4<T>(p.dout, p.dvo), tid);
     stage_v(first);
     stage_tile<T, DP, C::kBM, kThr>(Qs, p.q, sq.bidx, h, sq.q0, m0, sq.sq, p.dqk, rows_vec4<T>(p.q, p.dqk), tid);
@@ -514,18 +572,20 @@ __device__ __forceinline__ void tiled_bwd_dq(const Params& p, float* smem, int z
   }
   const int wm = m0 + (tid >> 5) * kWarpRows;
   if (wm < sq.sq) key_range(p, sq, wm, min(wm + kWarpRows, sq.sq) - 1, w_lo, w_hi);
-  if (n_hi >= n_lo) zero_dbias_outside<T>(p, sq, h, m0, C::kBM, n_lo / C::kBN * C::kBN, (n_hi / C::kBN + 1) * C::kBN);
-  else zero_dbias_outside<T>(p, sq, h, m0, C::kBM, 0, 0);
+  if (rank == 0) {
+    if (n_hi >= n_lo) zero_dbias_outside<T>(p, sq, h, m0, C::kBM, n_lo / C::kBN * C::kBN, (n_hi / C::kBN + 1) * C::kBN);
+    else zero_dbias_outside<T>(p, sq, h, m0, C::kBM, 0, 0);
+  }
   const int dq4 = (p.dqk + 3) >> 2, dv4 = (p.dvo + 3) >> 2;
   stage_wait<2>();      // dO and V
   __syncthreads();
-  for (int n0 = first; n0 <= n_hi; n0 += C::kBN) {
-    const bool more = n0 + C::kBN <= n_hi;
+  for (int n0 = first; n0 <= n_hi; n0 += SPLIT * C::kBN) {
+    const bool more = n0 + SPLIT * C::kBN <= n_hi;
     float s[4][C::kNC], dp[4][C::kNC];
     tile_dots<DP>(dp, dOs, Vs, dv4, ty, tx);
     stage_wait<0>();
     __syncthreads();      // V has been read, K (and Q) is there
-    if (more) stage_v(n0 + C::kBN);
+    if (more) stage_v(n0 + SPLIT * C::kBN);
     tile_dots<DP>(s, Qs, Ks, dq4, ty, tx);
     const uint32_t keep = p.dropout_on ? tile_keep_bits<C::kNC>(dctx, m0 + ty * 4, n0, tx) : 0xffffffffu;
 #pragma unroll
@@ -555,7 +615,27 @@ __device__ __forceinline__ void tiled_bwd_dq(const Params& p, float* smem, int z
     tile_accumulate<DP>(adq, dSs, Ks, k0, k1, ty, tx);
     stage_wait<0>();
     __syncthreads();      // K has been read, the next V is there
-    if (more) stage_k(n0 + C::kBN);
+    if (more) stage_k(n0 + SPLIT * C::kBN);
+  }
+  if constexpr (SPLIT == 2) {      // the first CTA finishes two of a thread's rows, the second the others (K's and V's tiles are free)
+    float4 mine[2 * C::kND], theirs[2 * C::kND];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < C::kND; ++j) {
+        mine[i * C::kND + j] = rank == 0 ? adq[i][j] : adq[i + 2][j];
+        theirs[i * C::kND + j] = rank == 0 ? adq[i + 2][j] : adq[i][j];
+      }
+    pair_exchange<2 * C::kND>(Ks, mine, theirs, rank);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int m = m0 + ty * 4 + 2 * (int)rank + i;
+      float4 row[C::kND];
+#pragma unroll
+      for (int j = 0; j < C::kND; ++j) row[j] = mine[i * C::kND + j];
+      if (m < sq.sq) store_acc_row<T, DP>(row_ptr_mut<T>(p.dq, sq.bidx, h, sq.q0 + m), row, p.sm_scale, p.dqk, tx);
+    }
+    return;
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -568,23 +648,25 @@ __device__ __forceinline__ void tiled_bwd_dq(const Params& p, float* smem, int z
 // Hq, batch), last rows first.  3: both in one launch, x alternating between the two (neither reads what the other
 // writes); joint_backward() says when.  At the sizes single precision is used at, each of the two alone leaves most of the chip idle: 2 x 8
 // heads x 500 tokens are 256 CTAs of four warps, 7 warps an SM, waiting for their own loads and barriers.
-template <typename T, int DP, int WHICH>
-__global__ void __launch_bounds__(128, DP <= 64 || WHICH == 2 ? 3 : 2) tiled_bwd_kernel(const __grid_constant__ Params p) {
+template <typename T, int DP, int WHICH, int SPLIT>
+__global__ void __cluster_dims__(SPLIT, 1, 1) __launch_bounds__(128, DP <= 64 || WHICH == 2 ? 3 : 2)
+tiled_bwd_kernel(const __grid_constant__ Params p) {
   wait_for_earlier_grids();
   extern __shared__ float smem[];
   constexpr int kBM = Tiled<DP>::kBM;
+  const int nx = (int)gridDim.x / SPLIT;
   int x, h, z;
-  tile_of_block<false>((int)gridDim.x, (int)gridDim.y, (int)gridDim.z, x, h, z);
+  tile_of_block<false>((int)blockIdx.x / SPLIT, nx, (int)gridDim.y, (int)gridDim.z, x, h, z);
   if constexpr (WHICH == 1) {
-    tiled_bwd_dkdv<T, DP>(p, smem, z, h, x * kBM);
+    tiled_bwd_dkdv<T, DP, SPLIT>(p, smem, z, h, x * kBM);
   } else if constexpr (WHICH == 2) {
-    tiled_bwd_dq<T, DP>(p, smem, z, h, (int)(gridDim.x - 1 - x) * kBM);
+    tiled_bwd_dq<T, DP, SPLIT>(p, smem, z, h, (nx - 1 - x) * kBM);
   } else {
     if (x & 1) {
-      const int m0 = ((int)gridDim.x / 2 - 1 - (x >> 1)) * kBM;
-      if (m0 < p.max_sq) tiled_bwd_dq<T, DP>(p, smem, z, h, m0);
+      const int m0 = (nx / 2 - 1 - (x >> 1)) * kBM;
+      if (m0 < p.max_sq) tiled_bwd_dq<T, DP, SPLIT>(p, smem, z, h, m0);
     } else if (h < p.hk) {
-      tiled_bwd_dkdv<T, DP>(p, smem, z, h, (x >> 1) * kBM);
+      tiled_bwd_dkdv<T, DP, SPLIT>(p, smem, z, h, (x >> 1) * kBM);
     }
   }
 }

@@ -46,6 +46,22 @@ def test_edges(sq, sk, causal, dt, D):
         torch.testing.assert_close(a.double(), b, atol=ATOL[dt], rtol=ATOL[dt], msg=lambda m: f"{name}: {m}")
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("heads", [1, 24])
+def test_split_row_tiles(heads, D):
+    """Few row tiles: two CTAs share the blocks of one (1 x 1024 rows); many (24 heads): one CTA each.  Grouped heads, so that the
+    blocks run over several of them."""
+    from aotriton_b200 import autograd
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    mk = lambda h: torch.randn(1, h, 1024, D, generator=g, device="cuda")
+    q, k, v, do = mk(2 * heads), mk(heads), mk(heads), mk(2 * heads)
+    ref = _reference(q, k, v, do, torch.ones(1024, 1024, dtype=torch.bool, device="cuda").tril())
+    ins = [t.clone().requires_grad_() for t in (q, k, v)]
+    out = autograd.attention(*ins, causal=True)
+    for name, a, b in zip(("out", "dq", "dk", "dv"), (out.detach(),) + torch.autograd.grad(out, ins, do), ref):
+        torch.testing.assert_close(a.double(), b, atol=1e-4, rtol=1e-4, msg=lambda m: f"{name}: {m}")
+
+
 @pytest.mark.parametrize("D", [32, 64, 100, 128])
 @pytest.mark.parametrize("rows", [1, 5, 127, 500, 2000])
 def test_fp32_delta(rows, D):
