@@ -763,10 +763,11 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           tmem_ld16f(dp_col, dp[0]);
           tmem_wait_ld();
           if (threadIdx.x == AB200_TRACE_TID) AB200_STAMP(G, 10);
+          const float2 ds2 = make_float2(p.dropout_scale, p.dropout_scale);
 #pragma unroll
           for (int c = 0; c < 16; ++c) {
-            pk[c] = pack2<T>(pr[2 * c], pr[2 * c + 1]);
-            if constexpr ((FEAT & kDropout) != 0) pk[c] &= keep_mask(keep, c);      // (1 / (1 - p) follows at the write-out of dV)
+            if constexpr ((FEAT & kDropout) != 0) pk[c] = dropout_p_pair<T>(make_float2(pr[2 * c], pr[2 * c + 1]), ds2, keep_mask(keep, c));
+            else pk[c] = pack2<T>(pr[2 * c], pr[2 * c + 1]);
           }
           tmem_st16(dp_col, pk);
           tmem_wait_st();
@@ -774,7 +775,6 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars[L::bPFull]);
           tmem_ld16f(dp_col + 16, dp[1]);
-          const float2 ds2 = make_float2(p.dropout_scale, p.dropout_scale);
 #pragma unroll
           for (int c4 = 0; c4 < 8; ++c4) {
             if (c4 == 4) tmem_wait_ld();
@@ -852,7 +852,7 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         tc_fence_after();
         tmem_ld32f(tmem_base + lane_addr + kColAcc0 + d0, v);
         tmem_wait_ld();
-        stage_put32<T>(stage, r, d0, v, (FEAT & kDropout) ? p.dropout_scale : 1.0f, HD * 2);
+        stage_put32<T>(stage, r, d0, v, 1.0f, HD * 2);
         __syncwarp();
         warp_copy_out<T, 4>(stage, reinterpret_cast<T*>(p.dv.ptr) + (int64_t)sq.bidx * p.dv.s[0] + (int64_t)hk * p.dv.s[1] +
                                        (sq.k0 + it.n0) * p.dv.s[2],

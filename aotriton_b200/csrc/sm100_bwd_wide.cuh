@@ -474,17 +474,17 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
         tc_fence_after();
         const uint32_t a_col = tmem_base + lane_addr + kColDPW + (uint32_t)s * 64u + cbase;
         uint32_t pk[16];
+        const float2 ds2 = make_float2(p.dropout_scale, p.dropout_scale);
         if constexpr (MODE == kWideDV) {
 #pragma unroll
           for (int c = 0; c < 16; ++c) {
-            pk[c] = pack2<T>(pr[2 * c], pr[2 * c + 1]);
-            if constexpr ((FEAT & kDropout) != 0) pk[c] &= keep_mask(keep, c);      // (1 / (1 - p) follows at the write-out)
+            if constexpr ((FEAT & kDropout) != 0) pk[c] = dropout_p_pair<T>(make_float2(pr[2 * c], pr[2 * c + 1]), ds2, keep_mask(keep, c));
+            else pk[c] = pack2<T>(pr[2 * c], pr[2 * c + 1]);
           }
         } else {
           float dp[32];
           tmem_ld32f(a_col, dp);
           tmem_wait_ld();
-          const float2 ds2 = make_float2(p.dropout_scale, p.dropout_scale);
 #pragma unroll
           for (int c4 = 0; c4 < 8; ++c4) {
             const float4 d4 = lds128(dlt + 16u * c4);
@@ -623,7 +623,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
       const int nrows = min(kBlk, rows_total - r0);
       T* dst = reinterpret_cast<T*>(outv.ptr) + (int64_t)sq.bidx * outv.s[0] + (int64_t)hrow * outv.s[1] +
                (row_tok0 + r0) * outv.s[2];
-      const float scale = MODE != kWideDV ? p.sm_scale : ((FEAT & kDropout) ? p.dropout_scale : 1.0f);
+      const float scale = MODE != kWideDV ? p.sm_scale : 1.0f;
       for (int c = (warp - 4) >> 2; c * 32 < d_out; c += 2 * kGroups) {
         float v[32];
         tmem_ld32f(tmem_base + lane_addr + kWColAcc + c * 32, v);
