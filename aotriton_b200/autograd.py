@@ -56,10 +56,16 @@ def __getattr__(name):
     raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
+def _int64(x):
+    return type(x) is int and -(1 << 63) <= x < 1 << 63
+
+
 def _attend(q, k, v, b, cu_q, cu_k, max_q, max_k, sm_scale, dropout_p, causal, return_lse, seed, offset1, op):
     """The native route (csrc/torch_ops.cc): the result, or None where the call is not an ordinary one -- other tensors, modes
     or argument types, graph capture by torch.compile.  Those go by the Function or the operators below."""
     if torch.compiler.is_compiling():
+        return None
+    if op and not (_int64(seed) and _int64(offset1)):      # (the operators take both, used or not, as 64-bit signed numbers)
         return None
     ct, wl, wr = flash.translate_causal(causal)
     if type(offset1) is int and 0 <= offset1 < 1 << 64:
