@@ -138,7 +138,8 @@ struct Attend : torch::autograd::Function<Attend> {
     const Tensor b = bias.value_or(Tensor()), cu_q = seqs_q.value_or(Tensor()), cu_k = seqs_k.value_or(Tensor());
     Tensor out, lse, seed;
     ::forward(c, q, k, v, b, cu_q, cu_k, true, out, lse, seed);
-    ctx->save_for_backward({q, k, v, b, out, lse, seed, cu_q, cu_k});
+    ctx->save_for_backward({q, k, v, b, out, lse, cu_q, cu_k});
+    if (seed.defined()) ctx->saved_data["seed"] = seed;      // (a number of the call, nothing for a saved-tensor hook to change)
     ctx->saved_data["numbers"] = std::vector<int64_t>{c.causal_type, c.left, c.right, c.max_q, c.max_k, (int64_t)c.seed,
                                                       (int64_t)c.offset, c.packed, c.op};
     ctx->saved_data["scales"] = std::vector<double>{c.sm_scale, c.dropout_p};
@@ -148,7 +149,9 @@ struct Attend : torch::autograd::Function<Attend> {
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &b = saved[3], &out = saved[4], &lse = saved[5], &seed = saved[6];
+    const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &b = saved[3], &out = saved[4], &lse = saved[5], &cu_q = saved[6], &cu_k = saved[7];
+    const auto found = ctx->saved_data.find("seed");
+    const Tensor seed = found == ctx->saved_data.end() ? Tensor() : found->second.toTensor();
     const auto n = ctx->saved_data["numbers"].toIntVector();
     const auto s = ctx->saved_data["scales"].toDoubleVector();
     const Call c{s[0], s[1], n[0], n[1], n[2], n[3], n[4], (uint64_t)n[5], (uint64_t)n[6], n[7] != 0, n[8] != 0};
@@ -158,7 +161,7 @@ struct Attend : torch::autograd::Function<Attend> {
       operator_backward(c, q, k, v, b, out, dout, lse, seed, r);
       return r;
     }
-    for (const Tensor& t : {q, k, v, b, out, lse, seed})      // (a saved-tensor hook may have handed back something else)
+    for (const Tensor& t : {q, k, v, b, out, lse})      // (a saved-tensor hook may have handed back something else)
       TORCH_CHECK(!t.defined() || (t.is_cuda() && t.numel() > 0 && t.stride(-1) == 1), "attention: a saved tensor has changed its form");
     if (dout.stride(-1) != 1) dout = dout.contiguous();
     const aotriton::DType dt = dtype_of(q.scalar_type());
@@ -180,7 +183,7 @@ struct Attend : torch::autograd::Function<Attend> {
       p.DQ_ACC.cookie = &acc;
       p.DQ_ACC.acquire = &DqAcc::acquire;
     }
-    fill_common(p, c, saved[7], saved[8], seed);
+    fill_common(p, c, cu_q, cu_k, seed);
     check(flash::attn_bwd(p, flash::attn_bwd_params::kVersion, current_stream(), &options), c.packed ? "attn_bwd (varlen)" : "attn_bwd");
     g_last_bwd_family.store(ab200_last_bwd_family(), std::memory_order_relaxed);
     return r;
