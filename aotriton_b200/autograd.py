@@ -75,6 +75,32 @@ def _attend(q, k, v, b, cu_q, cu_k, max_q, max_k, sm_scale, dropout_p, causal, r
     return _native.attend(q, k, v, b, cu_q, cu_k, max_q, max_k, sm_scale, dropout_p, ct, wl, wr, return_lse, seed, offset1, op)
 
 
+def _backward(q, k, v, b, o, do, L, cu_q, cu_k, seed, offset1, offset2, sm_scale, dropout_p, causal, max_q, max_k):
+    """(dq, dk, dv, dbias) of a dense or, with cumulative lengths, a token-packed call."""
+    do = do if do.stride(-1) == 1 else do.contiguous()
+    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    db = torch.empty_like(b) if b is not None else None
+    delta = torch.empty_like(L)
+    if cu_q is None:
+        _check(flash.attn_bwd(q, k, v, b, sm_scale, o, do, dq, dk, dv, db, None, L, flash.eager_delta(delta), dropout_p, seed, offset1,
+                              offset2, causal), "attn_bwd")
+    else:
+        _check(flash.attn_bwd_varlen(q, k, v, cu_q, cu_k, max_q, max_k, None, None, None, sm_scale, o, do, dq, dk, dv, None, None, L,
+                                     flash.eager_delta(delta), dropout_p, seed, offset1, offset2, causal, "compact"), "attn_bwd (varlen)")
+    _native.note_bwd_family()
+    return dq, dk, dv, db
+
+
+def _native_backward(q, k, v, b, o, do, L, cu_q, cu_k, seed, offset, sm_scale, dropout_p, causal_type, wl, wr, max_q, max_k):
+    """The backward of a native call whose gradient, saved tensors or modes are not ordinary ones (csrc/torch_ops.cc)."""
+    causal = (wl, wr) if causal_type == flash.CausalType.WINDOWED else False
+    return _backward(q, k, v, b, o, do, L, cu_q, cu_k, seed.view(torch.uint64) if seed is not None else _NULL_SCALAR, _NULL_SCALAR,
+                     offset if seed is not None else 0, sm_scale, dropout_p, causal, max_q, max_k)
+
+
+_native.set_python_backward(_native_backward)
+
+
 class _Attention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, b, causal, sm_scale, dropout_p, return_lse=False,
@@ -92,13 +118,8 @@ class _Attention(torch.autograd.Function):
     @staticmethod
     def backward(ctx, do, *unused):
         q, k, v, b, o, L = ctx.saved_tensors
-        do = do if do.stride(-1) == 1 else do.contiguous()
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        db = torch.empty_like(b) if b is not None else None
-        delta = torch.empty_like(L)
-        _check(flash.attn_bwd(q, k, v, b, ctx.sm_scale, o, do, dq, dk, dv, db, None, L, flash.eager_delta(delta),
-                              ctx.dropout_p, ctx.philox_seed, ctx.philox_offset, 0, ctx.causal), "attn_bwd")
-        _native.note_bwd_family()
+        dq, dk, dv, db = _backward(q, k, v, b, o, do, L, None, None, ctx.philox_seed, ctx.philox_offset, 0, ctx.sm_scale, ctx.dropout_p,
+                                   ctx.causal, 0, 0)
         return dq, dk, dv, db, None, None, None, None, None, None
 
 
@@ -132,14 +153,8 @@ class _VarlenAttention(torch.autograd.Function):
     @staticmethod
     def backward(ctx, do, *unused):
         q, k, v, o, L, cu_q, cu_k = ctx.saved_tensors
-        do = do if do.stride(-1) == 1 else do.contiguous()
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        delta = torch.empty_like(L)
-        _check(flash.attn_bwd_varlen(q, k, v, cu_q, cu_k, ctx.max_seqlens[0], ctx.max_seqlens[1], None, None, None,
-                                     ctx.sm_scale, o, do, dq, dk, dv, None, None, L, flash.eager_delta(delta),
-                                     ctx.dropout_p, ctx.philox_seed, ctx.philox_offset, 0, ctx.causal,
-                                     "compact"), "attn_bwd (varlen)")
-        _native.note_bwd_family()
+        dq, dk, dv, _ = _backward(q, k, v, None, o, do, L, cu_q, cu_k, ctx.philox_seed, ctx.philox_offset, 0, ctx.sm_scale, ctx.dropout_p,
+                                  ctx.causal, *ctx.max_seqlens)
         return (dq, dk, dv) + (None,) * 10
 
 

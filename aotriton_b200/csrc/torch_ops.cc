@@ -1,7 +1,7 @@
 // The autograd entry points' native route: attention on ordinary torch tensors, forward and backward, without Python in
 // between.  Outputs, gradients and scratch come from torch's caching allocator, launches go to torch's current stream
-// through the C++ operator API (include/aotriton/flash.h), the backward is a torch::autograd::Function, so that
-// saved-tensor hooks, version checks and CUDA-graph capture see what they see of the Python Function.
+// through the C++ operator API (include/aotriton/flash.h), the backward is a torch::autograd::Function: version checks and CUDA-graph
+// capture see what they see of the Python Function, saved-tensor hooks the inputs, the output and the log-sum-exp.
 //
 // What bounds a small call is the host: measured per training step of 2 x 4 heads x 128 tokens of 64 (25 us of kernels), the
 // Python Function took 160 us, this takes 86; cross attention through the operators written in Python, 4 x 8 heads x 1024 x 77
@@ -9,7 +9,8 @@
 //
 // attend() returns None for whatever is not ordinary, and the caller then goes the Python way: tensors that are not plain CUDA tensors of
 // one type on the current device with unit innermost stride, and every mode in which an operator call means more than its kernels
-// (dispatch and function modes, functorch transforms, forward-mode gradients, tracing).
+// (dispatch and function modes, functorch transforms, forward-mode gradients, tracing).  The backward asks the same of its
+// gradient, of what was saved and of the modes it runs under, and otherwise leaves itself to the operator or to the Python Function's.
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -41,6 +42,9 @@ namespace {
 // Kernel family of the most recent backward: the library keeps it per thread, and autograd runs backwards on a thread of
 // its own.
 std::atomic<int> g_last_bwd_family{0};
+
+// The Function's backward as Python has it (autograd.py), for what Attend::backward leaves to it.  Set once, at import.
+PyObject* g_python_backward = nullptr;
 
 // A call's numbers.  `packed`: token-packed sequences (cu_q, cu_k); `op`: the call stands for the registered operators, whose
 // backward may use the fused form and is itself an operator.
@@ -131,6 +135,26 @@ struct DqAcc {
   }
 };
 
+bool plain_modes() {
+  const auto& tls = c10::impl::tls_local_dispatch_key_set();
+  return !c10::impl::TorchDispatchModeTLS::any_modes_set() && !at::impl::torch_function_mode_enabled() && !torch::jit::tracer::isTracing() &&
+         !tls.included_.has(c10::DispatchKey::Python) && !tls.included_.has(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) &&
+         !tls.included_.has(c10::DispatchKey::Functionalize);
+}
+
+// Nothing but a strided CUDA tensor on device `dev`, with elements, without a forward-mode gradient.
+bool plain(const Tensor& t, int dev) {
+  static const uint64_t allowed =
+      (c10::DispatchKeySet(c10::DispatchKey::CUDA) | c10::DispatchKeySet(c10::DispatchKey::AutogradCUDA) |
+       c10::DispatchKeySet(c10::DispatchKey::ADInplaceOrView) | c10::DispatchKeySet(c10::DispatchKey::AutocastCUDA)).raw_repr();
+  return t.defined() && (t.key_set().raw_repr() & ~allowed) == 0 && t.is_cuda() && t.get_device() == dev && t.layout() == at::kStrided &&
+         t.numel() != 0 && !t._fw_grad(0).defined();
+}
+// ... of this type and rank, with a unit innermost stride
+bool plain_operand(const Tensor& t, int dev, at::ScalarType type, int64_t dim) {
+  return plain(t, dev) && t.scalar_type() == type && t.dim() == dim && t.stride(-1) == 1;
+}
+
 struct Attend : torch::autograd::Function<Attend> {
   using Maybe = std::optional<Tensor>;      // (an undefined Tensor is no argument to apply())
   static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Maybe& bias,
@@ -157,12 +181,18 @@ struct Attend : torch::autograd::Function<Attend> {
     const Call c{s[0], s[1], n[0], n[1], n[2], n[3], n[4], (uint64_t)n[5], (uint64_t)n[6], n[7] != 0, n[8] != 0};
     variable_list r(8);
     Tensor dout = grads[0].defined() ? grads[0] : at::zeros_like(out);
-    if (c.op && at::GradMode::is_enabled()) {      // create_graph: the operator, which knows that it has no derivative
+    // create_graph: the operator, which knows that it has no derivative
+    if (c.op && at::GradMode::is_enabled()) {
       operator_backward(c, q, k, v, b, out, dout, lse, seed, r);
       return r;
     }
-    for (const Tensor& t : {q, k, v, b, out, lse})      // (a saved-tensor hook may have handed back something else)
-      TORCH_CHECK(!t.defined() || (t.is_cuda() && t.numel() > 0 && t.stride(-1) == 1), "attention: a saved tensor has changed its form");
+    // A gradient that is not an ordinary tensor (a batch of them under vmap), a mode that only this pass runs under, or a saved-tensor
+    // hook that handed back something else than it was given: what the call stands for deals with it.
+    if (!as_saved(q, k, v, b, out, dout, lse, cu_q, cu_k)) {
+      if (c.op) operator_backward(c, q, k, v, b, out, dout, lse, seed, r);
+      else python_backward(c, q, k, v, b, out, dout, lse, cu_q, cu_k, seed, r);
+      return r;
+    }
     if (dout.stride(-1) != 1) dout = dout.contiguous();
     const aotriton::DType dt = dtype_of(q.scalar_type());
     r[0] = gradient_of(q);
@@ -189,6 +219,39 @@ struct Attend : torch::autograd::Function<Attend> {
     return r;
   }
 
+  static bool as_saved(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& out, const Tensor& dout,
+                       const Tensor& lse, const Tensor& cu_q, const Tensor& cu_k) {
+    if (!plain_modes()) return false;
+    const int dev = c10::cuda::current_device();
+    const auto type = q.scalar_type();
+    for (const Tensor* t : {&q, &k, &v, &out})
+      if (!plain_operand(*t, dev, type, 4)) return false;
+    for (const Tensor* t : {&cu_q, &cu_k})
+      if (t->defined() && !plain_operand(*t, dev, at::kInt, 1)) return false;
+    return (!b.defined() || plain_operand(b, dev, type, 4)) && plain_operand(lse, dev, at::kFloat, 2) && lse.is_contiguous() &&
+           lse.numel() == q.size(0) * q.size(1) * q.size(2) && plain(dout, dev) && dout.scalar_type() == type && dout.sizes() == out.sizes();
+  }
+
+  static void python_backward(const Call& c, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& out,
+                              const Tensor& dout, const Tensor& lse, const Tensor& cu_q, const Tensor& cu_k, const Tensor& seed,
+                              variable_list& r) {
+    pybind11::gil_scoped_acquire gil;
+    auto wrap = [](const Tensor& t) {
+      return t.defined() ? pybind11::reinterpret_steal<pybind11::object>(THPVariable_Wrap(t)) : pybind11::object(pybind11::none());
+    };
+    const pybind11::object t[] = {wrap(q), wrap(k), wrap(v), wrap(b), wrap(out), wrap(dout), wrap(lse), wrap(cu_q), wrap(cu_k), wrap(seed)};
+    const auto result = pybind11::reinterpret_steal<pybind11::object>(PyObject_CallFunction(
+        g_python_backward, "OOOOOOOOOOKddLLLLL", t[0].ptr(), t[1].ptr(), t[2].ptr(), t[3].ptr(), t[4].ptr(), t[5].ptr(), t[6].ptr(), t[7].ptr(),
+        t[8].ptr(), t[9].ptr(), (unsigned long long)c.offset, c.sm_scale, c.dropout_p, (long long)c.causal_type, (long long)c.left,
+        (long long)c.right, (long long)c.max_q, (long long)c.max_k));
+    if (!result) {
+      python_error e;
+      e.persist();
+      throw e;
+    }
+    for (int i = 0; i < (b.defined() ? 4 : 3); ++i) r[i] = THPVariable_Unpack(PyTuple_GET_ITEM(result.ptr(), i));
+  }
+
   static void operator_backward(const Call& c, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& b, const Tensor& out,
                                 const Tensor& dout, const Tensor& lse, const Tensor& seed, variable_list& r) {
     const auto one = lse.options().dtype(at::kLong);
@@ -209,24 +272,11 @@ struct Attend : torch::autograd::Function<Attend> {
 
 // ---- from Python ------------------------------------------------------------------------------------------
 
-bool plain_modes() {
-  const auto& tls = c10::impl::tls_local_dispatch_key_set();
-  return !c10::impl::TorchDispatchModeTLS::any_modes_set() && !at::impl::torch_function_mode_enabled() && !torch::jit::tracer::isTracing() &&
-         !tls.included_.has(c10::DispatchKey::Python) && !tls.included_.has(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) &&
-         !tls.included_.has(c10::DispatchKey::Functionalize);
-}
-
-// A torch.Tensor or Parameter (no subclass) that is nothing but a strided CUDA tensor on device `dev`, without a forward-mode
-// gradient.  The tensor itself goes to *out.
+// A torch.Tensor or Parameter (no subclass) that is plain().  The tensor itself goes to *out.
 bool plain_tensor(PyObject* o, int dev, Tensor* out) {
-  static const uint64_t allowed =
-      (c10::DispatchKeySet(c10::DispatchKey::CUDA) | c10::DispatchKeySet(c10::DispatchKey::AutogradCUDA) |
-       c10::DispatchKeySet(c10::DispatchKey::ADInplaceOrView) | c10::DispatchKeySet(c10::DispatchKey::AutocastCUDA)).raw_repr();
   if (!THPVariable_CheckExact(o)) return false;
   const Tensor& t = THPVariable_Unpack(o);
-  if (!t.defined() || (t.key_set().raw_repr() & ~allowed) != 0 || !t.is_cuda() || t.get_device() != dev || t.layout() != at::kStrided)
-    return false;
-  if (t.numel() == 0 || t.stride(-1) != 1 || t._fw_grad(0).defined()) return false;
+  if (!plain(t, dev) || t.stride(-1) != 1) return false;
   *out = t;
   return true;
 }
@@ -314,7 +364,17 @@ PyObject* note_bwd_family(PyObject*, PyObject*) {
   Py_RETURN_NONE;
 }
 
+// The Function's backward: (q, k, v, bias, out, dout, logsumexp, cu_seqlens_q, cu_seqlens_k, seed, offset, sm_scale, dropout_p, causal_type,
+// window_left, window_right, max_seqlen_q, max_seqlen_k) -> (dq, dk, dv, dbias).  Kept for the life of the process.
+PyObject* set_python_backward(PyObject*, PyObject* fn) {
+  Py_INCREF(fn);
+  std::swap(g_python_backward, fn);
+  Py_XDECREF(fn);
+  Py_RETURN_NONE;
+}
+
 PyMethodDef kMethods[] = {{"attend", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&attend)), METH_FASTCALL, nullptr},
+                          {"set_python_backward", &set_python_backward, METH_O, nullptr},
                           {"last_bwd_family", &last_bwd_family, METH_NOARGS, nullptr},
                           {"note_bwd_family", &note_bwd_family, METH_NOARGS, nullptr},
                           {nullptr, nullptr, 0, nullptr}};
