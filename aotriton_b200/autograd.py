@@ -7,12 +7,37 @@ values it actually used to the backward; the backward allocates dQ/dK/dV(/dB) an
 """
 from __future__ import annotations
 
+import warnings
+
 import torch
 
-from . import flash, load_torch_ops
+from . import cabi, flash, load_torch_ops
 from .flash import hipError_t
 
-_native = load_torch_ops()
+try:
+    _native = load_torch_ops()
+except ImportError as e:      # (built where torch was missing, had no CUDA or was another version)
+    if torch.version.cuda is not None:
+        warnings.warn(f"aotriton_b200: {e}; attention calls take the Python way, which costs the host more", RuntimeWarning)
+
+    class _native:
+        _family = 0
+
+        @staticmethod
+        def attend(*args):
+            return None
+
+        @staticmethod
+        def set_python_backward(fn):
+            pass
+
+        @classmethod
+        def note_bwd_family(cls):
+            cls._family = int(cabi.lib().ab200_last_bwd_family())
+
+        @classmethod
+        def last_bwd_family(cls):
+            return cls._family
 
 DEFAULT_PHILOX_SEED = 0x1BF52
 DEFAULT_PHILOX_OFFSET_1 = 0x1D4000

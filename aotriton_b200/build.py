@@ -6,7 +6,8 @@ Products, all written next to this file so that they are found without installat
                                (include/aotriton/*.h); the name follows the reference's
                                library (v3src/CMakeLists.txt:383-387)
   pyaotriton.<abi>.so          pybind11 module with the reference's Python surface
-  _torch_ops.<abi>.so          the autograd entry points' native route (links libtorch)
+  _torch_ops.<abi>.so          the autograd entry points' native route (links libtorch; left out where torch is missing or has no
+                               CUDA, the entry points then take the Python way)
 
 `python -m aotriton_b200.build` rebuilds what is out of date.  Set AOTRITON_NAME_SUFFIX
 to compile namespace aotriton<suffix> the way the reference's cmake option does.
@@ -137,8 +138,13 @@ def torch_ops_path() -> Path:
     return PKG / ("_torch_ops" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 
-def build_torch_ops() -> Path:
-    import torch
+def build_torch_ops() -> Path | None:
+    try:
+        import torch
+    except ImportError:
+        return None
+    if torch.version.cuda is None:
+        return None
     from torch.utils.cpp_extension import include_paths
 
     OBJ.mkdir(exist_ok=True)
@@ -169,4 +175,4 @@ def build_all(verbose_ptxas: bool = False) -> None:
 if __name__ == "__main__":
     os.environ.setdefault("AB200_BUILD_VERBOSE", "1")
     build_all(verbose_ptxas="-v" in sys.argv)
-    print("built", LIB, pymodule_path(), "and", torch_ops_path())
+    print("built", *(p for p in (LIB, pymodule_path(), torch_ops_path()) if p.exists()))
