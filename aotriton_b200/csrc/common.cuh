@@ -181,18 +181,32 @@ __device__ __forceinline__ int64_t lse_offset(const Params& p, const Seq& s, int
   return ((int64_t)s.bidx * p.hq + h) * s.lse_row + s.q0;
 }
 
-// The elements of a warp's row segment of N columns that lie outside [lo, hi] (relative to its first column) become `fill`.  Where no
-// row of the warp has a lower bound inside the segment (`no_lo`, warp-uniform: a causal mask, a sequence's end) one comparison an
-// element is enough.  (Measured, with blocks that a warp sees nothing of left out of the forward's softmax: 24 packed prompts of 32 to
-// 2048 tokens, 32:8 heads of 128, 339 -> 331 us; training step of 16 x 12 x 391 of 64 with dropout 291.5 -> 288.5.)
-template <int N>
-__device__ __forceinline__ void mask_columns(float* x, int lo, int hi, bool no_lo, float fill) {
-  if (no_lo) {
+// The elements of a warp's row segment (columns first..first + N - 1) that lie outside [lo, hi] become `fill`.  Where no row of the warp has
+// a lower bound inside the segment (`no_lo`, warp-uniform: a causal mask, a sequence's end) one comparison an element is enough, with
+// code for either.  ONE_BOUND false: two comparisons always, one piece of code.
+// ONE_BOUND pays except beside bias and dropout together, where its second piece of code is spilled for around every block.  Measured, device us,
+// two comparisons / one: forward, 4 x 16:8 heads x 2048 causal of 64 95.6 / 90.6, of 128 105.9 / 101.5; with bias and dropout, not causal, of 64
+// 483.8 / 490.9, of 72 490 / 502 (1000 tokens of 64, which end inside a block, 151.6 / 149.2); dQ there, of 72, 556 / 577, of 128 548 / 577;
+// dV of 256, in a whole backward, 1453 / 1462, but its dQ 703 / 696.  (To leave out of the forward's softmax the blocks that a warp sees nothing
+// of costs registers as well: with one comparison, without and with it, of 128 101.5 / 103.2 causal, 164 / 170 not; bias and dropout of 72 490 / 546.)
+template <int N, bool ONE_BOUND>
+__device__ __forceinline__ void mask_columns(float* x, int first, int lo, int hi, bool no_lo, float fill) {
+  if constexpr (ONE_BOUND) {
+    lo -= first;
+    hi -= first;
+    if (no_lo) {
 #pragma unroll
-    for (int c = 0; c < N; ++c) x[c] = c <= hi ? x[c] : fill;
+      for (int c = 0; c < N; ++c) x[c] = c <= hi ? x[c] : fill;
+    } else {
+#pragma unroll
+      for (int c = 0; c < N; ++c) x[c] = (c >= lo && c <= hi) ? x[c] : fill;
+    }
   } else {
 #pragma unroll
-    for (int c = 0; c < N; ++c) x[c] = (c >= lo && c <= hi) ? x[c] : fill;
+    for (int c = 0; c < N; ++c) {
+      const int n = first + c;
+      x[c] = (n >= lo && n <= hi) ? x[c] : fill;
+    }
   }
 }
 

@@ -731,7 +731,7 @@ sm100_bwd_dkdv_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           }
         }
         if (any_mask) {
-          mask_columns<32>(pr, col_lo - mbase, col_hi - mbase, mbase >= warp_lo, 0.f);
+          mask_columns<32, FEAT != kAll>(pr, mbase, col_lo, col_hi, mbase >= warp_lo, 0.f);
         }
         if (threadIdx.x == AB200_TRACE_TID) AB200_STAMP(G, 7);
         uint32_t keep = 0xffffffffu;
@@ -1233,7 +1233,7 @@ sm100_bwd_dq_kernel(const __grid_constant__ Params p, const __grid_constant__ CU
         for (int c = 0; c < 32; ++c) pr[c] = ex2(pr[c] - lse2);
       }
       if (any_mask) {
-        mask_columns<32>(pr, row_lo - nbase, row_hi - nbase, nbase >= warp_lo, 0.f);
+        mask_columns<32, FEAT != kAll>(pr, nbase, row_lo, row_hi, nbase >= warp_lo, 0.f);
       }
       uint32_t keep = 0xffffffffu;
       if (shared) {

@@ -447,7 +447,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           }
         }
         if (any_mask) {
-          mask_columns<32>(pr, v_lo - mbase, v_hi - mbase, mbase >= warp_lo, 0.f);
+          mask_columns<32, FEAT != kAll>(pr, mbase, v_lo, v_hi, mbase >= warp_lo, 0.f);
         }
         uint32_t keep = 0xffffffffu;
         if (shared) {
@@ -565,7 +565,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
           for (int c = 0; c < 32; ++c) pr[c] = ex2(pr[c] - lse2);
         }
         if (any_mask) {
-          mask_columns<32>(pr, v_lo - nbase, v_hi - nbase, nbase >= warp_lo, 0.f);
+          mask_columns<32, true>(pr, nbase, v_lo, v_hi, nbase >= warp_lo, 0.f);
         }
         uint32_t keep = 0xffffffffu;
         if (shared) {

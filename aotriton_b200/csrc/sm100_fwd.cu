@@ -418,9 +418,9 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
       if (lo > row_lo) row_lo = (int)(lo > 0x7fffffffLL ? 0x7fffffffLL : lo);
       if (hi < row_hi) row_hi = (int)(hi < -1 ? -1 : hi);
     }
+    constexpr bool kOneBound = FEAT != kAll || HD > 128;      // (mask_columns)
     // the tightest bounds over the warp's rows: a block needs masking iff it is not inside them
     const int warp_lo = __reduce_max_sync(0xffffffffu, row_lo), warp_hi = __reduce_min_sync(0xffffffffu, row_hi);
-    const int dead_lo = __reduce_min_sync(0xffffffffu, row_lo), dead_hi = __reduce_max_sync(0xffffffffu, row_hi);      // (the widest)
     DropoutCtx dctx;
     if (L::kTiles == 2 && drop_on) dctx = dropout_ctx(p, z, h);
     const int row0 = m0 + t * kBM + quarter * 32;      // the warp's tiles of bias start in this row
@@ -449,23 +449,6 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
         }
       }
       if (!mbar_wait(&bars[L::bSFull + t], par, abort_flag, status, 0x700 + 2 * j + t)) { ok = false; break; }
-      // A block that none of the warp's rows sees (a causal problem's last one, for the first tile): P is zero, and that is all.
-      if ((n0 > dead_hi || n0 + kBN - 1 < dead_lo) && !(L::kTiles == 1 && drop_on)) {
-        tc_fence_after();
-        uint32_t zero[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) zero[i] = 0u;
-        tmem_st32(s_addr, zero);
-        tmem_st32(s_addr + 32, zero);
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(&bars[L::bPHalf + t]);
-          mbar_arrive(&bars[L::bPFull + t]);
-        }
-        continue;
-      }
       AB200_FSTAMP(j, 0);
       tc_fence_after();
       float sc[128];
@@ -494,9 +477,7 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
       bool simple = !bias_on && p.qk_scale > 0.f;
       float mx;
       if (simple) {
-        if (any_mask) {
-          mask_columns<128>(sc, row_lo - n0, row_hi - n0, n0 >= warp_lo, -INFINITY);
-        }
+        if (any_mask) mask_columns<128, kOneBound>(sc, n0, row_lo, row_hi, n0 >= warp_lo, -INFINITY);
         float m8[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) m8[c] = fmaxf(sc[2 * c], sc[2 * c + 1]);
@@ -512,9 +493,7 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
 #pragma unroll
           for (int c = 0; c < 128; ++c) sc[c] *= p.qk_scale;
         }
-        if (any_mask) {
-          mask_columns<128>(sc, row_lo - n0, row_hi - n0, n0 >= warp_lo, -INFINITY);
-        }
+        if (any_mask) mask_columns<128, kOneBound>(sc, n0, row_lo, row_hi, n0 >= warp_lo, -INFINITY);
         float m8[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) m8[c] = fmaxf(sc[2 * c], sc[2 * c + 1]);
