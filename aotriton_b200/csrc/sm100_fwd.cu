@@ -116,6 +116,8 @@ __device__ void write_dead_rows(const Params& p, const Seq& sq, int h, int m0, i
 // FEAT (features()): with code for dropout in the loop a call with bias alone, and with code for either a call with
 // neither, spills around every block.  Measured, us, dropout's instantiation against the call's own, neither: 4 x 32 heads
 // x 4096 of 128, causal, 583 -> 571; 8 x 16 heads x 2048 of 64 260 -> 241; bias, 4 x 8 heads x 1024 of 64 41.6 -> 40.8.
+// Bias' instantiation against the call's own, neither, of 256: 4 x 16:8 heads x 2048 327 -> 317, causal 201 -> 197, 2 x 16 x 4096 causal
+// 333 -> 329, 8 x 16 x 2048 637 -> 640.
 template <typename T, int HD, bool EXACT, int FEAT>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUtensorMap tm_q,
@@ -741,10 +743,7 @@ template <typename T, int HD>
 cudaError_t launch_fwd_T(const Params& p, cudaStream_t st) {
   const bool exact = exact_tiles(p, HD);
   switch (features(p)) {
-    case kPlain:
-      // (Whole tiles of 256 columns: ptxas spills 320 bytes in the instantiation without bias, 268 in the one with it.
-      // Measured, 8 x 16 heads x 2048, not causal: 642 us against 628.)
-      return exact ? launch_fwd_TE<T, HD, true, HD == 256 ? kBias : kPlain>(p, st) : launch_fwd_TE<T, HD, false, kPlain>(p, st);
+    case kPlain: return exact ? launch_fwd_TE<T, HD, true, kPlain>(p, st) : launch_fwd_TE<T, HD, false, kPlain>(p, st);
     case kBias: return exact ? launch_fwd_TE<T, HD, true, kBias>(p, st) : launch_fwd_TE<T, HD, false, kBias>(p, st);
     case kDropout: return exact ? launch_fwd_TE<T, HD, true, kDropout>(p, st) : launch_fwd_TE<T, HD, false, kDropout>(p, st);
     default: return exact ? launch_fwd_TE<T, HD, true, kAll>(p, st) : launch_fwd_TE<T, HD, false, kAll>(p, st);
