@@ -15,6 +15,7 @@
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include "indexing.h"
 
 namespace ab200 {
 
@@ -61,6 +62,7 @@ struct Params {
   int32_t drop_copy;              // test hook of the bounded waits: the producer leaves out one tile copy
                                   // (1 = first V block of the forward, 2 = first Q/dO block of dK/dV, 3 = first V block of dQ)
   int32_t packed_tiles;           // token-packed: the grid counts row tiles of all sequences instead of max_sq's per sequence
+  int32_t hw_order;               // the forward's CTAs in the hardware's order: a grid of 2^24 or more, beyond quick_div
   unsigned int* ticket;           // dK/dV's ticket counter, zeroed by the preprocess kernel of the same call (null: by the launch itself)
   int32_t dk_from_db;             // dK = sm_scale * dBias^T Q, after the dQ kernel has written dBias (sm100_bwd_dk_db.cuh)
   int32_t keep_tiles, keep_shift; // keep bits of the first keep_tiles 32-key tiles pass through dQ's rows (0: none), or, with
@@ -76,16 +78,6 @@ enum : int { kPlain = 0, kBias = 1, kDropout = 2, kAll = 3 };      // bias, and 
 inline int features(const Params& p) {
   if (p.has_dbias && !p.has_bias) return kAll;
   return (p.has_bias ? kBias : 0) | (p.dropout_on ? kDropout : 0);
-}
-
-// a / b for 0 <= a, 0 < b and a quotient below 2^21, by the fp32 reciprocal and two corrections: at the start of a CTA every
-// cycle of an integer division is waited for.
-__device__ __forceinline__ int quick_div(int a, int b) {
-  int q = (int)((float)a * __frcp_rn((float)b));
-  int r = a - q * b;
-  if (r < 0) { --q; r += b; }
-  if (r >= b) ++q;
-  return q;
 }
 
 struct Seq {

@@ -214,26 +214,6 @@ __device__ __forceinline__ const T* bias_at(const Params& p, const Seq& sq, int 
          (int64_t)m * p.bias.s[2] + (int64_t)n * p.bias.s[3];
 }
 
-// Which (row tile counted from the last, head, batch) a CTA takes: heads in groups of 32, inside a group the row tiles
-// slowest, so that the long tiles of a causal problem start together and first.  SNAKE: the CTAs that find room at once are dealt out
-// a round of all SMs at a time, so every other round runs from the short tiles to the long ones; in the same order the SM with the
-// longest first tile also had the longest second one.  Measured, forward, fp32, 2 x 8 x 500 x 64 causal: 35 -> 31 us.  (The backward's
-// time is its longest CTA's, whichever SM that is on.)
-template <bool SNAKE>
-__device__ __forceinline__ void tile_of_block(int bx, int nx, int nh, int nz, int& x, int& h, int& z) {
-  constexpr int kHeadGroup = 32, kSms = 148;
-  int lin = bx + nx * ((int)blockIdx.y + nh * (int)blockIdx.z);
-  if constexpr (SNAKE) {
-    const int round = lin / kSms, round0 = round * kSms;
-    if (round & 1) lin = round0 + min(kSms, nx * nh * nz - round0) - 1 - (lin - round0);
-  }
-  const int grp = lin / (kHeadGroup * nx), r = lin - grp * (kHeadGroup * nx), gsize = min(kHeadGroup, nh * nz - grp * kHeadGroup);
-  x = r / gsize;
-  const int hz = grp * kHeadGroup + (r - x * gsize);
-  z = hz / nh;
-  h = hz - z * nh;
-}
-
 // Forward.  grid = (cdiv(max_sq, 32), Hq, batch).  Two groups of four warps take every other block of the keys, each with
 // tiles of its own, and merge at the end: a row tile's chain of blocks, which is what a small grid waits for, is half
 // as long, and an SM has 16 warps instead of 12.  Within a group the copy of V runs under the scores, that of the next K
@@ -257,7 +237,7 @@ __global__ void __launch_bounds__(kFwdGroups * 128, 2) tiled_fwd_kernel(const __
     if (p.off_out) *p.off_out = p.off2 + (p.off1_ptr ? *p.off1_ptr : 0ull);
   }
   int x, h, z;
-  tile_of_block<true>((int)blockIdx.x, (int)gridDim.x, (int)gridDim.y, (int)gridDim.z, x, h, z);
+  tile_of_block<true>((int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, (int)gridDim.x, (int)gridDim.y, (int)gridDim.z, x, h, z);
   const int m0 = ((int)gridDim.x - 1 - x) * C::kBM;
   const Seq sq = resolve_seq(p, z);
   if (m0 >= sq.sq) return;
@@ -656,7 +636,7 @@ tiled_bwd_kernel(const __grid_constant__ Params p) {
   constexpr int kBM = Tiled<DP>::kBM;
   const int nx = (int)gridDim.x / SPLIT;
   int x, h, z;
-  tile_of_block<false>((int)blockIdx.x / SPLIT, nx, (int)gridDim.y, (int)gridDim.z, x, h, z);
+  tile_of_block<false>((int)blockIdx.x / SPLIT, (int)blockIdx.y, (int)blockIdx.z, nx, (int)gridDim.y, (int)gridDim.z, x, h, z);
   if constexpr (WHICH == 1) {
     tiled_bwd_dkdv<T, DP, SPLIT>(p, smem, z, h, x * kBM);
   } else if constexpr (WHICH == 2) {

@@ -210,7 +210,7 @@ __device__ __forceinline__ DkdvItem dkdv_item(const Params& p, int w) {
   DkdvItem it;
   const int per = p.batch * p.hk;
   const int nkb = (p.max_sk + kBlk - 1) / kBlk;
-  const int grp = quick_div(w, nkb * 8), r = w - grp * (nkb * 8);
+  const int grp = quick_div_any(w, nkb * 8), r = w - grp * (nkb * 8);
   const int kb = r >> 3, rem = grp * 8 + (r & 7);
   it.z = quick_div(min(rem, per - 1), p.hk);
   it.hk = min(rem, per - 1) - it.z * p.hk;

@@ -144,7 +144,7 @@ sm100_fwd_kernel(const __grid_constant__ Params p, const __grid_constant__ CUten
 #define AB200_FWD_HEAD_GROUP 32
 #endif
   int z = blockIdx.z, h = blockIdx.y, m0 = (int)(gridDim.x - 1 - blockIdx.x) * kCtaRows;
-  if constexpr (AB200_FWD_HEAD_GROUP > 0) {
+  if (AB200_FWD_HEAD_GROUP > 0 && !p.hw_order) {
     constexpr int kHeadGroup = AB200_FWD_HEAD_GROUP > 0 ? AB200_FWD_HEAD_GROUP : 1;
     const int nx = (int)gridDim.x, nh = (int)gridDim.y, nhz = nh * (int)gridDim.z;
     const int lin = (int)blockIdx.x + nx * ((int)blockIdx.y + nh * (int)blockIdx.z);
@@ -734,6 +734,7 @@ cudaError_t launch_fwd_TE(const Params& p, cudaStream_t st) {
   Params pp = p;
   pp.packed_tiles = packed_tiles_bound(p, L::kCtaRows);
   if (pp.packed_tiles > 0) grid = dim3(pp.packed_tiles * p.hq);
+  pp.hw_order = (int64_t)grid.x * grid.y * grid.z >= 1 << 24;
   e = launch_kernel(sm100_fwd_kernel<T, HD, EXACT, FEAT>, grid, dim3(kFwdThreads), L::kDynamic, st, pp, tq, tk, tv, status);
   if (e == cudaSuccess) count_launch();
   return e;
