@@ -142,22 +142,6 @@ __device__ __forceinline__ constexpr uint32_t mnmajor_step(int kk) { return (uin
 __device__ __forceinline__ uint32_t split_a_col(int kk) { return (uint32_t)(kWgCols * (kk >> 1) + (kk & 1) * 8); }
 
 template <typename T>
-__device__ __forceinline__ void store_row_chunk32(T* dst, const float* v, float scale, int d0, int dmax) {
-#pragma unroll
-  for (int v8 = 0; v8 < 4; ++v8) {
-    const int d = d0 + v8 * 8;
-    if (d < dmax) {
-      uint4 w;
-      w.x = pack2<T>(v[v8 * 8 + 0] * scale, v[v8 * 8 + 1] * scale);
-      w.y = pack2<T>(v[v8 * 8 + 2] * scale, v[v8 * 8 + 3] * scale);
-      w.z = pack2<T>(v[v8 * 8 + 4] * scale, v[v8 * 8 + 5] * scale);
-      w.w = pack2<T>(v[v8 * 8 + 6] * scale, v[v8 * 8 + 7] * scale);
-      *reinterpret_cast<uint4*>(dst + d) = w;
-    }
-  }
-}
-
-template <typename T>
 __device__ void zero_rows(const View4& v, int b, int h, int64_t tok0, int row0, int nrows, int d) {
   for (int r = threadIdx.x; r < kBlk; r += blockDim.x) {
     if (row0 + r >= nrows) continue;
