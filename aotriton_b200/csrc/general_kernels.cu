@@ -546,8 +546,8 @@ int64_t row_tiles(const Params& p) {      // of dQ, dK and dV together
 }
 // dK/dV and dQ in one launch, or in two.  Together they fill the chip where one alone does not, and share its last
 // wave.  What they lose is occupancy: a CTA of the joint launch asks for the shared memory of dK/dV (77 KB at head dims
-// above 64, two CTAs an SM) where dQ alone has room for three.  16-bit types there lose from 4096 row tiles on; single
-// precision is small as a rule, and keeps the one launch.
+// above 64, two CTAs an SM) where dQ alone has room for three.  16-bit types there take two launches from 4096 row tiles on
+// (around the line the two are within 2 %); single precision is small as a rule and keeps the one launch, which costs the largest calls up to 6 %.
 // Measured, dK/dV and dQ, joint against two launches, us (row tiles): fp32 2x8x8x500x64 causal (512) 74 / 81, 4x8x8x1024x128 (2048)
 // 1941 / 1971, 4x16x16x2048x64 (8192) 6535 / 6469, 4x16x16x2048x128 (8192) 14910 / 14062; fp16 4x16x16x2048x60 (8192) 7799 / 7759,
 // 4x8x8x1024x124 (2048) 2560 / 2624, 4x12x12x1024x124 (3072) 3844 / 3780, 4x16x16x1024x124 (4096) 4738 / 4712.
@@ -590,8 +590,9 @@ cudaError_t launch_tiled_T(int which, const Params& p, cudaStream_t st) {
 template <typename T>
 cudaError_t launch_general_D(int which, const Params& p, cudaStream_t st) {
   int d = p.dqk > p.dvo ? p.dqk : p.dvo;
-  if (d <= 64) return launch_tiled_T<T, 64>(which, p, st);
-  if (d <= 128) return launch_tiled_T<T, 128>(which, p, st);
+  // (the register-tiled kernels' largest grid: dK/dV and dQ in one launch)
+  const int64_t blocks = ((int64_t)(p.max_sq > p.max_sk ? p.max_sq : p.max_sk) + 31) / 32;
+  if (d <= 128 && !beyond_tile_order(2 * blocks, p.hq, p.batch)) return d <= 64 ? launch_tiled_T<T, 64>(which, p, st) : launch_tiled_T<T, 128>(which, p, st);
   if (which == 3) {
     const cudaError_t e = launch_general_D<T>(1, p, st);
     return e != cudaSuccess ? e : launch_general_D<T>(2, p, st);
