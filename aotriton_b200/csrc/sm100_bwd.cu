@@ -219,8 +219,8 @@ __device__ __forceinline__ DkdvItem dkdv_item(const Params& p, int w) {
 // MMA issuer's loop is latency-critical: even untaken branches and call sites in it cost several
 // per cent of the kernel's time).
 // FEAT (features()): at 96 registers a thread the compute warps' loop spills, and what dropout and bias keep there
-// (generator state, bias tile, pointers, strides) is most of it: at head dim 128 dK/dV stores 148 bytes with both, 124 with
-// dropout, 84 with bias, none with neither; dQ 28 with both, else none.  Measured, whole backward, us, the instantiation for both against the
+// (generator state, bias tile, pointers, strides) is most of it: at head dim 128 (fp16, whole tiles) dK/dV stores 156 bytes with both, 136 with
+// dropout, 24 with bias, 36 with neither; dQ at most 8.  Measured, whole backward, us, the instantiation for both against the
 // call's own: neither, dense causal 4 x 32 heads x 4096 of 128 1875 -> 1768, 64:8 heads x 16384, window 4096, 6530 -> 6200; bias,
 // 4 x 8 heads x 1024 of 64 131.5 -> 113.1, 4 x 8:2 heads x 1024 of 128 with dBias 228 -> 207; dropout, 16 packed sequences of 64 to 8192
 // tokens, 32:8 heads of 128, dK/dV 8980 -> 8713, dQ 5450 -> 4960; 16 x 12 x 391 of 64, training step, 324 -> 303.

@@ -18,7 +18,7 @@
 // live in two stages, so the dP' / S' GEMMs of block i+1 run while the compute warps work on block i.
 // Shared memory: 2 x 64 KB resident, 2 x 32 KB late, 32 KB early.  Tensor memory: [0,64) S', [64,128) and [128,192) two dP' buffers, whose first columns
 // then take the packed 16-bit P' / dS' (the A operand of the accumulating GEMM), [256,512) the
-// accumulator.  Twelve warps: TMA producer, MMA issuer, logsumexp/delta stager (dV, dK), one idle,
+// accumulator; with two compute groups [0,64) and [64,128) a buffer of S' each, [128,192) and [192,256) those of P'.  Twelve warps: TMA producer, MMA issuer, logsumexp/delta stager (dV, dK), one idle,
 // eight compute warps (thread = one row of the 128 x 64 score tile, two warpgroups split its columns
 // 32 apiece); dV with bias and dropout has eight more and two S' buffers (wide_groups).  The arithmetic is that of the 128-wide kernels (see the head of sm100_bwd.cu); dK and dV
 // recompute the probabilities separately, which is the price of the one-accumulator form.
@@ -26,7 +26,7 @@
 
 constexpr int kWideCompute = 8;        // warps of a compute group: 4..11, and 12..19 where there are two
 constexpr int kNB = 64;                // rows of a streamed block
-constexpr uint32_t kWColS = 0, kWColDP = 64, kWColAcc = 256;
+constexpr uint32_t kWColS = 0, kWColDP = 64, kWColAcc = 256;      // (two compute groups: kColDPW)
 constexpr int kWideDV = 0, kWideDK = 1, kWideDQ = 2;
 // Compute groups.  dV with dropout and bias is bound by its compute warps (they read the bias and draw the bits that the later
 // kernels get from it): two groups take every other streamed block, with a buffer of S' each, so that one's loads and
@@ -308,7 +308,7 @@ sm100_bwd_wide_kernel(const __grid_constant__ Params p, const __grid_constant__ 
       __syncwarp();
       return true;
     };
-    // order on the tensor pipe:  dP'_{i+1} S'_{i+1} | acc_i   (S' has one buffer: S'_{i+1} follows the
+    // order on the tensor pipe:  dP'_{i+1} S'_{i+1} | acc_i   (one compute group: S' has one buffer, S'_{i+1} follows the
     // compute warps' copy of S'_i into registers; dP'_{i+1} takes the buffer acc_{i-1} has read)
     bool ok = wait(L::bResFull, 0, 0x3700);
     if (ok) ok = issue_early(0);

@@ -3,9 +3,9 @@
 // through the C++ operator API (include/aotriton/flash.h), the backward is a torch::autograd::Function: version checks and CUDA-graph
 // capture see what they see of the Python Function, saved-tensor hooks the inputs, the output and the log-sum-exp.
 //
-// What bounds a small call is the host: measured per training step of 2 x 4 heads x 128 tokens of 64 (25 us of kernels), the
-// Python Function took 160 us, this takes 86; cross attention through the operators written in Python, 4 x 8 heads x 1024 x 77
-// of 80 (62 us of kernels), 332 and 85; one token of 4 sequences against 6007 keys, 32:8 heads of 128 (17 us), 33.5 and 22.5.
+// What bounds a small call is the host.  Measured, us a pass, the Python way against this: training step of 2 x 4 heads x 128 tokens of 64 (20
+// of kernels) 160 / 77; cross attention, 4 x 8 heads x 1024 x 77 of 80 (47 of kernels), 332 / 78; one token of 4 sequences against 6007
+// keys, 32:8 heads of 128 (14), 33.5 / 20.6.
 //
 // attend() returns None for whatever is not ordinary, and the caller then goes the Python way: tensors that are not plain CUDA tensors of
 // one type on the current device with unit innermost stride, and every mode in which an operator call means more than its kernels
